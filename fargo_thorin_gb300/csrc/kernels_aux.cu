@@ -521,10 +521,10 @@ __device__ __forceinline__ double planet_node(double s2, double dz, double mx, c
 {
   double d2 = s2 + dz * dz, taper = 1.0;
   if (d2 < P.rst2) {
-    const double dd = sqrt(d2);
+    const double dd = sqrt_fast(d2);
     taper = div_fast(-3.0 * d2 * d2, P.rst4) + div_fast(4.0 * dd * d2, P.rst3);
   }
-  const double iv = rsqrt(d2 + mx);
+  const double iv = rsqrt_fast(d2 + mx);
   return iv * iv * iv * taper;
 }
 
@@ -544,10 +544,10 @@ __device__ __forceinline__ void vert_quad(const double (&wq)[NV], double H, doub
   for (int m = 1; m <= NV; m++) {
     const double znode = ((double)m - 0.5) * deltaz, znode2 = znode * znode;
     const double sum = wq[m - 1];
-    double iv = rsqrt(r2 + znode2);
+    double iv = rsqrt_fast(r2 + znode2);
     is += sum * iv * iv * iv;
     if (peb) {
-      iv = rsqrt(r2 + znode2 * hc2);
+      iv = rsqrt_fast(r2 + znode2 * hc2);
       pis += sum * iv * iv * iv;
     }
     for (int k = 0; k < npl; k++) {
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRin
     double Hcorr = 0.0, pH = 0.0, pmcell = 0.0;
     if (peb) {
       pmcell = a.pdens[l] * g.r.Surf[i];
-      Hcorr = a.sqrt_pebble_alpha * rsqrt(a.tau[l]);        // sqrt(alpha / tau) without the division
+      Hcorr = a.sqrt_pebble_alpha * rsqrt_fast(a.tau[l]);        // sqrt(alpha / tau) without the division
       pH = H * Hcorr;
       const double p_H_avr = fr.p_H_avr[i];
       if (fabs(pH - p_H_avr) > 0.05 * p_H_avr) local = 1;
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRin
         }
       } else {
         mpl *= mass_taper;
-        double d2 = s2[k] + P.z * P.z + P.smoothing2, iv = rsqrt(d2), id3 = iv * iv * iv;
+        double d2 = s2[k] + P.z * P.z + P.smoothing2, iv = rsqrt_fast(d2), id3 = iv * iv * iv;
         tmp = (x - P.x) * id3;
         ax += -mpl * tmp;
         if (a.exclude_hill) tmp *= hillcut[k];
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRin
         acc[3 + 2 * k] += mcell * tmp;
         if (peb) {
           d2 += -P.smoothing2 + P.smoothing2 * Hcorr * Hcorr;
-          iv = rsqrt(d2); id3 = iv * iv * iv;
+          iv = rsqrt_fast(d2); id3 = iv * iv * iv;
           tmp = (x - P.x) * id3;
           pax += -mpl * tmp;
           if (a.pebble_gravity) { if (a.exclude_hill) tmp *= hillcut[k]; acc[2 + 2 * k] += pmcell * tmp; }

@@ -136,17 +136,17 @@ __global__ void k_visc_update(DevGrid g, double *__restrict__ vr, double *__rest
   const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
   if (i >= 1 && i < nr - 1) {
     const int lip = l + ns;
-    vt[l] += dt * g.r.InvRmed[i] *
-             ((g.r.Rsup[i] * trp[lip] - g.r.Rinf[i] * trp[l]) * g.r.InvDiffRsup[i] + (tpp[l] - tpp[ljm]) * invdphi +
-              0.5 * (trp[l] + trp[lip])) /
-             (0.5 * (rho[l] + rho[ljm]));
+    vt[l] += div_fast(dt * g.r.InvRmed[i] *
+                          ((g.r.Rsup[i] * trp[lip] - g.r.Rinf[i] * trp[l]) * g.r.InvDiffRsup[i] +
+                           (tpp[l] - tpp[ljm]) * invdphi + 0.5 * (trp[l] + trp[lip])),
+                      0.5 * (rho[l] + rho[ljm]));
   }
   if (i >= 1) {
     const int lim = l - ns;
-    vr[l] += dt * g.r.InvRinf[i] *
-             ((g.r.Rmed[i] * trr[l] - g.r.Rmed[i - 1] * trr[lim]) * g.r.InvDiffRmed[i] + (trp[ljp] - trp[l]) * invdphi -
-              0.5 * (tpp[l] + tpp[lim])) /
-             (0.5 * (rho[l] + rho[lim]));
+    vr[l] += div_fast(dt * g.r.InvRinf[i] *
+                          ((g.r.Rmed[i] * trr[l] - g.r.Rmed[i - 1] * trr[lim]) * g.r.InvDiffRmed[i] +
+                           (trp[ljp] - trp[l]) * invdphi - 0.5 * (tpp[l] + tpp[lim])),
+                      0.5 * (rho[l] + rho[lim]));
   }
   if (kepler_edges) {
     if (i == 0) vt[l] = vkep_in;
@@ -244,7 +244,7 @@ __global__ void k_eos(DevGrid g, const double *__restrict__ rho, const double *_
     double tmp1 = e * 1.0 * gm1;
     temper[l] = tmp1 * tmp2;
   }
-  cs[l] = sqrt(div_fast(gg1 * fabs(e), r));
+  cs[l] = sqrt_fast(div_fast(gg1 * fabs(e), r));
 }
 
 // Opacity laws, Opacity.c.
@@ -285,12 +285,12 @@ __device__ double opacity_BL94(double rho, double T)
     // t1 = (k1^-2 + k2^-2)^-2, x = k3 / (1 + 1e22 T^-10), k = (t1 + x^4)^(1/4),
     // rearranged to two divisions
     const double T2 = T * T, T4 = T2 * T2, T5 = T4 * T, T7 = T5 * T2, T10 = T5 * T5;
-    const double k3 = kappa[2] * sqrt(T);
+    const double k3 = kappa[2] * sqrt_fast(T);
     const double ik = div_fast(T4, __fma_rn(2.5e-33 * (T7 * T7), T4, 2.5e7));   // 1 / (k1^-2 + k2^-2) = T^4 / (2.5e7 + 2.5e-33 T^18)
     const double t1 = ik * ik;
     const double x = div_fast(k3 * T10, T10 + 1.0e22);
     const double x2 = x * x;
-    k = sqrt(sqrt(t1 + x2 * x2));
+    k = sqrt_fast(sqrt_fast(t1 + x2 * x2));
   } else if (T > 0.0 && rho > 0.0) {
     // T <= TEMPB(i, j) compared as logarithms: ln T <= (ln(kappa_j / kappa_i)
     // + (a_j - a_i) ln rho) / (b_i - b_j), one log each of rho and T; the
@@ -491,9 +491,9 @@ __device__ __forceinline__ double gradt_sq(const DevGrid &g, const double *T, in
 __device__ __forceinline__ double flux_limiter_sq(double g2, double c)
 {
   const double s2 = g2 * (c * c);
-  if (s2 <= 4.0) return div_fast(2.0, 3.0 + sqrt(9.0 + 10.0 * s2));
-  const double s = sqrt(g2) * c;
-  return div_fast(10.0, 10.0 * s + 9.0 + sqrt(81.0 + 180.0 * s));
+  if (s2 <= 4.0) return div_fast(2.0, 3.0 + sqrt_fast(9.0 + 10.0 * s2));
+  const double s = sqrt_fast(g2) * c;
+  return div_fast(10.0, 10.0 * s + 9.0 + sqrt_fast(81.0 + 180.0 * s));
 }
 
 // MidplaneVolumeDensity, OpacityProfile, CalculateQminus and the centred
@@ -1219,7 +1219,7 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
     const double r = rho[l], e = energy[l];
     const double tmp2 = div_fast(1.0, r);
     temper[l] = e * gm1 * tmp2;
-    cs[l] = sqrt(gg1 * fabs(e) * tmp2);
+    cs[l] = sqrt_fast(gg1 * fabs(e) * tmp2);
   }
 }
 

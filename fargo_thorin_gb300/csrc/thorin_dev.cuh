@@ -132,24 +132,84 @@ __device__ T block_reduce(T v, Op op, T identity)
   return v;
 }
 
+// Reciprocal and reciprocal square root estimates without the FP64 pipe.
+// GB300 issues an FP64 warp instruction every 76 cycles of a sub-partition
+// (1.68 lanes per clock and SM, any mix of adds, products and FMAs) and FP32
+// and integer ones in 1 to 4, so an estimate that takes about 25 of those and
+// no FP64 instruction is nearly free beside the FP64 work of any kernel here.
+// The mantissa m of the operand is split into a 24-bit FP32 part and an FP32
+// remainder, m = mh + ml; one Newton-Raphson step (to second order) from the
+// hardware's FP32 estimate y0 gives the correction y - y0 in FP32, which is
+// added to the bits of y0 as a 64-bit integer in units of 2^-53 of the
+// binade [0.5, 1].  Relative error below 2^-43 even for an FP32 estimate 2 ulp
+// off (the form before this, the hardware's FP64 estimate with one FP64
+// Newton-Raphson step, had 2^-40 and cost two FP64 instructions).  Operands: normal numbers with exponents in
+// [-500, 500] (the callers check).
+__device__ __forceinline__ double est_assemble(float y0, float corr, int hi_shift)
+{
+  const int k = __float2int_rn(corr * 4503599627370496.0f);            // corr * 2^52, |k| < 2^31
+  const int b = __float_as_int(y0);
+  const long long base = __double_as_longlong(__hiloint2double((b >> 3) + 0x38000000 + hi_shift, b << 29));
+  return __longlong_as_double(base + 2LL * (long long)k);
+}
+
+// 1 / d, d of either sign.
+__device__ __forceinline__ double recip_est(double d)
+{
+  const int H = __double2hiint(d), L = __double2loint(d);
+  const float mh = __int_as_float((__funnelshift_l(L, H, 3) & 0x007fffff) | 0x3f800000);
+  const float ml = __int2float_rn(L & 0x1fffffff) * 2.220446049250313e-16f;    // 2^-52
+  float y0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+  y0 = fminf(fmaxf(y0, 0.5f), 1.0f);                 // m in [1, 2): 1/m in (0.5, 1]
+  const float e = __fmaf_rn(-ml, y0, __fmaf_rn(-mh, y0, 1.0f));
+  const double y = est_assemble(y0, y0 * __fmaf_rn(e, e, e), 0x3ff00000 - (H & 0x7ff00000));
+  return __hiloint2double(__double2hiint(y) | (H & 0x80000000), __double2loint(y));
+}
+
+// 1 / sqrt(x), x > 0.
+__device__ __forceinline__ double rsqrt_est(double x)
+{
+  const int H = __double2hiint(x), L = __double2loint(x);
+  const int odd = ~(H >> 20) & 1;                    // the exponent's parity goes into the mantissa, m in [1, 4)
+  const float mh = __int_as_float((__funnelshift_l(L, H, 3) & 0x007fffff) | ((127 + odd) << 23));
+  const float ml = __int2float_rn(L & 0x1fffffff) * __int_as_float((75 + odd) << 23);   // 2^(odd - 52)
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+  y0 = fminf(fmaxf(y0, 0.5f), 1.0f);
+  const float t = mh * y0, tl = __fmaf_rn(mh, y0, -t);
+  float e = __fmaf_rn(-t, y0, 1.0f);                 // 1 - m y0^2
+  e = __fmaf_rn(-tl, y0, e);
+  e = __fmaf_rn(-(ml * y0), y0, e);
+  const float c = e * __fmaf_rn(0.375f, e, 0.5f);    // (1 - e)^(-1/2) - 1 to second order
+  return est_assemble(y0, y0 * c, (1023 + odd - (H >> 20)) << 19);
+}
+
+// x / 2 on the integer pipe (x normal, not near the smallest exponent).
+__device__ __forceinline__ double half_i(double x)
+{
+  return __hiloint2double(__double2hiint(x) - 0x00100000, __double2loint(x));
+}
+
+// Whether the exponent of x lies in [-500, 500] (zero, subnormals,
+// infinities, NaN: no).
+__device__ __forceinline__ bool exp_ok(double x)
+{
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 523u < 1001u;
+}
+
+__device__ __forceinline__ bool exp_zero(double x) { return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) == 0u; }
+
 // Quotient for the van Leer slopes only.  The harmonic-mean slope
 // 2 dq- dq+ / (dq- + dq+) enters a face value as a correction of at most
 // half a cell width times the slope, beside the cell value itself, so a
 // relative error e of the slope moves the face value by at most
-// e |dq| dx / |q|.  The reciprocal estimate with one Newton-Raphson step,
-// y = y + y(1 - d y), times x is two FP64 instructions shorter than
-// div_fast; thorin_selftest_slope_division measures its distance from IEEE
-// division on the GPU.  Same exponent guard as div_fast.
+// e |dq| dx / |q|.  x times the reciprocal estimate: one FP64 instruction.
+// thorin_selftest_slope_division measures its distance from IEEE division
+// on the GPU.
 __device__ __forceinline__ double div_slope(double x, double d)
 {
-  const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  const unsigned ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
-  if (((ex - 523u) < 1001u || ex == 0u) && (ed - 523u) < 1001u) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-    return x * y;
-  }
+  if ((exp_ok(x) || exp_zero(x)) && exp_ok(d)) return x * recip_est(d);
   return x / d;
 }
 
@@ -205,23 +265,19 @@ __device__ __forceinline__ double cube_rn(double x)
   return __dadd_rn(p, t);
 }
 
-// Division without the IEEE divide sequence, for the hot stencils.  The
-// hardware reciprocal estimate (rcp.approx.ftz.f64) gets one Newton-Raphson
-// step, y = y + y(1 - d y); the quotient q = x y then gets Markstein's
+// Division without the IEEE divide sequence, for the hot stencils: the
+// quotient q = x y with the reciprocal estimate y gets Markstein's
 // correction q + (x - d q) y with the residual formed exactly by an FMA
-// (P. W. Markstein, IBM J. Res. Dev. 34(1):111-119, 1990).  Operands whose
-// exponents lie in [2^-500, 2^500] (x may also be zero or subnormal) take this
-// path, anything else the IEEE division.  thorin_selftest_division measures
-// it against IEEE division on the GPU (no difference in 1e9 random quotients).
+// (P. W. Markstein, IBM J. Res. Dev. 34(1):111-119, 1990): three FP64
+// instructions (two for a reciprocal), where the form with an FP64
+// Newton-Raphson step took five.  Operands whose exponents lie in
+// [-500, 500] (x may also be zero or subnormal) take this path, anything
+// else the IEEE division.  thorin_selftest_division measures it against IEEE
+// division on the GPU.
 __device__ __forceinline__ double div_fast(double x, double d)
 {
-  const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  const unsigned ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
-  if (((ex - 523u) < 1001u || ex == 0u) && (ed - 523u) < 1001u) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = __fma_rn(-d, y, 1.0);
-    y = __fma_rn(y, e, y);
+  if ((exp_ok(x) || exp_zero(x)) && exp_ok(d)) {
+    const double y = recip_est(d);
     const double q = x * y;
     const double r = __fma_rn(-d, q, x);
     return __fma_rn(r, y, q);
@@ -229,3 +285,28 @@ __device__ __forceinline__ double div_fast(double x, double d)
   return x / d;
 }
 
+// Square root and reciprocal square root in three FP64 instructions each:
+// the estimate y of 1/sqrt(x), then s = x y with the residual x - s^2 formed
+// exactly (Markstein's correction as in div_fast), or one Newton-Raphson step
+// of y.  thorin_selftest_sqrt measures both on the GPU.
+__device__ __forceinline__ double sqrt_fast(double x)
+{
+  if (exp_ok(x) && __double2hiint(x) > 0) {
+    const double y = rsqrt_est(x);
+    const double s = x * y;
+    const double r = __fma_rn(-s, s, x);
+    return __fma_rn(r, half_i(y), s);
+  }
+  return sqrt(x);
+}
+
+__device__ __forceinline__ double rsqrt_fast(double x)
+{
+  if (exp_ok(x) && __double2hiint(x) > 0) {
+    const double y = rsqrt_est(x);
+    const double t = x * y;
+    const double e = __fma_rn(-t, y, 1.0);
+    return __fma_rn(half_i(y), e, y);
+  }
+  return rsqrt(x);
+}

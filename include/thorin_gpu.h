@@ -402,8 +402,8 @@ int thorin_gpu_init_pebbles(thorin_disk *d);
 int thorin_gpu_request_torques(thorin_disk *d);
 int thorin_gpu_get_torques(thorin_disk *d, thorin_torque *out, int max, int *n);
 
-/* Self-test of the kernels' division routine (reciprocal estimate, one
- * Newton-Raphson step, Markstein correction) against IEEE division on the
+/* Self-test of the kernels' division routine (reciprocal estimate, Markstein
+ * correction) against IEEE division on the
  * current GPU: n random quotients of values with exponents uniform in
  * [-max_exponent, max_exponent]; returns how many differ and the largest
  * difference in ulps.  No counterpart in the reference (its divisions are
@@ -411,12 +411,20 @@ int thorin_gpu_get_torques(thorin_disk *d, thorin_torque *out, int max, int *n);
 int thorin_selftest_division(long long n, unsigned long long seed, double max_exponent,
                              unsigned long long *mismatches, unsigned long long *max_ulp);
 
-/* Self-test of the van Leer slopes' shorter division (reciprocal estimate
- * and one Newton-Raphson step, no correction) against IEEE division: n
+/* Self-test of the van Leer slopes' shorter division (product with the
+ * reciprocal estimate, no correction) against IEEE division: n
  * random quotients as above; returns the largest difference in ulps.  No
  * counterpart in the reference. */
 int thorin_selftest_slope_division(long long n, unsigned long long seed, double max_exponent,
                                    unsigned long long *max_ulp);
+
+/* Compares the kernels' square root routine with IEEE square root on n
+ * random operands (exponents in [-max_exponent, max_exponent]) and the
+ * reciprocal square root with 1 / sqrt(x): results that differ from sqrt, the
+ * largest distance from it, and the largest distance of the reciprocal square
+ * root beyond one ulp (0: none). */
+int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_exponent, unsigned long long *mismatches,
+                         unsigned long long *max_ulp, unsigned long long *max_ulp_rsqrt);
 
 /* Self-test of the conditional CUDA graph nodes behind the SOR sweep loop:
  * a kernel that sets an IF node's condition to 0 must skip its body
