@@ -970,8 +970,7 @@ __global__ void k_rad_slope(DevGrid g, PtrPack8 pk)
       const double dqp = (qn - qc) * g.r.InvDiffRmed[i + 1];
       double sl = 0.0;
       if (i > 0) {
-        const double p = dqp * dqm;
-        if (__double_as_longlong(p) > 0LL) sl = div_slope(2.0 * p, dqp + dqm);     // p > 0.0
+        sl = 2.0 * vl_slope(dqm, dqp);
       }
       dst[l] = sl;
       dqm = dqp;
@@ -1071,20 +1070,13 @@ __global__ void __launch_bounds__(256) k_azi_rings(DevGrid g, const double *__re
 // save FP64 instructions: Work = Q * (1 / (RhoInt + 1e-20)), the slope's
 // 1/dxtheta folded into the face coefficient, the flux as Q* times
 // (dxrad RhoStar v); results differ from the reference's grouping in the
-// last bits only.
+// last bits only.  The FP64 pipe bounds it: six FP64 instructions per quantity
+// and pass (the quotient, its difference, the face value, the flux and two for
+// the update; the slopes run on the FP32 and integer pipes, vl_slope).
+// 512x1536: 231 -> 147 us with the gas's six quantities (151 -> 92 FP64
+// instructions a cell).
 #define AZ_HALO 4
 #define AZ_TMAX 512
-
-// Slope from the differences dqm = q_j - q_{j-1} and dqp = q_{j+1} - q_j;
-// each thread forms its own dqm and reads dqp from its right neighbour.
-__device__ __forceinline__ double azi_vl_slope_d(double dqm, double dqp)
-{
-  const double p = dqp * dqm;
-  const double s = dqp + dqm;
-  const bool pos = __double_as_longlong(p) > 0LL;                 // p > 0.0
-  const bool nz = (__double_as_longlong(s) << 1) != 0LL;          // s != 0.0
-  return (pos && nz) ? div_slope(p, s) : 0.0;
-}
 
 template <int NQ>
 __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, const double *__restrict__ vt,
@@ -1099,11 +1091,8 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
   const int j = (j0 + t - AZ_HALO + ns) % ns;
   const int tm = (t == 0) ? 0 : t - 1, tp = (t == T - 1) ? t : t + 1;   // edge threads only feed the halo
   const size_t rowo = (size_t)i * ns;
-  const double rmed = g.r.Rmed[i];
-  // ring constants from tables (the same values as 2 pi / ns * Rmed, its
-  // inverse and 1 / Surf, without three divisions per thread)
-  const double dxtheta = g.k.dpns * rmed;
-  const double invdxtheta = g.r.InvDxtheta[i];
+  // ring constants from tables
+  const double dtinvdx = dt * g.r.InvDxtheta[i];
   const double dxrad = (g.r.Rsup[i] - g.r.Rinf[i]) * dt;
   const double invsurf = g.r.InvSurf[i];
   double q[NQ];
@@ -1115,15 +1104,13 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
   const int npass = fast ? 2 : 1;
   for (int pass = 0; pass < npass; pass++) {
     const double v = (pass == 1) ? vuni : (vface - vsub);
-    const double ksi = v * dt;
-    const bool up = ksi > 0.0;                     // upwind cell of the left face is j-1
-    // face value q* = q_up +/- (dxtheta -/+ ksi) dq_up with the slope dq kept
-    // without its 1/dxtheta factor, which goes into cs instead.  The upwind
-    // choice differs between neighbouring cells, so it selects operands
-    // (integer moves) and every face value is one FMA, fma(+/-cs, dq_up,
-    // q_up), rather than two predicated ones.
-    const double cs = (dxtheta + (up ? -ksi : ksi)) * invdxtheta;
-    const double csg = __hiloint2double(__double2hiint(cs) ^ (up ? 0 : (int)0x80000000), __double2loint(cs));
+    const bool up = __double_as_longlong(v) > 0LL; // v > 0.0: upwind cell of the left face is j-1
+    // face value q* = q_up +/- (dxtheta -/+ v dt) dq_up with the slope dq kept
+    // without its 1/dxtheta factor, which goes into csg = +/-1 - v dt/dxtheta
+    // instead.  The upwind choice differs between neighbouring cells, so it
+    // selects operands (integer moves) and every face value is one FMA,
+    // fma(csg, dq_up, q_up), rather than two predicated ones.
+    const double csg = __fma_rn(-v, dtinvdx, up ? 1.0 : -1.0);
     // RhoStar at the left face (ComputeStarTheta of the density)
     const double rho = q[NQ - 1];
     s_a[t] = rho;
@@ -1132,7 +1119,7 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
     const double drm = rho - rho_m;
     s_b[t] = drm;
     __syncthreads();
-    const double drho = azi_vl_slope_d(drm, s_b[tp]);
+    const double drho = vl_slope(drm, s_b[tp]);
     s_c[t] = drho;
     __syncthreads();
     const double rs = __fma_rn(csg, up ? s_c[tm] : drho, up ? rho_m : rho);
@@ -1142,7 +1129,7 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
 #pragma unroll
     for (int k = 0; k < NQ; k++) {
       // VanLeerTheta: Work = Q / (RhoInt + 1e-20), its slope, the face value
-      const double w = q[k] * rcp;
+      const double w = (k < NQ - 1) ? q[k] * rcp : unit_quotient(rho);
       s_a[t] = w;
       __syncthreads();
       const double w_m = s_a[tm];
@@ -1151,7 +1138,7 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
         const double dm = w - w_m;
         s_b[t] = dm;
         __syncthreads();
-        const double dq = azi_vl_slope_d(dm, s_b[tp]);
+        const double dq = vl_slope(dm, s_b[tp]);
         s_c[t] = dq;
         __syncthreads();
         qs = __fma_rn(csg, up ? s_c[tm] : dq, up ? w_m : w);

@@ -213,6 +213,54 @@ __device__ __forceinline__ double div_slope(double x, double d)
   return x / d;
 }
 
+// The van Leer slope of the differences a and b on either side of a cell,
+// a b / (a + b) where they agree in sign, else 0, without an FP64
+// instruction: product, sum and quotient as FP32 pairs.  |a| and |b| are
+// scaled by the larger one's power of two and split like recip_est's operand
+// (24 bits and the remainder in FP32); the sum is a two-sum, the quotient
+// b / (a + b) the hardware's reciprocal estimate with one correction from the
+// exact FP32 residual, and the pair's low part is added to the high part's
+// bits in units of their last place.  Relative error below 2^-42.  Differences
+// more than 2^60 apart, zero, not finite or near the ends of the exponent
+// range take the FP64 form (div_slope).  About 60 FP32 and integer
+// instructions in place of three FP64 ones (228 cycles of a sub-partition).
+__device__ __forceinline__ double vl_slope(double a, double b)
+{
+  const int Ha = __double2hiint(a), Hb = __double2hiint(b);
+  if ((Ha ^ Hb) < 0) return 0.0;
+  const int ea = Ha & 0x7ff00000, eb = Hb & 0x7ff00000;
+  const int eM = max(ea, eb), em = min(ea, eb);
+  if (em >= (100 << 20) && eM < 0x7ff00000 && eM - em <= (60 << 20)) {
+    const int La = __double2loint(a), Lb = __double2loint(b);
+    const int sh = eM - (127 << 20);
+    const float ah = __int_as_float(__funnelshift_l(La, (Ha & 0x7fffffff) - sh, 3));
+    const float bh = __int_as_float(__funnelshift_l(Lb, (Hb & 0x7fffffff) - sh, 3));
+    const float al = __int2float_rn(La & 0x1fffffff) * __int_as_float((__float_as_int(ah) & 0x7f800000) - (52 << 23));
+    const float bl = __int2float_rn(Lb & 0x1fffffff) * __int_as_float((__float_as_int(bh) & 0x7f800000) - (52 << 23));
+    const float s = __fadd_rn(ah, bh), t = __fsub_rn(s, ah);
+    const float sl = __fadd_rn(__fadd_rn(__fsub_rn(ah, __fsub_rn(s, t)), __fsub_rn(bh, t)), __fadd_rn(al, bl));
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    const float qh = __fmul_rn(bh, y);
+    const float ql = __fmul_rn(__fadd_rn(__fmaf_rn(-qh, s, bh), __fmaf_rn(-qh, sl, bl)), y);
+    const float dh = __fmul_rn(ah, qh);
+    const float dl = __fmaf_rn(al, qh, __fmaf_rn(ah, ql, __fmaf_rn(ah, qh, -dh)));
+    // dh + dl as a float h and a remainder of the same sign, so that adding
+    // the remainder to the bits never crosses a power of two downwards
+    float h = __fadd_rn(dh, dl), l = __fadd_rn(__fsub_rn(dh, h), dl);
+    const int hb = __float_as_int(h) + (__float_as_int(l) >> 31);
+    l = __fadd_rn(__fsub_rn(h, __int_as_float(hb)), l);
+    const int k = __float2int_rn(l * __int_as_float((306 << 23) - (hb & 0x7f800000)));
+    const long long base =
+        __double_as_longlong(__hiloint2double(((hb >> 3) + sh) | (Ha & 0x80000000), hb << 29));
+    return __longlong_as_double(base + (long long)k);
+  }
+  const double p = a * b, s = a + b;
+  const bool pos = __double_as_longlong(p) > 0LL;                 // p > 0.0
+  const bool nz = (__double_as_longlong(s) << 1) != 0LL;          // s != 0.0
+  return (pos && nz) ? div_slope(p, s) : 0.0;
+}
+
 // |x| by clearing the sign bit on the integer pipe (same bits as fabs).
 __device__ __forceinline__ double abs_i(double x)
 {
@@ -309,4 +357,23 @@ __device__ __forceinline__ double rsqrt_fast(double x)
     return __fma_rn(half_i(y), e, y);
   }
   return rsqrt(x);
+}
+
+// r / (r + 1e-20), the density's own transported quotient (the reference
+// divides every transported quantity by Sigma + 1e-20): 1 where 1e-20 is
+// below half an ulp of r, else 1 - 1e-20 / r with the small quotient in FP32
+// (it is below 2^-31, so its FP32 error is below rounding) subtracted from the
+// bits of 1; very small, negative or non-finite r divide.
+__device__ __forceinline__ double unit_quotient(double r)
+{
+  const int H = __double2hiint(r);
+  if (H >= (1010 << 20) && H < 0x7ff00000) return 1.0;            // r >= 2^-13
+  if (H >= (988 << 20) && H < 0x7ff00000) {                       // r >= 2^-35
+    const float rf = __int_as_float(__funnelshift_l(__double2loint(r), H - 0x38000000, 3));
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(rf));
+    const int k = __float2int_rn(1.0e-20f * y * 9007199254740992.0f);   // units of 2^-53
+    return __longlong_as_double(0x3ff0000000000000LL - (long long)k);
+  }
+  return r * div_fast(1.0, r + 1e-20);
 }

@@ -1,5 +1,5 @@
 // thorin_selftest.cu -- on-device checks of the kernels' division and square
-// root routines (div_fast, div_slope, sqrt_fast, rsqrt_fast) against the IEEE
+// root routines (div_fast, div_slope, vl_slope, sqrt_fast, rsqrt_fast) against the IEEE
 // operations, conditional graph nodes, and the FP64 FMA peak.
 #include <string>
 #include "thorin_kernels.cuh"
@@ -331,6 +331,52 @@ extern "C" int thorin_selftest_slope_division(long long n, unsigned long long se
     return THORIN_ERR_CUDA;
   }
   *max_ulp = host;
+  return THORIN_OK;
+}
+
+// vl_slope against a (b / (a + b)) (0 where the signs differ), the two
+// operands' exponents within 2^emax of each other around a random common one;
+// unit_quotient against r / (r + 1e-20).
+__global__ void k_selftest_vl_slope(long long n, unsigned long long seed, double emax,
+                                    unsigned long long *__restrict__ out)
+{
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const unsigned long long key = seed + 3ULL * (unsigned long long)t;
+  const double c = exp2((double)(int)(st_mix(key) % 201ULL) - 100.0);
+  const double a = st_value(key + 1ULL, emax) * c, b = st_value(key + 2ULL, emax) * c;
+  const double ref = ((a > 0.0) == (b > 0.0)) ? a * (b / (a + b)) : 0.0;
+  const long long x = __double_as_longlong(ref), y = __double_as_longlong(vl_slope(a, b));
+  const unsigned long long u = (unsigned long long)(x > y ? x - y : y - x);
+  if (u) atomicMax(out, u);
+  const double r = fabs(st_value(key + 1ULL, emax));
+  const long long v = __double_as_longlong(r / (r + 1e-20)), w = __double_as_longlong(unit_quotient(r));
+  const unsigned long long z = (unsigned long long)(v > w ? v - w : w - v);
+  if (z) atomicMax(out + 1, z);
+}
+
+extern "C" int thorin_selftest_vl_slope(long long n, unsigned long long seed, double max_exponent,
+                                        unsigned long long *max_ulp, unsigned long long *max_ulp_quotient)
+{
+  if (n < 1 || !max_ulp || !max_ulp_quotient || !(max_exponent >= 0.0 && max_exponent <= 300.0)) {
+    g_last_error = "selftest_vl_slope: n >= 1, 0 <= max_exponent <= 300 and output pointers required";
+    return THORIN_ERR_ARG;
+  }
+  unsigned long long *dev = nullptr, host[2] = {0ULL, 0ULL};
+  cudaError_t e = cudaMalloc((void **)&dev, sizeof(host));
+  if (e == cudaSuccess) e = cudaMemset(dev, 0, sizeof(host));
+  if (e == cudaSuccess) {
+    k_selftest_vl_slope<<<(unsigned)((n + 255) / 256), 256>>>(n, seed, max_exponent, dev);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(host, dev, sizeof(host), cudaMemcpyDeviceToHost);
+  if (dev) cudaFree(dev);
+  if (e != cudaSuccess) {
+    g_last_error = std::string("selftest_vl_slope: ") + cudaGetErrorString(e);
+    return THORIN_ERR_CUDA;
+  }
+  *max_ulp = host[0];
+  *max_ulp_quotient = host[1];
   return THORIN_OK;
 }
 

@@ -418,6 +418,12 @@ int thorin_selftest_division(long long n, unsigned long long seed, double max_ex
 int thorin_selftest_slope_division(long long n, unsigned long long seed, double max_exponent,
                                    unsigned long long *max_ulp);
 
+/* Self-test of the van Leer slope a b / (a + b) in FP32 pairs and of the
+ * density's own quotient r / (r + 1e-20) against their FP64 forms: n random
+ * operands; returns the largest differences in ulps. */
+int thorin_selftest_vl_slope(long long n, unsigned long long seed, double max_exponent, unsigned long long *max_ulp,
+                             unsigned long long *max_ulp_quotient);
+
 /* Compares the kernels' square root routine with IEEE square root on n
  * random operands (exponents in [-max_exponent, max_exponent]) and the
  * reciprocal square root with 1 / sqrt(x): results that differ from sqrt, the

@@ -34,6 +34,21 @@ def test_slope_division_bound(max_exponent, seed):
     assert ulp.value <= 16384
 
 
+@pytest.mark.parametrize("max_exponent,seed", [(0.5, 9), (20.0, 10), (29.9, 11), (32.0, 12), (200.0, 13)])
+def test_van_leer_slope_bound(max_exponent, seed):
+    """The slope a b / (a + b) in FP32 pairs keeps the bound of the slopes'
+    division, 2^14 ulp, on both sides of its range (operands 2^60 apart) and
+    for both signs; the density's quotient r / (r + 1e-20) within 2 ulp."""
+    from fargo_thorin_gb300 import _lib
+    lib = _lib.load()
+    ulp, q = C.c_ulonglong(), C.c_ulonglong()
+    _lib.check(lib.thorin_selftest_vl_slope(1 << 26, seed, max_exponent, C.byref(ulp), C.byref(q)),
+               "selftest_vl_slope")
+    print("slope: max", ulp.value, "ulp; quotient:", q.value)
+    assert ulp.value <= 16384
+    assert q.value <= 2
+
+
 @pytest.mark.parametrize("max_exponent,seed", [(40.0, 6), (300.0, 7), (1000.0, 8)])
 def test_square_roots_match_ieee(max_exponent, seed):
     """sqrt_fast is Markstein-corrected like the division: at most one ulp
