@@ -897,37 +897,195 @@ __global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, doubl
 }
 
 // ---------------------------------------------------------------------------
-// Transport (TransportEuler.c).  Radial step: the six (gas) or five
-// (pebbles) transported quantities are updated out of place from the old
-// state, in four cell-parallel passes: quotients by the density, van Leer
-// slopes, upwind face values, flux divergence.
+// Transport (TransportEuler.c).  Radial step of one fluid in one kernel:
+// ComputeLRMomenta and the quotients by the density (TransportEuler.c:
+// 318-347), VanLeerRadial's slopes, ComputeStarRad's upwind face values
+// (:232-273) and the flux divergence (:384-415).
+//
+// A thread walks a chunk of rings of one column and keeps the quotients,
+// slopes and incoming fluxes of the current and the next ring in registers,
+// so the state is read once and the updated quantities are written once (four
+// kernels with about 70 field passes between them before this).  Like the
+// other stencils it is bound by the FP64 pipe, so the arithmetic is arranged
+// for few FP64 instructions (about 50 a cell for the gas, 41 for the pebbles):
+// * the quotients Q / (Sigma + 1e-20) of the momenta Sigma v and
+//   Sigma (v_theta + Omega r) r are the velocities times unit_quotient(Sigma),
+//   which is exactly 1 in all but thin gas;
+// * the slope of the quotients with ring spacings h,
+//   2 (d- / h-)(d+ / h+) / (d- / h- + d+ / h+) = 2 d- d+ / (h- (rho d- + d+)),
+//   rho = h+ / h-, comes from vl_slope without FP64; its 1 / h- goes into the
+//   face coefficient, +/-rho - v dt / h-, one FMA;
+// * each face's flux is formed once and shared by the two rings.
+// Slopes are zero in rings 0 and nr-1, the faces 0 and nr carry no flux.
+// Ring constants of the chunk are formed once per block in shared memory.
+// 512x1536: 150 us (gas) and 125 us (pebbles) in the four kernels, 90 and 73 us
+// here; 1024x3072: 335 and 270 us, 96% of the FP64 pipe's rate.
+#define RD_MAXRINGS 40
 
+struct RadialIO {
+  const double *rho, *vr, *vt, *energy, *label;
+  double *out[6];           // the four momenta, the density, the energy
+  double *ext;              // Sigma * label
+  int rings;                // rings per block
+};
 
-// ComputeLRMomenta (TransportEuler.c:318-347) + DivisePolarGrid quotients.
-__global__ void k_rad_prep(DevGrid g, int nq, const double *__restrict__ rho, const double *__restrict__ vr,
-                           const double *__restrict__ vt, const double *__restrict__ energy, double *rmp, double *rmm,
-                           double *tmp_, double *tmm, double *w0, double *w1, double *w2, double *w3, double *we,
-                           double *wr, const double *__restrict__ label, double *ext, double *wx)
+struct RdRing { double rm, cu, rho, dtinv, isd, rinf; float wh, wl; };
+
+// The ring's quotients: w[0..3] the momenta's, then energy, tracer.
+template <bool E, bool X>
+__device__ __forceinline__ void rd_load(const DevGrid &g, const RadialIO &io, const RdRing &c, int i, int j, int jp,
+                                        double vr_i, double &vr_ip, double &r, double &wr, double *w)
 {
-  const double omega_frame = g.ctl[CTL_OMEGA_FRAME];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const double r = rho[l], rm = g.r.Rmed[i];
-  const double a = r * vr[l + ns];
-  const double b = r * vr[l];
-  const double c = r * (vt[ljp] + rm * omega_frame) * rm;
-  const double d = r * (vt[l] + rm * omega_frame) * rm;
-  rmp[l] = a; rmm[l] = b; tmp_[l] = c; tmm[l] = d;
-  const double rcp = div_fast(1.0, r + 1e-20);    // quotients Q / (rho + 1e-20) as products
-  w0[l] = a * rcp; w1[l] = b * rcp; w2[l] = c * rcp; w3[l] = d * rcp;
-  if (energy) we[l] = energy[l] * rcp;
-  if (label) {                              // ComputeExtQty (TransportEuler.c:177-195)
-    const double x = r * label[l];
-    ext[l] = x;
-    wx[l] = x * rcp;
+  const int ns = g.ns, l = j + i * ns;
+  r = io.rho[l];
+  vr_ip = io.vr[l + ns];
+  const double u = __fma_rn(io.vt[l], c.rm, c.cu), ujp = __fma_rn(io.vt[jp + i * ns], c.rm, c.cu);
+  wr = unit_quotient(r);
+  w[0] = vr_ip; w[1] = vr_i; w[2] = ujp; w[3] = u;
+  double d = r;
+  if (X) w[4 + E] = io.label[l];
+  if (__double2hiint(wr) != 0x3ff00000) {          // thin gas
+    w[0] *= wr; w[1] *= wr; w[2] *= wr; w[3] *= wr;
+    if (X) w[4 + E] *= wr;
+    d = r + 1e-20;
   }
-  wr[l] = r * rcp;
+  if (E) w[4] = div_fast(io.energy[l], d);
+}
+
+template <bool E, bool X>
+__global__ void __launch_bounds__(BX, 4) k_radial(DevGrid g, RadialIO io)
+{
+  constexpr int NW = 4 + E + X;
+  __shared__ RdRing ring[RD_MAXRINGS + 4];
+  const double dt = g.ctl[CTL_DT];
+  const int ns = g.ns, nr = g.nr;
+  const int i0 = blockIdx.y * io.rings;
+  const int i1 = min(i0 + io.rings, nr);
+  // ring constants of rings i0-2 .. i1+1 (entry 0 is ring i0-2)
+  {
+    const int i = i0 - 2 + (int)threadIdx.x;
+    if (i >= 0 && i < nr && i <= i1 + 1) {
+      RdRing &c = ring[threadIdx.x];
+      c.rm = g.r.Rmed[i];
+      c.cu = c.rm * g.ctl[CTL_OMEGA_FRAME] * c.rm;
+      const double inv = g.r.InvDiffRmed[i];       // 0 in ring 0
+      c.dtinv = dt * inv;
+      c.rho = (i >= 1 && i < nr - 1) ? (g.r.Rmed[i + 1] - c.rm) * inv : 0.0;
+      c.wh = (float)c.rho;
+      c.wl = (float)(c.rho - (double)c.wh);
+      c.isd = dt * g.k.dpns * g.r.InvSurf[i];
+      c.rinf = g.r.Rinf[i];
+    }
+  }
+  __syncthreads();
+  const int j = blockIdx.x * BX + threadIdx.x;
+  if (j >= ns) return;
+  const int jp = (j == ns - 1) ? 0 : j + 1;
+  const RdRing *R = ring + 2 - i0;                  // R[i]: ring i
+  // cur: ring i, nxt: ring i+1; ds: differences between them
+  double wc[NW], wn[NW], ds[NW], sc[NW], fin[NW + 1];
+  double rc, rn, wrc, wrn, dr, srho = 0.0, vn, vf;
+  int i;
+#pragma unroll
+  for (int k = 0; k < NW; k++) sc[k] = 0.0;
+  if (i0 == 0) {
+    i = 0;
+    rd_load<E, X>(g, io, R[0], 0, j, jp, io.vr[j], vf, rc, wrc, wc);
+  } else {
+    // the face between rings i0-1 and i0 needs the slope of ring i0-1
+    i = i0 - 1;
+    double w0[NW], r0, wr0;
+    if (i >= 1) {
+      rd_load<E, X>(g, io, R[i - 1], i - 1, j, jp, io.vr[j + (i - 1) * ns], vf, r0, wr0, w0);
+    } else {
+      vf = io.vr[j + i * ns];
+    }
+    rd_load<E, X>(g, io, R[i], i, j, jp, vf, vf, rc, wrc, wc);
+    if (i >= 1) {
+#pragma unroll
+      for (int k = 0; k < NW; k++) sc[k] = wc[k] - w0[k];
+      srho = rc - r0;
+    }
+  }
+  // vf: v_r at face i+1
+  rd_load<E, X>(g, io, R[i + 1], i + 1, j, jp, vf, vn, rn, wrn, wn);
+#pragma unroll
+  for (int k = 0; k < NW; k++) ds[k] = wn[k] - wc[k];
+  dr = rn - rc;
+  if (i0 > 0 && i >= 1) {
+    const RdRing &c = R[i];
+#pragma unroll
+    for (int k = 0; k < NW; k++) sc[k] = vl_slope_t<true>(sc[k], ds[k], c.wh, c.wl, c.rho);
+    srho = vl_slope_t<true>(srho, dr, c.wh, c.wl, c.rho);
+  }
+#pragma unroll
+  for (int k = 0; k <= NW; k++) fin[k] = 0.0;
+  for (; i < i1; i++) {
+    const int l = j + i * ns;
+    double sn[NW], fout[NW + 1], sr = 0.0, w2[NW], r2 = 0.0, wr2 = 0.0, v2 = 0.0;
+#pragma unroll
+    for (int k = 0; k < NW; k++) sn[k] = 0.0;
+    if (i + 2 < nr) {                               // ring i+2, and the slope of ring i+1
+      rd_load<E, X>(g, io, R[i + 2], i + 2, j, jp, vn, v2, r2, wr2, w2);
+      const RdRing &c = R[i + 1];
+#pragma unroll
+      for (int k = 0; k < NW; k++) {
+        const double d2 = w2[k] - wn[k];
+        sn[k] = vl_slope_t<true>(ds[k], d2, c.wh, c.wl, c.rho);
+        ds[k] = d2;
+      }
+      const double d2 = r2 - rn;
+      sr = vl_slope_t<true>(dr, d2, c.wh, c.wl, c.rho);
+      dr = d2;
+    }
+    if (i + 1 < nr) {                               // the face between rings i and i+1
+      const RdRing &a = R[i], &b = R[i + 1];
+      const bool up = __double_as_longlong(vf) > 0LL;             // v > 0.0
+      const double c = __fma_rn(-vf, up ? a.dtinv : b.dtinv, up ? a.rho : -b.rho);
+      const double f = b.rinf * vf * __fma_rn(c, up ? srho : sr, up ? rc : rn);
+#pragma unroll
+      for (int k = 0; k < NW; k++) fout[k] = __fma_rn(c, up ? sc[k] : sn[k], up ? wc[k] : wn[k]) * f;
+      const double wu = up ? wrc : wrn;
+      fout[NW] = (__double2hiint(wu) == 0x3ff00000) ? f : wu * f;
+    } else {
+#pragma unroll
+      for (int k = 0; k <= NW; k++) fout[k] = 0.0;
+    }
+    if (i >= i0) {
+      const double isd = R[i].isd;
+      const double q = rc + 1e-20;                  // momenta Sigma v = (Sigma + 1e-20) w
+#pragma unroll
+      for (int k = 0; k < 4; k++) io.out[k][l] = __fma_rn(fin[k] - fout[k], isd, q * wc[k]);
+      if (E) io.out[5][l] = __fma_rn(fin[4] - fout[4], isd, io.energy[l]);
+      if (X) io.ext[l] = __fma_rn(fin[4 + E] - fout[4 + E], isd, rc * io.label[l]);
+      io.out[4][l] = __fma_rn(fin[NW] - fout[NW], isd, rc);
+    }
+#pragma unroll
+    for (int k = 0; k < NW; k++) { wc[k] = wn[k]; wn[k] = w2[k]; sc[k] = sn[k]; fin[k] = fout[k]; }
+    fin[NW] = fout[NW];
+    rc = rn; rn = r2; wrc = wrn; wrn = wr2; srho = sr; vf = vn; vn = v2;
+  }
+}
+
+// Rings per block of the radial step: the chunk length with the least work on
+// the busiest multiprocessor, which runs its blocks four at a time (the
+// registers' limit) and uses 50, 80 or 92% of the FP64 pipe with one, two or
+// three of them left; 1.3 rings per chunk are the slopes and the face that
+// neighbouring chunks both form.  Measured for the gas: 256x768 37 / 39 / 51 us
+// with 4 / 6 / 9 rings, 512x1536 105 / 95 / 90 / 103 us with 7 / 11 / 14 / 21,
+// 1024x3072 355 / 335 / 366 / 350 us with 10 / 14 / 20 / 27.
+static int rd_rings(int nr, int ns, int nsm)
+{
+  const double part[4] = {0.0, 1.0 / 0.5, 2.0 / 0.8, 3.0 / 0.92};
+  const long long nbx = (ns + BX - 1) / BX;
+  int best = 2;
+  double bestw = 1e300;
+  for (int r = 2; r <= RD_MAXRINGS; r++) {
+    const long long n = (nbx * ((nr + r - 1) / r) + nsm - 1) / nsm;
+    const double w = ((double)(n / 4 * 4) + part[n % 4]) * (r + 1.3);
+    if (w < bestw) { bestw = w; best = r; }
+  }
+  return best;
 }
 
 // ComputeSpeQty (TransportEuler.c:197-215): the tracer back from rho*label.
@@ -937,88 +1095,6 @@ __global__ void k_label_from_ext(DevGrid g, const double *__restrict__ rho, cons
   const int ns = g.ns;
   CELL_LOOP_2D
   label[l] = div_fast(ext[l], rho[l]);
-}
-
-// VanLeerRadial's slope (TransportEuler.c:384-415): with
-// dqm = (q_i - q_{i-1}) InvDiffRmed[i] and dqp = (q_{i+1} - q_i) InvDiffRmed[i+1],
-// 2 dqp dqm / (dqp + dqm) where dqp dqm > 0, else 0; 0 in rings 0 and nr-1.
-// One thread walks RS_RINGS rings of one column, so the difference between
-// rings i and i+1 (dqp of ring i) is formed once and reused as dqm of ring
-// i+1: the same values as a cell-by-cell evaluation, two FP64 instructions
-// fewer per cell and quantity.
-#define RS_RINGS 8
-
-__global__ void k_rad_slope(DevGrid g, PtrPack8 pk)
-{
-  const int ns = g.ns, nr = g.nr;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ns) return;
-  const int i0 = blockIdx.y * RS_RINGS;
-  const int i1 = (i0 + RS_RINGS < nr) ? i0 + RS_RINGS : nr;
-  for (int q = 0; q < pk.n; q++) {
-    const double *src = pk.src[q];
-    double *dst = pk.dst[q];
-    double qc = src[j + i0 * ns];
-    double dqm = (i0 >= 1) ? (qc - src[j + (i0 - 1) * ns]) * g.r.InvDiffRmed[i0] : 0.0;
-    for (int i = i0; i < i1; i++) {
-      const int l = j + i * ns;
-      if (i == nr - 1) {
-        dst[l] = 0.0;
-        break;
-      }
-      const double qn = src[l + ns];
-      const double dqp = (qn - qc) * g.r.InvDiffRmed[i + 1];
-      double sl = 0.0;
-      if (i > 0) {
-        sl = 2.0 * vl_slope(dqm, dqp);
-      }
-      dst[l] = sl;
-      dqm = dqp;
-      qc = qn;
-    }
-  }
-}
-
-// ComputeStarRad (TransportEuler.c:232-273): upwind face values at the inner
-// face of ring i (faces 0 and nr are zero).
-__global__ void k_rad_face(DevGrid g, PtrPack8 w, PtrPack8 dq, const double *__restrict__ vr)
-{
-  const double dt = g.ctl[CTL_DT];
-  const int ns = g.ns, nr = g.nr;
-  CELL_LOOP_2D
-  if (i == 0 || i == nr) {
-    for (int q = 0; q < w.n; q++) w.dst[q][l] = 0.0;
-    return;
-  }
-  const double v = vr[l];
-  if (v > 0.0) {
-    const double c = (g.r.Rmed[i] - g.r.Rmed[i - 1] - v * dt) * 0.5;
-    for (int q = 0; q < w.n; q++)
-      w.dst[q][l] = dq.src[q] ? w.src[q][l - ns] + c * dq.src[q][l - ns] : w.src[q][l - ns];
-  } else {
-    const double c = (g.r.Rmed[i + 1] - g.r.Rmed[i] + v * dt) * 0.5;
-    for (int q = 0; q < w.n; q++) w.dst[q][l] = dq.src[q] ? w.src[q][l] - c * dq.src[q][l] : w.src[q][l];
-  }
-}
-
-// VanLeerRadial update (TransportEuler.c:384-415).
-__global__ void k_rad_update(DevGrid g, PtrPack8 qf, const double *__restrict__ rhos, const double *__restrict__ vr,
-                             PtrPack8 io)
-{
-  const double dt = g.ctl[CTL_DT];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  const int lip = l + ns;
-  const double dtheta = g.k.dpns;
-  // the mass fluxes through the inner and outer faces are shared by all
-  // quantities: varq = q*_in fin - q*_out fout
-  const double fin = dt * dtheta * g.r.Rinf[i] * rhos[l] * vr[l];
-  const double fout = dt * dtheta * g.r.Rsup[i] * rhos[lip] * vr[lip];
-  const double is = g.r.InvSurf[i];
-  for (int q = 0; q < io.n; q++) {
-    const double varq = __fma_rn(qf.src[q][l], fin, -(qf.src[q][lip] * fout));
-    io.dst[q][l] = __fma_rn(varq, is, io.src[q][l]);
-  }
 }
 
 // Per-ring quantities of ComputeResiduals (TransportEuler.c:70-111): VMed,
@@ -1372,7 +1448,7 @@ void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double 
 }
 
 // Whole transport of one fluid.  q_in: rho, vr, vt, energy (NULL for
-// pebbles).  Scratch: 20 fields.  On return the caller's rho/energy pointers
+// pebbles).  On return the caller's rho/energy pointers
 // are swapped with the updated buffers and vr/vt hold the new velocities.
 
 void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, double **energy, double *label,
@@ -1388,42 +1464,19 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   if (energy) qi[nq++] = 4;
   if (label) qi[nq++] = 6;
   qi[nq++] = 5;
-  k_rad_prep<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, nq, *rho, vr, vt, energy ? *energy : nullptr, S.mom[0], S.mom[1],
-                                               S.mom[2], S.mom[3], S.w[0], S.w[1], S.w[2], S.w[3], S.w[4], S.w[5], label, S.ext, S.w[6]);
-  g_thorin_launches++;
-  // slopes of the quotients and of rho (slot 7)
-  PtrPack8 sl;
-  int n = 0;
-  // (the quotient rho / (rho + 1e-20) of the density is 1 to within
-  // 1e-20 / rho, so its slope term is below rounding and is left out)
-  for (int k = 0; k < nq; k++)
-    if (qi[k] != 5) { sl.src[n] = S.w[qi[k]]; sl.dst[n] = S.d[qi[k]]; n++; }
-  sl.src[n] = *rho; sl.dst[n] = S.d[7]; n++;
-  sl.n = n;
-  k_rad_slope<<<dim3((ns + BX - 1) / BX, (nr + RS_RINGS - 1) / RS_RINGS), BX, 0, s>>>(g, sl);
-  g_thorin_launches++;
-  // faces: quotients and rho
-  PtrPack8 wf, dqf;
-  n = 0;
-  for (int k = 0; k < nq; k++) {
-    wf.src[n] = S.w[qi[k]]; wf.dst[n] = S.f[qi[k]]; dqf.src[n] = (qi[k] == 5) ? nullptr : S.d[qi[k]]; n++;
-  }
-  wf.src[n] = *rho; wf.dst[n] = S.f[7]; dqf.src[n] = S.d[7]; n++;
-  wf.n = dqf.n = n;
-  k_rad_face<<<grid2d(ns, nr + 1, BX), BX, 0, s>>>(g, wf, dqf, vr);
-  g_thorin_launches++;
-  // flux divergence into the quotient buffers, which are free by now
-  PtrPack8 qf, io;
-  n = 0;
-  for (int k = 0; k < nq; k++) {
-    const int q = qi[k];
-    qf.src[n] = S.f[q];
-    io.src[n] = (q < 4) ? S.mom[q] : (q == 4) ? *energy : (q == 6) ? S.ext : *rho;
-    io.dst[n] = S.w[q];
-    n++;
-  }
-  qf.n = io.n = n;
-  k_rad_update<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, qf, S.f[7], vr, io);
+  // the radially transported quantities go to the w buffers
+  RadialIO rd;
+  rd.rho = *rho; rd.vr = vr; rd.vt = vt; rd.energy = energy ? *energy : nullptr; rd.label = label;
+  for (int q = 0; q < 4; q++) rd.out[q] = S.w[q];
+  rd.out[4] = S.w[5];
+  rd.out[5] = S.w[4];
+  rd.ext = S.w[6];
+  rd.rings = rd_rings(nr, ns, g.nsm);
+  const dim3 rgrid((ns + BX - 1) / BX, (nr + rd.rings - 1) / rd.rings);
+  if (energy && label) k_radial<true, true><<<rgrid, BX, 0, s>>>(g, rd);
+  else if (energy) k_radial<true, false><<<rgrid, BX, 0, s>>>(g, rd);
+  else if (label) k_radial<false, true><<<rgrid, BX, 0, s>>>(g, rd);
+  else k_radial<false, false><<<rgrid, BX, 0, s>>>(g, rd);
   g_thorin_launches++;
   // azimuthal step back into the momenta, the new energy, the tracer and
   // the new density
@@ -1432,7 +1485,7 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   AziIO az;
   for (int k = 0; k < nq; k++) {
     const int q = qi[k];
-    az.src[k] = io.dst[k];
+    az.src[k] = S.w[q];
     az.dst[k] = (q < 4) ? S.mom[q] : (q == 4) ? S.e_new : (q == 6) ? S.ext_new : S.rho_new;
   }
   az.n = nq;

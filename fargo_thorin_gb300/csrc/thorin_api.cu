@@ -437,15 +437,9 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   }
   for (int q = 0; q < 4; q++) RCHK(dfield(d, &d->ts.mom[q]));
   for (int q = 0; q < 6; q++) RCHK(dfield(d, &d->ts.w[q]));
-  for (int q = 0; q < 8; q++) {
-    if (q == 6 && !d->p.label_advection) { d->ts.d[q] = d->ts.f[q] = nullptr; continue; }
-    RCHK(dfield(d, &d->ts.d[q]));
-    RCHK(dfield(d, &d->ts.f[q]));
-  }
-  d->ts.w[6] = d->ts.ext = d->ts.ext_new = nullptr;
+  d->ts.w[6] = d->ts.ext_new = nullptr;
   if (d->p.label_advection) {
     RCHK(dfield(d, &d->ts.w[6]));
-    RCHK(dfield(d, &d->ts.ext));
     RCHK(dfield(d, &d->ts.ext_new));
     RCHK(dfield(d, &d->label));
   }
@@ -457,17 +451,11 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     TransportScratch &P = d->ts_peb;
     P = TransportScratch{};
     for (int q = 0; q < 4; q++) RCHK(dfield(d, &P.mom[q]));
-    for (int q = 0; q < 6; q++) RCHK(dfield(d, &P.w[q]));
-    // pebbles carry the four momenta (slots 0-3) and the density (slot 5,
-    // its slope in slot 7): no energy or tracer slots, no slope of the
-    // density quotient
-    for (int q = 0; q < 8; q++) {
-      const bool used = q < 4 || q == 5 || q == 7;
-      P.d[q] = P.f[q] = nullptr;
-      if (used && q != 5) RCHK(dfield(d, &P.d[q]));
-      if (used) RCHK(dfield(d, &P.f[q]));
+    for (int q = 0; q < 6; q++) {
+      P.w[q] = nullptr;
+      if (q != 4) RCHK(dfield(d, &P.w[q]));        // no energy
     }
-    P.w[6] = P.ext = P.ext_new = nullptr;
+    P.w[6] = P.ext_new = nullptr;
     RCHK(dalloc(d, (void **)&P.nshift, n1 * sizeof(int)));
     RCHK(dalloc(d, (void **)&P.vmed, n1 * sizeof(double)));
     RCHK(dalloc(d, (void **)&P.vtemp, n1 * sizeof(double)));

@@ -224,7 +224,10 @@ __device__ __forceinline__ double div_slope(double x, double d)
 // more than 2^60 apart, zero, not finite or near the ends of the exponent
 // range take the FP64 form (div_slope).  About 60 FP32 and integer
 // instructions in place of three FP64 ones (228 cycles of a sub-partition).
-__device__ __forceinline__ double vl_slope(double a, double b)
+// With WEIGHTED the sum is w a + b (the radial step's unequal ring spacings),
+// w = wh + wl as an FP32 pair, w64 the same in FP64.
+template <bool WEIGHTED>
+__device__ __forceinline__ double vl_slope_t(double a, double b, float wh, float wl, double w64)
 {
   const int Ha = __double2hiint(a), Hb = __double2hiint(b);
   if ((Ha ^ Hb) < 0) return 0.0;
@@ -237,8 +240,13 @@ __device__ __forceinline__ double vl_slope(double a, double b)
     const float bh = __int_as_float(__funnelshift_l(Lb, (Hb & 0x7fffffff) - sh, 3));
     const float al = __int2float_rn(La & 0x1fffffff) * __int_as_float((__float_as_int(ah) & 0x7f800000) - (52 << 23));
     const float bl = __int2float_rn(Lb & 0x1fffffff) * __int_as_float((__float_as_int(bh) & 0x7f800000) - (52 << 23));
-    const float s = __fadd_rn(ah, bh), t = __fsub_rn(s, ah);
-    const float sl = __fadd_rn(__fadd_rn(__fsub_rn(ah, __fsub_rn(s, t)), __fsub_rn(bh, t)), __fadd_rn(al, bl));
+    float ch = ah, cl = al;
+    if (WEIGHTED) {
+      ch = __fmul_rn(ah, wh);
+      cl = __fmaf_rn(al, wh, __fmaf_rn(ah, wl, __fmaf_rn(ah, wh, -ch)));
+    }
+    const float s = __fadd_rn(ch, bh), t = __fsub_rn(s, ch);
+    const float sl = __fadd_rn(__fadd_rn(__fsub_rn(ch, __fsub_rn(s, t)), __fsub_rn(bh, t)), __fadd_rn(cl, bl));
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
     const float qh = __fmul_rn(bh, y);
@@ -255,11 +263,13 @@ __device__ __forceinline__ double vl_slope(double a, double b)
         __double_as_longlong(__hiloint2double(((hb >> 3) + sh) | (Ha & 0x80000000), hb << 29));
     return __longlong_as_double(base + (long long)k);
   }
-  const double p = a * b, s = a + b;
+  const double p = a * b, s = WEIGHTED ? __fma_rn(w64, a, b) : a + b;
   const bool pos = __double_as_longlong(p) > 0LL;                 // p > 0.0
   const bool nz = (__double_as_longlong(s) << 1) != 0LL;          // s != 0.0
   return (pos && nz) ? div_slope(p, s) : 0.0;
 }
+
+__device__ __forceinline__ double vl_slope(double a, double b) { return vl_slope_t<false>(a, b, 0.f, 0.f, 0.0); }
 
 // |x| by clearing the sign bit on the integer pipe (same bits as fabs).
 __device__ __forceinline__ double abs_i(double x)

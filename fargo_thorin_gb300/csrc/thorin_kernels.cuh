@@ -49,15 +49,14 @@ struct SorCtl {
 
 // Transport scratch (device fields).
 struct TransportScratch {
-  double *mom[4];          // RadMomP, RadMomM, ThetaMomP, ThetaMomM (updated in place)
+  double *mom[4];          // RadMomP, RadMomM, ThetaMomP, ThetaMomM after the transport
   double *rho_new, *e_new;
-  double *ext, *ext_new;   // rho * label before and after the transport (LabelAdvection)
-  double *w[7], *d[8], *f[8];
+  double *ext_new;         // rho * label after the transport (LabelAdvection)
+  double *w[7];            // after the radial step: the momenta, energy, density, rho * label
   int *nshift;
   double *vmed, *vtemp;
 };
 
-struct PtrPack8 { const double *src[8]; double *dst[8]; int n; };
 struct AziIO { const double *src[7]; double *dst[7]; int n; };   // index n-1 is the density
 
 struct ViscParams {
