@@ -655,22 +655,20 @@ __device__ __forceinline__ double sor_resid_at(const double *T, const double *ml
   return __fma_rn(T[ljm], mljm[q], r);
 }
 
-#ifndef SOR_CPT
-#define SOR_CPT 4        // cells of one colour per thread
-#endif
-#ifndef SOR_BX
-#define SOR_BX 128       // threads per SOR block
-#endif
+#define SOR_CPT 4        // cells per thread of the start residual
+#define SOR_BX 128       // and its threads per block
+#define SOR_PX 256       // threads per block of a colour pass
+#define SOR_POCC 4       // and resident blocks per multiprocessor
 
 // Block sums of the pass's L1 residual and "changed" count, result in
 // thread 0.  The FP64 pipe bounds the SOR pass, so the first level goes
-// through shared memory: warp 0 adds the SOR_BX / 32 values of its lane's
-// column, then one shuffle tree finishes.  That is SOR_BX / 32 + 4 warp-wide
-// FP64 adds per block instead of 5 (SOR_BX / 32 + 1).  Fixed order.
+// through shared memory: warp 0 adds the SOR_PX / 32 values of its lane's
+// column, then one shuffle tree finishes.  That is SOR_PX / 32 + 4 warp-wide
+// FP64 adds per block instead of 5 (SOR_PX / 32 + 1).  Fixed order.
 __device__ __forceinline__ void sor_block_sums(double &a, int &c)
 {
-  __shared__ double sa[SOR_BX];
-  __shared__ int sc[SOR_BX];
+  __shared__ double sa[SOR_PX];
+  __shared__ int sc[SOR_PX];
   sa[threadIdx.x] = a;
   sc[threadIdx.x] = c;
   __syncthreads();
@@ -678,7 +676,7 @@ __device__ __forceinline__ void sor_block_sums(double &a, int &c)
     double s = sa[threadIdx.x];
     int t = sc[threadIdx.x];
 #pragma unroll
-    for (int k = 1; k < SOR_BX / 32; k++) {
+    for (int k = 1; k < SOR_PX / 32; k++) {
       s += sa[threadIdx.x + 32 * k];
       t += sc[threadIdx.x + 32 * k];
     }
@@ -752,15 +750,27 @@ __global__ void __launch_bounds__(SOR_BX) k_sor_resid0(DevGrid g, const double *
   }
 }
 
-// One colour pass of a sweep.  Each thread updates SOR_CPT cells of ring i
-// (k = base + m*blockDim, j = 2k + parity).  The pass is bound by the FP64
-// pipe, so each cell costs seven FP64 instructions: the residual as five
-// FMAs, its absolute value added to the L1 norm, and the update
-// T - resid * (omega/Ml) as one FMA (omega/Ml prepared once per solve by
-// k_sor_resid0); the change test delta > T*SORPRECISION runs on the integer
-// pipe (sor_changed).  The sweep number is counted on the device (c.niter),
-// so every sweep is the same two launches: the body of the sweep loop's
-// WHILE graph node.
+// One colour pass of a sweep.  Each cell costs seven FP64 instructions: the
+// residual as five FMAs, its absolute value added to the L1 norm, and the
+// update T - resid * (omega/Ml) as one FMA (omega/Ml prepared once per solve
+// by k_sor_resid0); the change test delta > T*SORPRECISION runs on the integer
+// pipe (sor_changed).  That is 22 us of the FP64 pipe for a pass of the
+// 1024x3072 disk, 17 us of DRAM traffic (seven coefficient arrays and T, 118
+// MB), and the latency of a pass's start and end, so:
+// * one wave of blocks strides over the colour's cells, 10 a thread on that
+//   disk, and a cell's coefficients are loaded while the cell before it is
+//   computed (with 1024 threads per multiprocessor and 64 registers a thread;
+//   more threads without the prefetch were slower);
+// * a pass's blocks start while the pass before drains (programmatic
+//   dependent launch) and load their first coefficients, which no pass
+//   writes, before they wait for it;
+// * the last block sums the block partials in one level.
+// 1024x3072: 25.6 us a pass (29.2 us with one cell in flight per thread, full
+// launches and a two-level sum; prefetch and launch give 1.5 us each), 512x1536
+// 13.2 -> 10.7 us, 128x384 7.6 -> 5.4 us.  Blocks of 512 x 2: 25.7 / 10.7 / 6.0 us,
+// 512 x 3 without prefetch 27.3 / 11.3 / 6.4 us, prefetching T too 25.8 us.
+// The sweep number is counted on the device (c.niter), so every sweep is the
+// same two launches: the body of the sweep loop's WHILE graph node.
 // delta > tn * SORPRECISION (SORPRECISION = 1e-15, between 2^-50 and 2^-49)
 // with delta = resid * cw, cw = omega / Ml > 0.  When resid, cw and tn are
 // positive normal numbers well inside the exponent range, delta lies in
@@ -782,84 +792,78 @@ __device__ __forceinline__ bool sor_changed(double resid, double cw, double tn)
   return __double_as_longlong(__fma_rn(-tn, TH_SORPRECISION, resid * cw)) > 0LL;
 }
 
-__global__ void __launch_bounds__(SOR_BX) k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml,
-                                                  const double *__restrict__ mlip, const double *__restrict__ mlim,
-                                                  const double *__restrict__ mljp, const double *__restrict__ mljm,
-                                                  const double *__restrict__ rhs, const double *__restrict__ cw,
-                                                  SorCtl c, double eps, int pass, int maxiters)
+// Programmatic dependent launch: the pass's blocks start while the pass before
+// drains; what a block does before sor_pdl_wait must not touch anything that
+// pass writes.
+__device__ __forceinline__ void sor_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void sor_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+struct SorRow { double ml, mlip, mlim, mljp, mljm, rhs, cw; };
+
+__global__ void __launch_bounds__(SOR_PX, SOR_POCC)
+k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, const double *__restrict__ mlip,
+           const double *__restrict__ mlim, const double *__restrict__ mljp, const double *__restrict__ mljm,
+           const double *__restrict__ rhs, const double *__restrict__ cw, SorCtl c, double eps, int pass, int maxiters)
 {
-  if (*((volatile int *)c.done)) return;
   const int ns = g.ns, half = ns >> 1;
   const int col = pass - 1;
-  const int cpt = SOR_BX * SOR_CPT;                // cells of one colour per tile
-  const int tpr = (half + cpt - 1) / cpt;          // tiles per ring
-  const int ntiles = tpr * (g.nr - 2);
+  const int total = half * (g.nr - 2);             // cell idx: ring idx / half + 1, k = idx % half of this colour
+  const int stride = gridDim.x * SOR_PX;
+  int idx = blockIdx.x * SOR_PX + threadIdx.x;
+  int r = idx / half, k = idx - r * half;
+  const int dr = stride / half, dk = stride - dr * half;
+  auto row_of = [&](int r, int k) {
+    const size_t q = (size_t)(((r + 1) << 1) + col) * half + k;
+    return SorRow{ml[q], mlip[q], mlim[q], mljp[q], mljm[q], rhs[q], cw[q]};
+  };
+  SorRow m;
+  if (idx < total) m = row_of(r, k);
+  sor_pdl_launch();
+  sor_pdl_wait();
+  if (*((volatile int *)c.done)) return;
   double a = 0.0;
   int ch = 0;
-  // grid-stride over (ring, tile): the grid is one wave of resident blocks
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int i = tile / tpr + 1, kx = tile - (i - 1) * tpr;
-    const int par = (col == 0) ? ((i - 1) & 1) : (i & 1);
-    const size_t pbase = (size_t)((i << 1) + col) * half;
-#pragma unroll
-    for (int m = 0; m < SOR_CPT; m++) {
-      const int k = kx * cpt + m * blockDim.x + threadIdx.x;
-      if (k < half) {
-        const int j = 2 * k + par;
-        const int l = j + i * ns;
-        const int ljp = (j == ns - 1) ? i * ns : l + 1;
-        const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-        const size_t q = pbase + k;
-        const double resid = sor_resid_at(T, ml, mlip, mlim, mljp, mljm, rhs, l, l + ns, l - ns, ljp, ljm, q);
-        a += abs_i(resid);
-        const double c = cw[q];
-        const double tn = __fma_rn(-resid, c, T[l]);     // T -= omega resid / Ml
-        T[l] = tn;
-        ch += sor_changed(resid, c, tn) ? 1 : 0;
-      }
-    }
+  while (idx < total) {
+    const int j = 2 * k + ((r + col) & 1);
+    const int row = (r + 1) * ns, l = row + j;
+    const int ljp = (j == ns - 1) ? row : l + 1;
+    const int ljm = (j == 0) ? row + ns - 1 : l - 1;
+    const double t = T[l], tip = T[l + ns], tim = T[l - ns], tjp = T[ljp], tjm = T[ljm];
+    idx += stride;
+    r += dr;
+    k += dk;
+    if (k >= half) { k -= half; r++; }
+    SorRow n;
+    if (idx < total) n = row_of(r, k);
+    // the reference's sum T ml + T_ip mlip + T_im mlim + T_jp mljp + T_jm mljm - rhs
+    double resid = __fma_rn(t, m.ml, -m.rhs);
+    resid = __fma_rn(tip, m.mlip, resid);
+    resid = __fma_rn(tim, m.mlim, resid);
+    resid = __fma_rn(tjp, m.mljp, resid);
+    resid = __fma_rn(tjm, m.mljm, resid);
+    a += abs_i(resid);
+    const double tn = __fma_rn(-resid, m.cw, t);     // T -= omega resid / Ml
+    T[l] = tn;
+    ch += sor_changed(resid, m.cw, tn) ? 1 : 0;
+    m = n;
   }
   sor_block_sums(a, ch);
-  const int chs = ch;
   const unsigned nb = gridDim.x;
   const int b = blockIdx.x;
-  const int slot = col * nb + b;
   if (threadIdx.x == 0) {
-    c.part[slot] = a;
-    c.ipart[slot] = chs;
+    c.part[col * nb + b] = a;
+    c.ipart[col * nb + b] = ch;
   }
   if (pass != 2) return;
-  // Completion in two levels so that no block sums thousands of partials
-  // while the GPU idles: the last block of each group of SOR_GROUP blocks
-  // sums the group's partials of both colours, the last group to finish sums
-  // the group sums and applies the exit tests.  The order of every sum is
-  // fixed, so the result does not depend on timing.
-  const unsigned grp = b / SOR_GROUP, g0 = grp * SOR_GROUP;
-  const unsigned gsize = (nb - g0 < SOR_GROUP) ? nb - g0 : SOR_GROUP;
-  if (!sor_last_block(c.gticket + grp * SOR_TSTRIDE, gsize)) return;
+  // The last block to finish sums both colours' partials in block order and
+  // applies the exit tests.
+  if (!sor_last_block(c.ticket, nb)) return;
   __threadfence();
   double s = 0.0;
   int cs = 0;
-  for (unsigned q = threadIdx.x; q < 2 * gsize; q += blockDim.x) {
-    const unsigned cc = q / gsize, bb = g0 + (q - cc * gsize);
-    s += __ldcg(c.part + cc * nb + bb);
-    cs += __ldcg(c.ipart + cc * nb + bb);
-  }
-  s = block_reduce(s, OpAdd(), 0.0);
-  cs = block_reduce(cs, OpAddI(), 0);
-  if (threadIdx.x == 0) {
-    c.gpart[grp] = s;
-    c.gipart[grp] = cs;
-    c.gticket[grp * SOR_TSTRIDE] = 0u;
-  }
-  const unsigned ng = (nb + SOR_GROUP - 1) / SOR_GROUP;
-  if (!sor_last_block(c.ticket, ng)) return;
-  __threadfence();
-  s = 0.0;
-  cs = 0;
-  for (unsigned q = threadIdx.x; q < ng; q += blockDim.x) {
-    s += __ldcg(c.gpart + q);
-    cs += __ldcg(c.gipart + q);
+  for (unsigned q = threadIdx.x; q < 2 * nb; q += SOR_PX) {
+    s += __ldcg(c.part + q);
+    cs += __ldcg(c.ipart + q);
   }
   s = block_reduce(s, OpAdd(), 0.0);
   cs = block_reduce(cs, OpAddI(), 0);
@@ -1382,32 +1386,23 @@ static int sor_occ_max()
   static std::atomic<int> occ_cache{0};
   int occ = occ_cache.load();
   if (occ == 0) {
-#ifdef SOR_CARVEOUT
-    cudaFuncSetAttribute(k_sor_pass, cudaFuncAttributePreferredSharedMemoryCarveout, SOR_CARVEOUT);
-#endif
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sor_pass, SOR_BX, 0) != cudaSuccess || occ < 1) occ = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sor_pass, SOR_PX, 0) != cudaSuccess || occ < 1) occ = 1;
     occ_cache.store(occ);
   }
   return occ;
 }
 
-// One wave of resident blocks striding over the (ring, tile) tiles, with at
-// most g.sor_tpsm threads per multiprocessor (default 1536: on the 1024x3072
-// disk the pass took 29.3 us with 12 blocks of 128 per SM, 30.4 us with the
-// 16 that fit, 31.6 us with 8; the ensemble autotuner may pick another cap
-// per disk).
+// One wave of resident blocks striding over the colour's cells, with at most
+// g.sor_tpsm threads per multiprocessor (the ensemble autotuner may pick a cap
+// per disk; the default is above what the pass's registers allow).
 static dim3 sor_grid_pass(const DevGrid &g, bool capped = true)
 {
   int occ = sor_occ_max();
   const int tpsm = g.sor_tpsm > 0 ? g.sor_tpsm : 1536;
-  if (capped && occ * SOR_BX > tpsm) occ = tpsm / SOR_BX > 0 ? tpsm / SOR_BX : 1;
-#ifdef SOR_OCC
-  occ = SOR_OCC;
-#endif
-  const int half = g.ns / 2;
-  const long long ntiles = (long long)((half + SOR_BX * SOR_CPT - 1) / (SOR_BX * SOR_CPT)) * (g.nr - 2);
+  if (capped && occ * SOR_PX > tpsm) occ = tpsm / SOR_PX > 0 ? tpsm / SOR_PX : 1;
+  const long long nblk = ((long long)(g.ns / 2) * (g.nr - 2) + SOR_PX - 1) / SOR_PX;
   const long long wave = (long long)g.nsm * occ;
-  return dim3((unsigned)(ntiles < wave ? ntiles : wave));
+  return dim3((unsigned)(nblk < wave ? nblk : wave));
 }
 
 static dim3 sor_grid_resid(const DevGrid &g)
@@ -1434,10 +1429,19 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
                       double eps, int count, int maxiters, cudaStream_t s)
 {
-  const dim3 grid = sor_grid_pass(g);
-  for (int n = 0; n < count; n++) {
-    k_sor_pass<<<grid, SOR_BX, 0, s>>>(g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, 1, maxiters);
-    k_sor_pass<<<grid, SOR_BX, 0, s>>>(g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, 2, maxiters);
+  // numbers of launches are counted by the caller
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = sor_grid_pass(g);
+  cfg.blockDim = dim3(SOR_PX);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  for (int n = 0; n < 2 * count; n++) {
+    // the first pass waits for whatever wrote its coefficients
+    cfg.numAttrs = (n > 0) ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_sor_pass, g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, (n & 1) + 1, maxiters);
   }
 }
 

@@ -498,10 +498,6 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     if (k >= 1 && k <= 64) d->sor_loop_k = k;
   }
   if (const char *ed = getenv("THORIN_SOR_DIRECT")) d->sor_direct = (atoi(ed) != 0);
-  const int ng = (sb + SOR_GROUP - 1) / SOR_GROUP;
-  RCHK(dalloc(d, (void **)&d->sor.gpart, (size_t)ng * sizeof(double)));
-  RCHK(dalloc(d, (void **)&d->sor.gipart, (size_t)ng * sizeof(int)));
-  RCHK(dalloc(d, (void **)&d->sor.gticket, (size_t)ng * SOR_TSTRIDE * sizeof(unsigned int)));
   fill_rings(d);
   {
     PlConst &c = d->plc;                 // constants of the planet side of a substep
