@@ -15,31 +15,21 @@ static const int BX = 128;
 
 // ---------------------------------------------------------------------------
 // Ring (azimuthal) means, mpi_make1Dprofile (mpiTasks.c:26-32) and the
-// other azimuthal averages of the loop.  One warp per ring sums in a fixed
-// tree (lanes take strided columns, then a butterfly), so results are
-// deterministic; they differ from the reference's left-to-right sum in the
-// last bits.  The only integer decision fed by a ring mean, the FARGO shift,
-// re-sums its ring in order when the mean lands near a rounding tie (see
-// k_azimuthal).  Output index is relative to ring0.
-// One warp's fixed-tree sum of a ring (all lanes return it).
-__device__ __forceinline__ double warp_ring_sum(const double *__restrict__ row, int ns, int lane)
+// other azimuthal averages of the loop.  One block per ring sums in a fixed
+// tree (ring_sum), so results are deterministic; they differ from the
+// reference's left-to-right sum in the last bits.  The only integer decision
+// fed by a ring mean, the FARGO shift, re-sums its ring in order when the mean
+// lands near a rounding tie (see k_azi_rings).  Output index is relative to
+// ring0.
+__global__ void __launch_bounds__(RING_T) k_ring_means(int ns, const double *__restrict__ f0,
+                                                       const double *__restrict__ f1, double *__restrict__ o0,
+                                                       double *__restrict__ o1, int ring0, int nf)
 {
-  double a = 0.0;
-  for (int j = lane; j < ns; j += 32) a += row[j];
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(TH_FULL, a, o);
-  return a;
-}
-
-__global__ void __launch_bounds__(256) k_ring_means(int ns, const double *__restrict__ f0,
-                                                    const double *__restrict__ f1, double *__restrict__ o0,
-                                                    double *__restrict__ o1, int ring0, int nrings, int nf)
-{
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= nrings) return;                         // whole warp
+  const int w = blockIdx.x;
   const size_t base = (size_t)(ring0 + w) * ns;
-  const double a0 = warp_ring_sum(f0 + base, ns, lane);
-  const double a1 = (nf > 1) ? warp_ring_sum(f1 + base, ns, lane) : 0.0;
-  if (lane == 0) {
+  const double a0 = ring_sum(f0 + base, ns);
+  const double a1 = (nf > 1) ? ring_sum(f1 + base, ns) : 0.0;
+  if (threadIdx.x == 0) {
     o0[w] = a0 / (double)ns;
     if (nf > 1) o1[w] = a1 / (double)ns;
   }
@@ -48,21 +38,21 @@ __global__ void __launch_bounds__(256) k_ring_means(int ns, const double *__rest
 // The same ring means at rings chosen on the device: ring info[slot] and,
 // with two, info[slot + 1] rings from there (else one ring when
 // info[slot] >= 0, none when it is negative).
-__global__ void __launch_bounds__(64) k_ring_means_at(int ns, const double *__restrict__ f, double *__restrict__ o,
-                                                      const int *__restrict__ info, int slot, int two)
+__global__ void __launch_bounds__(RING_T) k_ring_means_at(int ns, const double *__restrict__ f, double *__restrict__ o,
+                                                          const int *__restrict__ info, int slot, int two)
 {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = blockIdx.x;
   const int ring0 = info[slot];
   const int nrings = two ? info[slot + 1] : (ring0 >= 0 ? 1 : 0);
   if (ring0 < 0 || w >= nrings) return;
-  const double a = warp_ring_sum(f + (size_t)(ring0 + w) * ns, ns, lane);
-  if (lane == 0) o[w] = a / (double)ns;
+  const double a = ring_sum(f + (size_t)(ring0 + w) * ns, ns);
+  if (threadIdx.x == 0) o[w] = a / (double)ns;
 }
 
 void graph_ring_means_at(const DevGrid &g, const double *f, double *out, const int *ring_info, int slot, int two_slots,
                          cudaStream_t s)
 {
-  k_ring_means_at<<<1, 64, 0, s>>>(g.ns, f, out, ring_info, slot, two_slots);
+  k_ring_means_at<<<two_slots ? 2 : 1, RING_T, 0, s>>>(g.ns, f, out, ring_info, slot, two_slots);
   g_thorin_launches++;
 }
 
@@ -70,8 +60,7 @@ void aux_ring_means(const DevGrid &g, const double *f0, double *o0, const double
                     cudaStream_t s)
 {
   if (nrings <= 0) return;
-  const int blocks = (nrings * 32 + 255) / 256;
-  k_ring_means<<<blocks, 256, 0, s>>>(g.ns, f0, f1 ? f1 : f0, o0, o1 ? o1 : o0, ring0, nrings, f1 ? 2 : 1);
+  k_ring_means<<<nrings, RING_T, 0, s>>>(g.ns, f0, f1 ? f1 : f0, o0, o1 ? o1 : o0, ring0, f1 ? 2 : 1);
   g_thorin_launches++;
 }
 
@@ -390,7 +379,7 @@ __global__ void k_pebble_sources(DevGrid g, const double *__restrict__ pd, const
                                  const double *__restrict__ pvt, const double *__restrict__ tau,
                                  const double *__restrict__ vr, const double *__restrict__ vt,
                                  const double *__restrict__ pagr, const double *__restrict__ pagt,
-                                 double *__restrict__ paccr, double *__restrict__ pacct, double *__restrict__ dragr,
+                                 const double *__restrict__ colf, double *__restrict__ paccr, double *__restrict__ pacct, double *__restrict__ dragr,
                                  double *__restrict__ dragt, int back_reaction)
 {
   const double omega_frame = g.ctl[CTL_OMEGA_FRAME];
@@ -405,13 +394,13 @@ __global__ void k_pebble_sources(DevGrid g, const double *__restrict__ pd, const
     double vt2 = pvt[l] + pvt[ljp] + pvt[lim] + pvt[ljp - ns];
     vt2 = vt2 / 4.0 + g.r.Rinf[i] * omega_frame;
     vt2 = vt2 * vt2;
-    paccr[l] = vt2 * g.r.InvRinf[i] + 0.5 * (pagr[l] + pagr[lim]);
+    paccr[l] = vt2 * g.r.InvRinf[i] + 0.5 * (pagr[l] + pagr[lim]) + colf[j];
     if (back_reaction) {
       const double drag = (pvr[l] - vr[l]) * otau;
       dragr[l] = 0.5 * (pd[l] + pd[lim]) * drag;
     }
   }
-  pacct[l] = 0.5 * (pagt[l] + pagt[ljm]);
+  pacct[l] = 0.5 * (pagt[l] + pagt[ljm]) + colf[ns + j];
   if (back_reaction) {
     const double drag = (pvt[l] - vt[l]) * otau;
     dragt[l] = 0.5 * (pd[l] + pd[ljm]) * drag;
@@ -419,11 +408,11 @@ __global__ void k_pebble_sources(DevGrid g, const double *__restrict__ pd, const
 }
 
 void aux_pebble_sources(const DevGrid &g, const double *pd, const double *pvr, const double *pvt, const double *tau,
-                        const double *vr, const double *vt, const double *pagr, const double *pagt, double *paccr,
-                        double *pacct, double *dragr, double *dragt, int back_reaction,
+                        const double *vr, const double *vt, const double *pagr, const double *pagt, const double *col,
+                        double *paccr, double *pacct, double *dragr, double *dragt, int back_reaction,
                         cudaStream_t s)
 {
-  k_pebble_sources<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, pd, pvr, pvt, tau, vr, vt, pagr, pagt, paccr, pacct, dragr,
+  k_pebble_sources<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, pd, pvr, pvt, tau, vr, vt, pagr, pagt, col, paccr, pacct, dragr,
                                                          dragt, back_reaction);
   g_thorin_launches++;
 }
@@ -476,291 +465,537 @@ void aux_pebble_substep1(const DevGrid &g, double *pvr, double *pvt, const doubl
 }
 
 // ---------------------------------------------------------------------------
-// FillForcesArrays (Pframeforce.c:43-510).  Per ring: the azimuthal mean
-// sound speed and Stokes number (sums in order) and the 10-node vertical
-// averages of the star's pull for the ring-mean scale height.
-
-__global__ void k_force_rings(DevGrid g, ForceRings fr, int pebbles, double pebble_alpha)
+// FillForcesArrays (Pframeforce.c:43-510) in four kernels.
+//
+// k_force_rings, one block per ring: the ring-mean Stokes number, the scale
+// heights of the ring means and the 10-node vertical average of the star's
+// pull for the ring-mean column, one node per lane of the first warp.
+__global__ void __launch_bounds__(RING_T) k_force_rings(DevGrid g, ForceArgs a, ForceRings fr)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.nr) return;
-  const double cs_avr = g.r.csmean[i];       // the ring mean of c_s, summed in order
-  const double H_avr = cs_avr * g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
-  double tau_avr = 0.0, p_H_avr = 0.0, p_int = 0.0;
-  if (pebbles) {
-    tau_avr = fr.tau_avr[i];
-    p_H_avr = H_avr * sqrt(pebble_alpha / tau_avr);
-  }
+  const int i = blockIdx.x, lane = threadIdx.x;
+  const double H = g.r.csmean[i] * g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
   const double r2 = g.r.Rmed2[i];
-  const double H2 = H_avr * H_avr, zmax = 3.0 * H_avr, deltaz = zmax / 10.0;
-  double sig = 0.0, ist = 0.0;
-  for (int m = 1; m <= 10; m++) {
-    const double znode = ((double)m - 0.5) * deltaz;
-    double znode2 = znode * znode;
-    const double sum = exp(-(0.5 * znode2 / H2));
-    sig += sum;
-    double d2 = r2 + znode2, d = sqrt(d2), denom = d * d2;
-    ist += sum / denom;
-    if (pebbles) {
-      znode2 *= pebble_alpha / tau_avr;
-      d2 = r2 + znode2; d = sqrt(d2); denom = d * d2;
-      p_int += sum / denom;
+  double hc2 = 0.0;
+  if (a.pebbles) {
+    hc2 = ring_sum(a.tau + (size_t)i * g.ns, g.ns);
+    if (lane >= 32) return;
+    hc2 = div_fast(a.pebble_alpha, hc2 / (double)g.ns);
+  }
+  if (lane >= 32) return;
+  const int m = lane < 10 ? lane : 9;
+  const double z = ((double)m + 0.5) * (3.0 / 10.0) * H, z2 = z * z;
+  double s = a.wq10[m] * pow_m32(r2 + z2);
+  double p = a.wq10[m] * pow_m32(r2 + z2 * hc2);
+  if (lane >= 10) s = p = 0.0;
+  s = warp_reduce(s, OpAdd());
+  p = warp_reduce(p, OpAdd());
+  if (lane == 0) {
+    fr.H_avr[i] = H;
+    fr.p_H_avr[i] = a.pebbles ? H * sqrt(hc2) : 0.0;
+    const double f = s * a.isig10 * g.r.Rmed[i];
+    fr.agr0[i] = -f;
+    fr.pagr0[i] = a.pebbles ? -(p * a.isig10 * g.r.Rmed[i]) : 0.0;
+    fr.starw[i] = g.r.Surf[i] * f;
+  }
+}
+
+struct ForceRing {
+  double rm, surf, starw, agr0, pagr0, hc, H_avr, p_H_avr;
+  float hcf, havf, phavf;
+};
+
+// Whether |x - m| / m > 0.05, x and m from FP32 when they decide it (the FP32
+// values are within 1e-6 of the FP64 ones), else unknown (2).
+__device__ __forceinline__ int off_by_5pc(float x, float m)
+{
+  const float d = fabsf(x - m);
+  if (d > 0.05001f * m) return 1;
+  if (d < 0.04999f * m) return 0;
+  return 2;                                        // NaN as well
+}
+
+// FP32 value of a positive double of moderate exponent, truncated (0 outside
+// [2^-100, 2^100]).
+__device__ __forceinline__ float to_float_pos(double x)
+{
+  const int H = __double2hiint(x);
+  const float f = __int_as_float(__funnelshift_l(__double2loint(x), H - 0x38000000, 3));
+  return (unsigned)(H - (923 << 20)) < (unsigned)(200 << 20) ? f : 0.0f;
+}
+
+// k_forces: the accelerations of every cell whose scale height is within 5% of
+// the ring mean's and which is not near a planet (s < 10 H_pl or 5 r_Hill):
+// the star's pull is the ring's, a planet's is softened.  The other cells are
+// marked for k_forces_near.  A thread walks the rings of one column: in the
+// frame turned by the column's azimuth a planet lies at (pr, pt), the same for
+// all rings, so a cell at radius r sees it at (pr - r, pt); the radial and
+// azimuthal pull and the disk's pull on the planet need no rotation per cell,
+// and the sums over the column are turned once.  About 28 FP64 instructions a
+// cell with pebbles and a planet, where the form that worked in x and y took
+// 94; bound by the FP64 pipe.
+template <int NP>
+__global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRings fr)
+{
+  extern __shared__ char smem[];
+  ForceRing *ring = (ForceRing *)smem;
+  const double mass_taper = g.ctl[CTL_MASS_TAPER];
+  const int full_mass = (mass_taper == 1.0) ? 1 : 0;
+  const int ns = g.ns, peb = a.pebbles;
+  const int np = (NP == MAXPL_DEV) ? a.npl : NP;
+  const int i0 = blockIdx.y * a.rings_a, i1 = min(i0 + a.rings_a, g.nr);
+  for (int q = threadIdx.x; q < i1 - i0; q += 128) {
+    const int i = i0 + q;
+    ForceRing &R = ring[q];
+    R.rm = g.r.Rmed[i]; R.surf = g.r.Surf[i]; R.starw = fr.starw[i]; R.agr0 = fr.agr0[i];
+    R.hc = g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
+    R.H_avr = fr.H_avr[i];
+    R.hcf = (float)R.hc; R.havf = (float)R.H_avr;
+    if (peb) { R.pagr0 = fr.pagr0[i]; R.p_H_avr = fr.p_H_avr[i]; R.phavf = (float)R.p_H_avr; }
+  }
+  __syncthreads();
+  const int j = blockIdx.x * 128 + threadIdx.x;
+  double star = 0.0;
+  double W[NP > 0 ? NP : 1], Wu[NP > 0 ? NP : 1], pr[NP > 0 ? NP : 1], pt[NP > 0 ? NP : 1];
+  double c = 0.0, s = 0.0;
+#pragma unroll
+  for (int k = 0; k < NP; k++) W[k] = Wu[k] = pr[k] = pt[k] = 0.0;
+  if (j < ns) {
+    c = g.r.costab[j];
+    s = g.r.sintab[j];
+    double m[NP > 0 ? NP : 1], zz[NP > 0 ? NP : 1], sm2[NP > 0 ? NP : 1], sma[NP > 0 ? NP : 1], pt2[NP > 0 ? NP : 1],
+        lim[NP > 0 ? NP : 1];
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      if (k >= np) continue;
+      const DevPlanet &P = a.pl[k];
+      pr[k] = c * P.x + s * P.y;
+      pt[k] = c * P.y - s * P.x;
+      pt2[k] = pt[k] * pt[k];
+      m[k] = P.m * mass_taper;
+      zz[k] = P.z * P.z;
+      sm2[k] = P.smoothing2;
+      sma[k] = P.smoothing2 * a.pebble_alpha;
+      lim[k] = (P.near_h2 > P.near_hill2) ? P.near_h2 : P.near_hill2;
+      if (!full_mass) lim[k] = 0.0;
+    }
+    const float af = (float)a.pebble_alpha;
+    for (int i = i0; i < i1; i++) {
+      const ForceRing &R = ring[i - i0];
+      const int l = j + i * ns;
+      const double cs = a.cs[l], tau = peb ? a.tau[l] : 1.0;
+      const float Hf = to_float_pos(cs) * R.hcf;
+      int local = off_by_5pc(Hf, R.havf);
+      if (local == 2) {
+        const double H = cs * R.hc;
+        local = (fabs(H - R.H_avr) > 0.05 * R.H_avr) ? 1 : 0;
+      }
+      if (peb && !local) {
+        const float tf = to_float_pos(tau);
+        local = (tf > 0.0f) ? off_by_5pc(Hf * sqrtf(__fdividef(af, tf)), R.phavf) : 2;
+        if (local == 2) {
+          const double pH = cs * R.hc * sqrt(a.pebble_alpha / tau);
+          local = (fabs(pH - R.p_H_avr) > 0.05 * R.p_H_avr) ? 1 : 0;
+        }
+      }
+      double u[NP > 0 ? NP : 1], s2[NP > 0 ? NP : 1];
+#pragma unroll
+      for (int k = 0; k < NP; k++) {
+        if (k >= np) continue;
+        u[k] = R.rm - pr[k];
+        s2[k] = __fma_rn(u[k], u[k], pt2[k]);
+        if (__double_as_longlong(s2[k]) < __double_as_longlong(lim[k])) local = 1;   // both >= 0
+      }
+      a.near[l] = (unsigned char)local;
+      if (local) continue;
+      const double rho = a.rho[l];
+      star = __fma_rn(rho, R.starw, star);
+      double ar = R.agr0, at = 0.0, par = 0.0, pat = 0.0;
+      if (peb) par = R.pagr0;
+      if (NP > 0) {
+        const double mcell = rho * R.surf;
+        const double itau = peb ? div_fast(1.0, tau) : 0.0;
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+          if (k >= np) continue;
+          const double sz = s2[k] + zz[k];
+          const double id3 = pow_m32(sz + sm2[k]);
+          const double mi = m[k] * id3, w = mcell * id3;
+          ar = __fma_rn(-mi, u[k], ar);
+          at = __fma_rn(mi, pt[k], at);
+          W[k] += w;
+          Wu[k] = __fma_rn(w, u[k], Wu[k]);
+          if (peb) {
+            const double ip3 = pow_m32(__fma_rn(sma[k], itau, sz));
+            const double mp = m[k] * ip3;
+            par = __fma_rn(-mp, u[k], par);
+            pat = __fma_rn(mp, pt[k], pat);
+            if (a.pebble_gravity) {
+              const double wp = a.pdens[l] * R.surf * ip3;
+              W[k] += wp;
+              Wu[k] = __fma_rn(wp, u[k], Wu[k]);
+            }
+          }
+        }
+      }
+      a.agr[l] = ar;
+      a.agt[l] = at;
+      if (peb) { a.pagr[l] = par; a.pagt[l] = pat; }
     }
   }
-  fr.H_avr[i] = H_avr;
-  fr.sigma_avr[i] = sig;
-  fr.isigma_avr[i] = div_fast(1.0, sig);
-  fr.integstar_avr[i] = ist;
-  fr.p_H_avr[i] = p_H_avr;
-  fr.p_integstar_avr[i] = p_int;
+  const int b = blockIdx.x + blockIdx.y * gridDim.x, nb = a.nba + a.nbb;
+  double v = block_reduce_smem<128>(star * c, OpAdd());
+  if (threadIdx.x == 0) a.part[b] = v;
+  v = block_reduce_smem<128>(star * s, OpAdd());
+  if (threadIdx.x == 0) a.part[nb + b] = v;
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    if (k >= np) continue;
+    const double t = W[k] * pt[k];
+    v = block_reduce_smem<128>(c * Wu[k] + s * t, OpAdd());
+    if (threadIdx.x == 0) a.part[(size_t)(2 + 2 * k) * nb + b] = v;
+    v = block_reduce_smem<128>(s * Wu[k] - c * t, OpAdd());
+    if (threadIdx.x == 0) a.part[(size_t)(3 + 2 * k) * nb + b] = v;
+  }
 }
 
 // One quadrature node of a planet's potential (FillForcesArrays,
 // Pframeforce.c:300-372): cubic-spline taper inside rst, softened 1/d^3.
 __device__ __forceinline__ double planet_node(double s2, double dz, double mx, const DevPlanet &P)
 {
-  double d2 = s2 + dz * dz, taper = 1.0;
+  const double d2 = s2 + dz * dz;
   if (d2 < P.rst2) {
     const double dd = sqrt_fast(d2);
-    taper = div_fast(-3.0 * d2 * d2, P.rst4) + div_fast(4.0 * dd * d2, P.rst3);
+    return pow_m32(d2 + mx) * (div_fast(-3.0 * d2 * d2, P.rst4) + div_fast(4.0 * dd * d2, P.rst3));
   }
-  const double iv = rsqrt_fast(d2 + mx);
-  return iv * iv * iv * taper;
+  return pow_m32(d2 + mx);
 }
 
-// Vertical quadrature of one cell (FillForcesArrays, Pframeforce.c:260-372)
-// over NV nodes z_m = (m - 1/2) 3H/NV.  The Gaussian weights depend only on
-// m and NV and come precomputed; 1/d^3 comes from one reciprocal square root.
+// Vertical quadrature of a planet's pull on one cell over NV nodes
+// z_m = (m - 1/2) 3H/NV (Pframeforce.c:260-372).  A planet in the midplane
+// (P.z = 0) outside whose taper the whole column lies needs only
+// d2 = s2 + z_m^2 at each node.
 template <int NV>
-__device__ __forceinline__ void vert_quad(const double (&wq)[NV], double H, double r2, double Hcorr, double pH, int peb,
-                                          int npl, const int *with, const double *s2, double Rsup_Rinf2,
-                                          const DevPlanet *pl, double &integstar, double &p_integstar,
-                                          double *integpl, double *p_integpl)
+__device__ __forceinline__ double planet_quad(const double *wq, double H, double s2, double mx, const DevPlanet &P)
 {
-  const double deltaz = 3.0 * H / (double)NV;
-  const double hc2 = Hcorr * Hcorr;
-  double is = 0.0, pis = 0.0;
+  double sum = 0.0;
+  if (P.z == 0.0 && s2 >= P.rst2) {
+    const double H2 = H * H, b = s2 + mx;
 #pragma unroll
-  for (int m = 1; m <= NV; m++) {
-    const double znode = ((double)m - 0.5) * deltaz, znode2 = znode * znode;
-    const double sum = wq[m - 1];
-    double iv = rsqrt_fast(r2 + znode2);
-    is += sum * iv * iv * iv;
-    if (peb) {
-      iv = rsqrt_fast(r2 + znode2 * hc2);
-      pis += sum * iv * iv * iv;
+    for (int m = 0; m < NV; m++) {
+      const double z = ((double)m + 0.5) * (3.0 / (double)NV);
+      sum = __fma_rn(wq[m], pow_m32(__fma_rn(z * z, H2, b)), sum);
     }
-    for (int k = 0; k < npl; k++) {
-      if (!with[k]) continue;
-      const DevPlanet P = pl[k];
-      const double mx = (P.rsm2 > Rsup_Rinf2) ? P.rsm2 : Rsup_Rinf2;
-      integpl[k] += sum * planet_node(s2[k], znode - P.z, mx, P);
-      if (P.z < -0.05 * H || P.z > 0.05 * H) integpl[k] += sum * planet_node(s2[k], -znode - P.z, mx, P);
-      if (peb) {
-        const double zp = znode * Hcorr;
-        p_integpl[k] += sum * planet_node(s2[k], zp - P.z, mx, P);
-        if (P.z < -0.05 * pH || P.z > 0.05 * pH) p_integpl[k] += sum * planet_node(s2[k], -zp - P.z, mx, P);
+    return sum;
+  }
+  const bool off = (P.z < -0.05 * H || P.z > 0.05 * H);
+  const double deltaz = 3.0 * H / (double)NV;
+  for (int m = 0; m < NV; m++) {
+    const double z = ((double)m + 0.5) * deltaz;
+    double f = planet_node(s2, z - P.z, mx, P);
+    if (off) f += planet_node(s2, -z - P.z, mx, P);
+    sum += wq[m] * f;
+  }
+  return off ? 0.5 * sum : sum;
+}
+
+// The same by a warp, a node per lane; every lane gets the sum.
+__device__ __forceinline__ double planet_quad_warp(const double *wq, int nv, double H, double s2, double mx,
+                                                   const DevPlanet &P)
+{
+  const int lane = threadIdx.x & 31;
+  const bool off = (P.z < -0.05 * H || P.z > 0.05 * H);
+  const double z = ((double)lane + 0.5) * (3.0 * H / (double)nv);
+  double f = planet_node(s2, z - P.z, mx, P);
+  if (off) f += planet_node(s2, -z - P.z, mx, P);
+  f = (lane < nv) ? wq[lane < nv ? lane : 0] * f : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(TH_FULL, f, o);
+  return off ? 0.5 * f : f;
+}
+
+// r^3 times the star's vertical sum over nv nodes as a series in q = (H/r)^2,
+// or node by node in columns too thick for it.
+__device__ __forceinline__ double star_quad(const double *wq, const double *ck, int nv, double q)
+{
+  if (q <= FORCE_QMAX) {
+    double v = ck[FORCE_NC - 1];
+#pragma unroll
+    for (int k = FORCE_NC - 2; k >= 0; k--) v = __fma_rn(v, q, ck[k]);
+    return v;
+  }
+  double v = 0.0;
+  for (int m = 0; m < nv; m++) {
+    const double z = ((double)m + 0.5) * (3.0 / (double)nv);
+    v += wq[m] * pow_m32(1.0 + z * z * q);
+  }
+  return v;
+}
+
+// Whether the cell at (x, y) lies within two Hill radii of planet P, where the
+// vertical quadrature takes 30 nodes.  Rounded operations, so that every
+// kernel decides alike.
+__device__ __forceinline__ bool in_hill(double x, double y, const DevPlanet &P)
+{
+  const double dx = __dsub_rn(x, P.x), dy = __dsub_rn(y, P.y);
+  return __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) < P.rmorevert2;
+}
+
+// One of k_forces_near's cells with the NV-node vertical quadrature, by a
+// thread (WARP false, NV = 10) or by a warp whose lanes hold the nodes (NV =
+// 30; lane 0 writes and adds to acc).
+template <int NV, bool WARP>
+__device__ __forceinline__ void near_cell(const DevGrid &g, const ForceArgs &a, const ForceRings &fr, int i, int j,
+                                          double mass_taper, int full_mass, const double *wq, const double *ck,
+                                          double isig, double *acc)
+{
+  const int l = j + i * g.ns, peb = a.pebbles;
+  const bool add = !WARP || (threadIdx.x & 31) == 0;
+  const double c = g.r.costab[j], s = g.r.sintab[j], rm = g.r.Rmed[i], ir = g.r.InvRmed[i];
+  const double x = rm * c, y = rm * s;
+  const double H = a.cs[l] * (g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv), H2 = H * H;
+  const double mcell = a.rho[l] * g.r.Surf[i];
+  const double hc2 = peb ? div_fast(a.pebble_alpha, a.tau[l]) : 0.0;
+  const double q = H2 * (ir * ir), ir2 = ir * ir * isig;
+  const double f = star_quad(wq, ck, NV, q) * ir2;             // r sum_m w_m (r^2 + z_m^2)^(-3/2) / sigma
+  double ax = 0.0, ay = 0.0, pax = 0.0, pay = 0.0, par = 0.0;
+  if (add) {
+    acc[0] += mcell * f * c;
+    acc[1] += mcell * f * s;
+  }
+  if (peb) par = -star_quad(wq, ck, NV, q * hc2) * ir2;
+  for (int k = 0; k < a.npl; k++) {
+    const DevPlanet P = a.pl[k];
+    const double dx = x - P.x, dy = y - P.y;
+    const double s2 = dx * dx + dy * dy;
+    double id3, ip3 = 0.0, mpl = P.m, hillcut = 1.0;
+    if (full_mass && (s2 < P.near_h2 || s2 < P.near_hill2)) {
+      if (a.exclude_hill) {
+        const double d2 = s2 + P.z * P.z;
+        hillcut = 1.0 / (exp(-(sqrt(d2) / P.rhill - a.hillcut) / a.hillcut * 10.0) + 1.0);
+      }
+      const double mx = (P.rsm2 > fr.drsq[i]) ? P.rsm2 : fr.drsq[i];
+      if (WARP) {
+        id3 = planet_quad_warp(wq, NV, H, s2, mx, P) * isig;
+        if (peb) ip3 = planet_quad_warp(wq, NV, H * sqrt_fast(hc2), s2, mx, P) * isig;
+      } else {
+        id3 = planet_quad<NV>(wq, H, s2, mx, P) * isig;
+        if (peb) ip3 = planet_quad<NV>(wq, H * sqrt_fast(hc2), s2, mx, P) * isig;
+      }
+    } else {
+      mpl *= mass_taper;
+      const double sz = s2 + P.z * P.z;
+      id3 = pow_m32(sz + P.smoothing2);
+      if (peb) ip3 = pow_m32(sz + P.smoothing2 * hc2);
+    }
+    double tx = dx * id3, ty = dy * id3;
+    ax -= mpl * tx;
+    ay -= mpl * ty;
+    if (add) {
+      acc[2 + 2 * k] += mcell * (tx * hillcut);
+      acc[3 + 2 * k] += mcell * (ty * hillcut);
+    }
+    if (peb) {
+      tx = dx * ip3; ty = dy * ip3;
+      pax -= mpl * tx;
+      pay -= mpl * ty;
+      if (a.pebble_gravity && add) {
+        const double pm = a.pdens[l] * g.r.Surf[i];
+        acc[2 + 2 * k] += pm * (tx * hillcut);
+        acc[3 + 2 * k] += pm * (ty * hillcut);
       }
     }
   }
-  integstar = is;
-  p_integstar = pis;
+  if (!add) return;
+  a.agr[l] = c * ax + s * ay - f;
+  a.agt[l] = c * ay - s * ax;
+  if (peb) {
+    a.pagr[l] = c * pax + s * pay + par;
+    a.pagt[l] = c * pay - s * pax;
+  }
 }
 
-#define FORCE_CPT 4     // cells per thread: one block reduction per 4*128 cells
-
-__global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRings fr)
+// k_forces_near: the cells k_forces left out, with the vertical quadrature of
+// the star's pull and of the planets near the cell: about 180 FP64
+// instructions a cell for 10 nodes and one planet (370 before the star's
+// series and the shorter powers).  They lie together around the planets (7% of
+// the cells for one planet at r = 1), so the kernel has its own grid, with few
+// rings per block.  The cells within two Hill radii take 30 nodes, and the
+// taper next to the planet: a few hundred cells whose chains of dependent
+// FP64 instructions would hold up the rest, so the last blocks take them, a
+// warp per cell and a node per lane (cells w, w + W, ... of the annulus, 32
+// tested at a time).  512x1536: 70 us (238 us with two rings per thread and
+// the 30-node cells among the others); with k_forces' 66 us, 136 us where one
+// kernel for all cells took 340.
+__global__ void __launch_bounds__(128) k_forces_near(DevGrid g, ForceArgs a, ForceRings fr)
 {
   const double mass_taper = g.ctl[CTL_MASS_TAPER];
   const int full_mass = (mass_taper == 1.0) ? 1 : 0;
   const int ns = g.ns;
-  const int i = blockIdx.y;
-  const int npl = a.npl, peb = a.pebbles;
+  const int nq = 2 + 2 * a.npl, nb = a.nba + a.nbb, b = a.nba + blockIdx.x;
   double acc[2 + 2 * MAXPL_DEV];
-  for (int q = 0; q < 2 + 2 * npl; q++) acc[q] = 0.0;
-  for (int mc = 0; mc < FORCE_CPT; mc++) {
-    const int j = (blockIdx.x * FORCE_CPT + mc) * blockDim.x + threadIdx.x;
-    if (j >= ns) break;
-    const int l = j + i * ns;
-    const double omegainv = g.r.OmegaInv[i], r2 = g.r.Rmed2[i];
-    const double Rsup_Rinf2 = fr.drsq[i];
-    const double x = g.r.Rmed[i] * g.r.costab[j];
-    const double y = g.r.Rmed[i] * g.r.sintab[j];
-    const double mcell = a.rho[l] * g.r.Surf[i];
-    const double H = a.cs[l] * omegainv * g.k.sqrt_adiabind_inv;
-    const double H_avr = fr.H_avr[i];
-    int local = (fabs(H - H_avr) > 0.05 * H_avr) ? 1 : 0;      // |H - H_avr| / H_avr > 0.05
-    double Hcorr = 0.0, pH = 0.0, pmcell = 0.0;
-    if (peb) {
-      pmcell = a.pdens[l] * g.r.Surf[i];
-      Hcorr = a.sqrt_pebble_alpha * rsqrt_fast(a.tau[l]);        // sqrt(alpha / tau) without the division
-      pH = H * Hcorr;
-      const double p_H_avr = fr.p_H_avr[i];
-      if (fabs(pH - p_H_avr) > 0.05 * p_H_avr) local = 1;
-    }
-    double s2[MAXPL_DEV], integpl[MAXPL_DEV], p_integpl[MAXPL_DEV], hillcut[MAXPL_DEV];
-    int with[MAXPL_DEV];
-    int Nvert = 10;
-    for (int k = 0; k < npl; k++) {
-      const DevPlanet P = a.pl[k];
-      s2[k] = (x - P.x) * (x - P.x) + (y - P.y) * (y - P.y);
-      hillcut[k] = 1.0;
-      integpl[k] = 0.0;
-      p_integpl[k] = 0.0;
-      if (full_mass && (s2[k] < P.near_h2 || s2[k] < P.near_hill2)) {
-        local = 1;
-        with[k] = 1;
-        if (a.exclude_hill) {
-          const double d2 = s2[k] + P.z * P.z;
-          hillcut[k] = 1.0 / (exp(-(sqrt(d2) / P.rhill - a.hillcut) / a.hillcut * 10.0) + 1.0);
-        }
-      } else {
-        with[k] = 0;
-      }
-      if (s2[k] < P.rmorevert2) Nvert = 30;
-    }
-    double isig, integstar, p_integstar = 0.0;       // 1 / sigma from tables
-    if (local) {
-      if (Nvert == 10) {
-        isig = a.isig10;
-        vert_quad<10>(a.wq10, H, r2, Hcorr, pH, peb, npl, with, s2, Rsup_Rinf2, a.pl, integstar, p_integstar,
-                      integpl, p_integpl);
-      } else {
-        isig = a.isig30;
-        vert_quad<30>(a.wq30, H, r2, Hcorr, pH, peb, npl, with, s2, Rsup_Rinf2, a.pl, integstar, p_integstar,
-                      integpl, p_integpl);
-      }
-    } else {
-      isig = fr.isigma_avr[i];
-      integstar = fr.integstar_avr[i];
-      if (peb) p_integstar = fr.p_integstar_avr[i];
-    }
-    double tmp = integstar * isig;
-    double agr = -g.r.Rmed[i] * tmp;            // 0.0 + ar
-    acc[0] += mcell * tmp * x;
-    acc[1] += mcell * tmp * y;
-    double pagr = 0.0;
-    if (peb) { const double pt = p_integstar * isig; pagr = -g.r.Rmed[i] * pt; }
-    double ax = 0.0, ay = 0.0, pax = 0.0, pay = 0.0;
-    for (int k = 0; k < npl; k++) {
-      const DevPlanet P = a.pl[k];
-      double mpl = P.m;
-      if (with[k]) {
-        const bool off = (P.z < -0.05 * H || P.z > 0.05 * H);
-        tmp = (x - P.x) * integpl[k] * (off ? 0.5 * isig : isig);
-        ax += -mpl * tmp;
-        if (a.exclude_hill) tmp *= hillcut[k];
-        acc[2 + 2 * k] += mcell * tmp;
-        tmp = (y - P.y) * integpl[k] * (off ? 0.5 * isig : isig);
-        ay += -mpl * tmp;
-        if (a.exclude_hill) tmp *= hillcut[k];
-        acc[3 + 2 * k] += mcell * tmp;
-        if (peb) {
-          const bool poff = (P.z < -0.05 * pH || P.z > 0.05 * pH);
-          tmp = (x - P.x) * p_integpl[k] * (poff ? 0.5 * isig : isig);
-          pax += -mpl * tmp;
-          if (a.pebble_gravity) { if (a.exclude_hill) tmp *= hillcut[k]; acc[2 + 2 * k] += pmcell * tmp; }
-          tmp = (y - P.y) * p_integpl[k] * (poff ? 0.5 * isig : isig);
-          pay += -mpl * tmp;
-          if (a.pebble_gravity) { if (a.exclude_hill) tmp *= hillcut[k]; acc[3 + 2 * k] += pmcell * tmp; }
-        }
-      } else {
-        mpl *= mass_taper;
-        double d2 = s2[k] + P.z * P.z + P.smoothing2, iv = rsqrt_fast(d2), id3 = iv * iv * iv;
-        tmp = (x - P.x) * id3;
-        ax += -mpl * tmp;
-        if (a.exclude_hill) tmp *= hillcut[k];
-        acc[2 + 2 * k] += mcell * tmp;
-        tmp = (y - P.y) * id3;
-        ay += -mpl * tmp;
-        if (a.exclude_hill) tmp *= hillcut[k];
-        acc[3 + 2 * k] += mcell * tmp;
-        if (peb) {
-          d2 += -P.smoothing2 + P.smoothing2 * Hcorr * Hcorr;
-          iv = rsqrt_fast(d2); id3 = iv * iv * iv;
-          tmp = (x - P.x) * id3;
-          pax += -mpl * tmp;
-          if (a.pebble_gravity) { if (a.exclude_hill) tmp *= hillcut[k]; acc[2 + 2 * k] += pmcell * tmp; }
-          tmp = (y - P.y) * id3;
-          pay += -mpl * tmp;
-          if (a.pebble_gravity) { if (a.exclude_hill) tmp *= hillcut[k]; acc[3 + 2 * k] += pmcell * tmp; }
-        }
+  for (int q = 0; q < nq; q++) acc[q] = 0.0;
+  int any = 0;
+  if ((int)blockIdx.x < a.nbn) {
+    const int nbx = (ns + 127) / 128, by = blockIdx.x / nbx;
+    const int j = (blockIdx.x - by * nbx) * 128 + threadIdx.x;
+    const int i0 = by * a.rings_b, i1 = min(i0 + a.rings_b, g.nr);
+    if (j < ns) {
+      const double c = g.r.costab[j], s = g.r.sintab[j];
+      for (int i = i0; i < i1; i++) {
+        if (!a.near[j + i * ns]) continue;
+        const double x = __dmul_rn(g.r.Rmed[i], c), y = __dmul_rn(g.r.Rmed[i], s);
+        bool hill = false;
+        for (int k = 0; k < a.npl; k++) hill = hill || in_hill(x, y, a.pl[k]);
+        if (hill) continue;
+        any = 1;
+        near_cell<10, false>(g, a, fr, i, j, mass_taper, full_mass, a.wq10, a.c10, a.isig10, acc);
       }
     }
-    const double ir = g.r.InvRmed[i];
-    a.agr[l] = agr + (x * ax + y * ay) * ir;
-    a.agt[l] = 0.0 + (x * ay - y * ax) * ir;
-    if (peb) {
-      a.pagr[l] = pagr + (x * pax + y * pay) * ir;
-      a.pagt[l] = 0.0 + (x * pay - y * pax) * ir;
+  } else {
+    const int lane = threadIdx.x & 31, nw = (a.nbb - a.nbn) * 4;
+    const int gw = (blockIdx.x - a.nbn) * 4 + (threadIdx.x >> 5);
+    for (int k = 0; k < a.npl; k++) {
+      const DevPlanet &P = a.pl[k];
+      if (!(P.rmorevert2 > 0.0)) continue;
+      // rings that reach within two Hill radii of the planet's radius
+      const double rp = sqrt(P.x * P.x + P.y * P.y), rh = 2.001 * P.rhill;
+      int lo = 0, hi = g.nr;
+      while (lo < hi) {                              // first ring with Rsup >= rp - rh
+        const int mid = (lo + hi) >> 1;
+        if (g.r.Rsup[mid] < rp - rh) lo = mid + 1;
+        else hi = mid;
+      }
+      const int imin = lo;
+      hi = g.nr;
+      while (lo < hi) {                              // first ring with Rinf > rp + rh
+        const int mid = (lo + hi) >> 1;
+        if (g.r.Rinf[mid] <= rp + rh) lo = mid + 1;
+        else hi = mid;
+      }
+      const long long ncells = (long long)(lo - imin) * ns;
+      for (long long base = gw; base < ncells; base += 32LL * nw) {   // warp-uniform
+        const long long q = base + (long long)lane * nw;
+        int i = 0, j = 0;
+        bool mine = false;
+        if (q < ncells) {
+          i = imin + (int)(q / ns);
+          j = (int)(q - (q / ns) * ns);
+          if (a.near[j + i * ns]) {
+            const double x = __dmul_rn(g.r.Rmed[i], g.r.costab[j]), y = __dmul_rn(g.r.Rmed[i], g.r.sintab[j]);
+            mine = in_hill(x, y, P);
+            for (int k2 = 0; k2 < k; k2++) mine = mine && !in_hill(x, y, a.pl[k2]);
+          }
+        }
+        unsigned bal = __ballot_sync(TH_FULL, mine);
+        while (bal) {
+          const int src = __ffs(bal) - 1;
+          bal &= bal - 1u;
+          any = 1;
+          near_cell<30, true>(g, a, fr, __shfl_sync(TH_FULL, i, src), __shfl_sync(TH_FULL, j, src), mass_taper,
+                              full_mass, a.wq30, a.c30, a.isig30, acc);
+        }
+      }
     }
   }
-  const int nq = 2 + 2 * npl;
-  const int b = blockIdx.x + blockIdx.y * gridDim.x;
+  if (!__syncthreads_or(any)) {
+    if (threadIdx.x < nq) a.part[(size_t)threadIdx.x * nb + b] = 0.0;
+    return;
+  }
   for (int q = 0; q < nq; q++) {
     const double v = block_reduce_smem<128>(acc[q], OpAdd());
-    if (threadIdx.x == 0) a.part[(size_t)b * nq + q] = v;
+    if (threadIdx.x == 0) a.part[(size_t)q * nb + b] = v;
   }
 }
 
-__global__ void __launch_bounds__(1024) k_forces_final(const double *__restrict__ part, int nb, int nq, double *__restrict__ scal)
+// The sums over the blocks in a fixed order, one block per quantity, and, by
+// the last of them, the indirect term (Pframeforce.c:488-509): in the frame
+// of a column it is (c ax + s ay, c ay - s ax) at every radius, so it is kept
+// per column, the azimuthal part as the mean of the columns either side of a
+// cell's left face, and added where the accelerations are used (a pass over
+// four fields and 14 FP64 instructions a cell before).
+__global__ void __launch_bounds__(1024) k_forces_final(DevGrid g, ForceArgs a, double *__restrict__ scal)
 {
-  // one block; quantity q summed over blocks in a fixed order
-  for (int q = 0; q < nq; q++) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += part[(size_t)b * nq + q];
-    s = block_reduce(s, OpAdd(), 0.0);
-    if (threadIdx.x == 0) {
-      if (q == 0) scal[SC_INDX] = -s;
-      else if (q == 1) scal[SC_INDY] = -s;
-      else scal[SC_PLANET_A + (q - 2)] = s;
-    }
-    __syncthreads();
+  __shared__ bool last;
+  const int q = blockIdx.x, nb = a.nba + a.nbb;
+  const double *p = a.part + (size_t)q * nb;
+  double s = 0.0;
+  for (int b = threadIdx.x; b < nb; b += 1024) s += p[b];
+  s = block_reduce_smem<1024>(s, OpAdd());
+  if (threadIdx.x == 0) {
+    scal[q == 0 ? SC_INDX : q == 1 ? SC_INDY : SC_PLANET_A + (q - 2)] = (q < 2) ? -s : s;
+    __threadfence();
+    last = (atomicAdd(a.ticket, 1u) == gridDim.x - 1);
   }
-}
-
-// Indirect term added to every cell (Pframeforce.c:488-509).
-__global__ void k_forces_indirect(DevGrid g, double *__restrict__ agr, double *__restrict__ agt,
-                                  double *__restrict__ pagr, double *__restrict__ pagt, const double *__restrict__ scal, int pebbles)
-{
-  const double indx_pl = g.ctl[CTL_INDX_PL], indy_pl = g.ctl[CTL_INDY_PL];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *a.ticket = 0u;
+  const double axi = __ldcg(scal + SC_INDX) + g.ctl[CTL_INDX_PL], ayi = __ldcg(scal + SC_INDY) + g.ctl[CTL_INDY_PL];
   const int ns = g.ns;
-  CELL_LOOP_2D
-  const double axi = scal[SC_INDX] + indx_pl, ayi = scal[SC_INDY] + indy_pl;
-  const double x = g.r.Rmed[i] * g.r.costab[j], y = g.r.Rmed[i] * g.r.sintab[j];
-  const double ar = (x * axi + y * ayi) * g.r.InvRmed[i];
-  const double at = (x * ayi - y * axi) * g.r.InvRmed[i];
-  agr[l] += ar;
-  agt[l] += at;
-  if (pebbles) { pagr[l] += ar; pagt[l] += at; }
+  for (int j = threadIdx.x; j < ns; j += 1024) {
+    const double c = g.r.costab[j], sn = g.r.sintab[j];
+    const int jm = (j == 0) ? ns - 1 : j - 1;
+    a.col[j] = c * axi + sn * ayi;
+    a.col[ns + j] = 0.5 * ((c + g.r.costab[jm]) * ayi - (sn + g.r.sintab[jm]) * axi);
+  }
+}
+
+template <int NP>
+static void launch_forces(const DevGrid &g, const ForceArgs &a, const ForceRings &fr, dim3 grid, cudaStream_t s)
+{
+  k_forces<NP><<<grid, 128, a.rings_a * sizeof(ForceRing), s>>>(g, a, fr);
 }
 
 void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
                 double *scal, cudaStream_t s)
 {
-  if (a0.pebbles) aux_ring_means(g, a0.tau, fr.tau_avr, nullptr, nullptr, 0, g.nr, s);
-  k_force_rings<<<(g.nr + 127) / 128, 128, 0, s>>>(g, fr, a0.pebbles, a0.pebble_alpha);
-  g_thorin_launches++;
   ForceArgs a = a0;
   for (int pass = 0; pass < 2; pass++) {
     const int nv = pass ? 30 : 10;
-    double *w = pass ? a.wq30 : a.wq10, sig = 0.0;
+    double *w = pass ? a.wq30 : a.wq10, *ck = pass ? a.c30 : a.c10, sig = 0.0;
     const double deltaz = 3.0 / (double)nv;          // H = 1
+    for (int k = 0; k < FORCE_NC; k++) ck[k] = 0.0;
     for (int m = 1; m <= nv; m++) {
       const double z = ((double)m - 0.5) * deltaz;
       w[m - 1] = exp(-(0.5 * (z * z)));
       sig += w[m - 1];
+      double t = w[m - 1];
+      for (int k = 0; k < FORCE_NC; k++) {           // binomial(-3/2, k) w_m z_m^2k
+        ck[k] += t;
+        t *= z * z * (-1.5 - k) / (k + 1.0);
+      }
     }
-    if (pass) { a.sig30 = sig; a.isig30 = 1.0 / sig; }
-    else { a.sig10 = sig; a.isig10 = 1.0 / sig; }
+    if (pass) a.isig30 = 1.0 / sig;
+    else a.isig10 = 1.0 / sig;
   }
-  dim3 grid = grid2d(g.ns, g.nr, 128 * FORCE_CPT);
-  k_forces<<<grid, 128, 0, s>>>(g, a, fr);
+  // rings per block: chunks long enough that the block sums and the ring
+  // constants are a small part, and at least about six blocks per
+  // multiprocessor; for the near cells fewer, as all their work may lie in a
+  // few chunks
+  const int nbx = (g.ns + 127) / 128;
+  auto rings = [&](int blocks, int lo, int hi) {
+    const int r = (int)((long long)g.nr * nbx / (g.nsm * blocks));
+    return r < lo ? lo : (r > hi ? hi : r);
+  };
+  a.rings_a = rings(6, 4, 32);
+  a.rings_b = rings(40, 1, 4);
+  const dim3 ga(nbx, (g.nr + a.rings_a - 1) / a.rings_a);
+  a.nba = ga.x * ga.y;
+  a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
+  a.nbb = a.nbn + (a.npl > 0 ? g.nsm : 0);
+  k_force_rings<<<g.nr, RING_T, 0, s>>>(g, a, fr);
   g_thorin_launches++;
-  k_forces_final<<<1, 1024, 0, s>>>(a0.part, grid.x * grid.y, 2 + 2 * a0.npl, scal);
+  switch (a.npl) {
+  case 0: launch_forces<0>(g, a, fr, ga, s); break;
+  case 1: launch_forces<1>(g, a, fr, ga, s); break;
+  case 2: launch_forces<2>(g, a, fr, ga, s); break;
+  case 3: launch_forces<3>(g, a, fr, ga, s); break;
+  default: launch_forces<MAXPL_DEV>(g, a, fr, ga, s); break;
+  }
   g_thorin_launches++;
-  k_forces_indirect<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, a0.agr, a0.agt, a0.pagr, a0.pagt, scal,
-                                                          a0.pebbles);
+  k_forces_near<<<a.nbb, 128, 0, s>>>(g, a, fr);
+  g_thorin_launches++;
+  k_forces_final<<<2 + 2 * a.npl, 1024, 0, s>>>(g, a, scal);
   g_thorin_launches++;
 }
 

@@ -26,7 +26,7 @@ __global__ void k_substep1(DevGrid g, const double *__restrict__ rho, const doub
                            const double *__restrict__ vtheta, const double *__restrict__ energy,
                            const double *__restrict__ press,
                            const double *__restrict__ agr, const double *__restrict__ agt,
-                           const double *__restrict__ dragr, const double *__restrict__ dragt,
+                           const double *__restrict__ colf, const double *__restrict__ dragr, const double *__restrict__ dragt,
                            double *__restrict__ vradint, double *__restrict__ vthetaint,
                            double *__restrict__ gaccr, double *__restrict__ gacct, double gm1, int pebbles, int back_reaction,
                            const double *__restrict__ supp_torque, const double *__restrict__ invdxtheta_r)
@@ -45,7 +45,7 @@ __global__ void k_substep1(DevGrid g, const double *__restrict__ rho, const doub
     double vt2 = vtheta[l] + vtheta[ljp] + vtheta[lim] + vtheta[ljp - ns];
     vt2 = vt2 / 4.0 + g.r.Rinf[i] * omega_frame;
     vt2 = vt2 * vt2;
-    double tmp = -gradp + 0.5 * (agr[l] + agr[lim]) + vt2 * g.r.InvRinf[i];
+    double tmp = -gradp + 0.5 * (agr[l] + agr[lim]) + colf[j] + vt2 * g.r.InvRinf[i];
     double v = vrad[l] + dt * tmp;
     if (pebbles) {
       double acc = tmp;
@@ -63,7 +63,7 @@ __global__ void k_substep1(DevGrid g, const double *__restrict__ rho, const doub
     const double pljm = press ? press[ljm] : gm1 * energy[ljm];
     const double it2 = div_fast(2.0, rho[l] + rho[ljm]);     // 2 / (rho_l + rho_ljm), shared
     double gradp = (pl - pljm) * it2 * invdxtheta;
-    double tmp = -gradp + 0.5 * (agt[l] + agt[ljm]);
+    double tmp = -gradp + 0.5 * (agt[l] + agt[ljm]) + colf[ns + j];
     double v = vtheta[l] + dt * tmp;
     v += dt * supp_torque[i];
     if (pebbles) {
@@ -1103,31 +1103,28 @@ __global__ void k_label_from_ext(DevGrid g, const double *__restrict__ rho, cons
 
 // Per-ring quantities of ComputeResiduals (TransportEuler.c:70-111): VMed,
 // the ring mean of v_theta; the integer FARGO shift Nshift; the uniform
-// residual velocity of the second pass.  One warp per ring.  The mean is a
-// fixed butterfly sum (every lane ends with the same bits); when
-// Ntilde + 1/2 lies within 1e-9 of an integer, the ring is summed again left
-// to right, the reference's order, so that the integer shift is exactly the
-// reference's.
-__global__ void __launch_bounds__(256) k_azi_rings(DevGrid g, const double *__restrict__ vt,
-                                                   int *__restrict__ nshift, double *__restrict__ vmed,
-                                                   double *__restrict__ vtemp)
+// residual velocity of the second pass.  One block per ring.  The mean is a
+// fixed tree sum (ring_sum); when Ntilde + 1/2 lies within 1e-9 of an integer,
+// the ring is summed again left to right, the reference's order, so that the
+// integer shift is exactly the reference's.
+__global__ void __launch_bounds__(RING_T) k_azi_rings(DevGrid g, const double *__restrict__ vt,
+                                                      int *__restrict__ nshift, double *__restrict__ vmed,
+                                                      double *__restrict__ vtemp)
 {
   const double dt = g.ctl[CTL_DT];
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (i >= g.nr) return;                           // whole warp
+  const int i = blockIdx.x;
   const int ns = g.ns;
   const double *row = vt + (size_t)i * ns;
-  double a = 0.0;
-  for (int j = lane; j < ns; j += 32) a += row[j];
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(TH_FULL, a, o);
-  double vm = a / (double)ns;
+  double vm = ring_sum(row, ns);
+  if (threadIdx.x >= 32) return;
+  vm /= (double)ns;
   double Ntilde = vm * g.r.InvRmed[i] * dt * (double)ns / 2.0 / TH_PI;
   const double frac = Ntilde + 0.5 - floor(Ntilde + 0.5);
   if (frac < 1e-9 || frac > 1.0 - 1e-9) {
     vm = warp_seq_sum(row, ns) / (double)ns;
     Ntilde = vm * g.r.InvRmed[i] * dt * (double)ns / 2.0 / TH_PI;
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     const double Nround = floor(Ntilde + 0.5);
     const double invdt = 1.0 / dt, dpinvns = 2.0 * TH_PI / (double)ns;
     vmed[i] = vm;
@@ -1293,12 +1290,12 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
 // ---------------------------------------------------------------------------
 // Launch wrappers
 void hydro_substep1(const DevGrid &g, const double *rho, const double *vrad, const double *vtheta,
-                    const double *energy, const double *press, const double *agr, const double *agt,
+                    const double *energy, const double *press, const double *agr, const double *agt, const double *col,
                     const double *dragr, const double *dragt, double *vradint, double *vthetaint, double *gaccr,
                     double *gacct, double gm1, int pebbles, int back_reaction,
                     const double *supp_torque, const double *invdxtheta_r, cudaStream_t s)
 {
-  k_substep1<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, vrad, vtheta, energy, press, agr, agt, dragr, dragt, vradint,
+  k_substep1<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, vrad, vtheta, energy, press, agr, agt, col, dragr, dragt, vradint,
                                                    vthetaint, gaccr, gacct, gm1, pebbles,
                                                    back_reaction, supp_torque, invdxtheta_r);
   g_thorin_launches++;
@@ -1484,7 +1481,7 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   g_thorin_launches++;
   // azimuthal step back into the momenta, the new energy, the tracer and
   // the new density
-  k_azi_rings<<<(nr * 32 + 255) / 256, 256, 0, s>>>(g, vt, S.nshift, S.vmed, S.vtemp);
+  k_azi_rings<<<nr, RING_T, 0, s>>>(g, vt, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   AziIO az;
   for (int k = 0; k < nq; k++) {

@@ -113,8 +113,8 @@ enum {  // ring arrays kept on the device
   R_RINF, R_RSUP, R_RMED, R_SURF, R_INVRMED, R_INVSURF, R_INVDIFFRMED, R_INVDIFFRSUP, R_INVRINF, R_OMEGAINV, R_RMED2,
   R_WAVEKILLER, R_RMED15, R_RINF15, R_RSUP15, R_COSTAB, R_SINTAB, R_SIGMAMED, R_ENERGYMED, R_VTHETAMED, R_PEBDENS0,
   R_PEBVRAD0, R_PEBVTHETA0, R_CSMEAN, R_TEMPMEAN, R_NUMED, R_NUINF, R_INVDXTHETA, R_INVDXTHETA2, R_SUPPTORQUE,
-  R_DELTAR2, R_CFLDXRAD, R_CFLDXTHETA, R_CFLMINDX, R_CFLDEN5, R_VMOY, R_PVTMED, R_HAVR, R_SIGAVR, R_ISTAVR, R_PHAVR,
-  R_PISTAVR, R_VMED, R_TAUAVR, R_VTEMP, R_DAMPVR0, R_CSISO, R_COOLT, R_QPLUSMED, R_ISIGAVR, R_DRSQ, R_OMEGA,
+  R_DELTAR2, R_CFLDXRAD, R_CFLDXTHETA, R_CFLMINDX, R_CFLDEN5, R_VMOY, R_PVTMED, R_HAVR, R_PHAVR, R_AGR0, R_PAGR0,
+  R_STARW, R_VMED, R_VTEMP, R_DAMPVR0, R_CSISO, R_COOLT, R_QPLUSMED, R_DRSQ, R_OMEGA,
   R_COUNT
 };
 
@@ -143,6 +143,8 @@ struct thorin_disk {
   double *partials, *scal;
   int *iscal, *nshift, *heat_idx_d, *damp_rings_d;
   double *heat_val_d;
+  double *force_col;                 // indirect term per column (ForceArgs::col)
+  unsigned char *force_near;         // cells of k_forces_near
   unsigned int *ticket;
   DevPlanet *planets_d;
   double *ctl;                       // control block (CTL_*), also d->g.ctl
@@ -384,9 +386,8 @@ static void build_grid(thorin_disk *d)
   k.sqrt3 = sqrt(3.0);
   d->cfl.dxrad = R[R_CFLDXRAD]; d->cfl.dxtheta = R[R_CFLDXTHETA]; d->cfl.mindx = R[R_CFLMINDX];
   d->cfl.den5 = R[R_CFLDEN5]; d->cfl.vmoy = R[R_VMOY]; d->cfl.pvtmed = R[R_PVTMED];
-  d->fr.H_avr = R[R_HAVR]; d->fr.sigma_avr = R[R_SIGAVR]; d->fr.integstar_avr = R[R_ISTAVR];
-  d->fr.p_H_avr = R[R_PHAVR]; d->fr.p_integstar_avr = R[R_PISTAVR]; d->fr.tau_avr = R[R_TAUAVR];
-  d->fr.isigma_avr = R[R_ISIGAVR]; d->fr.drsq = R[R_DRSQ];
+  d->fr.H_avr = R[R_HAVR]; d->fr.p_H_avr = R[R_PHAVR]; d->fr.agr0 = R[R_AGR0]; d->fr.pagr0 = R[R_PAGR0];
+  d->fr.starw = R[R_STARW]; d->fr.drsq = R[R_DRSQ];
 }
 
 static int check_supported(const thorin_params &p)
@@ -464,7 +465,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     CUCHK(cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming));
   }
   // reduction scratch: enough partials for every reduction kernel
-  const size_t nb = (size_t)((d->ns + 127) / 128 + 2) * (size_t)(d->nr + 2);
+  const size_t nb = (size_t)((d->ns + 127) / 128 + 2) * (size_t)(d->nr + 2) + (size_t)d->g.nsm;
   RCHK(dalloc(d, (void **)&d->partials, nb * (2 + 2 * MAXPL_DEV + 6) * sizeof(double)));
   RCHK(dalloc(d, (void **)&d->scal, 256 * sizeof(double)));
   RCHK(dalloc(d, (void **)&d->iscal, 64 * sizeof(int)));
@@ -473,6 +474,8 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   RCHK(dalloc(d, (void **)&d->heat_val_d, THORIN_MAXPLANETS * sizeof(double)));
   RCHK(dalloc(d, (void **)&d->damp_rings_d, n1 * sizeof(int)));
   RCHK(dalloc(d, (void **)&d->planets_d, MAXPL_DEV * sizeof(DevPlanet)));
+  RCHK(dalloc(d, (void **)&d->force_col, 2 * (size_t)d->ns * sizeof(double)));
+  RCHK(dalloc(d, (void **)&d->force_near, (size_t)d->nr * d->ns));
   CUCHK(cudaMallocHost((void **)&d->scal_h, 256 * sizeof(double)));
   CUCHK(cudaMallocHost((void **)&d->iscal_h, 64 * sizeof(int)));
   CUCHK(cudaMallocHost((void **)&d->csmean_h, n1 * sizeof(double)));
@@ -1385,10 +1388,12 @@ static ForceArgs force_args(const thorin_disk *d, int npl)
   a.rho = d->rho; a.cs = d->cs; a.tau = d->tau; a.pdens = d->pdens;
   a.agr = d->agr; a.agt = d->agt; a.pagr = d->pagr; a.pagt = d->pagt;
   a.part = d->partials;
+  a.col = d->force_col;
+  a.near = d->force_near;
+  a.ticket = d->ticket + 8;
   a.pl = d->planets_d;
   a.npl = npl; a.pebbles = p.pebbles; a.exclude_hill = p.exclude_hill; a.pebble_gravity = p.pebble_gravity;
   a.pebble_alpha = p.pebble_alpha; a.hillcut = p.hillcut;
-  a.sqrt_pebble_alpha = sqrt(p.pebble_alpha);
   return a;
 }
 
@@ -1758,12 +1763,12 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
   // SourceTermsPebbles (Pebbles.c:550-613)
   if (p.pebbles) {
     aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s);
-    aux_pebble_sources(d->g, d->pdens, d->pvrad, d->pvtheta, d->tau, d->vrad, d->vtheta, d->pagr, d->pagt, d->paccr,
-                       d->pacct, d->dragr, d->dragt, p.back_reaction, d->s);
+    aux_pebble_sources(d->g, d->pdens, d->pvrad, d->pvtheta, d->tau, d->vrad, d->vtheta, d->pagr, d->pagt, d->force_col,
+                       d->paccr, d->pacct, d->dragr, d->dragt, p.back_reaction, d->s);
   }
   // SubStep1 with viscous terms (SourceEuler.c:319-415)
-  hydro_substep1(d->g, d->rho, d->vrad, d->vtheta, d->energy, p.energy_eq ? nullptr : d->press, d->agr, d->agt, d->dragr, d->dragt, d->vrad_int,
-                 d->vtheta_int, d->gaccr, d->gacct, d->gm1, p.pebbles, p.back_reaction,
+  hydro_substep1(d->g, d->rho, d->vrad, d->vtheta, d->energy, p.energy_eq ? nullptr : d->press, d->agr, d->agt,
+                 d->force_col, d->dragr, d->dragt, d->vrad_int, d->vtheta_int, d->gaccr, d->gacct, d->gm1, p.pebbles, p.back_reaction,
                  d->ring[R_SUPPTORQUE], d->ring[R_INVDXTHETA], d->s);
   hydro_stress(d->g, d->vrad_int, d->vtheta_int, d->rho, d->divv, d->trr, d->tpp, d->trp, d->invdphi, d->s);
   const int kepler = (!p.damping) || (p.damping && p.damp_vrad);

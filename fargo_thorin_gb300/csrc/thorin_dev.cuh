@@ -132,6 +132,35 @@ __device__ T block_reduce(T v, Op op, T identity)
   return v;
 }
 
+// Sum of a ring by a block of RING_T threads, valid in the first warp: each
+// thread takes every RING_T-th column, the first warp adds the other warps'
+// values of its lanes and a butterfly finishes.  A fixed tree, and every lane
+// returns the same bits.  (One warp per ring, the form before, left most
+// multiprocessors idle: 10 us for the rings of a 512x1536 disk, and the same
+// for a single ring.)
+#define RING_T 128
+__device__ __forceinline__ double ring_sum(const double *__restrict__ row, int ns)
+{
+  __shared__ double sh[RING_T];
+  double a = 0.0, b = 0.0;
+  int j = threadIdx.x;
+  for (; j + RING_T < ns; j += 2 * RING_T) {
+    a += row[j];
+    b += row[j + RING_T];
+  }
+  if (j < ns) a += row[j];
+  a += b;
+  __syncthreads();
+  sh[threadIdx.x] = a;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int w = 1; w < RING_T / 32; w++) a += sh[threadIdx.x + 32 * w];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(TH_FULL, a, o);
+  }
+  return a;
+}
+
 // Reciprocal and reciprocal square root estimates without the FP64 pipe.
 // GB300 issues an FP64 warp instruction every 76 cycles of a sub-partition
 // (1.68 lanes per clock and SM, any mix of adds, products and FMAs) and FP32
@@ -367,6 +396,30 @@ __device__ __forceinline__ double rsqrt_fast(double x)
     return __fma_rn(half_i(y), e, y);
   }
   return rsqrt(x);
+}
+
+// x^(-3/2), x > 0, in three FP64 instructions: y from rsqrt_est, y^2 and y^3
+// as rounded products, and the factor 1 + 3/2 (1 - x y^2) as an integer added
+// to the bits of y^3 (below 2^12 ulp, formed in FP32 to a 2^-8th of an ulp;
+// the residual 1 - x y^2 is exact).  Within 2 ulp; the cube of a rounded
+// reciprocal square root, five instructions, was within 5.
+__device__ __forceinline__ double pow_m32(double x)
+{
+  if (exp_ok(x) && __double2hiint(x) > 0) {
+    const double y = rsqrt_est(x);
+    const double y2 = y * y;
+    const double e = __fma_rn(-x, y2, 1.0);
+    const double y3 = y2 * y;
+    const int H = __double2hiint(e), M = H & 0x7fffffff;
+    const float ef = (M < 0x39000000) ? 0.0f       // below 2^-111
+                                      : __int_as_float(__funnelshift_l(__double2loint(e), M - 0x38000000, 3) |
+                                                       (H & 0x80000000));
+    const float mf = __int_as_float(0x3f800000 | ((__double2hiint(y3) & 0x000fffff) << 3));
+    const int k = __float2int_rn(ef * mf * 6755399441055744.0f);       // 1.5 * 2^52
+    return __longlong_as_double(__double_as_longlong(y3) + (long long)k);
+  }
+  const double iv = rsqrt(x);
+  return iv * iv * iv;
 }
 
 // r / (r + 1e-20), the density's own transported quotient (the reference

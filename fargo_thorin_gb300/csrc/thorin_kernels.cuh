@@ -70,23 +70,35 @@ struct CflFinal {
 };
 
 struct ForceRings {
-  double *H_avr, *sigma_avr, *integstar_avr, *p_H_avr, *p_integstar_avr, *tau_avr;
-  double *isigma_avr;          // 1 / sigma_avr
+  double *H_avr, *p_H_avr;     // ring-mean scale heights of the gas and the pebbles
+  double *agr0, *pagr0;        // the star's pull averaged over the ring-mean column
+  double *starw;               // its weight in the disk's pull on the star, Surf |agr0|
   const double *drsq;          // (Rsup - Rinf)^2
 };
+
+// Terms of the star's vertical average as a series in (H/r)^2, and the largest
+// (H/r)^2 it is used for: there the first term left out is below 8e-18.
+#define FORCE_NC 12
+#define FORCE_QMAX 0.0064
 
 struct ForceArgs {
   const double *rho, *cs, *tau, *pdens;
   double *agr, *agt, *pagr, *pagt;
-  double *part;               // [nblocks][2 + 2*npl]
+  double *part;               // [2 + 2*npl][nblocks]
+  double *col;                // [2][ns]: the indirect term of each column (radial, and azimuthal between j-1 and j)
+  unsigned char *near;        // cells left to k_forces_near
+  unsigned int *ticket;       // of k_forces_final
   const DevPlanet *pl;
   int npl, pebbles, exclude_hill, pebble_gravity;
   double pebble_alpha, hillcut;   // the mass taper is read from the control block
-  double sqrt_pebble_alpha;   // sqrt(pebble_alpha)
   // vertical quadrature weights exp(-z_m^2 / 2H^2) at z_m = (m - 1/2) 3H/N,
-  // which do not depend on H, and their sums (filled by aux_forces)
-  double wq10[10], wq30[30], sig10, sig30;
-  double isig10, isig30;      // 1 / sig10, 1 / sig30
+  // which do not depend on H, the inverses of their sums, and the series
+  // sum_k c_k (H/r)^2k of r^3 sum_m w_m (r^2 + z_m^2)^(-3/2) (filled by
+  // aux_forces)
+  double wq10[10], wq30[30], c10[FORCE_NC], c30[FORCE_NC];
+  double isig10, isig30;
+  int nba, nbb, nbn;          // blocks of k_forces and of k_forces_near, and those of the latter that walk rings
+  int rings_a, rings_b;       // rings per block of the two
 };
 
 struct GasAccArgs {           // one planet of AccreteOntoPlanets (Planet.c:34-166)
@@ -111,8 +123,8 @@ extern std::atomic<long long> g_thorin_launches;
 
 // kernels_hydro.cu
 void hydro_substep1(const DevGrid &g, const double *rho, const double *vrad, const double *vtheta,
-                    const double *energy, const double *press, const double *agr, const double *agt, const double *dragr, const double *dragt,
-                    double *vradint, double *vthetaint, double *gaccr, double *gacct,
+                    const double *energy, const double *press, const double *agr, const double *agt, const double *col,
+                    const double *dragr, const double *dragt, double *vradint, double *vthetaint, double *gaccr, double *gacct,
                     double gm1, int pebbles, int back_reaction, const double *supp_torque, const double *invdxtheta_r,
                     cudaStream_t s);
 void hydro_stress(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *trr,
@@ -189,7 +201,8 @@ void aux_iso_eos(const DevGrid &g, const double *rho, const double *csr, double 
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s);
 void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s);
 void aux_pebble_sources(const DevGrid &g, const double *pd, const double *pvr, const double *pvt, const double *tau,
-                        const double *vr, const double *vt, const double *pagr, const double *pagt, double *paccr,
+                        const double *vr, const double *vt, const double *pagr, const double *pagt, const double *col,
+                        double *paccr,
                         double *pacct, double *dragr, double *dragt, int back_reaction,
                         cudaStream_t s);
 void aux_pebble_substep1(const DevGrid &g, double *pvr, double *pvt, const double *tau, const double *vr, const double *vt,
