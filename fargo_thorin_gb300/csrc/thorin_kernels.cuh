@@ -22,7 +22,7 @@ enum {
   SC_DRAGCELL = 84,           // 6 values of the planet's cell for the aerodynamic drag
   SC_RCS = 96                 // device-resident DT: ring mean of c_s at each planet, taken before the hydro
 };
-enum { IS_NSUB = 0, IS_SOR_DONE, IS_SOR_NITER, IS_SOR_CHANGED, IS_CRASH, IS_COUNT };
+enum { IS_NSUB = 0, IS_SOR_DONE, IS_SOR_NITER, IS_SOR_CHANGED, IS_CRASH, IS_COUNT, IS_CFL_BOUND = 32 };
 
 // Red-black SOR control block (device pointers).
 struct SorCtl {
