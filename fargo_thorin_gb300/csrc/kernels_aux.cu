@@ -124,7 +124,7 @@ __global__ void k_stokes(DevGrid g, const double *__restrict__ rho, const double
 {
   const int ns = g.ns;
   CELL_LOOP_2D
-  tau[l] = div_fast(2.0 * g.k.pebbulkdens * psize[l], rho[l]) * g.k.sqrt_adiabind_inv;
+  tau[l] = div_fast((2.0 * g.k.pebbulkdens * g.k.sqrt_adiabind_inv) * psize[l], rho[l]);
 }
 
 void aux_stokes(const DevGrid &g, const double *rho, const double *psize, double *tau, cudaStream_t s)
@@ -145,17 +145,6 @@ void aux_stokes(const DevGrid &g, const double *rho, const double *psize, double
 struct OpMaxI64 { __device__ long long operator()(long long a, long long b) const { return b > a ? b : a; } };
 
 #define CFL_CPT 4       // cells per thread
-
-// FP32 value of x, truncated; 0 below 2^-100 in size, infinite above 2^100
-// (and for a NaN, so that a bound formed from it excludes nothing).
-__device__ __forceinline__ float to_float_trunc(double x)
-{
-  const int H = __double2hiint(x), M = H & 0x7fffffff;
-  float f = __int_as_float(__funnelshift_l(__double2loint(x), M - 0x38000000, 3));
-  if (M < (923 << 20)) f = 0.0f;
-  if (M > (1123 << 20)) f = __int_as_float(0x7f800000);
-  return __int_as_float(__float_as_int(f) | (H & 0x80000000));
-}
 
 // The sums of squared rates of one cell in FP64 (the reference's expressions).
 __device__ __forceinline__ void cfl_cell(const DevGrid &g, const double *vr, const double *vt, const double *cs,
@@ -278,76 +267,71 @@ __global__ void __launch_bounds__(256) k_cfl_bounds(DevGrid g, const double *__r
   }
 }
 
-// Second pass: the block maxima of the sums in FP64, of the blocks that can
-// hold the disk's largest.
+// Second pass: the maxima of the sums in FP64, over the columns that can hold
+// the disk's largest (all of them without bounds: upper NULL).  The sums are
+// >= 0, so the maxima of the grid are taken on their bits, exactly and in any
+// order; a block whose maximum is not a number, as only a crashed state holds,
+// does not count.  A block takes a quarter of a block of the first pass: the
+// rings that are evaluated fall on several multiprocessors.
 __global__ void __launch_bounds__(256) k_cfl_cells(DevGrid g, const double *__restrict__ vr,
                                                    const double *__restrict__ vt, const double *__restrict__ cs,
                                                    const double *__restrict__ pvr, const double *__restrict__ pvt,
                                                    CflRings cr, int pebbles, int fast, int viscous,
                                                    const float *__restrict__ upper, const int *__restrict__ bound,
-                                                   double *__restrict__ part)
+                                                   unsigned long long *__restrict__ top)
 {
   const int ns = g.ns;
   const int i = blockIdx.y + 1;                    // rings One_or_active .. Max_or_active-1
-  const int b = blockIdx.x + blockIdx.y * gridDim.x;
-  const bool dog = upper[2 * b] >= __int_as_float(bound[0]);
-  const bool dop = pebbles && upper[2 * b + 1] >= __int_as_float(bound[1]);
-  if (!dog && !dop) {
-    if (threadIdx.x == 0) {
-      part[2 * b] = 0.0;
-      part[2 * b + 1] = pebbles ? 0.0 : -1.0e30;
-    }
-    return;
+  if (upper) {
+    const int b = blockIdx.x / CFL_CPT + blockIdx.y * ((gridDim.x + CFL_CPT - 1) / CFL_CPT);
+    if (!(upper[2 * b] >= __int_as_float(bound[0])) && !(pebbles && upper[2 * b + 1] >= __int_as_float(bound[1])))
+      return;
   }
   const double dxrad = cr.dxrad[i], dxtheta = cr.dxtheta[i], mindx = cr.mindx[i];
   const double invdt5 = viscous ? div_fast(g.r.nu_med[i] * 4., cr.den5[i]) : 1e-30;
   // the per-cell rates divide by ring constants: multiply by their reciprocals
   const double idxrad = div_fast(1.0, dxrad), idxtheta = div_fast(1.0, dxtheta), imindx = div_fast(1.0, mindx);
-  long long gas = 0, peb = 0;
-  for (int m = 0; m < CFL_CPT; m++) {
-    const int j = (blockIdx.x * CFL_CPT + m) * blockDim.x + threadIdx.x;
-    if (j >= ns) break;
-    double sg, sp;
-    cfl_cell(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, i, j, idxrad, idxtheta, imindx, invdt5, sg, sp);
-    const long long bg = __double_as_longlong(sg), bp = __double_as_longlong(sp);
-    gas = bg > gas ? bg : gas;
-    peb = bp > peb ? bp : peb;
-  }
-  const long long mg = block_reduce(gas, OpMaxI64(), 0LL);
-  const long long mp = pebbles ? block_reduce(peb, OpMaxI64(), 0LL) : 0LL;
+  double sg = 0.0, sp = 0.0;
+  const int j = blockIdx.x * 256 + threadIdx.x;
+  if (j < ns) cfl_cell(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, i, j, idxrad, idxtheta, imindx, invdt5, sg, sp);
+  const long long mg = block_reduce(__double_as_longlong(sg), OpMaxI64(), 0LL);
+  const long long mp = pebbles ? block_reduce(__double_as_longlong(sp), OpMaxI64(), 0LL) : 0LL;
   if (threadIdx.x == 0) {
-    part[2 * b] = __longlong_as_double(mg);
-    part[2 * b + 1] = pebbles ? __longlong_as_double(mp) : -1.0e30;
+    if (mg <= 0x7ff0000000000000LL) atomicMax(top, (unsigned long long)mg);
+    if (pebbles && mp <= 0x7ff0000000000000LL) atomicMax(top + 1, (unsigned long long)mp);
   }
 }
 
-__global__ void __launch_bounds__(1024) k_cfl_final(DevGrid g, const double *__restrict__ part, CflRings cr, CflFinal f,
-                            double *__restrict__ scal, int *__restrict__ iscal, int *__restrict__ bound)
+// The shear step over the rings, as a 64-bit integer minimum, and the time step.
+struct OpMinI64 { __device__ long long operator()(long long a, long long b) const { return b < a ? b : a; } };
+
+__global__ void __launch_bounds__(1024) k_cfl_final(DevGrid g, CflRings cr, CflFinal f, double *__restrict__ scal,
+                                                    int *__restrict__ iscal, int *__restrict__ bound,
+                                                    unsigned long long *__restrict__ top)
 {
-  if (threadIdx.x < 2) bound[threadIdx.x] = 0;     // for the next call's k_cfl_bounds
   // the remaining part of the DT and MinStepForRebound's rate come from the
   // disk's control block; so does the CFL's substep length, written back
-  const double deltaT = g.ctl[CTL_DELTAT], invdtreb_sq = g.ctl[CTL_INVDTREB];
-  double mg = 0.0, mp = -1.0e30, shear = 1e30;
-  for (int b = threadIdx.x; b < f.nb; b += blockDim.x) {
-    const double a = part[2 * b], c = part[2 * b + 1];
-    if (a > mg) mg = a;
-    if (c > mp) mp = c;
-  }
+  const double deltaT = g.ctl[CTL_DELTAT], invdtreb_sq = g.ctl[CTL_INVDTREB], dts = scal[SC_DTSTELLAR];
+  const unsigned long long mg = top[0], mp = top[1];
+  long long shear = __double_as_longlong(1e30);
   for (int i = threadIdx.x; i < g.nr - 1; i += blockDim.x) {
-    const double dt = f.twopi_cfl_ns / fabs(cr.vmoy[i] * g.r.InvRmed[i] - cr.vmoy[i + 1] * g.r.InvRmed[i + 1]);
-    if (dt < shear) shear = dt;
+    const double w = fabs(cr.vmoy[i] * g.r.InvRmed[i] - cr.vmoy[i + 1] * g.r.InvRmed[i + 1]);
+    const long long dt = __double_as_longlong(div_fast(f.twopi_cfl_ns, w));
+    if (dt >= 0 && dt < shear) shear = dt;
   }
-  mg = block_reduce(mg, OpMax(), 0.0);
-  mp = block_reduce(mp, OpMax(), -1.0e30);
-  shear = block_reduce(shear, OpMin(), 1e30);
+  shear = block_reduce(shear, OpMinI64(), __double_as_longlong(1e30));
+  if (threadIdx.x < 2) {                           // for the next call
+    bound[threadIdx.x] = 0;
+    top[threadIdx.x] = 0ULL;
+  }
   if (threadIdx.x == 0) {
+    const double dmg = __longlong_as_double((long long)mg), dmp = f.pebbles ? __longlong_as_double((long long)mp) : -1.0e30,
+                 dshear = __longlong_as_double(shear);
     double newdt;
-    if (!f.pebbles) newdt = TH_CFLSECURITY / sqrt(mg + invdtreb_sq);
-    else newdt = TH_CFLSECURITY / sqrt(mg + mp + invdtreb_sq);
+    if (!f.pebbles) newdt = div_fast(TH_CFLSECURITY, sqrt_fast(dmg + invdtreb_sq));
+    else newdt = div_fast(TH_CFLSECURITY, sqrt_fast(dmg + dmp + invdtreb_sq));
     if (newdt > 1e30) newdt = 1e30;
-    if (shear < newdt) newdt = shear;
-    const double dts = scal[SC_DTSTELLAR];
+    if (dshear < newdt) newdt = dshear;
     if (newdt > dts) {
       const double m = (1.0 * dts > f.minimum_step) ? 1.0 * dts : f.minimum_step;
       newdt = (newdt < m) ? newdt : m;
@@ -356,7 +340,7 @@ __global__ void __launch_bounds__(1024) k_cfl_final(DevGrid g, const double *__r
     if (f.first_call && f.first_step > 0.0) newdt = f.first_step;
     if (deltaT < newdt) newdt = deltaT;
     scal[SC_NEWDT] = newdt;
-    scal[SC_INVDTPEB] = mp;
+    scal[SC_INVDTPEB] = dmp;
     const int n = (int)(ceil(deltaT / newdt));
     iscal[IS_NSUB] = n;
     g.ctl[CTL_DT] = deltaT / (double)n;
@@ -369,16 +353,21 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
 {
   if (pebbles && fast) aux_ring_means(g, vt, cr.vmoy, pvt, cr.pvtmed, 0, g.nr, s);
   else aux_ring_means(g, vt, cr.vmoy, nullptr, nullptr, 0, g.nr, s);
-  dim3 grid = grid2d(g.ns, g.nr - 1, 256 * CFL_CPT);
-  CflFinal f = f0;
-  f.nb = grid.x * grid.y;
-  float *upper = (float *)(part + 2 * (size_t)f.nb);
+  float *upper = (float *)part;
   int *bound = iscal + IS_CFL_BOUND;
-  k_cfl_bounds<<<grid, 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper, bound);
+  unsigned long long *top = (unsigned long long *)(scal + SC_CFLTOP);
+  // on small grids the FP64 of every cell takes less than a launch (128x384:
+  // 3.4 us; 256x768: 13 us)
+  if ((long long)g.nr * g.ns < (1 << 17)) upper = nullptr;
+  if (upper) {
+    k_cfl_bounds<<<grid2d(g.ns, g.nr - 1, 256 * CFL_CPT), 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast,
+                                                                      viscous, upper, bound);
+    g_thorin_launches++;
+  }
+  k_cfl_cells<<<grid2d(g.ns, g.nr - 1, 256), 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
+                                                          bound, top);
   g_thorin_launches++;
-  k_cfl_cells<<<grid, 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper, bound, part);
-  g_thorin_launches++;
-  k_cfl_final<<<1, 1024, 0, s>>>(g, part, cr, f, scal, iscal, bound);
+  k_cfl_final<<<1, 1024, 0, s>>>(g, cr, f0, scal, iscal, bound, top);
   g_thorin_launches++;
 }
 
@@ -500,97 +489,6 @@ void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s)
   int blocks = (n + 255) / 256;
   if (blocks > 1216) blocks = 1216;
   k_crash<<<blocks, 256, 0, s>>>(n, f, flag);
-  g_thorin_launches++;
-}
-
-// ---------------------------------------------------------------------------
-// SourceTermsPebbles (Pebbles.c:550-613), after DampPebbles.
-__global__ void k_pebble_sources(DevGrid g, const double *__restrict__ pd, const double *__restrict__ pvr,
-                                 const double *__restrict__ pvt, const double *__restrict__ tau,
-                                 const double *__restrict__ vr, const double *__restrict__ vt,
-                                 const double *__restrict__ pagr, const double *__restrict__ pagt,
-                                 const double *__restrict__ colf, double *__restrict__ paccr, double *__restrict__ pacct, double *__restrict__ dragr,
-                                 double *__restrict__ dragt, int back_reaction)
-{
-  const double omega_frame = g.ctl[CTL_OMEGA_FRAME];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  const double Omega = g.r.Omega[i];
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  const double otau = back_reaction ? div_fast(Omega, tau[l]) : 0.0;    // Omega / tau_s
-  if (i >= 1) {
-    const int lim = l - ns;
-    const int ljp = (j == ns - 1) ? i * ns : l + 1;
-    double vt2 = pvt[l] + pvt[ljp] + pvt[lim] + pvt[ljp - ns];
-    vt2 = vt2 / 4.0 + g.r.Rinf[i] * omega_frame;
-    vt2 = vt2 * vt2;
-    paccr[l] = vt2 * g.r.InvRinf[i] + 0.5 * (pagr[l] + pagr[lim]) + colf[j];
-    if (back_reaction) {
-      const double drag = (pvr[l] - vr[l]) * otau;
-      dragr[l] = 0.5 * (pd[l] + pd[lim]) * drag;
-    }
-  }
-  pacct[l] = 0.5 * (pagt[l] + pagt[ljm]) + colf[ns + j];
-  if (back_reaction) {
-    const double drag = (pvt[l] - vt[l]) * otau;
-    dragt[l] = 0.5 * (pd[l] + pd[ljm]) * drag;
-  }
-}
-
-void aux_pebble_sources(const DevGrid &g, const double *pd, const double *pvr, const double *pvt, const double *tau,
-                        const double *vr, const double *vt, const double *pagr, const double *pagt, const double *col,
-                        double *paccr, double *pacct, double *dragr, double *dragt, int back_reaction,
-                        cudaStream_t s)
-{
-  k_pebble_sources<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, pd, pvr, pvt, tau, vr, vt, pagr, pagt, col, paccr, pacct, dragr,
-                                                         dragt, back_reaction);
-  g_thorin_launches++;
-}
-
-// SubStep1Pebbles (Pebbles.c:617-652) followed by ParticleDiffusion
-// (Pebbles.c:656-698): both only change the pebble velocities of cell l.
-__global__ void k_pebble_substep1(DevGrid g, double *__restrict__ pvr, double *__restrict__ pvt,
-                                  const double *__restrict__ tau, const double *__restrict__ vr,
-                                  const double *__restrict__ vt, const double *__restrict__ paccr,
-                                  const double *__restrict__ pacct, const double *__restrict__ gaccr,
-                                  const double *__restrict__ gacct, const double *__restrict__ rho,
-                                  const double *__restrict__ pd, int diffusion, double schmidt,
-                                  const double *__restrict__ invdxtheta_r)
-{
-  const double dt = g.ctl[CTL_DT];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  const double Omega = g.r.Omega[i];
-  const double t = tau[l];
-  const double efac = exp(div_fast(-dt * Omega, t));
-  double a = pvr[l], b = pvt[l];
-  const double oinv = g.r.OmegaInv[i];               // x / Omega as x * OmegaInv
-  if (i > 0) a = a * efac + gaccr[l] * dt + (vr[l] + (paccr[l] - gaccr[l]) * t * oinv) * (1.0 - efac);
-  b = b * efac + gacct[l] * dt + (vt[l] + (pacct[l] - gacct[l]) * t * oinv) * (1.0 - efac);
-  if (diffusion) {
-    if (i >= 1) {
-      const int lim = l - ns;
-      double corr = div_fast(-g.r.nu_inf[i], schmidt);
-      corr *= div_fast(rho[l] + rho[lim], pd[l] + pd[lim]);
-      corr *= (div_fast(pd[l], rho[l]) - div_fast(pd[lim], rho[lim])) * g.r.InvDiffRmed[i];
-      a += corr;
-    }
-    const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-    double corr = div_fast(-g.r.nu_med[i], schmidt);
-    corr *= div_fast(rho[l] + rho[ljm], pd[l] + pd[ljm]);
-    corr *= (div_fast(pd[l], rho[l]) - div_fast(pd[ljm], rho[ljm])) * invdxtheta_r[i];
-    b += corr;
-  }
-  pvr[l] = a;
-  pvt[l] = b;
-}
-
-void aux_pebble_substep1(const DevGrid &g, double *pvr, double *pvt, const double *tau, const double *vr, const double *vt,
-                         const double *paccr, const double *pacct, const double *gaccr, const double *gacct,
-                         const double *rho, const double *pd, int diffusion, double schmidt,
-                         const double *invdxtheta_r, cudaStream_t s)
-{
-  k_pebble_substep1<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, pvr, pvt, tau, vr, vt, paccr, pacct, gaccr, gacct, rho, pd, diffusion, schmidt, invdxtheta_r);
   g_thorin_launches++;
 }
 

@@ -18,64 +18,161 @@
 static inline dim3 grid2d(int ns, int rows, int bx) { return dim3((ns + bx - 1) / bx, rows); }
 static const int BX = 128;
 
+// Rings per block of a kernel whose threads walk the rings of a column: the
+// chunk length with the least work on the busiest multiprocessor, which runs
+// its blocks four at a time and uses 50, 80 or 92% of the FP64 pipe with one,
+// two or three of them left; `extra` is the work at a chunk's start, in rings.
+static int chunk_rings(int nr, int ns, int nsm, int most, double extra)
+{
+  const double part[4] = {0.0, 1.0 / 0.5, 2.0 / 0.8, 3.0 / 0.92};
+  const long long nbx = (ns + BX - 1) / BX;
+  int best = 2;
+  double bestw = 1e300;
+  for (int r = 2; r <= most; r++) {
+    const long long n = (nbx * ((nr + r - 1) / r) + nsm - 1) / nsm;
+    const double w = ((double)(n / 4 * 4) + part[n % 4]) * (r + extra);
+    if (w < bestw) { bestw = w; best = r; }
+  }
+  return best;
+}
+
 // ---------------------------------------------------------------------------
 // SubStep1 velocity predictor (SourceEuler.c:319-407), pressure from the
 // energy (ComputePressureField, SourceEuler.c:740-762) or, in isothermal
-// runs, the pressure field formed at the start of the substep.
-__global__ void k_substep1(DevGrid g, const double *__restrict__ rho, const double *__restrict__ vrad,
-                           const double *__restrict__ vtheta, const double *__restrict__ energy,
-                           const double *__restrict__ press,
-                           const double *__restrict__ agr, const double *__restrict__ agt,
-                           const double *__restrict__ colf, const double *__restrict__ dragr, const double *__restrict__ dragt,
-                           double *__restrict__ vradint, double *__restrict__ vthetaint,
-                           double *__restrict__ gaccr, double *__restrict__ gacct, double gm1, int pebbles, int back_reaction,
-                           const double *__restrict__ supp_torque, const double *__restrict__ invdxtheta_r)
+// runs, the pressure field formed at the start of the substep; with pebbles
+// also SourceTermsPebbles (Pebbles.c:550-613), SubStep1Pebbles (:617-652) and
+// ParticleDiffusion (:656-698), whose new velocities go to pvrn, pvtn (the
+// neighbours' old ones are read here).  Their accelerations and drags are used
+// at the cell that forms them, so they stay in registers: six fields written
+// and read less, and three launches in one.
+//
+// A thread walks the rings of a column and keeps what the next ring shares
+// (pressure, half of the velocity average, the pebble-to-gas ratio); quotients
+// by the same sums of densities share a reciprocal; the difference of the
+// ratios of two columns is one quotient.  FP64-bound: about 30 FP64
+// instructions a cell for the gas (40 before) and 97 with pebbles (135 in three
+// kernels).  512x1536: 161 us, 213 us in three kernels.
+#define SRC_MAXRINGS 24
+
+struct SrcRing { double inv2, invrinf, ro, invdx2, supp, omega, oinv, cr, ct; };
+
+template <bool PEB>
+__global__ void __launch_bounds__(BX) k_sources(DevGrid g, SourceIO io)
 {
-  const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const double pl = press ? press[l] : gm1 * energy[l];
-  if (i >= 1) {
-    const int lim = l - ns;
-    const double plim = press ? press[lim] : gm1 * energy[lim];
-    const double ir2 = div_fast(2.0, rho[l] + rho[lim]);     // 2 / (rho_l + rho_lim), shared
-    double gradp = (pl - plim) * ir2 * g.r.InvDiffRmed[i];
-    double vt2 = vtheta[l] + vtheta[ljp] + vtheta[lim] + vtheta[ljp - ns];
-    vt2 = vt2 / 4.0 + g.r.Rinf[i] * omega_frame;
-    vt2 = vt2 * vt2;
-    double tmp = -gradp + 0.5 * (agr[l] + agr[lim]) + colf[j] + vt2 * g.r.InvRinf[i];
-    double v = vrad[l] + dt * tmp;
-    if (pebbles) {
-      double acc = tmp;
-      if (back_reaction) {
-        tmp = dragr[l] * ir2;
-        v += dt * tmp;
-        acc += tmp;
-      }
-      gaccr[l] = acc;
+  __shared__ SrcRing ring[SRC_MAXRINGS];
+  __shared__ double tab[64];
+  const double dt = g.ctl[CTL_DT];
+  const int ns = g.ns, nr = g.nr;
+  const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
+  if ((int)threadIdx.x < i1 - i0) {
+    const int i = i0 + threadIdx.x;
+    SrcRing &R = ring[threadIdx.x];
+    R.inv2 = 2.0 * g.r.InvDiffRmed[i];
+    R.invrinf = g.r.InvRinf[i];
+    R.ro = g.r.Rinf[i] * g.ctl[CTL_OMEGA_FRAME];
+    R.invdx2 = 2.0 * io.invdxtheta[i];
+    R.supp = io.supp_torque[i];
+    if (PEB) {
+      R.omega = g.r.Omega[i];
+      R.oinv = g.r.OmegaInv[i];
+      R.cr = div_fast(-g.r.nu_inf[i], io.schmidt) * g.r.InvDiffRmed[i];
+      R.ct = div_fast(-g.r.nu_med[i], io.schmidt) * io.invdxtheta[i];
     }
-    vradint[l] = v;
   }
-  {
-    const double invdxtheta = invdxtheta_r[i];
-    const double pljm = press ? press[ljm] : gm1 * energy[ljm];
-    const double it2 = div_fast(2.0, rho[l] + rho[ljm]);     // 2 / (rho_l + rho_ljm), shared
-    double gradp = (pl - pljm) * it2 * invdxtheta;
-    double tmp = -gradp + 0.5 * (agt[l] + agt[ljm]) + colf[ns + j];
-    double v = vtheta[l] + dt * tmp;
-    v += dt * supp_torque[i];
-    if (pebbles) {
-      double acc = tmp + supp_torque[i];
-      if (back_reaction) {
-        tmp = dragt[l] * it2;
-        v += dt * tmp;
-        acc += tmp;
-      }
-      gacct[l] = acc;
+  if (PEB && threadIdx.x >= 64) tab[threadIdx.x - 64] = c_exp64[threadIdx.x - 64];
+  __syncthreads();
+  const int j = blockIdx.x * BX + threadIdx.x;
+  if (j >= ns) return;
+  const int jm = (j == 0) ? ns - 1 : j - 1, jp = (j == ns - 1) ? 0 : j + 1;
+  const double colr = io.col[j], colt = io.col[ns + j];
+  const double *pres = io.press ? io.press : io.energy;
+  const double pscale = io.press ? 1.0 : io.gm1;
+  // of the ring below: density, pressure, v_theta sum, acceleration
+  double rho_m = 1.0, p_m = 0.0, vts_m = 0.0, ag_m = 0.0;
+  double pd_m = 1.0, ratio_m = 0.0, pvts_m = 0.0, pag_m = 0.0;
+  if (i0 > 0) {
+    const int l = j + (i0 - 1) * ns, lp = jp + (i0 - 1) * ns;
+    rho_m = io.rho[l];
+    p_m = pscale * pres[l];
+    vts_m = io.vt[l] + io.vt[lp];
+    ag_m = io.agr[l];
+    if (PEB) {
+      pd_m = io.pd[l];
+      ratio_m = div_fast(pd_m, rho_m);
+      pvts_m = io.pvt[l] + io.pvt[lp];
+      pag_m = io.pagr[l];
     }
-    vthetaint[l] = v;
+  }
+  for (int i = i0; i < i1; i++) {
+    const SrcRing &R = ring[i - i0];
+    const int row = i * ns, l = j + row, ljm = jm + row, ljp = jp + row;
+    const double rho = io.rho[l], rho_jm = io.rho[ljm], p = pscale * pres[l], vr = io.vr[l], vt = io.vt[l];
+    const double vts = vt + io.vt[ljp], ag = io.agr[l];
+    double pd = 0.0, ratio = 0.0, pvts = 0.0, pag = 0.0, otau = 0.0, toinv = 0.0, ef = 0.0, ef1 = 0.0, pvr = 0.0,
+           pvt = 0.0;
+    if (PEB) {
+      const double tau = io.tau[l];
+      pd = io.pd[l];
+      pvr = io.pvr[l];
+      pvt = io.pvt[l];
+      pvts = pvt + io.pvt[ljp];
+      pag = io.pagr[l];
+      otau = div_fast(R.omega, tau);
+      toinv = tau * R.oinv;
+      ef = exp_fast(-dt * otau, tab);
+      ef1 = 1.0 - ef;
+      if (io.diffusion) ratio = div_fast(pd, rho);
+    }
+    if (i >= 1) {
+      const double den = rho + rho_m, ir = div_fast(1.0, den);
+      double w = __fma_rn(vts + vts_m, 0.25, R.ro);
+      double acc = __fma_rn(w * w, R.invrinf, -((p - p_m) * ir * R.inv2));
+      acc = __fma_rn(0.5, ag + ag_m, acc) + colr;
+      double v = __fma_rn(dt, acc, vr);
+      if (PEB) {
+        const double pds = pd + pd_m;
+        if (io.back_reaction) {
+          const double drag = (pvr - vr) * otau * (pds * ir);
+          v = __fma_rn(dt, drag, v);
+          acc += drag;
+        }
+        w = __fma_rn(pvts + pvts_m, 0.25, R.ro);
+        const double pacc = __fma_rn(0.5, pag + pag_m, w * w * R.invrinf) + colr;
+        double a = __fma_rn(__fma_rn(pacc - acc, toinv, vr), ef1, __fma_rn(acc, dt, pvr * ef));
+        if (io.diffusion) a += div_fast(R.cr * (ratio - ratio_m) * den, pds);
+        io.pvrn[l] = a;
+      }
+      io.vrint[l] = v;
+    } else if (PEB) {
+      io.pvrn[l] = pvr;
+    }
+    {
+      const double den = rho + rho_jm, it = div_fast(1.0, den);
+      double acc = __fma_rn(0.5, io.agt[l] + io.agt[ljm], -((p - pscale * pres[ljm]) * it * R.invdx2)) + colt;
+      double v = __fma_rn(dt, acc, vt);
+      if (R.supp != 0.0) {
+        v = __fma_rn(dt, R.supp, v);
+        acc += R.supp;
+      }
+      if (PEB) {
+        const double pd_jm = io.pd[ljm], pds = pd + pd_jm;
+        if (io.back_reaction) {
+          const double drag = (pvt - vt) * otau * (pds * it);
+          v = __fma_rn(dt, drag, v);
+          acc += drag;
+        }
+        const double pacc = __fma_rn(0.5, io.pagt[l] + io.pagt[ljm], colt);
+        double b = __fma_rn(__fma_rn(pacc - acc, toinv, vt), ef1, __fma_rn(acc, dt, pvt * ef));
+        // (pd/rho - pd_jm/rho_jm) (rho + rho_jm) / (pd + pd_jm) as one quotient
+        if (io.diffusion)
+          b += div_fast(R.ct * __fma_rn(-pd_jm, rho, pd * rho_jm) * den, rho * rho_jm * pds);
+        io.pvtn[l] = b;
+      }
+      io.vtint[l] = v;
+    }
+    if (PEB && i == nr - 1) io.pvrn[l + ns] = io.pvr[l + ns];     // row nrad as it was
+    rho_m = rho; p_m = p; vts_m = vts; ag_m = ag;
+    if (PEB) { pd_m = pd; ratio_m = ratio; pvts_m = pvts; pag_m = pag; }
   }
 }
 
@@ -924,6 +1021,10 @@ __global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, doubl
 // Ring constants of the chunk are formed once per block in shared memory.
 // 512x1536: 150 us (gas) and 125 us (pebbles) in the four kernels, 90 and 73 us
 // here; 1024x3072: 335 and 270 us, 96% of the FP64 pipe's rate.
+// Rings per block (chunk_rings): 1.3 rings per chunk are the slopes and the
+// face that neighbouring chunks both form.  Measured for the gas: 256x768
+// 37 / 39 / 51 us with 4 / 6 / 9 rings, 512x1536 105 / 95 / 90 / 103 us with 7 / 11 /
+// 14 / 21, 1024x3072 355 / 335 / 366 / 350 us with 10 / 14 / 20 / 27.
 #define RD_MAXRINGS 40
 
 struct RadialIO {
@@ -1069,27 +1170,6 @@ __global__ void __launch_bounds__(BX, 4) k_radial(DevGrid g, RadialIO io)
     fin[NW] = fout[NW];
     rc = rn; rn = r2; wrc = wrn; wrn = wr2; srho = sr; vf = vn; vn = v2;
   }
-}
-
-// Rings per block of the radial step: the chunk length with the least work on
-// the busiest multiprocessor, which runs its blocks four at a time (the
-// registers' limit) and uses 50, 80 or 92% of the FP64 pipe with one, two or
-// three of them left; 1.3 rings per chunk are the slopes and the face that
-// neighbouring chunks both form.  Measured for the gas: 256x768 37 / 39 / 51 us
-// with 4 / 6 / 9 rings, 512x1536 105 / 95 / 90 / 103 us with 7 / 11 / 14 / 21,
-// 1024x3072 355 / 335 / 366 / 350 us with 10 / 14 / 20 / 27.
-static int rd_rings(int nr, int ns, int nsm)
-{
-  const double part[4] = {0.0, 1.0 / 0.5, 2.0 / 0.8, 3.0 / 0.92};
-  const long long nbx = (ns + BX - 1) / BX;
-  int best = 2;
-  double bestw = 1e300;
-  for (int r = 2; r <= RD_MAXRINGS; r++) {
-    const long long n = (nbx * ((nr + r - 1) / r) + nsm - 1) / nsm;
-    const double w = ((double)(n / 4 * 4) + part[n % 4]) * (r + 1.3);
-    if (w < bestw) { bestw = w; best = r; }
-  }
-  return best;
 }
 
 // ComputeSpeQty (TransportEuler.c:197-215): the tracer back from rho*label.
@@ -1289,15 +1369,14 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
 
 // ---------------------------------------------------------------------------
 // Launch wrappers
-void hydro_substep1(const DevGrid &g, const double *rho, const double *vrad, const double *vtheta,
-                    const double *energy, const double *press, const double *agr, const double *agt, const double *col,
-                    const double *dragr, const double *dragt, double *vradint, double *vthetaint, double *gaccr,
-                    double *gacct, double gm1, int pebbles, int back_reaction,
-                    const double *supp_torque, const double *invdxtheta_r, cudaStream_t s)
+void hydro_sources(const DevGrid &g, const SourceIO &io0, cudaStream_t s)
 {
-  k_substep1<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, vrad, vtheta, energy, press, agr, agt, col, dragr, dragt, vradint,
-                                                   vthetaint, gaccr, gacct, gm1, pebbles,
-                                                   back_reaction, supp_torque, invdxtheta_r);
+  SourceIO io = io0;
+  // 0.15 rings a chunk: the ring below is read again, and the ring constants
+  io.rings = chunk_rings(g.nr, g.ns, g.nsm, SRC_MAXRINGS, 0.15);
+  const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
+  if (io.pd) k_sources<true><<<grid, BX, 0, s>>>(g, io);
+  else k_sources<false><<<grid, BX, 0, s>>>(g, io);
   g_thorin_launches++;
 }
 
@@ -1452,8 +1531,8 @@ void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double 
 // pebbles).  On return the caller's rho/energy pointers
 // are swapped with the updated buffers and vr/vt hold the new velocities.
 
-void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, double **energy, double *label,
-                     const TransportScratch &S, int fast, int damp_vrad, double drin,
+void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
+                     double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,
                      double drout, double *temper, double *cs, double gm1, double gg1, cudaStream_t s)
 {
   const int ns = g.ns, nr = g.nr;
@@ -1467,12 +1546,12 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   qi[nq++] = 5;
   // the radially transported quantities go to the w buffers
   RadialIO rd;
-  rd.rho = *rho; rd.vr = vr; rd.vt = vt; rd.energy = energy ? *energy : nullptr; rd.label = label;
+  rd.rho = *rho; rd.vr = vr_in; rd.vt = vt_in; rd.energy = energy ? *energy : nullptr; rd.label = label;
   for (int q = 0; q < 4; q++) rd.out[q] = S.w[q];
   rd.out[4] = S.w[5];
   rd.out[5] = S.w[4];
   rd.ext = S.w[6];
-  rd.rings = rd_rings(nr, ns, g.nsm);
+  rd.rings = chunk_rings(nr, ns, g.nsm, RD_MAXRINGS, 1.3);
   const dim3 rgrid((ns + BX - 1) / BX, (nr + rd.rings - 1) / rd.rings);
   if (energy && label) k_radial<true, true><<<rgrid, BX, 0, s>>>(g, rd);
   else if (energy) k_radial<true, false><<<rgrid, BX, 0, s>>>(g, rd);
@@ -1481,7 +1560,7 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   g_thorin_launches++;
   // azimuthal step back into the momenta, the new energy, the tracer and
   // the new density
-  k_azi_rings<<<nr, RING_T, 0, s>>>(g, vt, S.nshift, S.vmed, S.vtemp);
+  k_azi_rings<<<nr, RING_T, 0, s>>>(g, vt_in, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   AziIO az;
   for (int k = 0; k < nq; k++) {
@@ -1492,9 +1571,9 @@ void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, dou
   az.n = nq;
   const int T = azi_block(ns);
   const dim3 grid((ns + T - 2 * AZ_HALO - 1) / (T - 2 * AZ_HALO), nr);
-  if (nq == 7) k_azimuthal<7><<<grid, T, 0, s>>>(g, az, vt, fast, S.nshift, S.vmed, S.vtemp);
-  else if (nq == 6) k_azimuthal<6><<<grid, T, 0, s>>>(g, az, vt, fast, S.nshift, S.vmed, S.vtemp);
-  else k_azimuthal<5><<<grid, T, 0, s>>>(g, az, vt, fast, S.nshift, S.vmed, S.vtemp);
+  if (nq == 7) k_azimuthal<7><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else if (nq == 6) k_azimuthal<6><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else k_azimuthal<5><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   // velocities from the transported momenta
   k_velocities<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,

@@ -132,7 +132,7 @@ struct thorin_disk {
   double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *sor_cw, *tbackup, *flaring, *qirr;   // sor_cw = omega / ml
   double *press = nullptr;   // pressure field of isothermal runs (formed at the start of each substep)
   double *label = nullptr;   // passive tracer (LabelAdvection)
-  double *pdens, *pvrad, *pvtheta, *psize, *tau, *paccr, *pacct, *gaccr, *gacct, *dragr, *dragt, *macc;
+  double *pdens, *pvrad, *pvtheta, *psize, *tau, *pvrad_int, *pvtheta_int, *macc;
   double *t_rho_gas, *t_e_gas, *t_rho_peb;
   TransportScratch ts;
   // the pebble fluid's transport runs on its own stream with its own scratch,
@@ -429,12 +429,12 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   if (d->p.stellar_irradiation) { RCHK(dfield(d, &d->flaring)); RCHK(dfield(d, &d->qirr)); }
   else { d->flaring = d->qirr = nullptr; }
   if (d->p.pebbles) {
-    double **P[] = {&d->pagr, &d->pagt, &d->pdens, &d->pvrad, &d->pvtheta, &d->psize, &d->tau, &d->paccr, &d->pacct,
-                    &d->gaccr, &d->gacct, &d->dragr, &d->dragt, &d->macc, &d->t_rho_peb};
+    double **P[] = {&d->pagr, &d->pagt, &d->pdens, &d->pvrad, &d->pvtheta, &d->psize, &d->tau, &d->pvrad_int,
+                    &d->pvtheta_int, &d->macc, &d->t_rho_peb};
     for (auto f : P) RCHK(dfield(d, f));
   } else {
     d->pagr = d->pagt = d->pdens = d->pvrad = d->pvtheta = d->psize = d->tau = nullptr;
-    d->paccr = d->pacct = d->gaccr = d->gacct = d->dragr = d->dragt = d->macc = d->t_rho_peb = nullptr;
+    d->pvrad_int = d->pvtheta_int = d->macc = d->t_rho_peb = nullptr;
   }
   for (int q = 0; q < 4; q++) RCHK(dfield(d, &d->ts.mom[q]));
   for (int q = 0; q < 6; q++) RCHK(dfield(d, &d->ts.w[q]));
@@ -1717,8 +1717,9 @@ static int energy_step(thorin_disk *d, double dt)
   return capped ? THORIN_ERR_SOR_MAXIT : THORIN_OK;
 }
 
-static void transport_fluid(thorin_disk *d, double **rho, double *vr, double *vt, double **energy, double **rho_scratch,
-                            double dt, int gas, const TransportScratch &scratch, cudaStream_t stream)
+// vr_in, vt_in: the velocities before the step (for the gas, vr and vt themselves)
+static void transport_fluid(thorin_disk *d, double **rho, const double *vr_in, const double *vt_in, double *vr,
+                            double *vt, double **energy, double **rho_scratch, double dt, int gas, const TransportScratch &scratch, cudaStream_t stream)
 {
   TransportScratch S = scratch;
   S.rho_new = *rho_scratch;
@@ -1727,7 +1728,7 @@ static void transport_fluid(thorin_disk *d, double **rho, double *vr, double *vt
   // the velocity kernel when it is the only boundary condition
   const thorin_params &p = d->p;
   const int fused = p.damping && p.damp_vrad && !(p.open_inner || p.open_outer || p.non_reflecting || p.outer_source_mass);
-  hydro_transport(d->g, rho, vr, vt, energy, (gas && p.label_advection) ? d->label : nullptr, S,
+  hydro_transport(d->g, rho, vr_in, vt_in, vr, vt, energy, (gas && p.label_advection) ? d->label : nullptr, S,
                   p.fast_transport, gas && fused, d->drin, d->drout, gas ? d->temper : nullptr, d->cs, d->gm1, d->gg1,
                   stream);
   std::swap(*rho, *rho_scratch);
@@ -1760,23 +1761,29 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
   CUCHK(cudaMemsetAsync(d->iscal + IS_CRASH, 0, sizeof(int), d->s));
   aux_crash(d->g, p.pebbles ? d->pdens : d->energy, d->iscal + IS_CRASH, d->s);
   if (!p.energy_eq) aux_iso_eos(d->g, d->rho, nullptr, d->cs, d->press, d->temper, 0, 1, 0, d->s);
-  // SourceTermsPebbles (Pebbles.c:550-613)
+  // SourceTermsPebbles (Pebbles.c:550-613), SubStep1 (SourceEuler.c:319-415),
+  // SubStep1Pebbles and ParticleDiffusion
+  if (p.pebbles) aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s);
+  SourceIO src = {};
+  src.rho = d->rho; src.vr = d->vrad; src.vt = d->vtheta; src.energy = d->energy;
+  src.press = p.energy_eq ? nullptr : d->press;
+  src.agr = d->agr; src.agt = d->agt; src.col = d->force_col;
+  src.supp_torque = d->ring[R_SUPPTORQUE]; src.invdxtheta = d->ring[R_INVDXTHETA];
+  src.vrint = d->vrad_int; src.vtint = d->vtheta_int;
+  src.gm1 = d->gm1; src.schmidt = p.schmidt_number;
+  src.back_reaction = p.back_reaction; src.diffusion = p.diffusive_particles;
   if (p.pebbles) {
-    aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s);
-    aux_pebble_sources(d->g, d->pdens, d->pvrad, d->pvtheta, d->tau, d->vrad, d->vtheta, d->pagr, d->pagt, d->force_col,
-                       d->paccr, d->pacct, d->dragr, d->dragt, p.back_reaction, d->s);
+    src.pd = d->pdens; src.pvr = d->pvrad; src.pvt = d->pvtheta; src.tau = d->tau;
+    src.pagr = d->pagr; src.pagt = d->pagt;
+    src.pvrn = d->pvrad_int; src.pvtn = d->pvtheta_int;
   }
-  // SubStep1 with viscous terms (SourceEuler.c:319-415)
-  hydro_substep1(d->g, d->rho, d->vrad, d->vtheta, d->energy, p.energy_eq ? nullptr : d->press, d->agr, d->agt,
-                 d->force_col, d->dragr, d->dragt, d->vrad_int, d->vtheta_int, d->gaccr, d->gacct, d->gm1, p.pebbles, p.back_reaction,
-                 d->ring[R_SUPPTORQUE], d->ring[R_INVDXTHETA], d->s);
+  hydro_sources(d->g, src, d->s);
+  // viscous terms
   hydro_stress(d->g, d->vrad_int, d->vtheta_int, d->rho, d->divv, d->trr, d->tpp, d->trp, d->invdphi, d->s);
   const int kepler = (!p.damping) || (p.damping && p.damp_vrad);
   hydro_visc_update(d->g, d->vrad_int, d->vtheta_int, d->rho, d->trr, d->tpp, d->trp, d->invdphi, kepler,
                     d->vkep_in - d->Rmed[0] * d->OmegaFrame, d->vkep_out - d->Rmed[d->nr - 1] * d->OmegaFrame, d->s);
   if (p.pebbles) {
-    aux_pebble_substep1(d->g, d->pvrad, d->pvtheta, d->tau, d->vrad, d->vtheta, d->paccr, d->pacct, d->gaccr, d->gacct,
-                        d->rho, d->pdens, p.diffusive_particles, p.schmidt_number, d->ring[R_INVDXTHETA], d->s);
     // EvolvePebbleDisk (Pebbles.c:702-708).  From here on the pebble fields
     // are read and written only by the pebble transport and the gas side
     // touches none of them, so it runs on the pebble stream while the gas
@@ -1784,8 +1791,9 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
     // streams join before this call returns.
     CUCHK(cudaEventRecord(d->ev_fork, d->s));
     CUCHK(cudaStreamWaitEvent(d->s_peb, d->ev_fork, 0));
-    aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s_peb);
-    transport_fluid(d, &d->pdens, d->pvrad, d->pvtheta, nullptr, &d->t_rho_peb, dt, 0, d->ts_peb, d->s_peb);
+    aux_damp_peb(d->g, d->pdens, d->pvrad_int, d->pvtheta_int, d->damp_rings_d, d->ndamp, d->s_peb);
+    transport_fluid(d, &d->pdens, d->pvrad_int, d->pvtheta_int, d->pvrad, d->pvtheta, nullptr, &d->t_rho_peb, dt, 0,
+                    d->ts_peb, d->s_peb);
     aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s_peb);
     CUCHK(cudaEventRecord(d->ev_join, d->s_peb));
   }
@@ -1805,7 +1813,7 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
     status = s;
   }
   // Transport, ApplyBoundaryCondition, ComputeTemperatureField, ComputeSoundSpeed
-  transport_fluid(d, &d->rho, d->vrad, d->vtheta, p.energy_eq ? &d->energy : nullptr, &d->t_rho_gas, dt, 1, d->ts, d->s);
+  transport_fluid(d, &d->rho, d->vrad, d->vtheta, d->vrad, d->vtheta, p.energy_eq ? &d->energy : nullptr, &d->t_rho_gas, dt, 1, d->ts, d->s);
   if (!d->capturing)
     CUCHK(cudaMemcpyAsync(d->nshift_h, d->nshift, d->nr * sizeof(int), cudaMemcpyDeviceToHost, d->s));
   if ((damp && !p.damp_vrad) || p.open_inner || p.open_outer || p.non_reflecting || p.outer_source_mass) {

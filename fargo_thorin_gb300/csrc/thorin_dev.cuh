@@ -418,8 +418,7 @@ __device__ __forceinline__ double pow_m32(double x)
     const int k = __float2int_rn(ef * mf * 6755399441055744.0f);       // 1.5 * 2^52
     return __longlong_as_double(__double_as_longlong(y3) + (long long)k);
   }
-  const double iv = rsqrt(x);
-  return iv * iv * iv;
+  return 1.0 / (x * sqrt(x));
 }
 
 // r / (r + 1e-20), the density's own transported quotient (the reference
@@ -439,4 +438,63 @@ __device__ __forceinline__ double unit_quotient(double r)
     return __longlong_as_double(0x3ff0000000000000LL - (long long)k);
   }
   return r * div_fast(1.0, r + 1e-20);
+}
+
+// exp(x) by table (P. T. P. Tang, ACM Trans. Math. Softw. 15(2):144-157,
+// 1989): n the integer nearest 64 x / ln 2, r = x - n ln 2 / 64 in two steps,
+// exp(x) = 2^(n div 64) 2^((n mod 64)/64) (1 + (r + r^2 (1/2 + r/6 + t))) with
+// the tail t = r^2/24 + r^3/120 + r^4/720, below 1.3e-6, in FP32.  Eight FP64
+// instructions.  tab: exp_table's 64 powers of 2^(1/64), in shared memory.
+__constant__ double c_exp64[64] = {
+    1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
+    1.0442737824274138, 1.0556451783605572, 1.0671404006768237, 1.0787607977571199,
+    1.0905077326652577, 1.102382583307841, 1.1143867425958924, 1.1265216186082418,
+    1.1387886347566916, 1.1511892299529827, 1.1637248587775775, 1.1763969916502812,
+    1.189207115002721, 1.202156731452703, 1.215247359980469, 1.22848053610687,
+    1.241857812073484, 1.255380757024691, 1.2690509571917332, 1.2828700160787783,
+    1.2968395546510096, 1.3109612115247644, 1.3252366431597413, 1.339667524053303,
+    1.3542555469368927, 1.3690024229745905, 1.383909881963832, 1.3989796725383112,
+    1.4142135623730951, 1.42961333839197, 1.4451808069770467, 1.460917794180647,
+    1.4768261459394993, 1.4929077282912648, 1.5091644275934228, 1.5255981507445384,
+    1.5422108254079407, 1.559004400237837, 1.5759808451078865, 1.593142151342267,
+    1.6104903319492543, 1.6280274218573478, 1.645755478153965, 1.6636765803267364,
+    1.681792830507429, 1.7001063537185235, 1.718619298122478, 1.7373338352737062,
+    1.7562521603732995, 1.7753764925265212, 1.7947090750031072, 1.8142521755003989,
+    1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
+    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
+
+__device__ __forceinline__ double float_to_double(float f)
+{
+  const int b = __float_as_int(f);                   // 0 becomes 2^-127
+  return __hiloint2double((((b & 0x7fffffff) >> 3) + 0x38000000) | (b & 0x80000000), b << 29);
+}
+
+// FP32 value of x, truncated; 0 below 2^-100 in size, infinite above 2^100
+// (and for a NaN).
+__device__ __forceinline__ float to_float_trunc(double x)
+{
+  const int H = __double2hiint(x), M = H & 0x7fffffff;
+  float f = __int_as_float(__funnelshift_l(__double2loint(x), M - 0x38000000, 3));
+  if (M < (923 << 20)) f = 0.0f;
+  if (M > (1123 << 20)) f = __int_as_float(0x7f800000);
+  return __int_as_float(__float_as_int(f) | (H & 0x80000000));
+}
+
+__device__ __forceinline__ double exp_fast(double x, const double *tab)
+{
+  const float xf = to_float_trunc(x);
+  if (fabsf(xf) < 600.0f) {
+    const int n = __float2int_rn(xf * 92.332482616893656f);
+    const double nd = float_to_double(__int2float_rn(n));
+    double r = __fma_rn(nd, -0.01083042469326756, x);
+    r = __fma_rn(nd, -2.9815858269852933e-12, r);
+    const float rf = to_float_trunc(r);
+    const float t = rf * rf * __fmaf_rn(rf, __fmaf_rn(rf, 1.3888889e-3f, 8.3333333e-3f), 4.1666667e-2f);
+    const double q = __fma_rn(r, 0.16666666666666666, 0.5) + float_to_double(t);
+    const double e = __fma_rn(r * r, q, r);
+    const double T = tab[n & 63];
+    const double y = __fma_rn(T, e, T);
+    return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
+  }
+  return exp(x);
 }

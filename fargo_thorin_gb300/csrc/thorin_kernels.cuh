@@ -20,7 +20,8 @@ enum {
   SC_TORQUE = 56,             // 2 per planet: ring means of Sigma either side of the planet (UpdateLog)
   SC_GASACC = 80,             // dM, dPx, dPy of the gas accretion onto one planet
   SC_DRAGCELL = 84,           // 6 values of the planet's cell for the aerodynamic drag
-  SC_RCS = 96                 // device-resident DT: ring mean of c_s at each planet, taken before the hydro
+  SC_RCS = 96,                // device-resident DT: ring mean of c_s at each planet, taken before the hydro
+  SC_CFLTOP = 104             // bits of the CFL's largest sums of squared rates (gas, pebbles)
 };
 enum { IS_NSUB = 0, IS_SOR_DONE, IS_SOR_NITER, IS_SOR_CHANGED, IS_CRASH, IS_COUNT, IS_CFL_BOUND = 32 };
 
@@ -51,6 +52,15 @@ struct TransportScratch {
   double *vmed, *vtemp;
 };
 
+// Arguments of the source step (pd NULL: no pebbles).
+struct SourceIO {
+  const double *rho, *vr, *vt, *energy, *press, *agr, *agt, *col, *supp_torque, *invdxtheta;
+  const double *pd, *pvr, *pvt, *tau, *pagr, *pagt;
+  double *vrint, *vtint, *pvrn, *pvtn;
+  double gm1, schmidt;
+  int back_reaction, diffusion, rings;
+};
+
 struct AziIO { const double *src[7]; double *dst[7]; int n; };   // index n-1 is the density
 
 struct ViscParams {
@@ -65,7 +75,7 @@ struct CflRings {
 };
 
 struct CflFinal {
-  int nb, pebbles, first_call;
+  int pebbles, first_call;
   double deltaT, invdtreb_sq, minimum_step, maximum_step, first_step, twopi_cfl_ns;
 };
 
@@ -122,11 +132,7 @@ struct AccArgs {
 extern std::atomic<long long> g_thorin_launches;
 
 // kernels_hydro.cu
-void hydro_substep1(const DevGrid &g, const double *rho, const double *vrad, const double *vtheta,
-                    const double *energy, const double *press, const double *agr, const double *agt, const double *col,
-                    const double *dragr, const double *dragt, double *vradint, double *vthetaint, double *gaccr, double *gacct,
-                    double gm1, int pebbles, int back_reaction, const double *supp_torque, const double *invdxtheta_r,
-                    cudaStream_t s);
+void hydro_sources(const DevGrid &g, const SourceIO &io, cudaStream_t s);
 void hydro_stress(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *trr,
                   double *tpp, double *trp, double invdphi, cudaStream_t s);
 void hydro_visc_update(const DevGrid &g, double *vr, double *vt, const double *rho, const double *trr, const double *tpp,
@@ -164,8 +170,8 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
                       double eps, int count, int maxiters, cudaStream_t s);
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s);
-void hydro_transport(const DevGrid &g, double **rho, double *vr, double *vt, double **energy, double *label,
-                     const TransportScratch &S, int fast, int damp_vrad, double drin,
+void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
+                     double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,
                      double drout, double *temper, double *cs, double gm1, double gg1, cudaStream_t s);
 
 // kernels_aux.cu
@@ -200,15 +206,6 @@ void aux_iso_eos(const DevGrid &g, const double *rho, const double *csr, double 
                  int set_cs, int set_press, int set_temper, cudaStream_t s);
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s);
 void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s);
-void aux_pebble_sources(const DevGrid &g, const double *pd, const double *pvr, const double *pvt, const double *tau,
-                        const double *vr, const double *vt, const double *pagr, const double *pagt, const double *col,
-                        double *paccr,
-                        double *pacct, double *dragr, double *dragt, int back_reaction,
-                        cudaStream_t s);
-void aux_pebble_substep1(const DevGrid &g, double *pvr, double *pvt, const double *tau, const double *vr, const double *vt,
-                         const double *paccr, const double *pacct, const double *gaccr, const double *gacct,
-                         const double *rho, const double *pd, int diffusion, double schmidt,
-                         const double *invdxtheta_r, cudaStream_t s);
 void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
                 double *scal, cudaStream_t s);
 // AccArgs go to the device first (a_dev), the kernels read them there.

@@ -334,6 +334,53 @@ extern "C" int thorin_selftest_slope_division(long long n, unsigned long long se
   return THORIN_OK;
 }
 
+// exp_fast against exp over [-range, range] (x cubed in part, so that small
+// arguments are met too), pow_m32 against 1 / (x sqrt(x)).
+__global__ void k_selftest_exp(long long n, unsigned long long seed, double range, double emax,
+                               unsigned long long *__restrict__ out)
+{
+  __shared__ double tab[64];
+  if (threadIdx.x < 64) tab[threadIdx.x] = c_exp64[threadIdx.x];
+  __syncthreads();
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const double u = 2.0 * ((double)(st_mix(seed + (unsigned long long)t) >> 11) * (1.0 / 9007199254740992.0)) - 1.0;
+  const double x = range * ((t & 1) ? u : u * u * u);
+  const long long a = __double_as_longlong(exp(x)), b = __double_as_longlong(exp_fast(x, tab));
+  const unsigned long long d = (unsigned long long)(a > b ? a - b : b - a);
+  if (d) atomicMax(out, d);
+  const double y = fabs(st_value(seed + (unsigned long long)t, emax));
+  const long long c = __double_as_longlong(1.0 / (y * sqrt(y))), e = __double_as_longlong(pow_m32(y));
+  const unsigned long long f = (unsigned long long)(c > e ? c - e : e - c);
+  if (f) atomicMax(out + 1, f);
+}
+
+extern "C" int thorin_selftest_exp(long long n, unsigned long long seed, double range, double max_exponent,
+                                   unsigned long long *max_ulp_exp, unsigned long long *max_ulp_pow)
+{
+  if (n < 1 || !max_ulp_exp || !max_ulp_pow || !(range >= 0.0 && range <= 700.0) ||
+      !(max_exponent >= 0.0 && max_exponent <= 600.0)) {
+    g_last_error = "selftest_exp: n >= 1, 0 <= range <= 700, 0 <= max_exponent <= 600 and output pointers required";
+    return THORIN_ERR_ARG;
+  }
+  unsigned long long *dev = nullptr, host[2] = {0ULL, 0ULL};
+  cudaError_t e = cudaMalloc((void **)&dev, sizeof(host));
+  if (e == cudaSuccess) e = cudaMemset(dev, 0, sizeof(host));
+  if (e == cudaSuccess) {
+    k_selftest_exp<<<(unsigned)((n + 255) / 256), 256>>>(n, seed, range, max_exponent, dev);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(host, dev, sizeof(host), cudaMemcpyDeviceToHost);
+  if (dev) cudaFree(dev);
+  if (e != cudaSuccess) {
+    g_last_error = std::string("selftest_exp: ") + cudaGetErrorString(e);
+    return THORIN_ERR_CUDA;
+  }
+  *max_ulp_exp = host[0];
+  *max_ulp_pow = host[1];
+  return THORIN_OK;
+}
+
 // vl_slope against a (b / (a + b)) (0 where the signs differ), the two
 // operands' exponents within 2^emax of each other around a random common one;
 // unit_quotient against r / (r + 1e-20).

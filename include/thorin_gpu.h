@@ -424,6 +424,12 @@ int thorin_selftest_slope_division(long long n, unsigned long long seed, double 
 int thorin_selftest_vl_slope(long long n, unsigned long long seed, double max_exponent, unsigned long long *max_ulp,
                              unsigned long long *max_ulp_quotient);
 
+/* Self-test of the kernels' exponential on [-range, range] and of x^(-3/2)
+ * against CUDA's exp and 1 / (x sqrt(x)): n random operands; returns the
+ * largest differences in ulps. */
+int thorin_selftest_exp(long long n, unsigned long long seed, double range, double max_exponent,
+                        unsigned long long *max_ulp_exp, unsigned long long *max_ulp_pow);
+
 /* Compares the kernels' square root routine with IEEE square root on n
  * random operands (exponents in [-max_exponent, max_exponent]) and the
  * reciprocal square root with 1 / sqrt(x): results that differ from sqrt, the

@@ -34,6 +34,21 @@ def test_slope_division_bound(max_exponent, seed):
     assert ulp.value <= 16384
 
 
+@pytest.mark.parametrize("span,max_exponent,seed", [(0.01, 1.0, 20), (1.0, 40.0, 21), (50.0, 200.0, 22),
+                                                     (599.0, 300.0, 23), (700.0, 600.0, 24)])
+def test_exp_and_power_match_cuda(span, max_exponent, seed):
+    """The exponential by table is within one ulp of exp, as CUDA's is: at
+    most 2 ulp apart.  x^(-3/2) is within 2 ulp and 1 / (x sqrt(x)) has three
+    roundings (2 ulp): at most 4 ulp apart."""
+    from fargo_thorin_gb300 import _lib
+    lib = _lib.load()
+    ue, up = C.c_ulonglong(), C.c_ulonglong()
+    _lib.check(lib.thorin_selftest_exp(1 << 26, seed, span, max_exponent, C.byref(ue), C.byref(up)), "selftest_exp")
+    print("exp:", ue.value, "ulp; x^-3/2:", up.value)
+    assert ue.value <= 2
+    assert up.value <= 4
+
+
 @pytest.mark.parametrize("max_exponent,seed", [(0.5, 9), (20.0, 10), (29.9, 11), (32.0, 12), (200.0, 13)])
 def test_van_leer_slope_bound(max_exponent, seed):
     """The slope a b / (a + b) in FP32 pairs keeps the bound of the slopes'
