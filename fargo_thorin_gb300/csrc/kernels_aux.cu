@@ -542,15 +542,6 @@ __device__ __forceinline__ int off_by_5pc(float x, float m)
   return 2;                                        // NaN as well
 }
 
-// FP32 value of a positive double of moderate exponent, truncated (0 outside
-// [2^-100, 2^100]).
-__device__ __forceinline__ float to_float_pos(double x)
-{
-  const int H = __double2hiint(x);
-  const float f = __int_as_float(__funnelshift_l(__double2loint(x), H - 0x38000000, 3));
-  return (unsigned)(H - (923 << 20)) < (unsigned)(200 << 20) ? f : 0.0f;
-}
-
 // k_forces: the accelerations of every cell whose scale height is within 5% of
 // the ring mean's and which is not near a planet (s < 10 H_pl or 5 r_Hill):
 // the star's pull is the ring's, a planet's is softened.  The other cells are
@@ -1374,21 +1365,6 @@ void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const 
   k_integrals<<<grid, 256, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, pebbles, part);
   g_thorin_launches++;
   k_integrals_final<<<1, 1024, 0, s>>>(part, grid.x * grid.y, scal);
-  g_thorin_launches++;
-}
-
-// Final minimum of block partials (DiffusionTimestep's MPI_MIN).
-__global__ void __launch_bounds__(1024) k_min_final(const double *__restrict__ part, int nb, double *__restrict__ out)
-{
-  double m = 1.0e38;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) m = (part[b] < m) ? part[b] : m;
-  m = block_reduce(m, OpMin(), 1.0e38);
-  if (threadIdx.x == 0) *out = m;
-}
-
-void aux_min_final(const double *part, int nb, double *out, cudaStream_t s)
-{
-  k_min_final<<<1, 1024, 0, s>>>(part, nb, out);
   g_thorin_launches++;
 }
 

@@ -20,17 +20,17 @@ static const int BX = 128;
 
 // Rings per block of a kernel whose threads walk the rings of a column: the
 // chunk length with the least work on the busiest multiprocessor, which runs
-// its blocks four at a time and uses 50, 80 or 92% of the FP64 pipe with one,
-// two or three of them left; `extra` is the work at a chunk's start, in rings.
-static int chunk_rings(int nr, int ns, int nsm, int most, double extra)
+// its blocks `slots` at a time and uses 1 - (1 - n / slots)^2 of the FP64 pipe
+// with n of them left; `extra` is the work at a chunk's start, in rings.
+static int chunk_rings(int nr, int ns, int nsm, int most, double extra, int slots = 4)
 {
-  const double part[4] = {0.0, 1.0 / 0.5, 2.0 / 0.8, 3.0 / 0.92};
   const long long nbx = (ns + BX - 1) / BX;
   int best = 2;
   double bestw = 1e300;
   for (int r = 2; r <= most; r++) {
     const long long n = (nbx * ((nr + r - 1) / r) + nsm - 1) / nsm;
-    const double w = ((double)(n / 4 * 4) + part[n % 4]) * (r + extra);
+    const double full = (double)(n / slots * slots), part = (double)(n % slots), q = 1.0 - part / slots;
+    const double w = (full + (part > 0.0 ? part / (1.0 - q * q) : 0.0)) * (r + extra);
     if (w < bestw) { bestw = w; best = r; }
   }
   return best;
@@ -331,28 +331,27 @@ __global__ void k_qplus_row0(DevGrid g, double *__restrict__ qplus, double lr01,
 // Energy equation (EnergySources.c)
 // ComputeTemperatureField + ComputeSoundSpeed (SourceEuler.c:715-792).
 __global__ void k_eos(DevGrid g, const double *__restrict__ rho, const double *__restrict__ energy,
-                      double *__restrict__ temper, double *__restrict__ cs, double gm1, double gg1)
+                      double *__restrict__ temper, double *__restrict__ cs, double gm1, double gamma)
 {
   const int ns = g.ns;
   CELL_LOOP_2D
-  const double r = rho[l], e = energy[l];
-  if (temper) {                             // NULL: ComputeSoundSpeed alone
-    double tmp2 = div_fast(1.0, r * 1.0);
-    double tmp1 = e * 1.0 * gm1;
-    temper[l] = tmp1 * tmp2;
-  }
-  cs[l] = sqrt_fast(div_fast(gg1 * fabs(e), r));
+  // c_s = sqrt(gamma (gamma - 1) |e| / rho) = sqrt(gamma |T|)
+  const double t = div_fast(energy[l] * gm1, rho[l]);
+  if (temper) temper[l] = t;                // NULL: ComputeSoundSpeed alone
+  cs[l] = sqrt_fast(gamma * abs_i(t));
 }
 
 // Opacity laws, Opacity.c.
 // Bell & Lin (Opacity.c:31-75).  The thresholds T(i,j) solve
 // kappa_i rho^a_i T^b_i = kappa_j rho^a_j T^b_j.  The first branch
 // (T <= T(2,3), grains) covers almost the whole disk; its test
-// T <= (kappa_3/kappa_2 rho)^(1/24.5) is decided as T^49 <= (kappa_3/kappa_2
-// rho)^2 unless the two sides are within 1e-12, when the threshold itself is
-// evaluated with pow as in the reference.  The grain branch's integer and
-// half powers are products, quotients and square roots (each within a few
-// ulp of pow); the other branches keep pow.
+// T <= (kappa_3/kappa_2 rho)^(1/24.5) is decided by FP32 logarithms unless the
+// two sides are within 0.01 of each other in log2, then as T^49 <=
+// (kappa_3/kappa_2 rho)^2 unless those are within 1e-12, when the threshold
+// itself is evaluated with pow as in the reference.  The grain branch's integer
+// and half powers are products, quotients and roots (each within a few ulp of
+// pow); it does not use rho, so rho = vd * rho2cgs is formed only where it is
+// needed.
 __device__ __forceinline__ double pow_int_pos(double x, int n)
 {
   double r = 1.0, b = x;
@@ -360,34 +359,44 @@ __device__ __forceinline__ double pow_int_pos(double x, int n)
   return r;
 }
 
-__device__ double opacity_BL94(double rho, double T)
+__device__ double opacity_BL94(double vd, double rho2cgs, double T)
 {
   const double kappa[8] = {2.0e-4, 2.0e16, 0.1, 2.0e81, 1.0e-8, 1.0e-36, 1.5e20, 0.348};
   const double a[8] = {0.0, 0.0, 0.0, 1.0, 2.0 / 3.0, 1.0 / 3.0, 1.0, 0.0};
   const double b[8] = {2.0, -7.0, 0.5, -24.0, 3.0, 10.0, -2.5, 0.0};
 #define TEMPB(i, j) pow(kappa[j] / kappa[i] * pow(rho, a[j] - a[i]), 1.0 / (b[i] - b[j]))
   bool grains;
-  const double c23 = kappa[3] / kappa[2] * rho;            // (kappa_3/kappa_2) rho^(a_3-a_2), a_3-a_2 = 1
-  if (T > 0.0 && T < 1.0e5 && c23 > 0.0 && c23 < 1.0e150) {
-    const double lhs = pow_int_pos(T, 49), rhs = c23 * c23;
-    if (lhs < rhs * (1.0 - 1e-12)) grains = true;
-    else if (lhs > rhs * (1.0 + 1e-12)) grains = false;
-    else grains = (T <= TEMPB(2, 3));
+  // 49 log2 T against 2 log2(kappa_3/kappa_2 rho), each within 1e-4
+  const float Tf = to_float_pos(T), rf = to_float_pos(vd) * (float)rho2cgs;
+  const float d = (Tf > 0.0f && rf > 0.0f)
+                      ? 49.0f * __log2f(Tf) - 2.0f * (__log2f(rf) + 273.39788f) : 0.0f;    // log2(2e82)
+  double rho = 0.0;
+  if (fabsf(d) > 0.01f) {
+    grains = d < 0.0f;
+    if (!grains) rho = vd * rho2cgs;
   } else {
-    grains = (T <= TEMPB(2, 3));
+    rho = vd * rho2cgs;
+    const double c23 = kappa[3] / kappa[2] * rho;          // (kappa_3/kappa_2) rho^(a_3-a_2), a_3-a_2 = 1
+    if (T > 0.0 && T < 1.0e5 && c23 > 0.0 && c23 < 1.0e150) {
+      const double lhs = pow_int_pos(T, 49), rhs = c23 * c23;
+      if (lhs < rhs * (1.0 - 1e-12)) grains = true;
+      else if (lhs > rhs * (1.0 + 1e-12)) grains = false;
+      else grains = (T <= TEMPB(2, 3));
+    } else {
+      grains = (T <= TEMPB(2, 3));
+    }
   }
   double k;
   if (grains) {
     // k1 = kappa0 T^2, k2 = kappa1 T^-7, k3 = kappa2 T^0.5;
     // t1 = (k1^-2 + k2^-2)^-2, x = k3 / (1 + 1e22 T^-10), k = (t1 + x^4)^(1/4),
     // rearranged to two divisions
-    const double T2 = T * T, T4 = T2 * T2, T5 = T4 * T, T7 = T5 * T2, T10 = T5 * T5;
+    const double T2 = T * T, T4 = T2 * T2, T5 = T4 * T, T10 = T5 * T5, T14 = T10 * T4;
     const double k3 = kappa[2] * sqrt_fast(T);
-    const double ik = div_fast(T4, __fma_rn(2.5e-33 * (T7 * T7), T4, 2.5e7));   // 1 / (k1^-2 + k2^-2) = T^4 / (2.5e7 + 2.5e-33 T^18)
-    const double t1 = ik * ik;
+    const double ik = div_fast(T4, __fma_rn(2.5e-33 * T14, T4, 2.5e7));         // 1 / (k1^-2 + k2^-2) = T^4 / (2.5e7 + 2.5e-33 T^18)
     const double x = div_fast(k3 * T10, T10 + 1.0e22);
     const double x2 = x * x;
-    k = sqrt_fast(sqrt_fast(t1 + x2 * x2));
+    k = root4(__fma_rn(ik, ik, x2 * x2));
   } else if (T > 0.0 && rho > 0.0) {
     // T <= TEMPB(i, j) compared as logarithms: ln T <= (ln(kappa_j / kappa_i)
     // + (a_j - a_i) ln rho) / (b_i - b_j), one log each of rho and T; the
@@ -554,94 +563,149 @@ __device__ double opacity_SM03(const DevConst &k, double rho, double T_dust)
   return (aKext > kappa_gas) ? aKext : kappa_gas;
 }
 
-__device__ __forceinline__ double opacity_law(const DevConst &k, int law, double rho, double T, double parametric)
+template <int LAW>
+__device__ __forceinline__ double opacity_law(const DevConst &k, double vd, double T)
 {
-  switch (law) {
-  case THORIN_OPA_SM03: return opacity_SM03(k, rho, T);
-  case THORIN_OPA_ZHU12: return opacity_ZHU12(rho, T);
-  case THORIN_OPA_LP85: return opacity_LP85(rho, T);
-  case THORIN_OPA_CONST: return parametric;
-  default: return opacity_BL94(rho, T);
-  }
-}
-
-// |grad T|^2 at a cell centre (TemperatureGradient, EnergySources.c:609-653).
-__device__ __forceinline__ double gradt_sq(const DevGrid &g, const double *T, int i, int j, const double *invdxtheta_r)
-{
-  const int ns = g.ns, l = j + i * ns, lip = l + ns, lim = l - ns;
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  const double invdx = invdxtheta_r[i];
-  double gr_l = (T[l] - T[lim]) * g.r.InvDiffRmed[i];
-  double gr_lip = (T[lip] - T[l]) * g.r.InvDiffRmed[i + 1];
-  double gt_l = (T[l] - T[ljm]) * invdx;
-  double gt_ljp = (T[ljp] - T[l]) * invdx;
-  double r = 0.5 * (gr_lip + gr_l);
-  double t = 0.5 * (gt_ljp + gt_l);
-  return r * r + t * t;
-}
-
-// FluxLimiterValue (EnergySources.c:684-698) of s = sqrt(g2) * c, from
-// s^2 = g2 c^2: below s = 2 the limiter 2 / (3 + sqrt(9 + 10 s^2)) needs only
-// s^2, which saves the square root of |grad T| in optically thick cells (the
-// limiter is continuous at s = 2, where both forms give 1/5).
-__device__ __forceinline__ double flux_limiter_sq(double g2, double c)
-{
-  const double s2 = g2 * (c * c);
-  if (s2 <= 4.0) return div_fast(2.0, 3.0 + sqrt_fast(9.0 + 10.0 * s2));
-  const double s = sqrt_fast(g2) * c;
-  return div_fast(10.0, 10.0 * s + 9.0 + sqrt_fast(81.0 + 180.0 * s));
+  if (LAW == THORIN_OPA_SM03) return opacity_SM03(k, vd * k.rho2cgs, T);
+  if (LAW == THORIN_OPA_ZHU12) return opacity_ZHU12(vd * k.rho2cgs, T);
+  if (LAW == THORIN_OPA_LP85) return opacity_LP85(vd * k.rho2cgs, T);
+  return opacity_BL94(vd, k.rho2cgs, T);
 }
 
 // MidplaneVolumeDensity, OpacityProfile, CalculateQminus and the centred
 // diffusion coefficient of DiffusionCoefs (EnergySources.c:556-592,
-// 658-711, Opacity.c:231-266); block partial minima of DiffusionTimestep
-// (EnergySources.c:833-856).
-__global__ void k_diffcoef(DevGrid g, const double *__restrict__ rho, const double *__restrict__ T,
-                           const double *__restrict__ cs, double *__restrict__ opacity, double *__restrict__ qminus,
-                           double *__restrict__ dcen, double *__restrict__ dtmin_part, int law, double parametric_cu,
-                           double parametric_raw, double opacity_drop, double taueff_c, const double *__restrict__ invdxtheta_r,
-                           const double *__restrict__ deltar2_r)
+// 658-711, Opacity.c:231-266), and DiffusionTimestep (EnergySources.c:
+// 833-856).
+//
+// A thread walks the rings of a column, so the radial temperature difference
+// of a ring is formed once; |grad T|^2 (TemperatureGradient, :609-653) is
+// (R^2 + P^2) / 4, R = dT/dr at the two faces added, P the difference across the
+// two azimuthal neighbours over the cell width.  The flux limiter
+// (FluxLimiterValue, :684-698) of s = 4 |grad T| / (rho kappa T) needs only s^2
+// below s = 2, where it is 2 / (3 + sqrt(9 + 10 s^2)); both forms give 1/5 at
+// s = 2.  The diffusion coefficient's division and the limiter's are one.
+// FP64-bound: 81 FP64 instructions a cell with the Bell & Lin opacity, 120
+// before; 512x1536: 182 -> 138 us, with the minimum over the blocks.
+// Rings per block: chunks of at most 8, as the inner, hotter rings take the
+// longer opacity branches and short chunks spread them (512x1536: 133 / 138 / 157
+// us with 3 / 6 / 11 rings; 1024x3072: 486 / 500 / 543 us with 8 / 16 / 21).
+#define DC_MAXRINGS 8
+
+struct DcRing { double c1, inv, invp, invdx, deltar2; };
+
+template <int LAW>
+__global__ void __launch_bounds__(BX) k_diffcoef(DevGrid g, DiffusionIO io)
 {
+  __shared__ DcRing ring[DC_MAXRINGS];
+  __shared__ unsigned long long smax[BX / 32][DC_MAXRINGS];
+  __shared__ bool last;
   const int ns = g.ns, nr = g.nr;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  // DiffusionTimestep's min over the ring of deltar2 / D: deltar2 is a ring
-  // constant and correctly rounded division is monotone, so for D > 0 the
-  // minimum is deltar2 / max D, one division per block; other D (which only
-  // a crashed state holds) are divided cell by cell as the reference does
-  double dmax = 0.0, dtl = 1.0e38;
-  if (j < ns) {
-    const int l = j + i * ns;
-    const double H = cs[l] * g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
-    const double vd = div_fast(rho[l], H) * g.k.sqrt2pi_inv;
-    const double Tl = T[l];
-    double kap;
-    if (parametric_raw > 0.0) kap = parametric_cu;
-    else kap = opacity_law(g.k, law, vd * g.k.rho2cgs, Tl * g.k.t2si, parametric_raw) * g.k.opa2cu;
-    opacity[l] = kap;
-    const double tau = opacity_drop * 0.5 * kap * rho[l];
-    // Q- = 2 sigma T^3 / tau_eff, tau_eff = 3/8 tau + c + 1/(4 tau), as one quotient
-    const double T3 = cube_rn(Tl);
-    qminus[l] = div_fast(2.0 * g.k.sigma_sb * T3 * tau, __fma_rn(__fma_rn(0.375, tau, taueff_c), tau, 0.25));
-    const int ig = (i == 0) ? 1 : (i == nr - 1 ? nr - 2 : i);
-    const double g2 = gradt_sq(g, T, ig, j, invdxtheta_r);
-    // fac = 1 / (rho_mid kappa) and the limiter argument s = 4 |grad T| fac / T from one division
-    const double q = div_fast(1.0, vd * kap * Tl);
-    const double fac = q * Tl;
-    const double D = flux_limiter_sq(g2, 4.0 * q) * 16.0 * g.k.sigma_sb * T3 * fac;
-    dcen[l] = D;
-    if (__double_as_longlong(D) > 0LL) dmax = D;
-    else dtl = div_fast(deltar2_r[i], D);
+  const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
+  if ((int)threadIdx.x < i1 - i0) {
+    const int i = i0 + threadIdx.x;
+    DcRing &R = ring[threadIdx.x];
+    R.c1 = div_fast(g.k.sqrt2pi_inv, g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv);   // rho / H / sqrt(2 pi) = rho c1 / c_s
+    R.inv = g.r.InvDiffRmed[i];
+    R.invp = g.r.InvDiffRmed[i + 1];
+    R.invdx = io.invdxtheta[i];
+    R.deltar2 = io.deltar2[i];
   }
-  const double dm = block_reduce_smem<BX>(dmax, OpMax());
-  double m = block_reduce_smem<BX>(dtl, OpMin());
-  if (threadIdx.x == 0) {
-    if (dm > 0.0) {
-      const double q = div_fast(deltar2_r[i], dm);
-      if (q < m) m = q;
+  __syncthreads();
+  const int jt = blockIdx.x * BX + threadIdx.x;
+  const bool in = jt < ns;
+  const int j = in ? jt : ns - 1;
+  const int jm = (j == 0) ? ns - 1 : j - 1, jp = (j == ns - 1) ? 0 : j + 1;
+  const double sig2 = 2.0 * g.k.sigma_sb, sig32 = 32.0 * g.k.sigma_sb, drop = io.opacity_drop * 0.5;
+  const double *T = io.T;
+  // radial difference of ring i with the ring below, over their distance; the
+  // edge rings adopt their neighbour's gradient
+  double Tl = T[j + i0 * ns], below = 0.0, dtl = 1.0e38;
+  if (i0 > 0) below = (Tl - T[j + (i0 - 1) * ns]) * ring[0].inv;
+  for (int i = i0; i < i1; i++) {
+    const DcRing &R = ring[i - i0];
+    const int row = i * ns, l = j + row;
+    const double Tn = (i + 1 < nr) ? T[l + ns] : 0.0;
+    const double above = (i + 1 < nr) ? (Tn - Tl) * R.invp : 0.0;
+    double gr, gp;
+    if (i == 0 || i == nr - 1) {
+      const int k = (i == 0) ? 1 : nr - 2, lk = j + k * ns;
+      gr = (T[lk] - T[lk - ns]) * g.r.InvDiffRmed[k] + (T[lk + ns] - T[lk]) * g.r.InvDiffRmed[k + 1];
+      gp = (T[jp + k * ns] - T[jm + k * ns]) * io.invdxtheta[k];
+    } else {
+      gr = above + below;
+      gp = (T[jp + row] - T[jm + row]) * R.invdx;
     }
-    dtmin_part[blockIdx.x + blockIdx.y * gridDim.x] = m;
+    const double G = __fma_rn(gr, gr, gp * gp);                // 4 |grad T|^2
+    const double rho = io.rho[l];
+    const double vd = div_fast(rho * R.c1, io.cs[l]);
+    const double kap = (LAW == THORIN_OPA_CONST) ? io.parametric_cu
+                                                 : opacity_law<LAW>(g.k, vd, Tl * g.k.t2si) * g.k.opa2cu;
+    const double tau = drop * kap * rho;
+    const double T3 = cube_rn(Tl);
+    // Q- = 2 sigma T^3 / tau_eff, tau_eff = 3/8 tau + c + 1/(4 tau), as one quotient
+    const double qm = div_fast(sig2 * T3 * tau, __fma_rn(__fma_rn(0.375, tau, io.taueff_c), tau, 0.25));
+    // q = 1 / (rho_mid kappa T); s^2 = 16 |grad T|^2 q^2 = 4 G q^2
+    const double q = div_fast(1.0, vd * kap * Tl);
+    const double X = q * q * G;
+    const double num = sig32 * T3 * (q * Tl);                  // 2 * 16 sigma T^3 / (rho_mid kappa)
+    double D;
+    if (__double_as_longlong(X) <= __double_as_longlong(1.0)) {      // s <= 2
+      D = div_fast(num, 3.0 + sqrt_fast(__fma_rn(40.0, X, 9.0)));
+    } else {
+      const double s = 2.0 * sqrt_fast(X);
+      D = div_fast(5.0 * num, 10.0 * s + 9.0 + sqrt_fast(81.0 + 180.0 * s));
+    }
+    if (in) {
+      io.opacity[l] = kap;
+      io.qminus[l] = qm;
+      io.dcen[l] = D;
+    }
+    // DiffusionTimestep's min of deltar2 / D: deltar2 is a ring constant and
+    // correctly rounded division is monotone, so for D > 0 the minimum of a
+    // ring is deltar2 / max D; other D (which only a crashed state holds) are
+    // divided cell by cell as the reference does
+    unsigned hi = (unsigned)__double2hiint(D), lo = (unsigned)__double2loint(D);
+    if (!(__double_as_longlong(D) > 0LL)) {
+      hi = lo = 0u;
+      const double t = div_fast(R.deltar2, D);
+      if (in && t < dtl) dtl = t;
+    }
+    const unsigned mh = __reduce_max_sync(TH_FULL, hi);
+    const unsigned ml = __reduce_max_sync(TH_FULL, hi == mh ? lo : 0u);
+    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5][i - i0] = ((unsigned long long)mh << 32) | ml;
+    Tl = Tn;
+    below = above;
+  }
+  __syncthreads();
+  const int b = blockIdx.x + blockIdx.y * gridDim.x, nb = gridDim.x * gridDim.y;
+  if ((int)threadIdx.x < i1 - i0) {
+    unsigned long long m = 0ULL;
+#pragma unroll
+    for (int w = 0; w < BX / 32; w++) m = max(m, smax[w][threadIdx.x]);
+    const double dm = __longlong_as_double((long long)m);
+    if (dm > 0.0) {
+      const double t = div_fast(ring[threadIdx.x].deltar2, dm);
+      if (t < dtl) dtl = t;
+    }
+  }
+  const double m = block_reduce_smem<BX>(dtl, OpMin());
+  if (threadIdx.x == 0) {
+    io.part[b] = m;
+    __threadfence();
+    last = (atomicAdd(io.ticket, 1u) == (unsigned)nb - 1u);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 1.0e38;
+  for (int k = threadIdx.x; k < nb; k += BX) {
+    const double v = __ldcg(io.part + k);
+    t = (v < t) ? v : t;
+  }
+  t = block_reduce_smem<BX>(t, OpMin());
+  if (threadIdx.x == 0) {
+    *io.dtmin = t;
+    *io.ticket = 0u;
   }
 }
 
@@ -680,56 +744,6 @@ __global__ void k_irradiation(DevGrid g, const double *__restrict__ rho, const d
     }
     qirr[l] = q;
   }
-}
-
-// Matrix of the linearised implicit energy equation
-// (ImplicitRadiativeDiffusion, EnergySources.c:256-297), plus the
-// reciprocal of the diagonal used by the SOR update.
-__global__ void k_matrix(DevGrid g, const double *__restrict__ rho, const double *__restrict__ T,
-                         const double *__restrict__ cs, const double *__restrict__ dcen, const double *__restrict__ divv,
-                         const double *__restrict__ qminus, const double *__restrict__ qplus, const double *__restrict__ qirr,
-                         double *__restrict__ ml, double *__restrict__ mlip, double *__restrict__ mlim,
-                         double *__restrict__ mljp, double *__restrict__ mljm, double *__restrict__ rhs, double gm1, const double *__restrict__ invdxtheta2_r,
-                         int irradiation, int nheat, const int *__restrict__ heat_idx,
-                         const double *__restrict__ heat_val)
-{
-  const double dt = g.ctl[CTL_DT];
-  const int ns = g.ns;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y + 1;                   // rings 1 .. nr-2
-  if (j >= ns) return;
-  const int l = j + i * ns, lip = l + ns, lim = l - ns;
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  const double sqi = g.k.sqrt_adiabind_inv;
-  const double oi = g.r.OmegaInv[i];
-  const double idx2 = invdxtheta2_r[i];
-  // A at faces i and i+1, B at faces j and j+1
-  const double Dr_l = 0.5 * (dcen[l] + dcen[lim]);
-  const double Dr_lip = 0.5 * (dcen[lip] + dcen[l]);
-  const double A_l = Dr_l * g.r.Rinf[i] * g.r.InvDiffRmed[i];
-  const double A_lip = Dr_lip * g.r.Rinf[i + 1] * g.r.InvDiffRmed[i + 1];
-  const double H = cs[l] * oi * sqi;
-  const double Dt_l = 0.5 * (dcen[l] + dcen[ljm]);
-  const double B_l = Dt_l * idx2 * 2.0 * H;
-  const double Hjp = cs[ljp] * oi * sqi;
-  const double Dt_ljp = 0.5 * (dcen[ljp] + dcen[l]);
-  const double B_ljp = Dt_ljp * idx2 * 2.0 * Hjp;
-  const double bfac = div_fast(dt, rho[l] * g.k.cv);
-  const double afac = bfac * g.r.InvDiffRsup[i] * 2.0 * H * g.r.InvRmed[i];
-  const double Tl = T[l], qm = qminus[l];
-  const size_t q = sor_pidx(i, j, ns >> 1);
-  const double diag = 1.0 + divv[l] * gm1 * dt + 4.0 * bfac * qm + afac * (A_lip + A_l) + bfac * (B_ljp + B_l);
-  ml[q] = diag;
-  mlip[q] = -afac * A_lip;
-  mlim[q] = -afac * A_l;
-  mljp[q] = -bfac * B_ljp;
-  mljm[q] = -bfac * B_l;
-  double r = Tl + bfac * (qplus[l] + 3.0 * qm * Tl);
-  if (irradiation) r += bfac * qirr[l];
-  for (int k = 0; k < nheat; k++)
-    if (l == heat_idx[k]) r += bfac * heat_val[k];
-  rhs[q] = r;
 }
 
 // ---------------------------------------------------------------------------
@@ -796,30 +810,10 @@ __device__ __forceinline__ bool sor_last_block(unsigned int *ticket, unsigned nb
   return last;
 }
 
-__global__ void __launch_bounds__(SOR_BX) k_sor_resid0(DevGrid g, const double *__restrict__ T,
-                                                    const double *__restrict__ ml, const double *__restrict__ mlip,
-                                                    const double *__restrict__ mlim, const double *__restrict__ mljp,
-                                                    const double *__restrict__ mljm, const double *__restrict__ rhs,
-                                                    double *__restrict__ cw, SorCtl c)
+// The start residual's sums over the grid (the L1 norm and the warm start's
+// input scale) by the last block, which also resets the solve's counters.
+__device__ __forceinline__ void sor_resid_sums(const SorCtl &c, double a, double aj)
 {
-  const double omega = g.ctl[CTL_SOR_OMEGA];
-  const int ns = g.ns, half = ns >> 1;
-  const int i = blockIdx.y + 1;
-  double a = 0.0, aj = 0.0;
-  for (int m = 0; m < SOR_CPT; m++) {
-    const int j = blockIdx.x * blockDim.x * SOR_CPT + m * blockDim.x + threadIdx.x;
-    if (j < ns) {
-      const int l = j + i * ns;
-      const int ljp = (j == ns - 1) ? i * ns : l + 1;
-      const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-      const size_t q = sor_pidx(i, j, half);
-      const double r = abs_i(sor_resid_at(T, ml, mlip, mlim, mljp, mljm, rhs, l, l + ns, l - ns, ljp, ljm, q));
-      const double w = div_fast(omega, ml[q]);     // the sweeps' update is resid * omega / ml
-      cw[q] = w;
-      a += r;
-      aj += r * w;                                 // omega |resid / Ml|: the warm start's input scale
-    }
-  }
   a = block_reduce(a, OpAdd(), 0.0);
   aj = block_reduce(aj, OpAdd(), 0.0);
   const unsigned nb = gridDim.x * gridDim.y;
@@ -845,6 +839,125 @@ __global__ void __launch_bounds__(SOR_BX) k_sor_resid0(DevGrid g, const double *
       *c.ticket = 0u;
     }
   }
+}
+
+__global__ void __launch_bounds__(SOR_BX) k_sor_resid0(DevGrid g, const double *__restrict__ T,
+                                                    const double *__restrict__ ml, const double *__restrict__ mlip,
+                                                    const double *__restrict__ mlim, const double *__restrict__ mljp,
+                                                    const double *__restrict__ mljm, const double *__restrict__ rhs,
+                                                    double *__restrict__ cw, SorCtl c)
+{
+  const double omega = g.ctl[CTL_SOR_OMEGA];
+  const int ns = g.ns, half = ns >> 1;
+  const int i = blockIdx.y + 1;
+  double a = 0.0, aj = 0.0;
+  for (int m = 0; m < SOR_CPT; m++) {
+    const int j = blockIdx.x * blockDim.x * SOR_CPT + m * blockDim.x + threadIdx.x;
+    if (j < ns) {
+      const int l = j + i * ns;
+      const int ljp = (j == ns - 1) ? i * ns : l + 1;
+      const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
+      const size_t q = sor_pidx(i, j, half);
+      const double r = abs_i(sor_resid_at(T, ml, mlip, mlim, mljp, mljm, rhs, l, l + ns, l - ns, ljp, ljm, q));
+      const double w = div_fast(omega, ml[q]);     // the sweeps' update is resid * omega / ml
+      cw[q] = w;
+      a += r;
+      aj += r * w;                                 // omega |resid / Ml|: the warm start's input scale
+    }
+  }
+  sor_resid_sums(c, a, aj);
+}
+
+// Matrix of the linearised implicit energy equation
+// (ImplicitRadiativeDiffusion, EnergySources.c:256-297) and, with RESID, the
+// start of the SOR solve at the omega of the control block (what
+// k_sor_resid0 does for a system that is already in memory): omega/Ml and the
+// L1 residual of the start temperature.
+//
+// A thread walks the rings of a column: the radial face coefficient of a ring's
+// outer face is the next ring's inner one, and the azimuthal one of a cell's
+// right face comes from the neighbouring thread through shared memory (the
+// last thread of a block forms it).  The diagonal is 1 + the heating terms
+// minus the four neighbour coefficients.  FP64-bound: 40 FP64 instructions a
+// cell with the start residual, 60 in the two kernels before; 512x1536: 107 -> 74
+// us.
+#define MX_MAXRINGS 24
+
+struct MxRing { double ca, cb, ch; };
+
+template <bool RESID>
+__global__ void __launch_bounds__(BX) k_matrix(DevGrid g, MatrixIO io, SorCtl c)
+{
+  __shared__ MxRing ring[MX_MAXRINGS + 1];
+  __shared__ double sB[2][BX];
+  const double dt = g.ctl[CTL_DT], omega = RESID ? g.ctl[CTL_SOR_OMEGA] : 0.0;
+  const int ns = g.ns, half = ns >> 1;
+  const int i0 = 1 + blockIdx.y * io.rings, i1 = min(i0 + io.rings, g.nr - 1);     // rings 1 .. nr-2
+  if ((int)threadIdx.x <= i1 - i0) {
+    const int i = i0 + threadIdx.x;
+    MxRing &R = ring[threadIdx.x];
+    const double hc = g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;                     // H = c_s hc
+    R.ca = 0.5 * g.r.Rinf[i] * g.r.InvDiffRmed[i];
+    R.cb = io.invdxtheta2[i] * hc;
+    R.ch = 2.0 * g.r.InvDiffRsup[i] * g.r.InvRmed[i] * hc;
+  }
+  __syncthreads();
+  const int jt = blockIdx.x * BX + threadIdx.x;
+  const bool in = jt < ns;
+  const int j = in ? jt : ns - 1;
+  const int jm = (j == 0) ? ns - 1 : j - 1, jp = (j == ns - 1) ? 0 : j + 1;
+  const bool edge = threadIdx.x == BX - 1 || j == ns - 1;       // the right neighbour is in another block
+  const double dtc = div_fast(dt, g.k.cv), dtg = dt * io.gm1;
+  const double *T = io.T;
+  double D = io.dcen[j + i0 * ns];
+  double A = (D + io.dcen[j + (i0 - 1) * ns]) * ring[0].ca;     // inner face of ring i
+  double Tm = 0.0, Tl = T[j + i0 * ns], a = 0.0, aj = 0.0;
+  if (RESID) Tm = T[j + (i0 - 1) * ns];
+  for (int i = i0; i < i1; i++) {
+    const MxRing &R = ring[i - i0];
+    const int row = i * ns, l = j + row;
+    const double cs = io.cs[l];
+    const double B = (D + io.dcen[jm + row]) * (cs * R.cb);     // left face
+    double *s = sB[i & 1];
+    s[threadIdx.x] = B;
+    __syncthreads();
+    const double Bp = edge ? (io.dcen[jp + row] + D) * (io.cs[jp + row] * R.cb) : s[threadIdx.x + 1];
+    const double Dn = io.dcen[l + ns];
+    const double Ap = (Dn + D) * ring[i - i0 + 1].ca;           // outer face
+    const double bfac = div_fast(dtc, io.rho[l]);
+    const double afac = bfac * (cs * R.ch);
+    const double bq = bfac * io.qminus[l];
+    const double mip = -(afac * Ap), mim = -(afac * A), mjp = -(bfac * Bp), mjm = -(bfac * B);
+    const double diag = __fma_rn(4.0, bq, __fma_rn(io.divv[l], dtg, 1.0)) - (mip + mim) - (mjp + mjm);
+    double r = __fma_rn(3.0 * bq, Tl, __fma_rn(bfac, io.qplus[l], Tl));
+    if (io.qirr) r = __fma_rn(bfac, io.qirr[l], r);
+    for (int k = 0; k < io.nheat; k++)
+      if (l == io.heat_idx[k]) r = __fma_rn(bfac, io.heat_val[k], r);
+    const double Tn = T[l + ns];
+    if (in) {
+      const size_t q = sor_pidx(i, j, half);
+      io.ml[q] = diag;
+      io.mlip[q] = mip;
+      io.mlim[q] = mim;
+      io.mljp[q] = mjp;
+      io.mljm[q] = mjm;
+      io.rhs[q] = r;
+      if (RESID) {
+        double e = __fma_rn(Tl, diag, -r);
+        e = __fma_rn(Tn, mip, e);
+        e = __fma_rn(Tm, mim, e);
+        e = __fma_rn(T[jp + row], mjp, e);
+        e = __fma_rn(T[jm + row], mjm, e);
+        e = abs_i(e);
+        const double w = div_fast(omega, diag);
+        io.cw[q] = w;
+        a += e;
+        aj = __fma_rn(e, w, aj);
+      }
+    }
+    D = Dn; A = Ap; Tm = Tl; Tl = Tn;
+  }
+  if (RESID) sor_resid_sums(c, a, aj);
 }
 
 // One colour pass of a sweep.  Each cell costs seven FP64 instructions: the
@@ -1343,7 +1456,7 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
                              const double *__restrict__ rmm, const double *__restrict__ tmp_,
                              const double *__restrict__ tmm, double *__restrict__ vr, double *__restrict__ vt, int damp_vrad, double drin, double drout,
                              const double *__restrict__ energy, double *__restrict__ temper, double *__restrict__ cs,
-                             double gm1, double gg1)
+                             double gm1, double gamma)
 {
   const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
   const int ns = g.ns;
@@ -1360,10 +1473,9 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
   vr[l] = v;
   vt[l] = div_fast(tmp_[ljm] + tmm[l], rho[l] + rho[ljm] + 1e-15) * g.r.InvRmed[i] - rm * omega_frame;
   if (temper) {
-    const double r = rho[l], e = energy[l];
-    const double tmp2 = div_fast(1.0, r);
-    temper[l] = e * gm1 * tmp2;
-    cs[l] = sqrt_fast(gg1 * fabs(e) * tmp2);
+    const double t = div_fast(energy[l] * gm1, rho[l]);
+    temper[l] = t;
+    cs[l] = sqrt_fast(gamma * abs_i(t));
   }
 }
 
@@ -1416,19 +1528,23 @@ void hydro_qplus(const DevGrid &g, const double *vr, const double *vt, const dou
 void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double *temper, double *cs, double gm1,
                double gg1, cudaStream_t s)
 {
-  k_eos<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, energy, temper, cs, gm1, gg1);
+  k_eos<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, energy, temper, cs, gm1, gg1 / gm1);
   g_thorin_launches++;
 }
 
-int hydro_diffcoef_blocks(const DevGrid &g) { return ((g.ns + BX - 1) / BX) * g.nr; }
-
-void hydro_diffcoef(const DevGrid &g, const double *rho, const double *T, const double *cs, double *opacity,
-                    double *qminus, double *dcen, double *dtmin_part, int law, double parametric_cu,
-                    double parametric_raw, double opacity_drop, double taueff_c, const double *invdxtheta_r,
-                    const double *deltar2_r, cudaStream_t s)
+void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io0, int law, cudaStream_t s)
 {
-  k_diffcoef<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, T, cs, opacity, qminus, dcen, dtmin_part, law, parametric_cu,
-                                                   parametric_raw, opacity_drop, taueff_c, invdxtheta_r, deltar2_r);
+  DiffusionIO io = io0;
+  // 0.2 rings a chunk: the difference with the ring below and the ring constants
+  io.rings = chunk_rings(g.nr, g.ns, g.nsm, DC_MAXRINGS, 0.2, 8);
+  const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
+  switch (law) {
+  case THORIN_OPA_SM03: k_diffcoef<THORIN_OPA_SM03><<<grid, BX, 0, s>>>(g, io); break;
+  case THORIN_OPA_ZHU12: k_diffcoef<THORIN_OPA_ZHU12><<<grid, BX, 0, s>>>(g, io); break;
+  case THORIN_OPA_LP85: k_diffcoef<THORIN_OPA_LP85><<<grid, BX, 0, s>>>(g, io); break;
+  case THORIN_OPA_CONST: k_diffcoef<THORIN_OPA_CONST><<<grid, BX, 0, s>>>(g, io); break;
+  default: k_diffcoef<THORIN_OPA_BL94><<<grid, BX, 0, s>>>(g, io); break;
+  }
   g_thorin_launches++;
 }
 
@@ -1441,19 +1557,24 @@ void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, co
   g_thorin_launches++;
 }
 
-void hydro_matrix(const DevGrid &g, const double *rho, const double *T, const double *cs, const double *dcen,
-                  const double *divv, const double *qminus, const double *qplus, const double *qirr, double *ml,
-                  double *mlip, double *mlim, double *mljp, double *mljm, double *rhs,
-                  double gm1, const double *invdxtheta2_r, int irradiation, int nheat, const int *heat_idx,
-                  const double *heat_val, cudaStream_t s)
+// Rings per block of k_matrix; 0.3 rings a chunk are the first face and the
+// ring constants.
+static int matrix_rings(const DevGrid &g) { return chunk_rings(g.nr - 2, g.ns, g.nsm, MX_MAXRINGS, 0.3); }
+
+static dim3 matrix_grid(const DevGrid &g)
 {
-  if (g.nr < 3) return;
-  k_matrix<<<grid2d(g.ns, g.nr - 2, BX), BX, 0, s>>>(g, rho, T, cs, dcen, divv, qminus, qplus, qirr, ml, mlip, mlim, mljp,
-                                                     mljm, rhs, gm1, invdxtheta2_r, irradiation, nheat, heat_idx,
-                                                     heat_val);
-  g_thorin_launches++;
+  const int r = matrix_rings(g);
+  return dim3((g.ns + BX - 1) / BX, (g.nr - 2 + r - 1) / r);
 }
 
+void hydro_matrix(const DevGrid &g, const MatrixIO &io0, const SorCtl *resid, cudaStream_t s)
+{
+  MatrixIO io = io0;
+  io.rings = matrix_rings(g);
+  if (resid) k_matrix<true><<<matrix_grid(g), BX, 0, s>>>(g, io, *resid);
+  else k_matrix<false><<<matrix_grid(g), BX, 0, s>>>(g, io, SorCtl{});
+  g_thorin_launches++;
+}
 
 // Resident k_sor_pass blocks per multiprocessor that fit (occupancy API),
 // found once.
@@ -1488,9 +1609,9 @@ static dim3 sor_grid_resid(const DevGrid &g)
 
 int sor_blocks(const DevGrid &g)
 {
-  const dim3 a = sor_grid_pass(g, false), b = sor_grid_resid(g);
-  const int na = a.x * a.y, nb = b.x * b.y;
-  return na > nb ? na : nb;
+  const dim3 a = sor_grid_pass(g, false), b = sor_grid_resid(g), c = matrix_grid(g);
+  const int na = a.x * a.y, nb = b.x * b.y, nc = c.x * c.y;
+  return na > nb ? (na > nc ? na : nc) : (nb > nc ? nb : nc);
 }
 
 void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const double *mlip, const double *mlim,
@@ -1577,7 +1698,7 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
   g_thorin_launches++;
   // velocities from the transported momenta
   k_velocities<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,
-                                                 energy ? S.e_new : nullptr, energy ? temper : nullptr, cs, gm1, gg1);
+                                                 energy ? S.e_new : nullptr, energy ? temper : nullptr, cs, gm1, gg1 / gm1);
   g_thorin_launches++;
   if (label) {
     k_label_from_ext<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, S.rho_new, S.ext_new, label);

@@ -1542,13 +1542,16 @@ static int sor_loop_graph(thorin_disk *d)
 
 // SuccessiveOverrelaxation driver: the start residual (and the learned warm
 // start), then the sweep loop graph; one read of the exit state per solve.
-static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool learned = false)
+// started: the matrix kernel has formed the start residual at this omega.
+static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool learned = false, bool started = false)
 {
   // normres0 and the threshold always come from the start temperature as
   // the reference has it; a learned start only moves T before the sweeps
-  set_ctl(d, {{CTL_SOR_OMEGA, omega}});
-  hydro_sor_resid0(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor, d->s);
-  KCHECK("SOR residual kernel");
+  if (!started) {
+    set_ctl(d, {{CTL_SOR_OMEGA, omega}});
+    hydro_sor_resid0(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor, d->s);
+    KCHECK("SOR residual kernel");
+  }
   if (learned && d->ws_net && d->ws_mode == THORIN_WS_PREDICT) {
     // keep the start (for the update record after the solve), then move it
     CUCHK(cudaMemcpyAsync(d->tbackup, d->temper, (size_t)d->nr * d->ns * sizeof(double), cudaMemcpyDeviceToDevice,
@@ -1657,10 +1660,14 @@ static int energy_step(thorin_disk *d, double dt)
     return THORIN_ERR_STATE;
   }
   hydro_eos(d->g, d->rho, d->energy_int, d->temper, d->cs, d->gm1, d->gg1, d->s);
-  hydro_diffcoef(d->g, d->rho, d->temper, d->cs, d->opacity, d->qminus, d->dcen, d->partials, p.opacity_law,
-                 p.parametric_opacity * OPA2CU, p.parametric_opacity, p.opacity_drop, d->taueff_c,
-                 d->ring[R_INVDXTHETA], d->ring[R_DELTAR2], d->s);
-  aux_min_final(d->partials, hydro_diffcoef_blocks(d->g), d->scal + SC_DTSTELLAR, d->s);
+  DiffusionIO dif = {};
+  dif.rho = d->rho; dif.T = d->temper; dif.cs = d->cs;
+  dif.invdxtheta = d->ring[R_INVDXTHETA]; dif.deltar2 = d->ring[R_DELTAR2];
+  dif.opacity = d->opacity; dif.qminus = d->qminus; dif.dcen = d->dcen;
+  dif.part = d->partials; dif.dtmin = d->scal + SC_DTSTELLAR; dif.ticket = d->ticket + 9;
+  dif.parametric_cu = p.parametric_opacity * OPA2CU;
+  dif.opacity_drop = p.opacity_drop; dif.taueff_c = d->taueff_c;
+  hydro_diffcoef(d->g, dif, p.parametric_opacity > 0.0 ? THORIN_OPA_CONST : p.opacity_law, d->s);
   if (p.stellar_irradiation)
     hydro_irradiation(d->g, d->rho, d->cs, d->opacity, d->flaring, d->qirr, d->rstar, d->tirr4fac, p.opacity_drop,
                       d->taueff_c, d->ring[R_RINF15], d->ring[R_RSUP15], d->s);
@@ -1674,18 +1681,29 @@ static int energy_step(thorin_disk *d, double dt)
       CUCHK(cudaMemcpyAsync(d->heat_val_d, d->heatsrc, nheat * sizeof(double), cudaMemcpyHostToDevice, d->s));
     }
   }
-  hydro_matrix(d->g, d->rho, d->temper, d->cs, d->dcen, d->divv, d->qminus, d->qplus, d->qirr, d->ml, d->mlip, d->mlim,
-               d->mljp, d->mljm, d->rhs, d->gm1, d->ring[R_INVDXTHETA2], p.stellar_irradiation, nheat,
-               d->heat_idx_d, d->heat_val_d, d->s);
-  KCHECK("energy kernels");
+  MatrixIO mx = {};
+  mx.rho = d->rho; mx.T = d->temper; mx.cs = d->cs; mx.dcen = d->dcen; mx.divv = d->divv;
+  mx.qminus = d->qminus; mx.qplus = d->qplus; mx.qirr = p.stellar_irradiation ? d->qirr : nullptr;
+  mx.invdxtheta2 = d->ring[R_INVDXTHETA2];
+  mx.ml = d->ml; mx.mlip = d->mlip; mx.mlim = d->mlim; mx.mljp = d->mljp; mx.mljm = d->mljm; mx.rhs = d->rhs;
+  mx.cw = d->sor_cw;
+  mx.heat_idx = d->heat_idx_d; mx.heat_val = d->heat_val_d; mx.gm1 = d->gm1; mx.nheat = nheat;
   if (d->capturing) {                  // device-resident DT: schedule, solve loop and counters on the device
+    graph_sor_begin(d->capS, d->s);
+    hydro_matrix(d->g, mx, &d->sor, d->s);
+    KCHECK("energy kernels");
     RCHK(capture_sor(d));
     hydro_energy_from_t(d->g, d->rho, d->temper, d->energy_new, d->s);
     std::swap(d->energy, d->energy_new);
     return THORIN_OK;
   }
-  if (d->sor_first) {
+  // the omega schedule's next step is known before the matrix, which then
+  // starts the solve; a disk's first solve calibrates omega on the matrix
+  const bool first = d->sor_first;
+  if (first) {
     d->sor_first = 0;
+    hydro_matrix(d->g, mx, nullptr, d->s);
+    KCHECK("energy kernels");
     RCHK(iterate_relaxation(d));
     d->omega = d->omegabest;
     d->Niterlast = d->Niterbest;
@@ -1693,11 +1711,16 @@ static int energy_step(thorin_disk *d, double dt)
   d->omega += d->domega;
   if (d->omega > TH_OMEGAUPPER) { d->omega = TH_OMEGAUPPER; d->domega = -d->domega; }
   if (d->omega < 1.0) { d->omega = 1.0; d->domega = -d->domega; }
+  if (!first) {
+    set_ctl(d, {{CTL_SOR_OMEGA, d->omega}});
+    hydro_matrix(d->g, mx, &d->sor, d->s);
+    KCHECK("energy kernels");
+  }
   int Niter, capped;
   const bool train = d->ws_net && d->ws_mode == THORIN_WS_TRAIN;
   const size_t tbytes = (size_t)d->nr * d->ns * sizeof(double);
   if (train) CUCHK(cudaMemcpyAsync(d->tbackup, d->temper, tbytes, cudaMemcpyDeviceToDevice, d->s));
-  RCHK(sor_solve(d, d->omega, &Niter, &capped, true));
+  RCHK(sor_solve(d, d->omega, &Niter, &capped, true, !first));
   if (train) {
     // fit the network to this solve; energy_new is free until the energy is formed below
     RCHK(wn_sor_train(d->ws_net, d->nr, d->ns, d->ws_f, d->tbackup, d->temper, d->ml, d->mlip, d->mlim, d->mljp,
@@ -2056,14 +2079,12 @@ extern "C" int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys)
 // started in.  The first DT of a disk (omega calibration) runs on the host
 // path; planets are kept on the device for the DT.
 
-// Inserts the SOR sweep loop into the capture: the omega schedule, the start
-// residual, a WHILE node whose body (captured later into d->capS) holds the
-// sweeps, then the counters.
+// Inserts the SOR sweep loop into the capture, after the omega schedule and
+// the matrix with the start residual: the warm start, a WHILE node whose body
+// (captured later into d->capS) holds the sweeps, then the counters.
 static int capture_sor(thorin_disk *d)
 {
   StepDev &S = d->capS;
-  graph_sor_begin(S, d->s);
-  hydro_sor_resid0(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor, d->s);
   const bool predict = d->ws_net && d->ws_mode == THORIN_WS_PREDICT;
   const bool extrap = d->ws_mode == THORIN_WS_EXTRAPOLATE;
   if (predict || extrap) {  // the warm start moves T before the sweeps, as on the host path

@@ -398,10 +398,26 @@ __device__ __forceinline__ double rsqrt_fast(double x)
   return rsqrt(x);
 }
 
+// y (1 + rel) for |rel| below 2^-40: rel in units of y's last place, rounded to
+// an integer and added to y's bits (formed in FP32, to 2^-8 of an ulp).
+__device__ __forceinline__ double nudge(double y, float rel)
+{
+  const float mf = __int_as_float(0x3f800000 | ((__double2hiint(y) & 0x000fffff) << 3));
+  const int k = __float2int_rn(rel * mf * 4503599627370496.0f);          // 2^52
+  return __longlong_as_double(__double_as_longlong(y) + (long long)k);
+}
+
+// FP32 value of x, truncated, 0 below 2^-111 in size (x below 2^100).
+__device__ __forceinline__ float small_to_float(double x)
+{
+  const int H = __double2hiint(x), M = H & 0x7fffffff;
+  const float f = __int_as_float(__funnelshift_l(__double2loint(x), M - 0x38000000, 3) | (H & 0x80000000));
+  return (M < 0x39000000) ? 0.0f : f;
+}
+
 // x^(-3/2), x > 0, in three FP64 instructions: y from rsqrt_est, y^2 and y^3
-// as rounded products, and the factor 1 + 3/2 (1 - x y^2) as an integer added
-// to the bits of y^3 (below 2^12 ulp, formed in FP32 to a 2^-8th of an ulp;
-// the residual 1 - x y^2 is exact).  Within 2 ulp; the cube of a rounded
+// as rounded products, and the factor 1 + 3/2 (1 - x y^2) by nudge (the
+// residual 1 - x y^2 is exact).  Within 2 ulp; the cube of a rounded
 // reciprocal square root, five instructions, was within 5.
 __device__ __forceinline__ double pow_m32(double x)
 {
@@ -410,15 +426,29 @@ __device__ __forceinline__ double pow_m32(double x)
     const double y2 = y * y;
     const double e = __fma_rn(-x, y2, 1.0);
     const double y3 = y2 * y;
-    const int H = __double2hiint(e), M = H & 0x7fffffff;
-    const float ef = (M < 0x39000000) ? 0.0f       // below 2^-111
-                                      : __int_as_float(__funnelshift_l(__double2loint(e), M - 0x38000000, 3) |
-                                                       (H & 0x80000000));
-    const float mf = __int_as_float(0x3f800000 | ((__double2hiint(y3) & 0x000fffff) << 3));
-    const int k = __float2int_rn(ef * mf * 6755399441055744.0f);       // 1.5 * 2^52
-    return __longlong_as_double(__double_as_longlong(y3) + (long long)k);
+    return nudge(y3, 1.5f * small_to_float(e));
   }
   return 1.0 / (x * sqrt(x));
+}
+
+// x^(1/4), x > 0, in two FP64 instructions: q from two reciprocal square root
+// estimates, and the factor 1 + (x - q^4) / (4 x) by nudge.  Within an ulp.
+__device__ __forceinline__ double root4(double x)
+{
+  if (exp_ok(x) && __double2hiint(x) > 0) {
+    const double q = rsqrt_est(rsqrt_est(x));
+    const double q2 = q * q;
+    const double e = __fma_rn(-q2, q2, x);
+    // e / x from the two's own exponents: both scaled by x's power of two
+    const int sh = (__double2hiint(x) & 0x7ff00000) - 0x3ff00000;
+    const float xf = __int_as_float(0x3f800000 | ((__double2hiint(x) & 0x000fffff) << 3));
+    const int He = __double2hiint(e), Me = (He & 0x7fffffff) - sh;         // e 2^-E
+    const float ef = (Me < 0x39000000 || (He & 0x7ff00000) == 0)
+                         ? 0.0f
+                         : __int_as_float(__funnelshift_l(__double2loint(e), Me - 0x38000000, 3) | (He & 0x80000000));
+    return nudge(q, 0.25f * __fdividef(ef, xf));
+  }
+  return sqrt(sqrt(x));
 }
 
 // r / (r + 1e-20), the density's own transported quotient (the reference
@@ -497,4 +527,13 @@ __device__ __forceinline__ double exp_fast(double x, const double *tab)
     return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
   }
   return exp(x);
+}
+
+// FP32 value of a positive double of moderate exponent, truncated (0 outside
+// [2^-100, 2^100]).
+__device__ __forceinline__ float to_float_pos(double x)
+{
+  const int H = __double2hiint(x);
+  const float f = __int_as_float(__funnelshift_l(__double2loint(x), H - 0x38000000, 3));
+  return (unsigned)(H - (923 << 20)) < (unsigned)(200 << 20) ? f : 0.0f;
 }

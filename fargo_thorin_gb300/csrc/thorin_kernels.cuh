@@ -61,6 +61,25 @@ struct SourceIO {
   int back_reaction, diffusion, rings;
 };
 
+// Arguments of the opacity and diffusion coefficient step.
+struct DiffusionIO {
+  const double *rho, *T, *cs, *invdxtheta, *deltar2;
+  double *opacity, *qminus, *dcen, *part, *dtmin;   // dtmin: DiffusionTimestep's result
+  unsigned int *ticket;
+  double parametric_cu, opacity_drop, taueff_c;
+  int rings;
+};
+
+// Arguments of the implicit energy equation's matrix (qirr NULL: no irradiation).
+struct MatrixIO {
+  const double *rho, *T, *cs, *dcen, *divv, *qminus, *qplus, *qirr, *invdxtheta2;
+  double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *cw;
+  const int *heat_idx;
+  const double *heat_val;
+  double gm1;
+  int nheat, rings;
+};
+
 struct AziIO { const double *src[7]; double *dst[7]; int n; };   // index n-1 is the density
 
 struct ViscParams {
@@ -145,19 +164,12 @@ void hydro_qplus(const DevGrid &g, const double *vr, const double *vt, const dou
                  double invdphi, double lr01, double lr12, cudaStream_t s);
 void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double *temper, double *cs, double gm1,
                double gg1, cudaStream_t s);
-int hydro_diffcoef_blocks(const DevGrid &g);
-void hydro_diffcoef(const DevGrid &g, const double *rho, const double *T, const double *cs, double *opacity,
-                    double *qminus, double *dcen, double *dtmin_part, int law, double parametric_cu,
-                    double parametric_raw, double opacity_drop, double taueff_c, const double *invdxtheta_r,
-                    const double *deltar2_r, cudaStream_t s);
+void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io, int law, cudaStream_t s);
 void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, const double *opacity, double *flaring,
                        double *qirr, double rstar, double tirr4fac, double opacity_drop, double taueff_c,
                        const double *rinf15, const double *rsup15, cudaStream_t s);
-void hydro_matrix(const DevGrid &g, const double *rho, const double *T, const double *cs, const double *dcen,
-                  const double *divv, const double *qminus, const double *qplus, const double *qirr, double *ml,
-                  double *mlip, double *mlim, double *mljp, double *mljm, double *rhs,
-                  double gm1, const double *invdxtheta2_r, int irradiation, int nheat, const int *heat_idx,
-                  const double *heat_val, cudaStream_t s);
+// resid: also the start of the SOR solve (NULL: the matrix alone)
+void hydro_matrix(const DevGrid &g, const MatrixIO &io, const SorCtl *resid, cudaStream_t s);
 int sor_blocks(const DevGrid &g);
 void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const double *mlip, const double *mlim,
                       const double *mljp, const double *mljm, const double *rhs, double *cw,
@@ -221,4 +233,3 @@ int aux_accrete_blocks(const DevGrid &g, int imin, int imax);
 void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *e,
                    const double *pd, const double *pvt, double omega_frame, int pebbles, double *part, double *scal,
                    cudaStream_t s);
-void aux_min_final(const double *part, int nb, double *out, cudaStream_t s);
