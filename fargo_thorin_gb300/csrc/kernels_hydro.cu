@@ -177,154 +177,236 @@ __global__ void __launch_bounds__(BX) k_sources(DevGrid g, SourceIO io)
 }
 
 // UpdateDivVelocAndStressTensor (Viscosity.c:85-162): divergence and the
-// three stress components at cell l from the staggered velocities.
+// three stress components of a cell from the staggered velocities, with the
+// ring's constants folded into its coefficients.
+struct StressRing { double cr, cp, cv, rsup, rinf, cd, nu2, t1, t2; };
+
+__device__ __forceinline__ void stress_ring(const DevGrid &g, int i, double invdphi, StressRing &R)
+{
+  const double ir = g.r.InvRmed[i];
+  R.cr = g.r.InvDiffRsup[i];
+  R.cp = invdphi * ir;                       // (v_theta(j+1) - v_theta(j)) cp
+  R.cv = 0.5 * ir;                           // (v_r(i+1) + v_r(i)) cv
+  R.rsup = g.r.Rsup[i];
+  R.rinf = g.r.Rinf[i];
+  R.cd = R.cr * ir;
+  R.nu2 = 2.0 * g.r.nu_med[i];
+  // tau_rp = 2 rho_4/4 nu (r dOmega/dr + (v_r(j) - v_r(j-1)) / (r dphi)) / 2
+  const double n = 0.25 * g.r.nu_inf[i];
+  R.t1 = n * g.r.Rinf[i] * g.r.InvDiffRmed[i];
+  R.t2 = n * invdphi * g.r.InvRinf[i];
+}
+
 struct Stress { double divv, trr, tpp, trp; };
 
-__device__ __forceinline__ Stress stress_at(const DevGrid &g, const double *vr, const double *vt, const double *rho,
-                                            int i, int j, double invdphi)
+// om, om_m: v_theta / r of the cell and of the one below; rs, rs_m: the
+// densities of the cell and its left neighbour added, and those below.
+__device__ __forceinline__ Stress stress_cell(const StressRing &R, int i, double vr, double vr_ip, double vr_jm,
+                                              double vt, double vt_jp, double om, double om_m, double rho, double rs,
+                                              double rs_m)
 {
-  const int ns = g.ns, l = j + i * ns, lip = l + ns;
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const double onethird = 1.0 / 3.0;
   Stress s;
-  double Drr = (vr[lip] - vr[l]) * g.r.InvDiffRsup[i];
-  double Dpp = (vt[ljp] - vt[l]) * invdphi * g.r.InvRmed[i] + 0.5 * (vr[lip] + vr[l]) * g.r.InvRmed[i];
-  double dv = (vr[lip] * g.r.Rsup[i] - vr[l] * g.r.Rinf[i]) * g.r.InvDiffRsup[i] * g.r.InvRmed[i];
-  dv += (vt[ljp] - vt[l]) * invdphi * g.r.InvRmed[i];
-  s.divv = dv;
-  const double nu = g.r.nu_med[i];
-  s.trr = 2.0 * rho[l] * nu * (Drr - onethird * dv);
-  s.tpp = 2.0 * rho[l] * nu * (Dpp - onethird * dv);
-  if (i >= 1) {
-    const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1, lim = l - ns, ljmim = ljm - ns;
-    double Drp = 0.5 * (g.r.Rinf[i] * (vt[l] * g.r.InvRmed[i] - vt[lim] * g.r.InvRmed[i - 1]) * g.r.InvDiffRmed[i] +
-                        (vr[l] - vr[ljm]) * invdphi * g.r.InvRinf[i]);
-    s.trp = 2.0 * 0.25 * (rho[l] + rho[lim] + rho[ljm] + rho[ljmim]) * g.r.nu_inf[i] * Drp;
-  } else {
-    s.trp = 0.0;
-  }
+  const double dt = (vt_jp - vt) * R.cp;
+  const double Drr = (vr_ip - vr) * R.cr;
+  const double Dpp = __fma_rn(vr_ip + vr, R.cv, dt);
+  s.divv = __fma_rn(__fma_rn(vr_ip, R.rsup, -(vr * R.rinf)), R.cd, dt);
+  const double n = R.nu2 * rho;
+  s.trr = n * __fma_rn(-1.0 / 3.0, s.divv, Drr);
+  s.tpp = n * __fma_rn(-1.0 / 3.0, s.divv, Dpp);
+  s.trp = (i >= 1) ? (rs + rs_m) * __fma_rn(vr - vr_jm, R.t2, (om - om_m) * R.t1) : 0.0;
   return s;
 }
 
-__global__ void k_stress(DevGrid g, const double *__restrict__ vr, const double *__restrict__ vt,
-                         const double *__restrict__ rho, double *__restrict__ divv, double *__restrict__ trr,
-                         double *__restrict__ tpp, double *__restrict__ trp, double invdphi)
-{
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  Stress s = stress_at(g, vr, vt, rho, i, j, invdphi);
-  divv[l] = s.divv;
-  trr[l] = s.trr;
-  tpp[l] = s.tpp;
-  trp[l] = s.trp;
-}
+// The viscous terms and SubStep2 in one kernel: the stress tensor,
+// UpdateVelocityWithViscousTerms (Viscosity.c:165-218), ImposeKeplerianEdges
+// (:221-260) and the von Neumann-Richtmyer artificial viscosity with its
+// velocity and energy updates (SourceEuler.c:417-504).
+//
+// A thread walks the rings of a column; at ring k it forms the stress of ring
+// k, v_r of ring k, v_theta of ring k-1 and writes ring k-1.  Neighbours in
+// azimuth pass stress, v_theta and the artificial pressure through shared
+// memory, so a block of 128 threads covers 125 columns (two on the left and one
+// on the right only feed their neighbours).  The sums of densities and their reciprocals are
+// shared by both parts.  FP64-bound: about 58 FP64 instructions a cell plus 1.8
+// rings a chunk, where the three kernels took 103 and kept three fields between
+// them; 512x1536: 166 -> 133 us.
+#define VI_MAXRINGS 40
+#define VI_COLS (BX - 3)
 
-// UpdateVelocityWithViscousTerms (Viscosity.c:165-218) and
-// ImposeKeplerianEdges (Viscosity.c:221-260).
-__global__ void k_visc_update(DevGrid g, double *__restrict__ vr, double *__restrict__ vt,
-                              const double *__restrict__ rho, const double *__restrict__ trr,
-                              const double *__restrict__ tpp, const double *__restrict__ trp,
-                              double invdphi, int kepler_edges, double vkep_in, double vkep_out)
+struct ViscRing { StressRing s; double irm, a, b, c, ra, rm, rc, rt, sr, st, er, et; };
+
+__global__ void __launch_bounds__(BX) k_viscous(DevGrid g, ViscousIO io)
 {
+  __shared__ ViscRing ring[VI_MAXRINGS + 3];
+  __shared__ double s_tpp[2][BX], s_trp[2][BX], s_vt[BX], s_q[BX];
   const double dt = g.ctl[CTL_DT];
   const int ns = g.ns, nr = g.nr;
-  CELL_LOOP_2D
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  if (i >= 1 && i < nr - 1) {
-    const int lip = l + ns;
-    vt[l] += div_fast(dt * g.r.InvRmed[i] *
-                          ((g.r.Rsup[i] * trp[lip] - g.r.Rinf[i] * trp[l]) * g.r.InvDiffRsup[i] +
-                           (tpp[l] - tpp[ljm]) * invdphi + 0.5 * (trp[l] + trp[lip])),
-                      0.5 * (rho[l] + rho[ljm]));
+  const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
+  const int k0 = max(i0 - 2, 0);
+  for (int q = threadIdx.x; q <= min(i1, nr - 1) - k0; q += BX) {
+    const int i = k0 + q;
+    ViscRing &R = ring[q];
+    stress_ring(g, i, io.invdphi, R.s);
+    R.irm = g.r.InvRmed[i];
+    // v_theta += 2 dt / r (...) / (rho + rho_jm), v_r += 2 dt / r (...) / (rho + rho_im)
+    const double ct = 2.0 * dt * g.r.InvRmed[i], cr = 2.0 * dt * g.r.InvRinf[i];
+    R.a = ct * __fma_rn(g.r.Rsup[i], g.r.InvDiffRsup[i], 0.5);            // tau_rp(i+1)
+    R.b = ct * __fma_rn(-g.r.Rinf[i], g.r.InvDiffRsup[i], 0.5);           // tau_rp(i)
+    R.c = ct * io.invdphi;                                                // tau_pp - tau_pp(j-1)
+    R.ra = cr * g.r.Rmed[i] * g.r.InvDiffRmed[i];                         // tau_rr
+    R.rm = (i >= 1) ? -(cr * g.r.Rmed[i - 1] * g.r.InvDiffRmed[i]) : 0.0; // tau_rr(i-1)
+    R.rc = cr * io.invdphi;                                               // tau_rp(j+1) - tau_rp
+    R.rt = -0.5 * cr;                                                     // tau_pp + tau_pp(i-1)
+    R.sr = -2.0 * dt * g.r.InvDiffRmed[i];                                // q_r - q_r(i-1)
+    R.st = -2.0 * dt * io.invdxtheta[i];                                  // q_t - q_t(j-1)
+    R.er = -dt * g.r.InvDiffRsup[i];
+    R.et = -dt * io.invdxtheta[i];
   }
-  if (i >= 1) {
-    const int lim = l - ns;
-    vr[l] += div_fast(dt * g.r.InvRinf[i] *
-                          ((g.r.Rmed[i] * trr[l] - g.r.Rmed[i - 1] * trr[lim]) * g.r.InvDiffRmed[i] +
-                           (trp[ljp] - trp[l]) * invdphi - 0.5 * (tpp[l] + tpp[lim])),
-                      0.5 * (rho[l] + rho[lim]));
+  __syncthreads();
+  const int t = threadIdx.x, x = blockIdx.x * VI_COLS + t - 2;
+  const bool out = t >= 2 && t < BX - 1 && x < ns;
+  int j = x;                                       // wrapped column (ns >= 4)
+  if (j < 0) j += ns;
+  j %= ns;
+  const int jm = (j == 0) ? ns - 1 : j - 1, jp = (j == ns - 1) ? 0 : j + 1;
+  const int tm = (t == 0) ? 0 : t - 1, tp = (t == BX - 1) ? t : t + 1;
+  // of ring k-1: stress, rotation rate, density sums, old v_theta; of ring k-1 and k-2 after the viscous update
+  double trr_m = 0.0, tpp_m = 0.0, trp_m = 0.0, dtp_m = 0.0, om_m = 0.0, rs_m = 0.0, rho_m = 0.0, vt_m = 0.0;
+  double vr_m = 0.0, qr_m = 0.0, ir_m = 0.0;
+  if (k0 > 0) {
+    const int l = j + (k0 - 1) * ns;
+    om_m = io.vt[l] * g.r.InvRmed[k0 - 1];
+    rho_m = io.rho[l];
+    rs_m = rho_m + io.rho[jm + (k0 - 1) * ns];
   }
-  if (kepler_edges) {
-    if (i == 0) vt[l] = vkep_in;
-    if (i == nr - 1) vt[l] = vkep_out;
-  }
-}
-
-// SubStep2 (SourceEuler.c:417-504): von Neumann-Richtmyer artificial
-// viscosity, velocity and energy updates.  q_r, q_theta are recomputed at
-// the neighbouring cells instead of being stored.
-__device__ __forceinline__ double avisc(double dv, double rho)
-{
-  return (dv < 0.0) ? TH_CVNR * TH_CVNR * rho * dv * dv : 0.0;
-}
-
-__global__ void k_substep2(DevGrid g, const double *__restrict__ rho, const double *__restrict__ vr,
-                           const double *__restrict__ vt, const double *__restrict__ energy,
-                           double *__restrict__ vrnew, double *__restrict__ vtnew, double *__restrict__ eint, int energy_eq, const double *__restrict__ invdxtheta_r)
-{
-  const double dt = g.ctl[CTL_DT];
-  const int ns = g.ns, nr = g.nr;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  if (j >= ns) return;
-  const int l = j + i * ns;
-  if (i == nr) {                       // rows the reference never writes stay zero
-    vrnew[l] = 0.0;
-    vtnew[l] = 0.0;
-    return;
-  }
-  const int lip = l + ns;
-  const int ljp = (j == ns - 1) ? i * ns : l + 1;
-  const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-  const double qr = avisc(vr[lip] - vr[l], rho[l]);
-  const double qt = avisc(vt[ljp] - vt[l], rho[l]);
-  if (i >= 1) {
-    const int lim = l - ns;
-    const double qrm = avisc(vr[l] - vr[lim], rho[lim]);
-    vrnew[l] = vr[l] - div_fast(dt * 2.0, rho[l] + rho[lim]) * (qr - qrm) * g.r.InvDiffRmed[i];
-  } else {
-    vrnew[l] = 0.0;
-  }
-  const double invdxtheta = invdxtheta_r[i];
-  const double qtm = avisc(vt[l] - vt[ljm], rho[ljm]);
-  vtnew[l] = vt[l] - div_fast(dt * 2.0, rho[l] + rho[ljm]) * (qt - qtm) * invdxtheta;
-  if (energy_eq)
-    eint[l] = energy[l] - dt * qr * (vr[lip] - vr[l]) * g.r.InvDiffRsup[i] - dt * qt * (vt[ljp] - vt[l]) * invdxtheta;
-}
-
-// SubStep3 viscous heating (SourceEuler.c:541-554) from the stress of the
-// updated velocities (the second UpdateDivVelocAndStressTensor call,
-// SourceEuler.c:302).
-__global__ void k_qplus(DevGrid g, const double *__restrict__ vr, const double *__restrict__ vt,
-                        const double *__restrict__ rho, double *__restrict__ divv, double *__restrict__ qplus,
-                        double invdphi)
-{
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  Stress s = stress_at(g, vr, vt, rho, i, j, invdphi);
-  divv[l] = s.divv;
-  if (i >= 1) {
-    const double nu = g.r.nu_med[i];
-    double q;
-    if (nu != 0.0) {
-      q = div_fast(0.5, nu * rho[l]) * (s.trr * s.trr + 2.0 * s.trp * s.trp + s.tpp * s.tpp);
-      q += (2.0 / 9.0) * nu * rho[l] * s.divv * s.divv;
-    } else {
-      q = 0.0;
+  double vr = io.vr[j + k0 * ns];
+  const int k1 = i1;                               // ring k1 closes ring i1 - 1
+  for (int k = k0; k <= k1; k++) {
+    const int row = k * ns, l = j + row;
+    const bool body = k < nr;
+    double trr = 0.0, tpp = 0.0, trp = 0.0, om = 0.0, rs = 0.0, rho = 0.0, vt = 0.0, vr_ip = 0.0;
+    if (body) {
+      const ViscRing &R = ring[k - k0];
+      vr_ip = io.vr[l + ns];
+      vt = io.vt[l];
+      rho = io.rho[l];
+      rs = rho + io.rho[jm + row];
+      om = vt * R.irm;
+      const Stress s = stress_cell(R.s, k, vr, vr_ip, io.vr[jm + row], vt, io.vt[jp + row], om, om_m, rho, rs, rs_m);
+      trr = s.trr; tpp = s.tpp; trp = s.trp;
+      if (io.divv && out && k >= i0 && k < i1) io.divv[l] = s.divv;
     }
-    qplus[l] = q;
+    s_tpp[k & 1][t] = tpp;
+    s_trp[k & 1][t] = trp;
+    __syncthreads();
+    // v_r of ring k
+    double vrn = vr, ir = 0.0;
+    if (body && k >= 1) {
+      const ViscRing &R = ring[k - k0];
+      ir = div_fast(1.0, rho + rho_m);
+      const double w = __fma_rn(trr, R.ra, __fma_rn(trr_m, R.rm, __fma_rn(s_trp[k & 1][tp] - trp, R.rc, (tpp + tpp_m) * R.rt)));
+      vrn = __fma_rn(w, ir, vr);
+    }
+    // v_theta of ring k-1, then SubStep2 of ring k-1
+    const int m = k - 1;
+    if (m >= i0 - 1 && m >= k0) {
+      const ViscRing &R = ring[m - k0];
+      double vtn = vt_m, it = 0.0;
+      if (m >= i0) {
+        it = div_fast(1.0, rs_m);
+        if (m >= 1 && m < nr - 1) {
+          const double w = __fma_rn(trp, R.a, __fma_rn(trp_m, R.b, dtp_m * R.c));
+          vtn = __fma_rn(w, it, vt_m);
+        }
+        if (io.kepler) {
+          if (m == 0) vtn = io.vkep_in;
+          if (m == nr - 1) vtn = io.vkep_out;
+        }
+      }
+      const double dvr = vrn - vr_m;
+      const double cq = (TH_CVNR * TH_CVNR) * rho_m;
+      const double qr = (__double_as_longlong(dvr) < 0LL) ? cq * dvr * dvr : 0.0;
+      if (m >= i0) {                               // block-uniform
+        s_vt[t] = vtn;
+        __syncthreads();
+        const double dvt = s_vt[tp] - vtn;
+        const double qt = (__double_as_longlong(dvt) < 0LL) ? cq * dvt * dvt : 0.0;
+        s_q[t] = qt;
+        __syncthreads();
+        if (out) {
+          const int lm = l - ns;
+          io.vrnew[lm] = (m >= 1) ? __fma_rn((qr - qr_m) * ir_m, R.sr, vr_m) : 0.0;
+          io.vtnew[lm] = __fma_rn((qt - s_q[tm]) * it, R.st, vtn);
+          if (io.eint) io.eint[lm] = __fma_rn(qt * dvt, R.et, __fma_rn(qr * dvr, R.er, io.energy[lm]));
+        }
+      }
+      qr_m = qr;
+    }
+    dtp_m = tpp - s_tpp[k & 1][tm];
+    trr_m = trr; tpp_m = tpp; trp_m = trp; om_m = om; rs_m = rs; rho_m = rho; vt_m = vt;
+    vr_m = vrn;
+    ir_m = ir;
+    vr = vr_ip;
+  }
+  if (i1 == nr && out) {                           // rows the reference never writes stay zero
+    io.vrnew[j + nr * ns] = 0.0;
+    io.vtnew[j + nr * ns] = 0.0;
   }
 }
 
-// Power-law extrapolation of Q+ into ring 0 (SourceEuler.c:556-567).
-__global__ void k_qplus_row0(DevGrid g, double *__restrict__ qplus, double lr01, double lr12)
+// SubStep3 viscous heating (SourceEuler.c:541-567) from the stress of the
+// updated velocities (the second UpdateDivVelocAndStressTensor call,
+// SourceEuler.c:302), with its power-law extrapolation into ring 0, and the
+// temperature and sound speed of the energy equation's start
+// (ComputeTemperatureField, ComputeSoundSpeed; temper NULL: neither).  A thread
+// walks the rings of a column.  FP64-bound: 42 FP64 instructions a cell, 57 in
+// the three kernels before; 512x1536: 99 -> 71 us.
+#define HT_MAXRINGS 24
+
+__global__ void __launch_bounds__(BX) k_heating(DevGrid g, HeatingIO io)
 {
-  const int ns = g.ns;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ StressRing ring[HT_MAXRINGS];
+  const int ns = g.ns, nr = g.nr;
+  const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
+  if ((int)threadIdx.x < i1 - i0) stress_ring(g, i0 + threadIdx.x, io.invdphi, ring[threadIdx.x]);
+  __syncthreads();
+  const int j = blockIdx.x * BX + threadIdx.x;
   if (j >= ns) return;
-  double q1 = qplus[j + ns], q2 = qplus[j + 2 * ns];
-  qplus[j] = (g.r.nu_med[0] != 0.0) ? q1 * exp(log(q1 / q2) * lr01 / lr12) : 0.0;
+  const int jm = (j == 0) ? ns - 1 : j - 1, jp = (j == ns - 1) ? 0 : j + 1;
+  double om_m = 0.0, rs_m = 0.0, q1 = 0.0;
+  if (i0 > 0) {
+    const int l = j + (i0 - 1) * ns;
+    om_m = io.vt[l] * g.r.InvRmed[i0 - 1];
+    rs_m = io.rho[l] + io.rho[jm + (i0 - 1) * ns];
+  }
+  double vr = io.vr[j + i0 * ns];
+  for (int i = i0; i < i1; i++) {
+    const StressRing &R = ring[i - i0];
+    const int row = i * ns, l = j + row;
+    const double vr_ip = io.vr[l + ns], vt = io.vt[l], rho = io.rho[l];
+    const double rs = rho + io.rho[jm + row], om = vt * g.r.InvRmed[i];
+    const Stress s = stress_cell(R, i, vr, vr_ip, io.vr[jm + row], vt, io.vt[jp + row], om, om_m, rho, rs, rs_m);
+    io.divv[l] = s.divv;
+    if (i >= 1) {
+      double q = 0.0;
+      if (R.nu2 != 0.0) {
+        const double n = R.nu2 * rho;                          // 2 nu rho
+        q = div_fast(__fma_rn(s.trr, s.trr, __fma_rn(s.tpp, s.tpp, 2.0 * s.trp * s.trp)), n);
+        q = __fma_rn((1.0 / 9.0) * n * s.divv, s.divv, q);
+      }
+      io.qplus[l] = q;
+      if (i == 1) q1 = q;
+      if (i == 2)
+        io.qplus[j] = (g.r.nu_med[0] != 0.0) ? q1 * exp(log(q1 / q) * io.lr01 / io.lr12) : 0.0;
+    }
+    if (io.temper) {
+      const double T = div_fast(io.energy[l] * io.gm1, rho);
+      io.temper[l] = T;
+      io.cs[l] = sqrt_fast(io.gamma * abs_i(T));               // gamma (gamma - 1) e / rho = gamma T
+    }
+    om_m = om; rs_m = rs;
+    vr = vr_ip;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1492,36 +1574,22 @@ void hydro_sources(const DevGrid &g, const SourceIO &io0, cudaStream_t s)
   g_thorin_launches++;
 }
 
-void hydro_stress(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *trr,
-                  double *tpp, double *trp, double invdphi, cudaStream_t s)
+void hydro_viscous(const DevGrid &g, const ViscousIO &io0, cudaStream_t s)
 {
-  k_stress<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, vr, vt, rho, divv, trr, tpp, trp, invdphi);
+  ViscousIO io = io0;
+  io.rings = chunk_rings(g.nr, g.ns, g.nsm, VI_MAXRINGS, 1.8);
+  const dim3 grid((g.ns + VI_COLS - 1) / VI_COLS, (g.nr + io.rings - 1) / io.rings);
+  k_viscous<<<grid, BX, 0, s>>>(g, io);
   g_thorin_launches++;
 }
 
-void hydro_visc_update(const DevGrid &g, double *vr, double *vt, const double *rho, const double *trr, const double *tpp,
-                       const double *trp, double invdphi, int kepler, double vkin, double vkout,
-                       cudaStream_t s)
+void hydro_heating(const DevGrid &g, const HeatingIO &io0, cudaStream_t s)
 {
-  k_visc_update<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, vr, vt, rho, trr, tpp, trp, invdphi, kepler, vkin, vkout);
-  g_thorin_launches++;
-}
-
-void hydro_substep2(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *energy,
-                    double *vrnew, double *vtnew, double *eint, int energy_eq, const double *invdxtheta_r,
-                    cudaStream_t s)
-{
-  k_substep2<<<grid2d(g.ns, g.nr + 1, BX), BX, 0, s>>>(g, rho, vr, vt, energy, vrnew, vtnew, eint, energy_eq,
-                                                       invdxtheta_r);
-  g_thorin_launches++;
-}
-
-void hydro_qplus(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *qplus,
-                 double invdphi, double lr01, double lr12, cudaStream_t s)
-{
-  k_qplus<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, vr, vt, rho, divv, qplus, invdphi);
-  g_thorin_launches++;
-  k_qplus_row0<<<(g.ns + BX - 1) / BX, BX, 0, s>>>(g, qplus, lr01, lr12);
+  HeatingIO io = io0;
+  io.rings = chunk_rings(g.nr, g.ns, g.nsm, HT_MAXRINGS, 0.2);
+  if (io.rings < 3) io.rings = 3;                  // ring 0 is extrapolated by the thread of rings 1 and 2
+  const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
+  k_heating<<<grid, BX, 0, s>>>(g, io);
   g_thorin_launches++;
 }
 

@@ -128,7 +128,7 @@ struct thorin_disk {
   double *ring[R_COUNT];
   // fields
   double *rho, *vrad, *vtheta, *energy, *vrad_new, *vtheta_new, *energy_new, *vrad_int, *vtheta_int, *energy_int;
-  double *cs, *temper, *qplus, *qminus, *opacity, *divv, *trr, *trp, *tpp, *agr, *agt, *pagr, *pagt, *dcen;
+  double *cs, *temper, *qplus, *qminus, *opacity, *divv, *agr, *agt, *pagr, *pagt, *dcen;
   double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *sor_cw, *tbackup, *flaring, *qirr;   // sor_cw = omega / ml
   double *press = nullptr;   // pressure field of isothermal runs (formed at the start of each substep)
   double *label = nullptr;   // passive tracer (LabelAdvection)
@@ -422,7 +422,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   RCHK(dalloc(d, (void **)&d->acc_args_d, sizeof(AccArgs)));
   double **F[] = {&d->rho, &d->vrad, &d->vtheta, &d->energy, &d->vrad_new, &d->vtheta_new, &d->energy_new,
                   &d->vrad_int, &d->vtheta_int, &d->energy_int, &d->cs, &d->temper, &d->qplus, &d->qminus,
-                  &d->opacity, &d->divv, &d->trr, &d->trp, &d->tpp, &d->agr, &d->agt, &d->dcen, &d->ml, &d->mlip,
+                  &d->opacity, &d->divv, &d->agr, &d->agt, &d->dcen, &d->ml, &d->mlip,
                   &d->mlim, &d->mljp, &d->mljm, &d->rhs, &d->sor_cw, &d->tbackup, &d->t_rho_gas, &d->t_e_gas};
   for (auto f : F) RCHK(dfield(d, f));
   if (!d->p.energy_eq) RCHK(dfield(d, &d->press));
@@ -1647,7 +1647,13 @@ static int capture_sor(thorin_disk *d);
 static int energy_step(thorin_disk *d, double dt)
 {
   const thorin_params &p = d->p;
-  hydro_qplus(d->g, d->vrad, d->vtheta, d->rho, d->divv, d->qplus, d->invdphi, d->lr01, d->lr12, d->s);
+  HeatingIO heat = {};
+  heat.rho = d->rho; heat.vr = d->vrad; heat.vt = d->vtheta; heat.energy = d->energy_int;
+  heat.divv = d->divv; heat.qplus = d->qplus;
+  heat.invdphi = d->invdphi; heat.lr01 = d->lr01; heat.lr12 = d->lr12;
+  heat.gm1 = d->gm1; heat.gamma = p.adiabind;
+  if (!p.parametric_cooling) { heat.temper = d->temper; heat.cs = d->cs; }
+  hydro_heating(d->g, heat, d->s);
   if (p.parametric_cooling) {
     aux_parametric_cooling(d->g, d->rho, d->energy_int, d->qplus, d->divv, d->ring[R_COOLT], d->ring[R_QPLUSMED],
                            d->energy_new, d->gm1, d->s);
@@ -1659,7 +1665,6 @@ static int energy_step(thorin_disk *d, double dt)
     g_last_error = "OpacityTable SM03 needs the gas opacity table (thorin_gpu_set_opacity_table)";
     return THORIN_ERR_STATE;
   }
-  hydro_eos(d->g, d->rho, d->energy_int, d->temper, d->cs, d->gm1, d->gg1, d->s);
   DiffusionIO dif = {};
   dif.rho = d->rho; dif.T = d->temper; dif.cs = d->cs;
   dif.invdxtheta = d->ring[R_INVDXTHETA]; dif.deltar2 = d->ring[R_DELTAR2];
@@ -1801,17 +1806,12 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
     src.pvrn = d->pvrad_int; src.pvtn = d->pvtheta_int;
   }
   hydro_sources(d->g, src, d->s);
-  // viscous terms
-  hydro_stress(d->g, d->vrad_int, d->vtheta_int, d->rho, d->divv, d->trr, d->tpp, d->trp, d->invdphi, d->s);
-  const int kepler = (!p.damping) || (p.damping && p.damp_vrad);
-  hydro_visc_update(d->g, d->vrad_int, d->vtheta_int, d->rho, d->trr, d->tpp, d->trp, d->invdphi, kepler,
-                    d->vkep_in - d->Rmed[0] * d->OmegaFrame, d->vkep_out - d->Rmed[d->nr - 1] * d->OmegaFrame, d->s);
   if (p.pebbles) {
     // EvolvePebbleDisk (Pebbles.c:702-708).  From here on the pebble fields
     // are read and written only by the pebble transport and the gas side
     // touches none of them, so it runs on the pebble stream while the gas
-    // goes through SubStep2, the energy step and its own transport; the
-    // streams join before this call returns.
+    // goes through the viscous terms, SubStep2, the energy step and its own
+    // transport; the streams join before this call returns.
     CUCHK(cudaEventRecord(d->ev_fork, d->s));
     CUCHK(cudaStreamWaitEvent(d->s_peb, d->ev_fork, 0));
     aux_damp_peb(d->g, d->pdens, d->pvrad_int, d->pvtheta_int, d->damp_rings_d, d->ndamp, d->s_peb);
@@ -1820,9 +1820,18 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
     aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s_peb);
     CUCHK(cudaEventRecord(d->ev_join, d->s_peb));
   }
-  // SubStep2, ActualiseGas, ApplyBoundaryCondition
-  hydro_substep2(d->g, d->rho, d->vrad_int, d->vtheta_int, d->energy, d->vrad_new, d->vtheta_new, d->energy_int,
-                 p.energy_eq, d->ring[R_INVDXTHETA], d->s);
+  // viscous terms and SubStep2, ActualiseGas, ApplyBoundaryCondition
+  ViscousIO vis = {};
+  vis.rho = d->rho; vis.vr = d->vrad_int; vis.vt = d->vtheta_int; vis.energy = d->energy;
+  vis.invdxtheta = d->ring[R_INVDXTHETA];
+  vis.vrnew = d->vrad_new; vis.vtnew = d->vtheta_new;
+  vis.eint = p.energy_eq ? d->energy_int : nullptr;
+  vis.divv = p.energy_eq ? nullptr : d->divv;
+  vis.invdphi = d->invdphi;
+  vis.kepler = (!p.damping) || (p.damping && p.damp_vrad);
+  vis.vkep_in = d->vkep_in - d->Rmed[0] * d->OmegaFrame;
+  vis.vkep_out = d->vkep_out - d->Rmed[d->nr - 1] * d->OmegaFrame;
+  hydro_viscous(d->g, vis, d->s);
   std::swap(d->vrad, d->vrad_new);
   std::swap(d->vtheta, d->vtheta_new);
   boundary();

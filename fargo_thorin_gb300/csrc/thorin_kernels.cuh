@@ -61,6 +61,23 @@ struct SourceIO {
   int back_reaction, diffusion, rings;
 };
 
+// Arguments of the viscous terms and SubStep2 (eint NULL: no energy equation;
+// divv NULL: formed later, from the updated velocities).
+struct ViscousIO {
+  const double *rho, *vr, *vt, *energy, *invdxtheta;
+  double *vrnew, *vtnew, *eint, *divv;
+  double invdphi, vkep_in, vkep_out;
+  int kepler, rings;
+};
+
+// Arguments of the viscous heating (temper NULL: without the equation of state).
+struct HeatingIO {
+  const double *rho, *vr, *vt, *energy;
+  double *divv, *qplus, *temper, *cs;
+  double invdphi, lr01, lr12, gm1, gamma;
+  int rings;
+};
+
 // Arguments of the opacity and diffusion coefficient step.
 struct DiffusionIO {
   const double *rho, *T, *cs, *invdxtheta, *deltar2;
@@ -152,16 +169,8 @@ extern std::atomic<long long> g_thorin_launches;
 
 // kernels_hydro.cu
 void hydro_sources(const DevGrid &g, const SourceIO &io, cudaStream_t s);
-void hydro_stress(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *trr,
-                  double *tpp, double *trp, double invdphi, cudaStream_t s);
-void hydro_visc_update(const DevGrid &g, double *vr, double *vt, const double *rho, const double *trr, const double *tpp,
-                       const double *trp, double invdphi, int kepler, double vkin, double vkout,
-                       cudaStream_t s);
-void hydro_substep2(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *energy,
-                    double *vrnew, double *vtnew, double *eint, int energy_eq, const double *invdxtheta_r,
-                    cudaStream_t s);
-void hydro_qplus(const DevGrid &g, const double *vr, const double *vt, const double *rho, double *divv, double *qplus,
-                 double invdphi, double lr01, double lr12, cudaStream_t s);
+void hydro_viscous(const DevGrid &g, const ViscousIO &io, cudaStream_t s);
+void hydro_heating(const DevGrid &g, const HeatingIO &io, cudaStream_t s);
 void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double *temper, double *cs, double gm1,
                double gg1, cudaStream_t s);
 void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io, int law, cudaStream_t s);
