@@ -25,9 +25,9 @@ static const int BX = 128;
 static int chunk_rings(int nr, int ns, int nsm, int most, double extra, int slots = 4)
 {
   const long long nbx = (ns + BX - 1) / BX;
-  int best = 2;
+  int best = 1;
   double bestw = 1e300;
-  for (int r = 2; r <= most; r++) {
+  for (int r = 1; r <= most; r++) {
     const long long n = (nbx * ((nr + r - 1) / r) + nsm - 1) / nsm;
     const double full = (double)(n / slots * slots), part = (double)(n % slots), q = 1.0 - part / slots;
     const double w = (full + (part > 0.0 ? part / (1.0 - q * q) : 0.0)) * (r + extra);
@@ -1174,6 +1174,148 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
   }
 }
 
+// The whole solve of a small disk in one launch: a cluster of 16 blocks
+// (one per multiprocessor of a GPC, scheduled together by the hardware) keeps
+// the system in shared memory and separates the colour passes by cluster
+// barriers.  A pass as a launch of its own takes 4 to 5 us on a small disk,
+// nearly all of it the launch, the load latency and the completion, and the
+// sweep loop's graph runs up to seven sweeps too many; here a pass of a few
+// thousand cells takes 2.3 us, two thirds of it the L2 latency of the
+// neighbours, the chain of FP64 instructions (64 cycles each) and the barrier.
+// 24x72: a DT 321 -> 291 us.  Each block owns `per` consecutive cells
+// of each colour: their seven coefficients, temperatures and neighbour offsets
+// are in shared memory; the neighbours' temperatures come from L2 (__ldcg),
+// where every update is written before the barrier (release at the arrival,
+// acquire at the wait).  The L1 norm is summed per block in a fixed order,
+// handed to every block of the cluster through distributed shared memory, and
+// all blocks add the partials in the same order, so all take the same exit.
+// The loop ends at the iteration cap at the latest; no block waits for
+// anything but the hardware barrier.
+#define SOR_CLUSTER 16
+#define SOR_CLUSTER_CELLS 36000       // largest disk (cells of rings 1 .. nr-2)
+
+__device__ __forceinline__ void cluster_sync_all()
+{
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+// Store to the same shared variable of block `rank` of the cluster.
+__device__ __forceinline__ void cluster_store(double *p, unsigned rank, double v)
+{
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(512) k_sor_cluster(DevGrid g, double *__restrict__ T, const double *__restrict__ ml,
+                                                     const double *__restrict__ mlip, const double *__restrict__ mlim,
+                                                     const double *__restrict__ mljp, const double *__restrict__ mljm,
+                                                     const double *__restrict__ rhs, const double *__restrict__ cw,
+                                                     SorCtl c, double eps, int maxiters, int per)
+{
+  extern __shared__ double sm[];
+  __shared__ double red[512], part[2][SOR_CLUSTER], cpart[2][SOR_CLUSTER];
+  __shared__ int cnt, verdict;
+  double *co = sm;                                 // [7][2 per]
+  double *ts = sm + 14 * per;                      // [2 per]
+  int *li = (int *)(ts + 2 * per);                 // [2 per]: 4 l + (j == ns - 1) + 2 (j == 0)
+  const int ns = g.ns, half = ns >> 1, total = half * (g.nr - 2);
+  const unsigned rank = cluster_rank();
+  const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
+  const int first = (int)rank * per, n = min(per, total - first);      // may be <= 0
+  for (int q = t; q < 2 * per; q += nt) {
+    const int col = q / per, idx = first + (q - col * per);
+    if (idx >= total) continue;
+    const int r = idx / half, k = idx - r * half, i = r + 1;
+    const int j = 2 * k + ((r + col) & 1), l = j + i * ns;
+    const size_t p = (size_t)((i << 1) + col) * half + k;
+    const int w = 2 * per;
+    co[q] = ml[p]; co[w + q] = mlip[p]; co[2 * w + q] = mlim[p]; co[3 * w + q] = mljp[p]; co[4 * w + q] = mljm[p];
+    co[5 * w + q] = rhs[p]; co[6 * w + q] = cw[p];
+    ts[q] = T[l];
+    li[q] = 4 * l + (j == ns - 1 ? 1 : 0) + (j == 0 ? 2 : 0);
+  }
+  const double thr = eps * *c.normres0;
+  int it = 0, dn = 0;
+  cluster_sync_all();                              // every block of the cluster has started
+  while (!dn) {
+    it++;
+    const int buf = it & 1;
+    double a = 0.0;
+    int ch = 0;
+    if (t == 0) cnt = 0;
+#pragma unroll 1
+    for (int col = 0; col < 2; col++) {
+      const int w = 2 * per;
+      for (int q = t; q < n; q += nt) {
+        const int p = col * per + q, f = li[p], l = f >> 2;
+        const double tip = __ldcg(T + l + ns), tim = __ldcg(T + l - ns);
+        const double tjp = __ldcg(T + l + ((f & 1) ? 1 - ns : 1)), tjm = __ldcg(T + l + ((f & 2) ? ns - 1 : -1));
+        const double t0 = ts[p];
+        double resid = __fma_rn(t0, co[p], -co[5 * w + p]);
+        resid = __fma_rn(tip, co[w + p], resid);
+        resid = __fma_rn(tim, co[2 * w + p], resid);
+        resid = __fma_rn(tjp, co[3 * w + p], resid);
+        resid = __fma_rn(tjm, co[4 * w + p], resid);
+        a += abs_i(resid);
+        const double m = co[6 * w + p];
+        const double tn = __fma_rn(-resid, m, t0);
+        ts[p] = tn;
+        __stcg(T + l, tn);
+        ch += sor_changed(resid, m, tn) ? 1 : 0;
+      }
+      if (col == 0) cluster_sync_all();
+    }
+    red[t] = a;
+    ch = __reduce_add_sync(TH_FULL, ch);
+    __syncthreads();                               // red and the cleared count
+    if (lane == 0 && ch) atomicAdd(&cnt, ch);
+    if (warp < 4) {                                // one warp per sub-partition adds a quarter of the threads' values
+      const int nw = nt >> 5;
+      double s = 0.0;
+      for (int v = warp; v < nw; v += 4) s += red[32 * v + lane];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
+      a = s;
+    }
+    __syncthreads();
+    if (warp < 4 && lane == 0) red[warp] = a;
+    __syncthreads();
+    if (t < SOR_CLUSTER) {
+      const int nw = min(nt >> 5, 4);
+      double s = red[0];
+      for (int v = 1; v < nw; v++) s += red[v];
+      cluster_store(&part[buf][rank], t, s);
+      cluster_store(&cpart[buf][rank], t, (double)cnt);
+    }
+    cluster_sync_all();                            // temperatures and partials of the whole cluster
+    if (warp == 0) {
+      double s = (lane < SOR_CLUSTER) ? part[buf][lane] : 0.0, e = (lane < SOR_CLUSTER) ? cpart[buf][lane] : 0.0;
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
+      for (int o = 8; o > 0; o >>= 1) e += __shfl_xor_sync(TH_FULL, e, o);
+      if (lane == 0) {
+        dn = (s < thr || s < TH_SORMIN || e == 0.0) ? 1 : (it >= maxiters ? 2 : 0);
+        verdict = dn;
+        if (dn && rank == 0) {
+          *c.normres = s;
+          *c.changed = (int)e;
+          *c.niter = it;
+          *c.done = dn;
+        }
+      }
+    }
+    __syncthreads();
+    dn = verdict;
+    __syncthreads();                               // everyone has read it before the next sweep's writes
+  }
+}
+
 // After SOR: boundary rings adopt their neighbours' temperature and the
 // energy is rebuilt, E = rho T c_v (EnergySources.c:319-334).
 __global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, double *__restrict__ T,
@@ -1708,6 +1850,64 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
     cfg.numAttrs = (n > 0) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, k_sor_pass, g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, (n & 1) + 1, maxiters);
   }
+}
+
+// Cells of a colour per block of k_sor_cluster: an even number of whole warps'
+// worth at least.
+static int sor_cluster_per(const DevGrid &g)
+{
+  const long long total = (long long)(g.ns / 2) * (g.nr - 2);
+  const int per = (int)((total + SOR_CLUSTER - 1) / SOR_CLUSTER);
+  return per < 32 ? 32 : (per + 1) / 2 * 2;
+}
+
+static size_t sor_cluster_smem(int per) { return (size_t)per * (16 * sizeof(double) + 2 * sizeof(int)); }
+
+static void sor_cluster_config(const DevGrid &g, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, cudaStream_t s)
+{
+  const int per = sor_cluster_per(g), nt = (per + 31) / 32 * 32;
+  cfg = cudaLaunchConfig_t{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = SOR_CLUSTER;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(SOR_CLUSTER);
+  cfg.blockDim = dim3(nt > 512 ? 512 : nt);
+  cfg.dynamicSmemBytes = sor_cluster_smem(per);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+}
+
+// Whether a disk's solves run as one cluster launch each: the system fits the
+// shared memory of 16 blocks, 16 multiprocessors' FP64 is no slower than a
+// launch per pass on all of them (us a pass here and there: 24x72 2.3 / 4,
+// 96x288 4.2 / 5.2, 128x384 5.6 / 5.4), and the GPU can place the cluster.
+// Called once per disk; sets the kernel's launch limits in the current context.
+int hydro_sor_cluster_fits(const DevGrid &g)
+{
+  if ((long long)g.ns * (g.nr - 2) > SOR_CLUSTER_CELLS) return 0;
+  if (cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  sor_cluster_config(g, cfg, at, nullptr);
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_sor_cluster, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+  return n >= 1;
+}
+
+void hydro_sor_cluster(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                       double eps, int maxiters, cudaStream_t s)
+{
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  sor_cluster_config(g, cfg, at, s);
+  cudaLaunchKernelEx(&cfg, k_sor_cluster, g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, maxiters,
+                     sor_cluster_per(g));
 }
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)

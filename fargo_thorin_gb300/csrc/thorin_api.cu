@@ -208,6 +208,7 @@ struct thorin_disk {
   cudaGraphExec_t sor_loop = nullptr;
   int sor_loop_k = 8;            // sweeps per run of the loop body
   int sor_direct = 0;            // sweeps as plain stream launches (for kernel profilers)
+  int sor_cluster = 0;           // a solve is one cluster launch (small disks)
   double heatsrc[THORIN_MAXPLANETS];
   int heatsrc_index[THORIN_MAXPLANETS], heatsrc_max;
   double gm1, gg1, drin, drout, invdphi, lr01, lr12, taueff_c, tirr4fac, rstar;
@@ -501,6 +502,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     if (k >= 1 && k <= 64) d->sor_loop_k = k;
   }
   if (const char *ed = getenv("THORIN_SOR_DIRECT")) d->sor_direct = (atoi(ed) != 0);
+  d->sor_cluster = !d->sor_direct && hydro_sor_cluster_fits(d->g);
   fill_rings(d);
   {
     PlConst &c = d->plc;                 // constants of the planet side of a substep
@@ -1582,8 +1584,13 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
       if (d->iscal_h[IS_SOR_DONE] || first + d->sor_loop_k > d->p.sor_maxiters) break;
     }
   } else {
-    RCHK(sor_loop_graph(d));
-    CUCHK(cudaGraphLaunch(d->sor_loop, d->s));
+    if (d->sor_cluster) {
+      hydro_sor_cluster(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor,
+                        d->p.sor_eps, d->p.sor_maxiters, d->s);
+    } else {
+      RCHK(sor_loop_graph(d));
+      CUCHK(cudaGraphLaunch(d->sor_loop, d->s));
+    }
     KCHECK("SOR sweep kernels");
   }
   if (d->timing) CUCHK(cudaEventRecord(d->ev[1], d->s));
@@ -1596,7 +1603,7 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
   }
   *niter = n;
   *capped = (done == 2);
-  g_thorin_launches += 2LL * n;
+  g_thorin_launches += (d->sor_cluster && !d->sor_direct) ? 1LL : 2LL * n;
   if (d->timing) {
     float ms = 0.f;
     CUCHK(cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]));
@@ -2107,22 +2114,27 @@ static int capture_sor(thorin_disk *d)
                           d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->ctl + CTL_SOR_OMEGA, d->ws_jac,
                           d->ws_vq, d->ws_part, d->ws_step, d->g.nsm, d->s));
   }
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t cg;
-  const cudaGraphNode_t *deps = nullptr;
-  const cudaGraphEdgeData *edges = nullptr;
-  size_t ndeps = 0;
-  CUCHK(cudaStreamGetCaptureInfo(d->s, &cs, nullptr, &cg, &deps, &edges, &ndeps));
-  if (cs != cudaStreamCaptureStatusActive) { g_last_error = "SOR loop outside a capture"; return THORIN_ERR_STATE; }
-  cudaGraphNodeParams np = {};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = S.h_sor;
-  np.conditional.type = cudaGraphCondTypeWhile;
-  np.conditional.size = 1;
-  cudaGraphNode_t node;
-  CUCHK(cudaGraphAddNode(&node, cg, deps, edges, ndeps, &np));
-  d->capture_sor_body = np.conditional.phGraph_out[0];
-  CUCHK(cudaStreamUpdateCaptureDependencies(d->s, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+  if (d->sor_cluster) {
+    hydro_sor_cluster(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor,
+                      d->p.sor_eps, d->p.sor_maxiters, d->s);
+  } else {
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t cg;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t ndeps = 0;
+    CUCHK(cudaStreamGetCaptureInfo(d->s, &cs, nullptr, &cg, &deps, &edges, &ndeps));
+    if (cs != cudaStreamCaptureStatusActive) { g_last_error = "SOR loop outside a capture"; return THORIN_ERR_STATE; }
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = S.h_sor;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    CUCHK(cudaGraphAddNode(&node, cg, deps, edges, ndeps, &np));
+    d->capture_sor_body = np.conditional.phGraph_out[0];
+    CUCHK(cudaStreamUpdateCaptureDependencies(d->s, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+  }
   graph_sor_end(S, d->s);
   if ((predict || extrap) && d->ws_prev)   // this solve's update, an input of the next prediction
     RCHK(wn_record_update(d->nr, d->ns, d->temper, d->tbackup, d->ws_prev, d->ws_nh, d->ctl + CTL_DT, d->ws_dts, d->s));
@@ -2270,7 +2282,9 @@ static int build_dt_graph(thorin_disk *d, int npl)
     if (rc == THORIN_OK && e2 != cudaSuccess) e = e2;
   }
   // the substep body, with the SOR loop's node inside it
-  if (e == cudaSuccess && rc == THORIN_OK) e = cudaGraphConditionalHandleCreate(&S.h_sor, body, 1u, cudaGraphCondAssignDefault);
+  const bool loop = !d->sor_cluster;
+  S.sor_loop = loop;
+  if (loop && e == cudaSuccess && rc == THORIN_OK) e = cudaGraphConditionalHandleCreate(&S.h_sor, body, 1u, cudaGraphCondAssignDefault);
   if (e == cudaSuccess && rc == THORIN_OK) e = cudaStreamBeginCaptureToGraph(d->s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess && rc == THORIN_OK) {
     d->capturing = 1;
@@ -2280,11 +2294,11 @@ static int build_dt_graph(thorin_disk *d, int npl)
     cudaGraph_t tmp;
     const cudaError_t e2 = cudaStreamEndCapture(d->s, &tmp);
     if (rc == THORIN_OK && e2 != cudaSuccess) e = e2;
-    if (rc == THORIN_OK && e == cudaSuccess && !d->capture_sor_body) { g_last_error = "no SOR loop in the substep"; rc = THORIN_ERR_STATE; }
+    if (rc == THORIN_OK && e == cudaSuccess && !d->capture_sor_body && !d->sor_cluster) { g_last_error = "no SOR loop in the substep"; rc = THORIN_ERR_STATE; }
   }
   // the sweeps inside the SOR loop
-  if (e == cudaSuccess && rc == THORIN_OK) e = cudaStreamBeginCaptureToGraph(d->s, d->capture_sor_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess && rc == THORIN_OK) {
+  if (loop && e == cudaSuccess && rc == THORIN_OK) e = cudaStreamBeginCaptureToGraph(d->s, d->capture_sor_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  if (loop && e == cudaSuccess && rc == THORIN_OK) {
     SorCtl c = d->sor;
     c.cond = S.h_sor;
     c.has_cond = 1;

@@ -211,7 +211,7 @@ __global__ void k_g_sor_begin(StepDev S)
   if (omega < 1.0) { omega = 1.0; domega = -domega; }
   ctl[CTL_SOR_OMEGA] = omega;
   ctl[CTL_SOR_DOMEGA] = domega;
-  cudaGraphSetConditional(S.h_sor, 1u);
+  if (S.sor_loop) cudaGraphSetConditional(S.h_sor, 1u);
 }
 
 // After a solve (EnergySources.c:306-317): counters, and the schedule's

@@ -38,6 +38,7 @@ struct StepDev {
   SorCtl sor;
   double DT, evaporation_rate;
   int npl, pebbles, accret_heating, indirect_term;
+  int sor_loop;               // the solve's sweeps are a WHILE node (else one launch)
   cudaGraphConditionalHandle h_sub, h_sor;
 };
 

@@ -190,6 +190,11 @@ void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const
 void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
                       double eps, int count, int maxiters, cudaStream_t s);
+// The whole solve of a small disk in one launch, where hydro_sor_cluster_fits.
+int hydro_sor_cluster_fits(const DevGrid &g);
+void hydro_sor_cluster(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                       double eps, int maxiters, cudaStream_t s);
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s);
 void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
                      double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,

@@ -42,3 +42,30 @@ def test_grids_at_the_edges_of_the_tiles(kind, nr, ns, over):
             # the tolerance of the oracle comparisons (test_gpu_parity)
             assert H.rel_l2(d.get(H.FIELD_IDS[f])[:n], o.get(H.FIELD_IDS[f])[:n]) < 1e-11, f"{f} at DT {step}"
     d.close()
+
+
+@pytest.mark.parametrize("nr,ns", [(6, 10), (24, 72), (97, 366), (98, 370), (99, 374)])
+def test_cluster_solve_matches_the_launched_passes(nr, ns, monkeypatch):
+    """Small disks solve in one cluster launch (the largest that does has
+    36000 cells; 97x366 is below, 99x374 above); THORIN_SOR_DIRECT runs a
+    launch per colour pass.  Same updates, so the same bits and sweep counts,
+    on the host path and in the DT graph."""
+    from fargo_thorin_gb300.disk import GpuDisk
+    p = workloads.params_for("disk0", nr, ns)
+    out = []
+    for direct in ("0", "1"):
+        monkeypatch.setenv("THORIN_SOR_DIRECT", direct)
+        d = GpuDisk(p)
+        d.init_default()
+        H.start_state(d, p, {"dens": d.get(0), "temper": d.get(8)})
+        d.set_sor_state(1.3, 1e-3, 50)
+        s = workloads.make_planets(p, [workloads.PLANET0])
+        n = []
+        for k in range(3):
+            (d.algogas_graph if direct == "0" and k else d.algogas)(s)
+            n.append((d.stats().sor_last_niter, d.stats().substeps))
+        out.append((n, [d.get(f).copy() for f in (0, 1, 2, 3, 8)]))
+        d.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
