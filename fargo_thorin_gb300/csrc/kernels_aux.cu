@@ -1306,65 +1306,53 @@ void aux_accrete_kernels(const DevGrid &g, const AccArgs *a_dev, int nb_grid, do
 }
 
 // ---------------------------------------------------------------------------
-// Conservation integrals (GasTotalMass, GasMomentum, GasTotalEnergy,
-// SideEuler.c:26-80,523-565) and the same mass/momentum sums for pebbles.
-__global__ void k_integrals(DevGrid g, const double *__restrict__ rho, const double *__restrict__ vr,
-                            const double *__restrict__ vt, const double *__restrict__ e, const double *__restrict__ pd,
-                            const double *__restrict__ pvt, double omega_frame, int pebbles, double *__restrict__ part)
+// Conservation integrals: a block per ring (integral_ring), the rings' sums by
+// the block that finishes last.
+template <bool PEB>
+__global__ void __launch_bounds__(RING_T) k_integrals(DevGrid g, const double *__restrict__ rho, const double *__restrict__ vr,
+                                                      const double *__restrict__ vt, const double *__restrict__ e,
+                                                      const double *__restrict__ pd, const double *__restrict__ pvt,
+                                                      double omega_frame, double *__restrict__ part,
+                                                      double *__restrict__ scal, unsigned int *ticket)
 {
-  const int ns = g.ns;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  double m = 0, am = 0, en = 0, pm = 0, pam = 0;
-  if (j < ns) {
-    const int l = j + i * ns;
-    const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-    const int ljp = (j == ns - 1) ? i * ns : l + 1;
-    const double S = g.r.Surf[i], rm = g.r.Rmed[i];
-    m = S * rho[l];
-    am = S * (rho[l] + rho[ljm]) * rm * (vt[l] + omega_frame * rm);
-    double vrc = (rm - g.r.Rinf[i]) * vr[l + ns] + (g.r.Rsup[i] - rm) * vr[l];
-    vrc /= (g.r.Rsup[i] - g.r.Rinf[i]);
-    const double vtc = 0.5 * (vt[l] + vt[ljp]) + rm * omega_frame;
-    en = 0.5 * S * rho[l] * (vrc * vrc + vtc * vtc) + S * e[l];
-    if (pebbles) {
-      pm = S * pd[l];
-      pam = S * (pd[l] + pd[ljm]) * rm * (pvt[l] + omega_frame * rm);
-    }
-  }
-  m = block_reduce(m, OpAdd(), 0.0);
-  am = block_reduce(am, OpAdd(), 0.0);
-  en = block_reduce(en, OpAdd(), 0.0);
-  pm = block_reduce(pm, OpAdd(), 0.0);
-  pam = block_reduce(pam, OpAdd(), 0.0);
+  __shared__ bool last;
+  const int i = blockIdx.x, nr = g.nr, ns = g.ns;
+  const size_t row = (size_t)i * ns;
+  double sum[5];
+  integral_ring<PEB>(rho + row, vr + row, vr + row + ns, vt + row, e + row, pd + row, pvt + row, ns, g.r.Surf[i],
+                     g.r.Rmed[i], g.r.Rinf[i], g.r.Rsup[i], omega_frame, sum);
   if (threadIdx.x == 0) {
-    const int b = blockIdx.x + blockIdx.y * gridDim.x;
-    part[5 * b + 0] = m; part[5 * b + 1] = am; part[5 * b + 2] = en; part[5 * b + 3] = pm; part[5 * b + 4] = pam;
+#pragma unroll
+    for (int q = 0; q < 5; q++) part[(size_t)q * nr + i] = sum[q];
+    __threadfence();
+    last = (atomicAdd(ticket, 1u) == (unsigned)nr - 1u);
   }
-}
-
-__global__ void __launch_bounds__(1024) k_integrals_final(const double *__restrict__ part, int nb, double *__restrict__ scal)
-{
-  for (int q = 0; q < 5; q++) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += part[5 * b + q];
-    s = block_reduce(s, OpAdd(), 0.0);
-    if (threadIdx.x == 0) {
-      if (q == 1 || q == 4) s *= 0.5;
-      scal[SC_MASS + q] = s;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *ticket = 0u;
+  for (int q = threadIdx.x >> 5; q < 5; q += RING_T / 32) {
+    const double *p = part + (size_t)q * nr;
+    double a = 0.0, b = 0.0;
+    int k = threadIdx.x & 31;
+    for (; k + 32 < nr; k += 64) {
+      a += __ldcg(p + k);
+      b += __ldcg(p + k + 32);
     }
-    __syncthreads();
+    if (k < nr) a += __ldcg(p + k);
+    a = warp_reduce(a + b, OpAdd());
+    if ((threadIdx.x & 31) == 0) scal[SC_MASS + q] = (q == 1 || q == 4) ? 0.5 * a : a;
   }
 }
 
 void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *e,
                    const double *pd, const double *pvt, double omega_frame, int pebbles, double *part, double *scal,
-                   cudaStream_t s)
+                   unsigned int *ticket, cudaStream_t s)
 {
-  dim3 grid = grid2d(g.ns, g.nr, 256);
-  k_integrals<<<grid, 256, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, pebbles, part);
-  g_thorin_launches++;
-  k_integrals_final<<<1, 1024, 0, s>>>(part, grid.x * grid.y, scal);
+  if (pebbles)
+    k_integrals<true><<<g.nr, RING_T, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
+  else
+    k_integrals<false><<<g.nr, RING_T, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
   g_thorin_launches++;
 }
 

@@ -2523,7 +2523,7 @@ extern "C" int thorin_gpu_integrals(thorin_disk *d, double *mass, double *moment
                                     double *peb_momentum)
 {
   aux_integrals(d->g, d->rho, d->vrad, d->vtheta, d->energy, d->pdens, d->pvtheta, d->OmegaFrame, d->p.pebbles,
-                d->partials, d->scal, d->s);
+                d->partials, d->scal, d->ticket + 10, d->s);
   KCHECK("integral kernels");
   CUCHK(cudaMemcpyAsync(d->scal_h + SC_MASS, d->scal + SC_MASS, 5 * sizeof(double), cudaMemcpyDeviceToHost, d->s));
   CUCHK(cudaStreamSynchronize(d->s));

@@ -161,6 +161,59 @@ __device__ __forceinline__ double ring_sum(const double *__restrict__ row, int n
   return a;
 }
 
+// Conservation integrals of one ring (GasTotalMass, GasMomentum,
+// GasTotalEnergy, SideEuler.c:26-80,523-565, and the pebbles' mass and
+// momentum) by a block of RING_T threads: sum[] = mass, twice the momentum,
+// energy, pebble mass, twice the pebble momentum, valid in thread 0 (the
+// pebbles' only with PEB).  FP64 pipe bound, so what is constant in a ring is
+// taken out of its sums, and the momentum sum (rho_j + rho_j-1) w_j is summed
+// by parts to rho_j (w_j + w_j+1), whose factor the kinetic energy needs too:
+// 14 FP64 instructions a cell with pebbles, where a block reduction of five
+// values for every 256 cells and a division per cell took about 75.  A
+// 1024x3072 disk, the whole call: 425 -> 127 us (83 us of FP64 pipe; its reads
+// at copy speed take 24).
+template <bool PEB>
+__device__ __forceinline__ void integral_ring(const double *__restrict__ rho, const double *__restrict__ vr,
+                                              const double *__restrict__ vrp, const double *__restrict__ vt,
+                                              const double *__restrict__ e, const double *__restrict__ pd,
+                                              const double *__restrict__ pvt, int ns, double S, double rm, double ri,
+                                              double rs, double omega_frame, double sum[5])
+{
+  __shared__ double sh[5][RING_T];
+  const double w2 = 2.0 * (omega_frame * rm), wp = 2.0 * (rm - ri) / (rs - ri), wm = 2.0 * (rs - rm) / (rs - ri);
+  double m = 0.0, am = 0.0, ek = 0.0, ei = 0.0, pm = 0.0, pam = 0.0;
+#pragma unroll 4
+  for (int j = threadIdx.x; j < ns; j += RING_T) {
+    const int jp = (j == ns - 1) ? 0 : j + 1;
+    const double d = rho[j];
+    const double W = (vt[j] + vt[jp]) + w2;        // 2 v_theta of the cell's centre
+    const double V = wp * vrp[j] + wm * vr[j];     // 2 v_r
+    m += d;
+    am += d * W;
+    ek += d * (V * V + W * W);
+    ei += e[j];
+    if (PEB) {
+      const double q = pd[j];
+      pm += q;
+      pam += q * ((pvt[j] + pvt[jp]) + w2);
+    }
+  }
+  double v[5] = {S * m, S * rm * am, S * (0.125 * ek + ei), S * pm, S * rm * pam};
+#pragma unroll
+  for (int q = 0; q < (PEB ? 5 : 3); q++) sh[q][threadIdx.x] = v[q];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int q = 0; q < (PEB ? 5 : 3); q++) {
+      double a = v[q];
+#pragma unroll
+      for (int w = 1; w < RING_T / 32; w++) a += sh[q][threadIdx.x + 32 * w];
+      sum[q] = warp_reduce(a, OpAdd());
+    }
+    if (!PEB) sum[3] = sum[4] = 0.0;
+  }
+}
+
 // Reciprocal and reciprocal square root estimates without the FP64 pipe.
 // GB300 issues an FP64 warp instruction every 76 cycles of a sub-partition
 // (1.68 lanes per clock and SM, any mix of adds, products and FMAs) and FP32

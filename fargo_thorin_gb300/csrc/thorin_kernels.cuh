@@ -246,4 +246,4 @@ void aux_set_ctl(double *ctl, const CtlSet &v, cudaStream_t s);
 int aux_accrete_blocks(const DevGrid &g, int imin, int imax);
 void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *e,
                    const double *pd, const double *pvt, double omega_frame, int pebbles, double *part, double *scal,
-                   cudaStream_t s);
+                   unsigned int *ticket, cudaStream_t s);

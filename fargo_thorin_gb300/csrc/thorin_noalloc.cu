@@ -30,36 +30,22 @@
 
 static __device__ __align__(256) double g_noalloc_partials[NOALLOC_MAX_RINGS * NOALLOC_SLOTS];
 
-// GasTotalMass, GasMomentum, GasTotalEnergy (SideEuler.c:26-80, 523-565) of
-// one ring per block.
-__global__ void k_integrals_ring(const double *__restrict__ rho, const double *__restrict__ vr,
-                                 const double *__restrict__ vt, const double *__restrict__ e,
-                                 const double *__restrict__ surf, const double *__restrict__ rinf,
-                                 const double *__restrict__ rsup, const double *__restrict__ rmed, int ns,
-                                 double omega_frame, double *__restrict__ part)
+// The integrals of one ring per block (integral_ring).
+__global__ void __launch_bounds__(RING_T) k_integrals_ring(const double *__restrict__ rho, const double *__restrict__ vr,
+                                                           const double *__restrict__ vt, const double *__restrict__ e,
+                                                           const double *__restrict__ surf,
+                                                           const double *__restrict__ rinf,
+                                                           const double *__restrict__ rsup,
+                                                           const double *__restrict__ rmed, int ns, double omega_frame,
+                                                           double *__restrict__ part)
 {
   const int i = blockIdx.x;
-  const double S = surf[i], rm = rmed[i], ri = rinf[i], rs = rsup[i];
-  double m = 0.0, am = 0.0, en = 0.0;
-  for (int j = threadIdx.x; j < ns; j += blockDim.x) {
-    const int l = j + i * ns;
-    const int ljm = (j == 0) ? i * ns + ns - 1 : l - 1;
-    const int ljp = (j == ns - 1) ? i * ns : l + 1;
-    m += S * rho[l];
-    am += S * (rho[l] + rho[ljm]) * rm * (vt[l] + omega_frame * rm);
-    double vrc = (rm - ri) * vr[l + ns] + (rs - rm) * vr[l];
-    vrc /= (rs - ri);
-    const double vtc = 0.5 * (vt[l] + vt[ljp]) + rm * omega_frame;
-    en += 0.5 * S * rho[l] * (vrc * vrc + vtc * vtc) + S * e[l];
-  }
-  m = block_reduce(m, OpAdd(), 0.0);
-  am = block_reduce(am, OpAdd(), 0.0);
-  en = block_reduce(en, OpAdd(), 0.0);
-  if (threadIdx.x == 0) {
-    part[NOALLOC_SLOTS * i + 0] = m;
-    part[NOALLOC_SLOTS * i + 1] = am;
-    part[NOALLOC_SLOTS * i + 2] = en;
-  }
+  const size_t row = (size_t)i * ns;
+  double sum[5];
+  integral_ring<false>(rho + row, vr + row, vr + row + ns, vt + row, e + row, nullptr, nullptr, ns, surf[i], rmed[i],
+                       rinf[i], rsup[i], omega_frame, sum);
+  if (threadIdx.x == 0)
+    for (int q = 0; q < NOALLOC_SLOTS; q++) part[NOALLOC_SLOTS * i + q] = sum[q];
 }
 
 __global__ void __launch_bounds__(1024) k_integrals_rings_sum(const double *__restrict__ part, int nr, double *__restrict__ out)
@@ -150,7 +136,7 @@ extern "C" int thorin_integrals_static(const double *rho, const double *vrad, co
   int rc = noalloc_scratch(&part);
   if (rc != THORIN_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  k_integrals_ring<<<nrad, 256, 0, s>>>(rho, vrad, vtheta, energy, surf, rinf, rsup, rmed, nsec, omega_frame, part);
+  k_integrals_ring<<<nrad, RING_T, 0, s>>>(rho, vrad, vtheta, energy, surf, rinf, rsup, rmed, nsec, omega_frame, part);
   k_integrals_rings_sum<<<1, 1024, 0, s>>>(part, nrad, out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_noalloc_error = std::string("launch: ") + cudaGetErrorString(e); return THORIN_ERR_CUDA; }
