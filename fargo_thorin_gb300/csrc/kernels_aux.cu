@@ -35,24 +35,19 @@ __global__ void __launch_bounds__(RING_T) k_ring_means(int ns, const double *__r
   }
 }
 
-// The same ring means at rings chosen on the device: ring info[slot] and,
-// with two, info[slot + 1] rings from there (else one ring when
-// info[slot] >= 0, none when it is negative).
-__global__ void __launch_bounds__(RING_T) k_ring_means_at(int ns, const double *__restrict__ f, double *__restrict__ o,
-                                                          const int *__restrict__ info, int slot, int two)
+// The ring mean at a ring chosen on the device (none when *ring is negative).
+__global__ void __launch_bounds__(RING_T) k_ring_mean_at(int ns, const double *__restrict__ f, double *__restrict__ o,
+                                                         const int *__restrict__ ring)
 {
-  const int w = blockIdx.x;
-  const int ring0 = info[slot];
-  const int nrings = two ? info[slot + 1] : (ring0 >= 0 ? 1 : 0);
-  if (ring0 < 0 || w >= nrings) return;
-  const double a = ring_sum(f + (size_t)(ring0 + w) * ns, ns);
-  if (threadIdx.x == 0) o[w] = a / (double)ns;
+  const int i = *ring;
+  if (i < 0) return;
+  const double a = ring_sum(f + (size_t)i * ns, ns);
+  if (threadIdx.x == 0) *o = a / (double)ns;
 }
 
-void graph_ring_means_at(const DevGrid &g, const double *f, double *out, const int *ring_info, int slot, int two_slots,
-                         cudaStream_t s)
+void graph_ring_mean_at(const DevGrid &g, const double *f, double *out, const int *ring, cudaStream_t s)
 {
-  k_ring_means_at<<<two_slots ? 2 : 1, RING_T, 0, s>>>(g.ns, f, out, ring_info, slot, two_slots);
+  k_ring_mean_at<<<1, RING_T, 0, s>>>(g.ns, f, out, ring);
   g_thorin_launches++;
 }
 
@@ -1024,75 +1019,111 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
 // the effective accretion radius give up pebbles up to the model rate.
 
 // Trapzd and IntegrateColumnMass (Pebbles.c:302-349) for one cell, evaluated
-// by a whole warp: the it = 2^(n-2) midpoints of level n are spread over the
-// lanes (lane k takes points k, k + 32, ...), point j at a + (j + 1/2)
-// spacing, and the level's sum is an xor butterfly over the lanes' partial
-// sums, so every lane holds the same bits of the integral and takes the same
-// exit.  The levels, the refinement integral = (integral + (b - a) sum / it)
-// / 2 and the exit test after level 5 are the reference's; only the order of
+// by a whole warp.  Levels 2 to 6, before which the reference makes no exit
+// test that can pass, have 1, 2, 4, 8 and 16 midpoints: level n's are taken
+// at once by the lanes 2^(n-2) to 2^(n-1) - 1 and the lower end by lane 0, so
+// five levels cost one exponential a lane and one butterfly (with a pass each
+// they were most of the 22 us of this kernel).  From level 7 on the 2^(n-2)
+// midpoints are spread over the lanes.  Point j is a + (j + 1/2) spacing and
+// a level's sum an xor butterfly over its lanes' partial sums, so every lane
+// holds the same bits of the integral and takes the same exit.  The levels,
+// the refinement integral = (integral + (b - a) sum / it) / 2 and the exit
+// test after level 5 are the reference's (1 / it is exact); only the order of
 // the midpoint sum and the rounding of the abscissae differ from its
-// sequential loop (x += spacing), by relative amounts of order 1e-16.  Before
-// this the reference's loop ran in one thread per cell, up to 2^14
-// dependent exponentials each.
+// sequential loop (x += spacing), by relative amounts of order 1e-16.
 __device__ double column_mass_warp(double a, double b, double Hpeb)
 {
   const int lane = threadIdx.x & 31;
-  const double H2 = Hpeb * Hpeb;
-  double integral = 0.5 * (b - a) * (exp(div_fast(-0.5 * a * a, H2)) + exp(div_fast(-0.5 * b * b, H2)));
+  const double H2 = Hpeb * Hpeb, w = b - a;
+  const int own = (lane == 0) ? 1 : 1 << (31 - __clz(lane));      // points of the lane's level
+  double x = (lane == 0) ? a : a + ((double)(lane - own) + 0.5) * (w * (1.0 / own));
+  double sum = exp(div_fast(-0.5 * x * x, H2));
+  double fb = __shfl_sync(TH_FULL, sum, 0);
+  double integral = fb;
+  if (a != -b) fb = exp(div_fast(-0.5 * b * b, H2));
+  integral = 0.5 * w * (integral + fb);
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const double t = __shfl_xor_sync(TH_FULL, sum, o);
+    if (own > o) sum += t;
+  }
   double iold = integral;
-  for (int n = 2; n <= 16; n++) {
+#pragma unroll
+  for (int n = 2; n <= 6; n++) {
+    const double it_inv = 1.0 / (double)(1 << (n - 2));
+    iold = integral;
+    integral = 0.5 * (integral + w * __shfl_sync(TH_FULL, sum, 1 << (n - 2)) * it_inv);
+  }
+  for (int n = 7; n <= 17; n++) {
+    if (fabs(integral - iold) < 1.0e-4 * fabs(iold) || (integral == 0.0 && iold == 0.0)) return integral;
+    if (n > 16) break;
     const int it = 1 << (n - 2);
-    const double iter = it, spacing = (b - a) / iter;
-    double sum = 0.0;
+    const double it_inv = ldexp(1.0, 2 - n), spacing = w * it_inv;
+    sum = 0.0;
     for (int j = lane; j < it; j += 32) {
-      const double x = a + ((double)j + 0.5) * spacing;
+      x = a + ((double)j + 0.5) * spacing;
       sum += exp(div_fast(-0.5 * x * x, H2));
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(TH_FULL, sum, o);
-    integral = 0.5 * (integral + (b - a) * sum / iter);
-    if (n > 5)
-      if (fabs(integral - iold) < 1.0e-4 * fabs(iold) || (integral == 0.0 && iold == 0.0)) return integral;
     iold = integral;
+    integral = 0.5 * (integral + w * sum * it_inv);
   }
   return __longlong_as_double(0x7ff8000000000000ULL);   // the reference aborts here
 }
 
-// The annulus work runs on many blocks in three grid passes (mean Stokes
-// number, upper limits per cell, application of the limiter), each followed
-// by a one-block kernel that sums the block partials in a fixed order and
-// does the scalar steps of the reference.
-// acc[] scalars: 0 Reff, 1 vrel, 2 Mt, 3 limiter.
+// The annulus work runs in three launches on many blocks (mean Stokes number,
+// upper limits per cell, application of the limiter); the block that finishes
+// last sums the block partials in a fixed order and does the scalar steps of
+// the reference.  A launch on a small disk is mostly latency: the nine
+// launches before this, with the arguments, the ring means and each sum a
+// launch of its own, took 91 us of a substep at 128x384, these take
+// 67 (a third of it the copy of the result and the wait for it).
+// acc[] scalars: 0 Reff, 1 vrel, 2 Mt, 3 limiter, 4-5 the ring means.
 
-__global__ void __launch_bounds__(ACC_BX) k_acc_tau(DevGrid g, const AccArgs *__restrict__ ap)
+__device__ __forceinline__ bool acc_last_block(unsigned int *ticket)
 {
-  const AccArgs &a = *ap;
-  if ((int)blockIdx.x >= a.nb) return;           // grid sized for the widest annulus
-  const int ncells = (a.imax - a.imin + 1) * g.ns;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  double t = (q < ncells) ? a.tau[(size_t)a.imin * g.ns + q] : 0.0;
-  t = block_reduce(t, OpAdd(), 0.0);
-  if (threadIdx.x == 0) a.part[blockIdx.x] = t;
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
+    if (last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
 }
 
-__global__ void __launch_bounds__(ACC_BX) k_acc_reff(DevGrid g, const AccArgs *__restrict__ ap)
+// Sum over the annulus of the Stokes number by all blocks but two, which form
+// the ring means of v_theta at the two rings bracketing the planet; then the
+// effective accretion radius (Pebbles.c:375-437).  With SET the arguments come
+// by value and are left for the other two kernels.
+template <bool SET>
+__global__ void __launch_bounds__(RING_T) k_acc_reff(DevGrid g, AccArgs av, AccArgs *ap)
 {
-  const AccArgs &a = *ap;
-  const int nb = a.nb;
-  if (nb == 0) return;                       // no annulus (only the device-resident DT launches this)
-  const int ns = g.ns;
-  __shared__ double sh[2];
-  if (threadIdx.x == 0) {                    // vt1D at the two rings bracketing the planet
-    sh[0] = a.acc[4];
-    sh[1] = (a.iflow + 1 < g.nr) ? a.acc[5] : 0.0;   // vt1D[nrad] is zero in the reference
+  const AccArgs &a = SET ? av : *ap;
+  if (a.nb == 0) return;                         // no annulus (only the device-resident DT launches this)
+  const int ns = g.ns, ncells = (a.imax - a.imin + 1) * ns, nb = gridDim.x - 2;
+  if (blockIdx.x >= 2) {
+    const double *tau = a.tau + (size_t)a.imin * ns;
+    double t = 0.0;
+    for (int q = (blockIdx.x - 2) * RING_T + threadIdx.x; q < ncells; q += nb * RING_T) t += tau[q];
+    t = block_reduce(t, OpAdd(), 0.0);
+    if (threadIdx.x == 0) a.part[blockIdx.x - 2] = t;
+  } else {
+    const int i = a.iflow + blockIdx.x;          // vt1D[nrad] is zero in the reference
+    double m = 0.0;
+    if (i >= 0 && i < g.nr) m = ring_sum(a.vt + (size_t)i * ns, ns);
+    if (threadIdx.x == 0) a.acc[4 + blockIdx.x] = m / (double)ns;
+    if (SET && threadIdx.x == 0 && blockIdx.x == 0) *ap = av;
   }
+  if (!acc_last_block(a.ticket)) return;
   double ts = 0.0;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) ts += a.part[b];
+  for (int b = threadIdx.x; b < nb; b += RING_T) ts += __ldcg(a.part + b);
   ts = block_reduce(ts, OpAdd(), 0.0);
   if (threadIdx.x == 0) {
-    const int ncells = (a.imax - a.imin + 1) * ns;
     const double tau_mean = ts / (double)ncells;
-    const double flow = sh[0] * (1.0 - a.frac) + sh[1] * a.frac + a.Rp * a.omega_frame;
+    const double flow = __ldcg(a.acc + 4) * (1.0 - a.frac) + __ldcg(a.acc + 5) * a.frac + a.Rp * a.omega_frame;
     const double flowx = -flow * a.Yp / a.Rp, flowy = flow * a.Xp / a.Rp;
     const double vrel = sqrt((a.VXp - flowx) * (a.VXp - flowx) + (a.VYp - flowy) * (a.VYp - flowy) + a.VZp * a.VZp);
     const double Mt = sqrt(1.0 / 3.0) * cube_rn(vrel) / a.Omegap;
@@ -1113,9 +1144,7 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_reff(DevGrid g, const AccArgs *_
 // Annulus cell q (0 .. (imax - imin + 1) ns - 1) of the accretion step: true
 // when its midplane distance to the planet is within the effective accretion
 // radius, with the pebble scale height and the column's ends inside the
-// sphere (Pebbles.c:445-453).  The operations are spelled out as
-// round-to-nearest intrinsics so that the two kernels that call this get the
-// same bits.
+// sphere (Pebbles.c:445-453).
 __device__ __forceinline__ bool acc_cell(const DevGrid &g, const AccArgs &a, int q, int &i, int &l, double &Hpeb,
                                          double &zmin, double &zmax)
 {
@@ -1136,13 +1165,15 @@ __device__ __forceinline__ bool acc_cell(const DevGrid &g, const AccArgs &a, int
   return true;
 }
 
-// Column integrals of the annulus cells inside the sphere (IntegrateColumnMass
-// of Pebbles.c:456), one warp per cell, into macc[l] (zero outside the
-// accretion step).  Warp w of the grid takes the annulus cells w, w + W,
-// w + 2W, ... (W warps in all), 32 of them tested at a time, so the cells of
-// the sphere, which lie together around the planet, fall on many
-// multiprocessors.
-__global__ void __launch_bounds__(ACC_BX) k_acc_column(DevGrid g, const AccArgs *__restrict__ ap)
+// Upper limit of the mass each annulus cell inside the sphere can give up
+// (Pebbles.c:454-462) into macc[l] (zero outside the accretion step), with
+// its column integral (IntegrateColumnMass of Pebbles.c:456) by one warp per
+// cell, and the limiter from the sums of the limit, the scale height, the
+// pebble density and the cell count.  Warp w of the grid takes the annulus
+// cells w, w + W, w + 2W, ... (W warps in all), 32 of them tested at a time,
+// so the cells of the sphere, which lie together around the planet, fall on
+// many multiprocessors.
+__global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *__restrict__ ap)
 {
   const AccArgs &a = *ap;
   if (a.nb == 0) return;                         // no annulus
@@ -1150,62 +1181,39 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_column(DevGrid g, const AccArgs 
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (ACC_BX / 32);
   const int gw = blockIdx.x * (ACC_BX / 32) + (threadIdx.x >> 5);
+  double v[4] = {0.0, 0.0, 0.0, 0.0};            // limit, scale height, pebble density, cells
   for (long long base = gw; base < ncells; base += 32LL * nw) {   // warp-uniform
     const long long c = base + (long long)lane * nw;
     int i = 0, l = 0;
-    double Hpeb = 0.0, zmin = 0.0, zmax = 0.0;
+    double Hpeb = 0.0, zmin = 0.0, zmax = 0.0, cm = 0.0;
     const bool inside = c < ncells && acc_cell(g, a, (int)c, i, l, Hpeb, zmin, zmax);
     unsigned bal = __ballot_sync(TH_FULL, inside);
     while (bal) {
       const int src = __ffs(bal) - 1;
       bal &= bal - 1u;
-      const double cm = column_mass_warp(__shfl_sync(TH_FULL, zmin, src), __shfl_sync(TH_FULL, zmax, src),
-                                         __shfl_sync(TH_FULL, Hpeb, src));
-      if (lane == src) a.macc[l] = cm;
+      const double m = column_mass_warp(__shfl_sync(TH_FULL, zmin, src), __shfl_sync(TH_FULL, zmax, src),
+                                        __shfl_sync(TH_FULL, Hpeb, src));
+      if (lane == src) cm = m;
+    }
+    if (inside) {
+      const double pd = a.pdens[l];
+      const double mcell = g.r.Surf[i] * pd;
+      const double vdp = pd / Hpeb * g.k.sqrt2pi_inv;
+      double dM = vdp * g.r.Surf[i] * cm;
+      if (dM > mcell) dM = 0.99999999 * mcell;
+      a.macc[l] = dM;
+      v[0] += dM; v[1] += Hpeb; v[2] += pd; v[3] += 1.0;
     }
   }
-}
-
-// Upper limit of the mass each annulus cell inside the sphere can give up
-// (Pebbles.c:454-462), from its column integral (k_acc_column), and the
-// block partials of the limit, the scale height, the pebble density and the
-// cell count.
-__global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *__restrict__ ap)
-{
-  const AccArgs &a = *ap;
-  if ((int)blockIdx.x >= a.nb) return;           // grid sized for the widest annulus
-  const int ncells = (a.imax - a.imin + 1) * g.ns;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  double dmu = 0.0, hpm = 0.0, pdm = 0.0, nc = 0.0;
-  int i = 0, l = 0;
-  double Hpeb = 0.0, zmin = 0.0, zmax = 0.0;
-  if (q < ncells && acc_cell(g, a, q, i, l, Hpeb, zmin, zmax)) {
-    const double pd = a.pdens[l];
-    const double mcell = g.r.Surf[i] * pd;
-    const double vdp = pd / Hpeb * g.k.sqrt2pi_inv;
-    double dM = vdp * g.r.Surf[i] * a.macc[l];
-    if (dM > mcell) dM = 0.99999999 * mcell;
-    a.macc[l] = dM;
-    dmu = dM; hpm = Hpeb; pdm = pd; nc = 1.0;
-  }
-  dmu = block_reduce(dmu, OpAdd(), 0.0);
-  hpm = block_reduce(hpm, OpAdd(), 0.0);
-  pdm = block_reduce(pdm, OpAdd(), 0.0);
-  nc = block_reduce(nc, OpAdd(), 0.0);
-  if (threadIdx.x == 0) {
-    a.part[4 * blockIdx.x + 0] = dmu; a.part[4 * blockIdx.x + 1] = hpm;
-    a.part[4 * blockIdx.x + 2] = pdm; a.part[4 * blockIdx.x + 3] = nc;
-  }
-}
-
-__global__ void __launch_bounds__(ACC_BX) k_acc_limiter(const AccArgs *__restrict__ ap, double pi, double sqrt2pi_inv)
-{
-  const AccArgs &a = *ap;
-  const int nb = a.nb;
-  if (nb == 0) return;
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int k = 0; k < 4; k++) v[k] += a.part[4 * b + k];
+  if (__syncthreads_or(v[3] > 0.0))
+    for (int k = 0; k < 4; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 4; k++) a.part[4 * blockIdx.x + k] = v[k];
+  if (!acc_last_block(a.ticket)) return;
+  const int nb = gridDim.x;
+  for (int k = 0; k < 4; k++) v[k] = 0.0;
+  for (int b = threadIdx.x; b < nb; b += ACC_BX)
+    for (int k = 0; k < 4; k++) v[k] += __ldcg(a.part + 4 * b + k);
   for (int k = 0; k < 4; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
   if (threadIdx.x == 0) {
     const double dmu = v[0];
@@ -1216,52 +1224,48 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_limiter(const AccArgs *__restric
     const double veloc = (a.Mp < Mt) ? vrel : Reff * a.Omegap;
     double dM_model;
     if (Hpeb_mean < Reff) dM_model = 2.0 * Reff * veloc * pdens_mean;
-    else dM_model = pi * Reff * Reff * veloc * pdens_mean / Hpeb_mean * sqrt2pi_inv;
+    else dM_model = TH_PI * Reff * Reff * veloc * pdens_mean / Hpeb_mean * g.k.sqrt2pi_inv;
     dM_model *= a.dt;
     a.acc[3] = (dmu > dM_model) ? dM_model / dmu : 1.0;
   }
 }
 
-__global__ void __launch_bounds__(ACC_BX) k_acc_apply(DevGrid g, const AccArgs *__restrict__ ap)
+// The accreted mass out of the cells (Pebbles.c:479-520) and its sum and
+// momentum.
+__global__ void __launch_bounds__(ACC_BX) k_acc_apply(DevGrid g, const AccArgs *__restrict__ ap, double *__restrict__ scal)
 {
   const AccArgs &a = *ap;
-  if ((int)blockIdx.x >= a.nb) return;           // grid sized for the widest annulus
+  if (a.nb == 0) return;                         // no annulus
   const int ns = g.ns;
   const int ncells = (a.imax - a.imin + 1) * ns;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const double limiter = a.acc[3];
-  double dM_s = 0.0, dPx = 0.0, dPy = 0.0;
-  if (q < ncells) {
+  double v[3] = {0.0, 0.0, 0.0};                 // mass and momentum
+  for (int q = blockIdx.x * ACC_BX + threadIdx.x; q < ncells; q += gridDim.x * ACC_BX) {
     const int i = a.imin + q / ns, j = q - (q / ns) * ns, l = j + i * ns;
-    if (a.macc[l] > 0.0) {
+    const double up = a.macc[l];
+    if (up > 0.0) {
       const double xc = g.r.Rmed[i] * g.r.costab[j], yc = g.r.Rmed[i] * g.r.sintab[j];
       const double vtcorr = g.r.Rmed[i] * a.omega_frame;
       const double vrc = a.pvr[l], vtc = a.pvt[l] + vtcorr;
       const double vxc = (vrc * xc - vtc * yc) * g.r.InvRmed[i], vyc = (vrc * yc + vtc * xc) * g.r.InvRmed[i];
-      const double dM = a.macc[l] * limiter;
+      const double dM = up * limiter;
       a.macc[l] = 0.0;
       const double mcell = g.r.Surf[i] * a.pdens[l];
       double pd = (mcell - dM) / g.r.Surf[i];
       if (pd < 0.0) pd = 1.e-20;
       a.pdens[l] = pd;
-      dM_s = dM; dPx = dM * vxc; dPy = dM * vyc;
+      v[0] += dM; v[1] += dM * vxc; v[2] += dM * vyc;
     }
   }
-  dM_s = block_reduce(dM_s, OpAdd(), 0.0);
-  dPx = block_reduce(dPx, OpAdd(), 0.0);
-  dPy = block_reduce(dPy, OpAdd(), 0.0);
-  if (threadIdx.x == 0) {
-    a.part[3 * blockIdx.x + 0] = dM_s; a.part[3 * blockIdx.x + 1] = dPx; a.part[3 * blockIdx.x + 2] = dPy;
-  }
-}
-
-__global__ void __launch_bounds__(ACC_BX) k_acc_sum(const AccArgs *__restrict__ ap, double *__restrict__ scal)
-{
-  const AccArgs &a = *ap;
-  const int nb = a.nb;
-  double v[3] = {0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int k = 0; k < 3; k++) v[k] += a.part[3 * b + k];
+  if (__syncthreads_or(v[0] != 0.0))
+    for (int k = 0; k < 3; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 3; k++) a.part[3 * blockIdx.x + k] = v[k];
+  if (!acc_last_block(a.ticket)) return;
+  const int nb = gridDim.x;
+  for (int k = 0; k < 3; k++) v[k] = 0.0;
+  for (int b = threadIdx.x; b < nb; b += ACC_BX)
+    for (int k = 0; k < 3; k++) v[k] += __ldcg(a.part + 3 * b + k);
   for (int k = 0; k < 3; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
   if (threadIdx.x == 0) { scal[SC_ACC_DM] = v[0]; scal[SC_ACC_DPX] = v[1]; scal[SC_ACC_DPY] = v[2]; }
 }
@@ -1272,36 +1276,15 @@ int aux_accrete_blocks(const DevGrid &g, int imin, int imax)
   return (ncells + ACC_BX - 1) / ACC_BX;
 }
 
-__global__ void k_set_accargs(AccArgs a, AccArgs *__restrict__ dst)
+void aux_accrete(const DevGrid &g, const AccArgs *a0, AccArgs *a_dev, int nb, double *scal, cudaStream_t s)
 {
-  if (threadIdx.x == 0) *dst = a;
-}
-
-void aux_accrete(const DevGrid &g, const AccArgs &a0, AccArgs *a_dev, double *scal, cudaStream_t s)
-{
-  AccArgs a = a0;
-  a.nb = aux_accrete_blocks(g, a.imin, a.imax);
-  k_set_accargs<<<1, 32, 0, s>>>(a, a_dev);
+  const int grid = nb < 2 * g.nsm ? nb : 2 * g.nsm;
+  if (a0) k_acc_reff<true><<<2 + grid, RING_T, 0, s>>>(g, *a0, a_dev);
+  else k_acc_reff<false><<<2 + grid, RING_T, 0, s>>>(g, AccArgs(), a_dev);
   g_thorin_launches++;
-  aux_ring_means(g, a.vt, a.acc + 4, nullptr, nullptr, a.iflow, (a.iflow + 1 < g.nr) ? 2 : 1, s);
-  aux_accrete_kernels(g, a_dev, a.nb, scal, s);
-}
-
-void aux_accrete_kernels(const DevGrid &g, const AccArgs *a_dev, int nb_grid, double *scal, cudaStream_t s)
-{
-  k_acc_tau<<<nb_grid, ACC_BX, 0, s>>>(g, a_dev);
+  k_acc_upper<<<2 * g.nsm, ACC_BX, 0, s>>>(g, a_dev);
   g_thorin_launches++;
-  k_acc_reff<<<1, ACC_BX, 0, s>>>(g, a_dev);
-  g_thorin_launches++;
-  k_acc_column<<<2 * g.nsm, ACC_BX, 0, s>>>(g, a_dev);
-  g_thorin_launches++;
-  k_acc_upper<<<nb_grid, ACC_BX, 0, s>>>(g, a_dev);
-  g_thorin_launches++;
-  k_acc_limiter<<<1, ACC_BX, 0, s>>>(a_dev, TH_PI, g.k.sqrt2pi_inv);
-  g_thorin_launches++;
-  k_acc_apply<<<nb_grid, ACC_BX, 0, s>>>(g, a_dev);
-  g_thorin_launches++;
-  k_acc_sum<<<1, ACC_BX, 0, s>>>(a_dev, scal);
+  k_acc_apply<<<grid, ACC_BX, 0, s>>>(g, a_dev, scal);
   g_thorin_launches++;
 }
 

@@ -1361,12 +1361,13 @@ extern "C" int thorin_gpu_accrete(thorin_disk *d, thorin_planets *sys, double dt
     a.vt = d->vtheta;
     a.part = d->partials;
     a.acc = d->scal + 64;
+    a.ticket = d->ticket + 11;
     pl_pebble_acc_prep(d->plc, d->Rinf.data(), d->Rsup.data(), d->GlobalRmed.data(), sys, k, d->OmegaFrame, dt,
                        ACC_BX, &a);
     const int imin = a.imin, imax = a.imax;
     double dMp = 0, dPx = 0, dPy = 0;
     if (imin <= imax) {
-      aux_accrete(d->g, a, d->acc_args_d, d->scal, d->s);
+      aux_accrete(d->g, &a, d->acc_args_d, a.nb, d->scal, d->s);
       KCHECK("accretion kernel");
       CUCHK(cudaMemcpyAsync(d->scal_h + SC_ACC_DM, d->scal + SC_ACC_DM, 3 * sizeof(double), cudaMemcpyDeviceToHost, d->s));
       CUCHK(cudaStreamSynchronize(d->s));
@@ -2176,8 +2177,7 @@ static int capture_substep(thorin_disk *d)
     const int nb_max = aux_accrete_blocks(d->g, 0, d->nr - 1);
     for (int k = 0; k < npl; k++) {
       graph_acc_prep(S, k, d->s);
-      graph_ring_means_at(d->g, d->vtheta, d->scal + 64 + 4, d->ring_info_d, 0, 1, d->s);
-      aux_accrete_kernels(d->g, S.acc, nb_max, d->scal, d->s);
+      aux_accrete(d->g, nullptr, S.acc, nb_max, d->scal, d->s);
       graph_acc_finish(S, k, d->s);
     }
     if (p.evaporation_rate > 0.0) aux_evaporate(d->g, d->temper, d->pdens, d->s);
@@ -2185,7 +2185,7 @@ static int capture_substep(thorin_disk *d)
   graph_force_prep(S, d->s);
   aux_forces(d->g, force_args(d, npl), d->fr, d->scal, d->s);
   for (int k = 0; k < npl; k++)
-    graph_ring_means_at(d->g, d->rho, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->ring_info_d, 2 + k, 0, d->s);
+    graph_ring_mean_at(d->g, d->rho, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->ring_info_d + k, d->s);
   // the planet kick and N-body step run beside the hydro substep, which does
   // not read the planets; the next substep's CFL waits for them
   CUCHK(cudaEventRecord(d->ev_pl_fork, d->s));
@@ -2242,7 +2242,7 @@ static int build_dt_graph(thorin_disk *d, int npl)
   if (!d->sys_d) {
     RCHK(dalloc(d, (void **)&d->sys_d, sizeof(thorin_planets)));
     RCHK(dalloc(d, (void **)&d->gst_d, sizeof(GraphStats)));
-    RCHK(dalloc(d, (void **)&d->ring_info_d, (2 + MAXPL_DEV) * sizeof(int)));
+    RCHK(dalloc(d, (void **)&d->ring_info_d, MAXPL_DEV * sizeof(int)));
     RCHK(dalloc(d, (void **)&d->acc_args_g, sizeof(AccArgs)));
     CUCHK(cudaMallocHost((void **)&d->sys_h, sizeof(thorin_planets)));
     CUCHK(cudaMallocHost((void **)&d->gst_h, sizeof(GraphStats)));
@@ -2260,6 +2260,7 @@ static int build_dt_graph(thorin_disk *d, int npl)
   a.vt = d->vtheta;
   a.part = d->partials;
   a.acc = d->scal + 64;
+  a.ticket = d->ticket + 11;
   CUCHK(cudaMemcpyAsync(d->acc_args_g, &a, sizeof(a), cudaMemcpyHostToDevice, d->s));
   CUCHK(cudaStreamSynchronize(d->s));
   StepDev &S = d->capS;

@@ -50,8 +50,7 @@ __global__ void k_g_acc_init(StepDev S)
   S.g.ctl[CTL_FACC_EVAP] = facc;
 }
 
-// AccretePebblesOntoPlanets' set-up for planet k; the ring means of v_theta
-// at the planet's ring follow from ring_info[0..1].
+// AccretePebblesOntoPlanets' set-up for planet k.
 __global__ void k_g_acc_prep(StepDev S, int k)
 {
   if (threadIdx.x != 0) return;
@@ -59,8 +58,6 @@ __global__ void k_g_acc_prep(StepDev S, int k)
   pl_pebble_acc_prep(S.c, S.g.r.Rinf, S.g.r.Rsup, S.g.r.Rmed, S.sys, k, S.g.ctl[CTL_OMEGA_FRAME], S.g.ctl[CTL_DT],
                      ACC_BX, &a);
   *S.acc = a;
-  S.ring_info[0] = a.nb > 0 ? a.iflow : -1;
-  S.ring_info[1] = (a.iflow + 1 < S.g.nr) ? 2 : 1;
 }
 
 // Heating1 and the planet's new mass and velocity after the accretion.
@@ -96,7 +93,7 @@ __global__ void k_g_force_prep(StepDev S)
     const double x = S.sys->x[k], y = S.sys->y[k];
     const double r = sqrt(x * x + y * y);
     const int i = (r >= S.c.rin && r <= S.c.rout) ? pl_ring_of(S.g.r.Rsup, S.c.nr, r) : -1;
-    S.ring_info[2 + k] = i;
+    S.ring_info[k] = i;
     // the planet step runs beside the hydro substep, which rewrites the
     // ring means of c_s at its end: DampingTW04's value is taken now
     S.scal[SC_RCS + k] = (i >= 0) ? S.g.r.csmean[i] : 0.0;
@@ -186,7 +183,7 @@ __global__ void __launch_bounds__(32) k_g_planet_step(StepDev S)
     for (int k = 0; k < S.npl; k++) {
       sys->ax[k] = S.scal[SC_PLANET_A + 2 * k];
       sys->ay[k] = S.scal[SC_PLANET_A + 2 * k + 1];
-      const int i = S.ring_info[2 + k];
+      const int i = S.ring_info[k];
       rrho[k] = (i >= 0) ? S.scal[SC_PLANET_A + 2 * MAXPL_DEV + k] : 0.0;
       rcs[k] = (i >= 0) ? S.scal[SC_RCS + k] : 0.0;
     }

@@ -30,7 +30,7 @@ struct StepDev {
   double *scal;
   int *iscal;
   AccArgs *acc;               // pointer fields set by the host once; the scalars per planet and substep
-  int *ring_info;             // [0,1]: accretion ring and ring count; [2 + k]: ring of planet k (-1 outside)
+  int *ring_info;             // ring of planet k (-1 outside)
   DevPlanet *pl;
   int *heat_idx;
   double *heat_val;
@@ -53,8 +53,5 @@ void graph_planet_step(const StepDev &S, cudaStream_t s);
 void graph_sor_begin(const StepDev &S, cudaStream_t s);
 void graph_sor_end(const StepDev &S, cudaStream_t s);
 void graph_sub_end(const StepDev &S, cudaStream_t s);
-// Ring mean of f at ring ring_info[slot] (count ring_info[slot + 1] when
-// two_slots, else 1 if the ring is >= 0), with the summation of
-// aux_ring_means; out[0..n).
-void graph_ring_means_at(const DevGrid &g, const double *f, double *out, const int *ring_info, int slot, int two_slots,
-                         cudaStream_t s);
+// Ring mean of f at ring *ring (device; none when it is negative).
+void graph_ring_mean_at(const DevGrid &g, const double *f, double *out, const int *ring, cudaStream_t s);

@@ -155,7 +155,8 @@ struct GasAccArgs {           // one planet of AccreteOntoPlanets (Planet.c:34-1
 struct AccArgs {
   double *pdens, *macc;
   double *part;               // block partials (4 per block)
-  double *acc;                // scalars: Reff, vrel, Mt, limiter
+  double *acc;                // scalars: Reff, vrel, Mt, limiter, ring means of v_theta
+  unsigned int *ticket;
   const double *pvr, *pvt, *tau, *cs, *vt;
   double Xp, Yp, Zp, VXp, VYp, VZp, Mp, Rp, Rhill, Omegap, Rp15, omega_frame, dt, pebble_alpha, frac;
   int imin, imax, iflow;
@@ -234,12 +235,9 @@ void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const 
 void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s);
 void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
                 double *scal, cudaStream_t s);
-// AccArgs go to the device first (a_dev), the kernels read them there.
-void aux_accrete(const DevGrid &g, const AccArgs &a, AccArgs *a_dev, double *scal, cudaStream_t s);
-// The accretion kernels alone over a grid of nb_grid blocks (at least the
-// annulus' aux_accrete_blocks; blocks beyond it return at once), arguments
-// and the two ring means of v_theta already on the device.
-void aux_accrete_kernels(const DevGrid &g, const AccArgs *a_dev, int nb_grid, double *scal, cudaStream_t s);
+// Pebble accretion with the arguments a0, which go to a_dev, or, with a0 NULL,
+// with those at a_dev; nb: aux_accrete_blocks of the widest annulus possible.
+void aux_accrete(const DevGrid &g, const AccArgs *a0, AccArgs *a_dev, int nb, double *scal, cudaStream_t s);
 // Control block writes (host path): up to 6 (index, value) pairs.
 struct CtlSet { int n; int idx[6]; double val[6]; };
 void aux_set_ctl(double *ctl, const CtlSet &v, cudaStream_t s);
