@@ -919,6 +919,8 @@ __device__ __forceinline__ void sor_resid_sums(const SorCtl &c, double a, double
       *c.done = 0;
       *c.niter = 0;
       *c.ticket = 0u;
+      *c.epoch += 1ULL;
+      *c.abort = 0;
     }
   }
 }
@@ -1174,145 +1176,232 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
   }
 }
 
-// The whole solve of a small disk in one launch: a cluster of 16 blocks
-// (one per multiprocessor of a GPC, scheduled together by the hardware) keeps
-// the system in shared memory and separates the colour passes by cluster
-// barriers.  A pass as a launch of its own takes 4 to 5 us on a small disk,
-// nearly all of it the launch, the load latency and the completion, and the
-// sweep loop's graph runs up to seven sweeps too many; here a pass of a few
-// thousand cells takes 2.3 us, two thirds of it the L2 latency of the
-// neighbours, the chain of FP64 instructions (64 cycles each) and the barrier.
-// 24x72: a DT 321 -> 291 us.  Each block owns `per` consecutive cells
-// of each colour: their seven coefficients, temperatures and neighbour offsets
-// are in shared memory; the neighbours' temperatures come from L2 (__ldcg),
-// where every update is written before the barrier (release at the arrival,
-// acquire at the wait).  The L1 norm is summed per block in a fixed order,
-// handed to every block of the cluster through distributed shared memory, and
-// all blocks add the partials in the same order, so all take the same exit.
-// The loop ends at the iteration cap at the latest; no block waits for
-// anything but the hardware barrier.
-#define SOR_CLUSTER 16
-#define SOR_CLUSTER_CELLS 36000       // largest disk (cells of rings 1 .. nr-2)
+// The whole solve in one cooperative launch, one block per multiprocessor.  A
+// pass as a launch of its own has 0.1 to 10 us of FP64 work on disks of up to
+// 700 x 2100 and takes 5.3 us (96x288) to 15 (700x2100); the rest is launch,
+// load latency and completion.  Here a block keeps its cells from sweep to
+// sweep (consecutive column pairs of one red and one black cell; temperatures
+// and, as far as they fit, coefficients in shared memory, the others streamed
+// from L2), and a cell whose neighbour belongs to another block waits for
+// that neighbour's value alone: every update goes to x as one 16-byte store of
+// the value and a tag (number of the solve, number of the sweep), which a
+// relaxed 16-byte load sees whole, so there is no barrier across the grid, no
+// fence and no flag.  No slot is written too early: a cell's next value needs
+// what every neighbour computed from this one.
+// The exit test runs beside the next sweep: a warp of its own in each block
+// sums the threads' |resid| of a sweep (in a fixed order, as all sums here),
+// that of block 0 adds the blocks' records and posts the verdict, which the
+// blocks take up at the end of the next sweep; the result is the sweep before,
+// still in the other of x's two buffers.  So a solve runs one sweep more than
+// it needs.  The updates are the passes' own, bit for bit.
+// All blocks are resident together (cooperative launch); each wait has a
+// limit, after which the solve ends without a verdict, and the caller reports
+// that.
+// us a pass, launches / here: 24x72 6.2 / 2.25, 128x384 5.7 / 1.9, 256x768 6.8 /
+// 2.5, 333x1002 8.0 / 3.3, 384x1152 8.6 / 3.9, 512x1536 10.8 / 6.0, 640x1920 12.9 /
+// 9.1, 700x2100 15.2 / 11.1, 850x2550 19.3 / 18.9, 1024x3072 25.8 / 28.2: there the
+// coefficients no longer fit in L2 beside x, so SOR_GRID_CELLS lies between the
+// last two.  Coefficients all streamed: 192x576 2.8 (2.1 in shared memory),
+// 333x1002 3.4, 640x1920 9.7.
+#define SOR_GRID_CELLS 2400000        // largest disk (cells of rings 1 .. nr-2)
+#define SOR_GRID_SPIN (1 << 22)       // loads of one wait, about 3 s
 
-__device__ __forceinline__ void cluster_sync_all()
+__device__ __forceinline__ void x_load(const ulonglong2 *p, unsigned long long &v, unsigned long long &tag)
 {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(v), "=l"(tag) : "l"(p) : "memory");
 }
 
-__device__ __forceinline__ unsigned cluster_rank()
+__device__ __forceinline__ void x_store(ulonglong2 *p, unsigned long long v, unsigned long long tag)
 {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+               ::"l"(p), "l"(v), "l"(tag) : "memory");
 }
 
-// Store to the same shared variable of block `rank` of the cluster.
-__device__ __forceinline__ void cluster_store(double *p, unsigned rank, double v)
+// Loads until the tag (shifted right) is there; false when the wait ran out.
+__device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long want, int shift, int *abort,
+                                       unsigned long long &v, unsigned long long &tag)
 {
-  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+  for (int n = 1; (tag >> shift) != want; n++) {
+    if ((n & 1023) == 0 && (n >= SOR_GRID_SPIN || *(volatile int *)abort)) {
+      *(volatile int *)abort = 1;
+      return false;
+    }
+    x_load(p, v, tag);
+  }
+  return true;
 }
 
-__global__ void __launch_bounds__(512) k_sor_cluster(DevGrid g, double *__restrict__ T, const double *__restrict__ ml,
-                                                     const double *__restrict__ mlip, const double *__restrict__ mlim,
-                                                     const double *__restrict__ mljp, const double *__restrict__ mljm,
-                                                     const double *__restrict__ rhs, const double *__restrict__ cw,
-                                                     SorCtl c, double eps, int maxiters, int per)
+struct SorSystem { const double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *cw; };
+
+__global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, SorCtl c, ulonglong2 *x, double eps,
+                                           int maxiters, int R, int res)
 {
   extern __shared__ double sm[];
-  __shared__ double red[512], part[2][SOR_CLUSTER], cpart[2][SOR_CLUSTER];
-  __shared__ int cnt, verdict;
-  double *co = sm;                                 // [7][2 per]
-  double *ts = sm + 14 * per;                      // [2 per]
-  int *li = (int *)(ts + 2 * per);                 // [2 per]: 4 l + (j == ns - 1) + 2 (j == 0)
-  const int ns = g.ns, half = ns >> 1, total = half * (g.nr - 2);
-  const unsigned rank = cluster_rank();
-  const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
-  const int first = (int)rank * per, n = min(per, total - first);      // may be <= 0
-  for (int q = t; q < 2 * per; q += nt) {
-    const int col = q / per, idx = first + (q - col * per);
-    if (idx >= total) continue;
-    const int r = idx / half, k = idx - r * half, i = r + 1;
-    const int j = 2 * k + ((r + col) & 1), l = j + i * ns;
-    const size_t p = (size_t)((i << 1) + col) * half + k;
-    const int w = 2 * per;
-    co[q] = ml[p]; co[w + q] = mlip[p]; co[2 * w + q] = mlim[p]; co[3 * w + q] = mljp[p]; co[4 * w + q] = mljm[p];
-    co[5 * w + q] = rhs[p]; co[6 * w + q] = cw[p];
-    ts[q] = T[l];
-    li[q] = 4 * l + (j == ns - 1 ? 1 : 0) + (j == 0 ? 2 : 0);
+  __shared__ int sdec[2];
+  const int ns = g.ns, half = ns >> 1, nr = g.nr, np = half * (nr - 2);
+  const int nb = gridDim.x, b = blockIdx.x, nt = blockDim.x - 32, tid = threadIdx.x;
+  const int g0 = (int)((long long)np * b / nb), P = (int)((long long)np * (b + 1) / nb) - g0;
+  const int Pm = (np + nb - 1) / nb;
+  double *sT = sm, *sA = sT + 2 * Pm, *sco = sA + 2 * nt;
+  int *sC = (int *)(sco + 14 * res), *sJ = sC + 2 * nt;
+  ulonglong2 *rec = x + 4 * (size_t)np, *verdict = rec + nb;
+  if (*(volatile int *)c.done) return;             // the same for all blocks: set at the end of a solve only
+  const unsigned long long ep = *(volatile unsigned long long *)c.epoch << 24;   // tag: solve, sweep
+  if (tid < 2) sdec[tid] = 0;
+
+  if (tid >= nt) {                                 // the exit test's warp
+    const int lane = tid - nt;
+    const double r0 = *c.normres0;
+    __syncthreads();
+    bool dead = false;
+    for (int n = 1;; n++) {
+      if (__syncthreads_or(dead)) return;          // end of sweep n
+      if (n > 1 && sdec[(n - 1) & 1]) return;
+      double s = 0.0;
+      int ch = 0;
+      for (int t = lane; t < nt; t += 32) {
+        s += sA[(n & 1) * nt + t];
+        ch += sC[(n & 1) * nt + t];
+      }
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
+      ch = __reduce_add_sync(TH_FULL, ch);
+      if (lane == 0)
+        x_store(rec + b, (unsigned long long)__double_as_longlong(s), ((ep | (unsigned)n) << 13) | (unsigned)min(ch, 8191));
+      const unsigned long long want = ((ep | (unsigned)n) << 13) >> 13;
+      unsigned long long v, tag = ~want << 13;
+      int dec = 0;
+      if (b == 0) {
+        s = 0.0;
+        ch = 0;
+        for (int k = lane; k < nb; k += 32) {
+          tag = ~want << 13;
+          if (!x_wait(rec + k, want, 13, c.abort, v, tag)) { dead = true; break; }
+          s += __longlong_as_double((long long)v);
+          ch += (int)(tag & 8191u);
+        }
+        dead = __any_sync(TH_FULL, dead);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
+        ch = __reduce_add_sync(TH_FULL, ch);
+        if (dead) continue;
+        dec = (s < eps * r0 || s < TH_SORMIN || ch == 0) ? 1 : (n >= maxiters ? 2 : 0);
+        if (lane == 0) {
+          if (dec) {
+            *c.normres = s;
+            *c.changed = ch;
+            *c.niter = n;
+            *c.done = dec;
+          }
+          x_store(verdict, (unsigned long long)dec, ep | (unsigned)n);
+        }
+      } else {
+        tag = ~(ep | (unsigned)n);
+        if (lane == 0) dead = !x_wait(verdict, ep | (unsigned)n, 0, c.abort, v, tag);
+        dead = __any_sync(TH_FULL, dead);
+        dec = dead ? 0 : (int)__shfl_sync(TH_FULL, (unsigned)v, 0);
+      }
+      if (lane == 0) sdec[n & 1] = dec;
+    }
   }
-  const double thr = eps * *c.normres0;
-  int it = 0, dn = 0;
-  cluster_sync_all();                              // every block of the cluster has started
-  while (!dn) {
-    it++;
-    const int buf = it & 1;
+
+  // Row q of the thread is the block's pair p = q nt + tid; sJ: 2 k of its ring
+  // plus the ring's parity, so that colour c sits in column sJ ^ c.  x: two
+  // buffers (sweep & 1) of the red and the black cells.
+  for (int q = 0; q < R; q++) {
+    const int p = q * nt + tid;
+    if (p >= P) break;
+    const int gg = g0 + p, r = gg / half, k = gg - r * half, j = 2 * k + (r & 1);
+    sJ[p] = j;
+    double t = 0.0;
+    for (int col = 0; col < 2; col++) {
+      t = T[(size_t)(r + 1) * ns + (j ^ col)];
+      sT[col * Pm + p] = t;
+      if (p < res) {
+        const size_t e = (size_t)2 * (gg + half) - k + col * half;             // sor_pidx
+        double *w = sco + col * 7 * res + p;
+        w[0] = m.ml[e]; w[res] = m.mlip[e]; w[2 * res] = m.mlim[e]; w[3 * res] = m.mljp[e];
+        w[4 * res] = m.mljm[e]; w[5 * res] = m.rhs[e]; w[6 * res] = m.cw[e];
+      }
+    }
+    x_store(x + np + gg, (unsigned long long)__double_as_longlong(t), ep);      // the black cells before sweep 1
+  }
+  __syncthreads();
+  bool dead = false;
+  int dec = 0, n = 0;
+  while (!dec) {
+    n++;
     double a = 0.0;
     int ch = 0;
-    if (t == 0) cnt = 0;
-#pragma unroll 1
     for (int col = 0; col < 2; col++) {
-      const int w = 2 * per;
-      for (int q = t; q < n; q += nt) {
-        const int p = col * per + q, f = li[p], l = f >> 2;
-        const double tip = __ldcg(T + l + ns), tim = __ldcg(T + l - ns);
-        const double tjp = __ldcg(T + l + ((f & 1) ? 1 - ns : 1)), tjm = __ldcg(T + l + ((f & 2) ? ns - 1 : -1));
-        const double t0 = ts[p];
-        double resid = __fma_rn(t0, co[p], -co[5 * w + p]);
-        resid = __fma_rn(tip, co[w + p], resid);
-        resid = __fma_rn(tim, co[2 * w + p], resid);
-        resid = __fma_rn(tjp, co[3 * w + p], resid);
-        resid = __fma_rn(tjm, co[4 * w + p], resid);
-        a += abs_i(resid);
-        const double m = co[6 * w + p];
-        const double tn = __fma_rn(-resid, m, t0);
-        ts[p] = tn;
-        __stcg(T + l, tn);
-        ch += sor_changed(resid, m, tn) ? 1 : 0;
-      }
-      if (col == 0) cluster_sync_all();
-    }
-    red[t] = a;
-    ch = __reduce_add_sync(TH_FULL, ch);
-    __syncthreads();                               // red and the cleared count
-    if (lane == 0 && ch) atomicAdd(&cnt, ch);
-    if (warp < 4) {                                // one warp per sub-partition adds a quarter of the threads' values
-      const int nw = nt >> 5;
-      double s = 0.0;
-      for (int v = warp; v < nw; v += 4) s += red[32 * v + lane];
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
-      a = s;
-    }
-    __syncthreads();
-    if (warp < 4 && lane == 0) red[warp] = a;
-    __syncthreads();
-    if (t < SOR_CLUSTER) {
-      const int nw = min(nt >> 5, 4);
-      double s = red[0];
-      for (int v = 1; v < nw; v++) s += red[v];
-      cluster_store(&part[buf][rank], t, s);
-      cluster_store(&cpart[buf][rank], t, (double)cnt);
-    }
-    cluster_sync_all();                            // temperatures and partials of the whole cluster
-    if (warp == 0) {
-      double s = (lane < SOR_CLUSTER) ? part[buf][lane] : 0.0, e = (lane < SOR_CLUSTER) ? cpart[buf][lane] : 0.0;
-      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(TH_FULL, s, o);
-      for (int o = 8; o > 0; o >>= 1) e += __shfl_xor_sync(TH_FULL, e, o);
-      if (lane == 0) {
-        dn = (s < thr || s < TH_SORMIN || e == 0.0) ? 1 : (it >= maxiters ? 2 : 0);
-        verdict = dn;
-        if (dn && rank == 0) {
-          *c.normres = s;
-          *c.changed = (int)e;
-          *c.niter = it;
-          *c.done = dn;
+      const int nw = n - 1 + col;                  // sweep of the neighbours' values
+      const unsigned long long want = ep | (unsigned)nw;
+      const ulonglong2 *xo = x + (size_t)(2 * (nw & 1) + 1 - col) * np + g0;    // by pair of the block
+      ulonglong2 *xn = x + (size_t)(2 * (n & 1) + col) * np + g0;
+      const double *so = sT + (1 - col) * Pm;
+      // the rows at the block's ends first: their values are what the other
+      // blocks wait for, and the rows between cover the way there
+      for (int z = 0; z < R; z++) {
+        const int q = (z & 1) ? R - 1 - (z >> 1) : (z >> 1), p = q * nt + tid;
+        if (p >= P) continue;
+        const int jr = sJ[p], k = jr >> 1;
+        const bool odd = (jr ^ col) & 1;
+        // the neighbour on the side away from the other cell of the pair
+        const int sd = odd ? (k == half - 1 ? p - half + 1 : p + 1) : (k == 0 ? p + half - 1 : p - 1);
+        const bool xup = p + half >= P && g0 + p + half < np, xdn = p < half && g0 + p >= half;
+        const bool xsd = (unsigned)sd >= (unsigned)P;
+        unsigned long long v0, v1, v2, t0, t1, t2;
+        if (xup) x_load(xo + p + half, v0, t0);
+        if (xdn) x_load(xo + p - half, v1, t1);
+        if (xsd) x_load(xo + sd, v2, t2);
+        SorRow w;
+        if (p < res) {
+          const double *s = sco + col * 7 * res + p;
+          w = SorRow{s[0], s[res], s[2 * res], s[3 * res], s[4 * res], s[5 * res], s[6 * res]};
+        } else {
+          const size_t e = (size_t)2 * (g0 + p + half) - k + col * half;
+          w = SorRow{m.ml[e], m.mlip[e], m.mlim[e], m.mljp[e], m.mljm[e], m.rhs[e], m.cw[e]};
         }
+        const double own = so[p], tc = sT[col * Pm + p];
+        double tip, tim, ts;
+        if (xup) {
+          if (!x_wait(xo + p + half, want, 0, c.abort, v0, t0)) dead = true;
+          tip = __longlong_as_double((long long)v0);
+        } else tip = (p + half < P) ? so[p + half] : T[(size_t)(nr - 1) * ns + (jr ^ col)];
+        if (xdn) {
+          if (!x_wait(xo + p - half, want, 0, c.abort, v1, t1)) dead = true;
+          tim = __longlong_as_double((long long)v1);
+        } else tim = (p >= half) ? so[p - half] : T[jr ^ col];
+        if (xsd) {
+          if (!x_wait(xo + sd, want, 0, c.abort, v2, t2)) dead = true;
+          ts = __longlong_as_double((long long)v2);
+        } else ts = so[sd];
+        double resid = __fma_rn(tc, w.ml, -w.rhs);
+        resid = __fma_rn(tip, w.mlip, resid);
+        resid = __fma_rn(tim, w.mlim, resid);
+        resid = __fma_rn(odd ? ts : own, w.mljp, resid);
+        resid = __fma_rn(odd ? own : ts, w.mljm, resid);
+        a += abs_i(resid);
+        const double tn = __fma_rn(-resid, w.cw, tc);
+        x_store(xn + p, (unsigned long long)__double_as_longlong(tn), ep | (unsigned)n);
+        sT[col * Pm + p] = tn;
+        ch += sor_changed(resid, w.cw, tn) ? 1 : 0;
       }
+      if (col == 0) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
     }
-    __syncthreads();
-    dn = verdict;
-    __syncthreads();                               // everyone has read it before the next sweep's writes
+    sA[(n & 1) * nt + tid] = a;
+    sC[(n & 1) * nt + tid] = ch;
+    if (__syncthreads_or(dead)) return;
+    if (n > 1) dec = sdec[(n - 1) & 1];
+  }
+  // the exit test passed on the sweep before this one
+  for (int q = 0; q < R; q++) {
+    const int p = q * nt + tid;
+    if (p >= P) break;
+    const int r = (g0 + p) / half;
+    for (int col = 0; col < 2; col++) {
+      const unsigned long long v = x[(size_t)(2 * ((n - 1) & 1) + col) * np + g0 + p].x;
+      T[(size_t)(r + 1) * ns + (sJ[p] ^ col)] = __longlong_as_double((long long)v);
+    }
   }
 }
 
@@ -1852,62 +1941,69 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
   }
 }
 
-// Cells of a colour per block of k_sor_cluster: an even number of whole warps'
-// worth at least.
-static int sor_cluster_per(const DevGrid &g)
+// k_sor_grid's launch: as many rows R of nt threads as hold a block's pairs,
+// the coefficients of its first res pairs (whole warps') in shared memory.
+// A solve alone on the GPU takes up to 1024 threads of a multiprocessor and
+// 200 KB of its memory; with shared set (disks of an ensemble advanced
+// together) it takes three quarters of the multiprocessors and at most half of
+// each, so that two solves and the other disks' kernels fit beside each other:
+// a DT of eight disks of 128 to 512 rings takes 12.7 ms (13.0 on all
+// multiprocessors, 14.2 with the larger blocks); alone the smaller blocks cost
+// 333x1002 3.85 us a pass instead of 3.3, 512x1536 6.8 instead of 6.1.
+struct SorGridShape { int nb, nt, R, res; size_t smem; };
+
+static SorGridShape sor_grid_shape(const DevGrid &g, int shared)
 {
-  const long long total = (long long)(g.ns / 2) * (g.nr - 2);
-  const int per = (int)((total + SOR_CLUSTER - 1) / SOR_CLUSTER);
-  return per < 32 ? 32 : (per + 1) / 2 * 2;
+  const int np = (g.ns >> 1) * (g.nr - 2), most = shared ? 480 : 992;
+  const int nsm = shared ? (3 * g.nsm + 3) / 4 : g.nsm;
+  SorGridShape q;
+  q.nb = (np + 31) / 32 < nsm ? (np + 31) / 32 : nsm;
+  const int pm = (np + q.nb - 1) / q.nb;
+  q.R = (pm + most - 1) / most;
+  q.nt = ((pm + q.R - 1) / q.R + 31) / 32 * 32;
+  const size_t room = (shared ? 110 : 200) * 1024, fixed = 20 * (size_t)pm + 24 * (size_t)q.nt;
+  q.res = fixed < room ? (int)((room - fixed) / (32 * 112)) * 32 : 0;
+  if (q.res > pm) q.res = (pm + 31) / 32 * 32;
+  q.smem = fixed + 112 * (size_t)q.res;
+  return q;
 }
 
-static size_t sor_cluster_smem(int per) { return (size_t)per * (16 * sizeof(double) + 2 * sizeof(int)); }
-
-static void sor_cluster_config(const DevGrid &g, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, cudaStream_t s)
+int hydro_sor_grid_fits(const DevGrid &g, int maxiters)
 {
-  const int per = sor_cluster_per(g), nt = (per + 31) / 32 * 32;
-  cfg = cudaLaunchConfig_t{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = SOR_CLUSTER;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(SOR_CLUSTER);
-  cfg.blockDim = dim3(nt > 512 ? 512 : nt);
-  cfg.dynamicSmemBytes = sor_cluster_smem(per);
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-}
-
-// Whether a disk's solves run as one cluster launch each: the system fits the
-// shared memory of 16 blocks, 16 multiprocessors' FP64 is no slower than a
-// launch per pass on all of them (us a pass here and there: 24x72 2.3 / 4,
-// 96x288 4.2 / 5.2, 128x384 5.6 / 5.4), and the GPU can place the cluster.
-// Called once per disk; sets the kernel's launch limits in the current context.
-int hydro_sor_cluster_fits(const DevGrid &g)
-{
-  if ((long long)g.ns * (g.nr - 2) > SOR_CLUSTER_CELLS) return 0;
-  if (cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024) != cudaSuccess) {
+  if (g.nr < 3 || (g.ns & 1) || (long long)g.ns * (g.nr - 2) > SOR_GRID_CELLS || maxiters >= (1 << 24) - 2) return 0;
+  const SorGridShape q = sor_grid_shape(g, 0);     // the larger blocks
+  if (q.smem > 227 * 1024 - 256 || q.nb >= SOR_GRID_RECORDS) return 0;
+  int dev = 0, coop = 0, sms = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || !coop) {
     cudaGetLastError();
     return 0;
   }
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at;
-  sor_cluster_config(g, cfg, at, nullptr);
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_sor_cluster, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
-  return n >= 1;
+  if (cudaFuncSetAttribute(k_sor_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 256) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sor_grid, q.nt + 32, q.smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n * sms >= q.nb;
 }
 
-void hydro_sor_cluster(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
-                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                       double eps, int maxiters, cudaStream_t s)
+void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                    const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                    void *x, double eps, int maxiters, int shared, cudaStream_t s)
 {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at;
-  sor_cluster_config(g, cfg, at, s);
-  cudaLaunchKernelEx(&cfg, k_sor_cluster, g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c, eps, maxiters,
-                     sor_cluster_per(g));
+  const SorGridShape q = sor_grid_shape(g, shared);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.gridDim = dim3(q.nb);
+  cfg.blockDim = dim3(q.nt + 32);
+  cfg.dynamicSmemBytes = q.smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const SorSystem m = {ml, mlip, mlim, mljp, mljm, rhs, cw};
+  cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res);
 }
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)

@@ -208,7 +208,9 @@ struct thorin_disk {
   cudaGraphExec_t sor_loop = nullptr;
   int sor_loop_k = 8;            // sweeps per run of the loop body
   int sor_direct = 0;            // sweeps as plain stream launches (for kernel profilers)
-  int sor_cluster = 0;           // a solve is one cluster launch (small disks)
+  int sor_one = 0;               // a solve is one cooperative launch
+  int sor_shared = 0;            // its blocks leave room for other disks' (set by the ensemble calls)
+  void *sor_x = nullptr;         // cells exchanged between the blocks of k_sor_grid
   double heatsrc[THORIN_MAXPLANETS];
   int heatsrc_index[THORIN_MAXPLANETS], heatsrc_max;
   double gm1, gg1, drin, drout, invdphi, lr01, lr12, taueff_c, tirr4fac, rstar;
@@ -490,10 +492,14 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   d->sor.normres0 = sp;
   d->sor.normres = sp + 1;
   d->sor.jscale = sp + 2;
+  d->sor.epoch = (unsigned long long *)(sp + 3);
   d->sor.ipart = ip + 8;
   d->sor.done = ip;
   d->sor.niter = ip + 1;
   d->sor.changed = ip + 2;
+  d->sor.abort = ip + 3;
+  CUCHK(cudaMemset(sp, 0, 8 * sizeof(double)));
+  CUCHK(cudaMemset(ip, 0, 8 * sizeof(int)));
   d->sor.ticket = d->ticket;
   d->sor.cond = 0;
   d->sor.has_cond = 0;
@@ -502,7 +508,12 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     if (k >= 1 && k <= 64) d->sor_loop_k = k;
   }
   if (const char *ed = getenv("THORIN_SOR_DIRECT")) d->sor_direct = (atoi(ed) != 0);
-  d->sor_cluster = !d->sor_direct && hydro_sor_cluster_fits(d->g);
+  d->sor_one = !d->sor_direct && hydro_sor_grid_fits(d->g, d->p.sor_maxiters);
+  if (d->sor_one) {
+    const size_t bytes = 16 * (2 * (size_t)(d->nr - 2) * d->ns + SOR_GRID_RECORDS);
+    RCHK(dalloc(d, &d->sor_x, bytes));
+    CUCHK(cudaMemset(d->sor_x, 0, bytes));
+  }
   fill_rings(d);
   {
     PlConst &c = d->plc;                 // constants of the planet side of a substep
@@ -1543,6 +1554,13 @@ static int sor_loop_graph(thorin_disk *d)
   return THORIN_OK;
 }
 
+// The sweeps of a solve as one launch (sor_one).
+static void sor_one_launch(thorin_disk *d)
+{
+  hydro_sor_grid(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor, d->sor_x,
+                 d->p.sor_eps, d->p.sor_maxiters, d->sor_shared, d->s);
+}
+
 // SuccessiveOverrelaxation driver: the start residual (and the learned warm
 // start), then the sweep loop graph; one read of the exit state per solve.
 // started: the matrix kernel has formed the start residual at this omega.
@@ -1585,9 +1603,8 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
       if (d->iscal_h[IS_SOR_DONE] || first + d->sor_loop_k > d->p.sor_maxiters) break;
     }
   } else {
-    if (d->sor_cluster) {
-      hydro_sor_cluster(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor,
-                        d->p.sor_eps, d->p.sor_maxiters, d->s);
+    if (d->sor_one) {
+      sor_one_launch(d);
     } else {
       RCHK(sor_loop_graph(d));
       CUCHK(cudaGraphLaunch(d->sor_loop, d->s));
@@ -1604,7 +1621,7 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
   }
   *niter = n;
   *capped = (done == 2);
-  g_thorin_launches += (d->sor_cluster && !d->sor_direct) ? 1LL : 2LL * n;
+  g_thorin_launches += (d->sor_one && !d->sor_direct) ? 1LL : 2LL * n;
   if (d->timing) {
     float ms = 0.f;
     CUCHK(cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]));
@@ -2115,9 +2132,8 @@ static int capture_sor(thorin_disk *d)
                           d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->ctl + CTL_SOR_OMEGA, d->ws_jac,
                           d->ws_vq, d->ws_part, d->ws_step, d->g.nsm, d->s));
   }
-  if (d->sor_cluster) {
-    hydro_sor_cluster(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor,
-                      d->p.sor_eps, d->p.sor_maxiters, d->s);
+  if (d->sor_one) {
+    sor_one_launch(d);
   } else {
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg;
@@ -2235,7 +2251,7 @@ static const char *graph_unsupported(const thorin_disk *d, const thorin_planets 
   return nullptr;
 }
 
-static int build_dt_graph(thorin_disk *d, int npl)
+static int capture_dt_graph(thorin_disk *d, int npl)
 {
   const thorin_params &p = d->p;
   if (d->dt_graph) { cudaGraphExecDestroy(d->dt_graph); d->dt_graph = nullptr; }
@@ -2283,7 +2299,7 @@ static int build_dt_graph(thorin_disk *d, int npl)
     if (rc == THORIN_OK && e2 != cudaSuccess) e = e2;
   }
   // the substep body, with the SOR loop's node inside it
-  const bool loop = !d->sor_cluster;
+  const bool loop = !d->sor_one;
   S.sor_loop = loop;
   if (loop && e == cudaSuccess && rc == THORIN_OK) e = cudaGraphConditionalHandleCreate(&S.h_sor, body, 1u, cudaGraphCondAssignDefault);
   if (e == cudaSuccess && rc == THORIN_OK) e = cudaStreamBeginCaptureToGraph(d->s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
@@ -2295,7 +2311,7 @@ static int build_dt_graph(thorin_disk *d, int npl)
     cudaGraph_t tmp;
     const cudaError_t e2 = cudaStreamEndCapture(d->s, &tmp);
     if (rc == THORIN_OK && e2 != cudaSuccess) e = e2;
-    if (rc == THORIN_OK && e == cudaSuccess && !d->capture_sor_body && !d->sor_cluster) { g_last_error = "no SOR loop in the substep"; rc = THORIN_ERR_STATE; }
+    if (rc == THORIN_OK && e == cudaSuccess && !d->capture_sor_body && !d->sor_one) { g_last_error = "no SOR loop in the substep"; rc = THORIN_ERR_STATE; }
   }
   // the sweeps inside the SOR loop
   if (loop && e == cudaSuccess && rc == THORIN_OK) e = cudaStreamBeginCaptureToGraph(d->s, d->capture_sor_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
@@ -2322,6 +2338,20 @@ static int build_dt_graph(thorin_disk *d, int npl)
   graph_roles(d, roles);
   for (int k = 0; k < 11; k++) d->cap_ptr[k] = *roles[k];
   return THORIN_OK;
+}
+
+static int build_dt_graph(thorin_disk *d, int npl)
+{
+  int rc = capture_dt_graph(d, npl);
+  if (rc != THORIN_OK && d->sor_one) {
+    // a conditional node's body takes no cooperative launch under MPS: the
+    // launches of the passes instead
+    const int one = d->sor_one;
+    d->sor_one = 0;
+    rc = capture_dt_graph(d, npl);
+    d->sor_one = one;
+  }
+  return rc;
 }
 
 // Uploads what the graph reads (planets, clock, frame, omega schedule) and
@@ -2434,6 +2464,9 @@ extern "C" int thorin_gpu_algogas_graph(thorin_disk *d, thorin_planets *sys)
   return graph_finish(d, sys);
 }
 
+// Whether other disks are advanced beside this one (sor_shared).
+void thorin_disk_share(thorin_disk *d, int shared) { d->sor_shared = shared; }
+
 // One DT of n disks: every disk's graph is launched on its own stream before
 // the first is waited for, so the disks run side by side on the GPU.
 extern "C" int thorin_ensemble_algogas_graph(thorin_disk **disks, thorin_planets **systems, int n, int *status)
@@ -2445,9 +2478,11 @@ extern "C" int thorin_ensemble_algogas_graph(thorin_disk **disks, thorin_planets
   std::vector<int> launched(n, 0);
   for (int k = 0; k < n; k++) {
     thorin_disk *d = disks[k];
+    thorin_disk_share(d, n > 1);                   // for the graph if it is built now
     int rc = thorin_gpu_graph_supported(d, systems[k]);
     if (rc == THORIN_OK && graph_host_dt(d)) rc = thorin_gpu_algogas(d, systems[k]);
     else if (rc == THORIN_OK) { rc = graph_launch(d, systems[k]); launched[k] = (rc == THORIN_OK); }
+    thorin_disk_share(d, 0);
     if (status) status[k] = rc;
     if (rc != THORIN_OK && rc != THORIN_ERR_SOR_MAXIT) worst = rc;
   }

@@ -12,6 +12,7 @@
 
 extern thread_local std::string g_last_error;
 long long thorin_disk_cells(const thorin_disk *d);
+void thorin_disk_share(thorin_disk *d, int shared);
 
 static std::vector<int> schedule(thorin_disk *const *disks, int n, int order)
 {
@@ -41,17 +42,19 @@ extern "C" int thorin_ensemble_algogas(thorin_disk *const *disks, thorin_planets
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int> next{0};
+  const int w = std::min(workers, n);
   auto work = [&]() {
     cudaSetDevice(dev);
     for (;;) {
       const int q = next.fetch_add(1);
       if (q >= n) break;
       const int k = idx[q];
+      thorin_disk_share(disks[k], w > 1);
       st[k] = thorin_gpu_algogas(disks[k], systems[k]);
+      thorin_disk_share(disks[k], 0);
       if (st[k] != THORIN_OK) err[k] = g_last_error;
     }
   };
-  const int w = std::min(workers, n);
   std::vector<std::thread> pool;
   for (int t = 1; t < w; t++) pool.emplace_back(work);
   work();

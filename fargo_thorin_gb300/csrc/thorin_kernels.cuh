@@ -36,6 +36,8 @@ struct SorCtl {
   double *normres;
   int *changed;
   double *jscale;         // sum over the start of |resid| * omega/Ml (k_sor_resid0)
+  unsigned long long *epoch;    // number of this solve (k_sor_grid's tags)
+  int *abort;             // a wait of k_sor_grid ran out
   // Condition of the graph's WHILE node around the sweeps: the completion
   // step sets it to 0 together with done (has_cond 0: no such node)
   cudaGraphConditionalHandle cond;
@@ -191,11 +193,15 @@ void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const
 void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
                       double eps, int count, int maxiters, cudaStream_t s);
-// The whole solve of a small disk in one launch, where hydro_sor_cluster_fits.
-int hydro_sor_cluster_fits(const DevGrid &g);
-void hydro_sor_cluster(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
-                       const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                       double eps, int maxiters, cudaStream_t s);
+// The whole solve in one cooperative launch, where
+// hydro_sor_grid_fits; x: 32 bytes a cell of rings 1 .. nr-2 and
+// 16 SOR_GRID_RECORDS more, zero at first; shared: other disks are at work on
+// the GPU.
+#define SOR_GRID_RECORDS 1024
+int hydro_sor_grid_fits(const DevGrid &g, int maxiters);
+void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                    const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                    void *x, double eps, int maxiters, int shared, cudaStream_t s);
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s);
 void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
                      double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,

@@ -44,12 +44,13 @@ def test_grids_at_the_edges_of_the_tiles(kind, nr, ns, over):
     d.close()
 
 
-@pytest.mark.parametrize("nr,ns", [(6, 10), (24, 72), (97, 366), (98, 370), (99, 374)])
-def test_cluster_solve_matches_the_launched_passes(nr, ns, monkeypatch):
-    """Small disks solve in one cluster launch (the largest that does has
-    36000 cells; 97x366 is below, 99x374 above); THORIN_SOR_DIRECT runs a
-    launch per colour pass.  Same updates, so the same bits and sweep counts,
-    on the host path and in the DT graph."""
+@pytest.mark.parametrize("nr,ns", [(4, 6), (6, 10), (24, 72), (97, 366), (6, 4000), (700, 40), (400, 804), (560, 1230)])
+def test_solve_in_one_launch_matches_the_launched_passes(nr, ns, monkeypatch):
+    """A solve is one cooperative launch; THORIN_SOR_DIRECT runs a launch per
+    colour pass.  Same updates, so the same bits and sweep counts, on the host
+    path and in the DT graph: fewer pairs than blocks, rings longer than a
+    block's share and shorter than it, one and several rows a thread, and
+    coefficients partly in shared memory (560x1230)."""
     from fargo_thorin_gb300.disk import GpuDisk
     p = workloads.params_for("disk0", nr, ns)
     out = []
