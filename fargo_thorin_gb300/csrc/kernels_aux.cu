@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(RING_T) k_ring_means(int ns, const double *__r
                                                        const double *__restrict__ f1, double *__restrict__ o0,
                                                        double *__restrict__ o1, int ring0, int nf)
 {
+  pdl_wait();
   const int w = blockIdx.x;
   const size_t base = (size_t)(ring0 + w) * ns;
   const double a0 = ring_sum(f0 + base, ns);
@@ -39,6 +40,7 @@ __global__ void __launch_bounds__(RING_T) k_ring_means(int ns, const double *__r
 __global__ void __launch_bounds__(RING_T) k_ring_mean_at(int ns, const double *__restrict__ f, double *__restrict__ o,
                                                          const int *__restrict__ ring)
 {
+  pdl_wait();
   const int i = *ring;
   if (i < 0) return;
   const double a = ring_sum(f + (size_t)i * ns, ns);
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(RING_T) k_ring_mean_at(int ns, const double *_
 
 void graph_ring_mean_at(const DevGrid &g, const double *f, double *out, const int *ring, cudaStream_t s)
 {
-  k_ring_mean_at<<<1, RING_T, 0, s>>>(g.ns, f, out, ring);
+  launch(k_ring_mean_at, 1, RING_T, 0, s, g.ns, f, out, ring);
   g_thorin_launches++;
 }
 
@@ -55,18 +57,19 @@ void aux_ring_means(const DevGrid &g, const double *f0, double *o0, const double
                     cudaStream_t s)
 {
   if (nrings <= 0) return;
-  k_ring_means<<<nrings, RING_T, 0, s>>>(g.ns, f0, f1 ? f1 : f0, o0, o1 ? o1 : o0, ring0, f1 ? 2 : 1);
+  launch(k_ring_means, nrings, RING_T, 0, s, g.ns, f0, f1 ? f1 : f0, o0, o1 ? o1 : o0, ring0, f1 ? 2 : 1);
   g_thorin_launches++;
 }
 
 __global__ void k_set_ctl(double *__restrict__ ctl, CtlSet v)
 {
+  pdl_wait();
   if (threadIdx.x < (unsigned)v.n) ctl[v.idx[threadIdx.x]] = v.val[threadIdx.x];
 }
 
 void aux_set_ctl(double *ctl, const CtlSet &v, cudaStream_t s)
 {
-  k_set_ctl<<<1, 32, 0, s>>>(ctl, v);
+  launch(k_set_ctl, 1, 32, 0, s, ctl, v);
   g_thorin_launches++;
 }
 
@@ -99,6 +102,7 @@ __device__ __forceinline__ double fvisc(const ViscParams &v, double rad, double 
 
 __global__ void k_viscosity_rings(DevGrid g, ViscParams v)
 {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.nr) return;
   const double cs = g.r.csmean[i], tm = g.r.tempmean[i];
@@ -108,7 +112,7 @@ __global__ void k_viscosity_rings(DevGrid g, ViscParams v)
 
 void aux_viscosity_rings(const DevGrid &g, const ViscParams &v, cudaStream_t s)
 {
-  k_viscosity_rings<<<(g.nr + 127) / 128, 128, 0, s>>>(g, v);
+  launch(k_viscosity_rings, (g.nr + 127) / 128, 128, 0, s, g, v);
   g_thorin_launches++;
 }
 
@@ -117,6 +121,7 @@ void aux_viscosity_rings(const DevGrid &g, const ViscParams &v, cudaStream_t s)
 __global__ void k_stokes(DevGrid g, const double *__restrict__ rho, const double *__restrict__ psize,
                          double *__restrict__ tau)
 {
+  pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
   tau[l] = div_fast((2.0 * g.k.pebbulkdens * g.k.sqrt_adiabind_inv) * psize[l], rho[l]);
@@ -124,7 +129,7 @@ __global__ void k_stokes(DevGrid g, const double *__restrict__ rho, const double
 
 void aux_stokes(const DevGrid &g, const double *rho, const double *psize, double *tau, cudaStream_t s)
 {
-  k_stokes<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, psize, tau);
+  launch(k_stokes, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, psize, tau);
   g_thorin_launches++;
 }
 
@@ -197,6 +202,7 @@ __global__ void __launch_bounds__(256) k_cfl_bounds(DevGrid g, const double *__r
                                                     CflRings cr, int pebbles, int fast, int viscous,
                                                     float *__restrict__ part, int *__restrict__ bound)
 {
+  pdl_wait();
   __shared__ float sh[4][8];
   const int ns = g.ns;
   const int i = blockIdx.y + 1;
@@ -275,6 +281,7 @@ __global__ void __launch_bounds__(256) k_cfl_cells(DevGrid g, const double *__re
                                                    const float *__restrict__ upper, const int *__restrict__ bound,
                                                    unsigned long long *__restrict__ top)
 {
+  pdl_wait();
   const int ns = g.ns;
   const int i = blockIdx.y + 1;                    // rings One_or_active .. Max_or_active-1
   if (upper) {
@@ -304,6 +311,7 @@ __global__ void __launch_bounds__(1024) k_cfl_final(DevGrid g, CflRings cr, CflF
                                                     int *__restrict__ iscal, int *__restrict__ bound,
                                                     unsigned long long *__restrict__ top)
 {
+  pdl_wait();
   // the remaining part of the DT and MinStepForRebound's rate come from the
   // disk's control block; so does the CFL's substep length, written back
   const double deltaT = g.ctl[CTL_DELTAT], invdtreb_sq = g.ctl[CTL_INVDTREB], dts = scal[SC_DTSTELLAR];
@@ -355,14 +363,14 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
   // 3.4 us; 256x768: 13 us)
   if ((long long)g.nr * g.ns < (1 << 17)) upper = nullptr;
   if (upper) {
-    k_cfl_bounds<<<grid2d(g.ns, g.nr - 1, 256 * CFL_CPT), 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast,
+    launch(k_cfl_bounds, grid2d(g.ns, g.nr - 1, 256 * CFL_CPT), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast,
                                                                       viscous, upper, bound);
     g_thorin_launches++;
   }
-  k_cfl_cells<<<grid2d(g.ns, g.nr - 1, 256), 256, 0, s>>>(g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
+  launch(k_cfl_cells, grid2d(g.ns, g.nr - 1, 256), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
                                                           bound, top);
   g_thorin_launches++;
-  k_cfl_final<<<1, 1024, 0, s>>>(g, cr, f0, scal, iscal, bound, top);
+  launch(k_cfl_final, 1, 1024, 0, s, g, cr, f0, scal, iscal, bound, top);
   g_thorin_launches++;
 }
 
@@ -370,6 +378,7 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
 // EvaporatePebbles (Pebbles.c:834-864).
 __global__ void k_evaporate(DevGrid g, const double *__restrict__ T, double *__restrict__ pdens)
 {
+  pdl_wait();
   const double facc = g.ctl[CTL_FACC_EVAP];
   const int ns = g.ns;
   CELL_LOOP_2D
@@ -382,7 +391,7 @@ __global__ void k_evaporate(DevGrid g, const double *__restrict__ T, double *__r
 
 void aux_evaporate(const DevGrid &g, const double *T, double *pdens, cudaStream_t s)
 {
-  k_evaporate<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, T, pdens);
+  launch(k_evaporate, grid2d(g.ns, g.nr, BX), BX, 0, s, g, T, pdens);
   g_thorin_launches++;
 }
 
@@ -392,6 +401,7 @@ void aux_evaporate(const DevGrid &g, const double *T, double *pdens, cudaStream_
 __global__ void k_damp_gas(DevGrid g, double *__restrict__ vrad, double *__restrict__ rho, double *__restrict__ vtheta,
                            double *__restrict__ energy, const int *__restrict__ rings, const double *__restrict__ vr0r, int damp_init, int damp_flux, int energy_eq)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
   const int ns = g.ns;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -416,7 +426,7 @@ void aux_damp_gas(const DevGrid &g, double *vrad, double *rho, double *vtheta, d
                   int energy_eq, cudaStream_t s)
 {
   if (nrings <= 0) return;
-  k_damp_gas<<<grid2d(g.ns, nrings, BX), BX, 0, s>>>(g, vrad, rho, vtheta, energy, rings, vr0r,
+  launch(k_damp_gas, grid2d(g.ns, nrings, BX), BX, 0, s, g, vrad, rho, vtheta, energy, rings, vr0r,
                                                      damp_init, damp_flux, energy_eq);
   g_thorin_launches++;
 }
@@ -431,6 +441,7 @@ __global__ void k_iso_eos(DevGrid g, const double *__restrict__ rho, const doubl
                           double *__restrict__ cs, double *__restrict__ press, double *__restrict__ temper, int set_cs,
                           int set_press, int set_temper)
 {
+  pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
   if (set_cs) cs[l] = csr[i];
@@ -441,13 +452,14 @@ __global__ void k_iso_eos(DevGrid g, const double *__restrict__ rho, const doubl
 void aux_iso_eos(const DevGrid &g, const double *rho, const double *csr, double *cs, double *press, double *temper,
                  int set_cs, int set_press, int set_temper, cudaStream_t s)
 {
-  k_iso_eos<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, csr, cs, press, temper, set_cs, set_press, set_temper);
+  launch(k_iso_eos, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, csr, cs, press, temper, set_cs, set_press, set_temper);
   g_thorin_launches++;
 }
 
 __global__ void k_damp_peb(DevGrid g, double *__restrict__ pd, double *__restrict__ pvr, double *__restrict__ pvt,
                            const int *__restrict__ rings)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
   const int ns = g.ns;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -465,13 +477,14 @@ __global__ void k_damp_peb(DevGrid g, double *__restrict__ pd, double *__restric
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s)
 {
   if (nrings <= 0) return;
-  k_damp_peb<<<grid2d(g.ns, nrings, BX), BX, 0, s>>>(g, pd, pvr, pvt, rings);
+  launch(k_damp_peb, grid2d(g.ns, nrings, BX), BX, 0, s, g, pd, pvr, pvt, rings);
   g_thorin_launches++;
 }
 
 // DetectCrash (SourceEuler.c:48-66): any negative value in rows 0..nr-1.
 __global__ void k_crash(int n, const double *__restrict__ f, int *flag)
 {
+  pdl_wait();
   int bad = 0;
   for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < n; l += gridDim.x * blockDim.x)
     if (f[l] < 0.0) bad = 1;
@@ -483,7 +496,7 @@ void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s)
   const int n = g.nr * g.ns;
   int blocks = (n + 255) / 256;
   if (blocks > 1216) blocks = 1216;
-  k_crash<<<blocks, 256, 0, s>>>(n, f, flag);
+  launch(k_crash, blocks, 256, 0, s, n, f, flag);
   g_thorin_launches++;
 }
 
@@ -495,6 +508,7 @@ void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s)
 // pull for the ring-mean column, one node per lane of the first warp.
 __global__ void __launch_bounds__(RING_T) k_force_rings(DevGrid g, ForceArgs a, ForceRings fr)
 {
+  pdl_wait();
   const int i = blockIdx.x, lane = threadIdx.x;
   const double H = g.r.csmean[i] * g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
   const double r2 = g.r.Rmed2[i];
@@ -550,6 +564,7 @@ __device__ __forceinline__ int off_by_5pc(float x, float m)
 template <int NP>
 __global__ void __launch_bounds__(128) k_forces(DevGrid g, ForceArgs a, ForceRings fr)
 {
+  pdl_wait();
   extern __shared__ char smem[];
   ForceRing *ring = (ForceRing *)smem;
   const double mass_taper = g.ctl[CTL_MASS_TAPER];
@@ -842,6 +857,7 @@ __device__ __forceinline__ void near_cell(const DevGrid &g, const ForceArgs &a, 
 // kernel for all cells took 340.
 __global__ void __launch_bounds__(128) k_forces_near(DevGrid g, ForceArgs a, ForceRings fr)
 {
+  pdl_wait();
   const double mass_taper = g.ctl[CTL_MASS_TAPER];
   const int full_mass = (mass_taper == 1.0) ? 1 : 0;
   const int ns = g.ns;
@@ -929,6 +945,7 @@ __global__ void __launch_bounds__(128) k_forces_near(DevGrid g, ForceArgs a, For
 // four fields and 14 FP64 instructions a cell before).
 __global__ void __launch_bounds__(1024) k_forces_final(DevGrid g, ForceArgs a, double *__restrict__ scal)
 {
+  pdl_wait();
   __shared__ bool last;
   const int q = blockIdx.x, nb = a.nba + a.nbb;
   const double *p = a.part + (size_t)q * nb;
@@ -957,7 +974,7 @@ __global__ void __launch_bounds__(1024) k_forces_final(DevGrid g, ForceArgs a, d
 template <int NP>
 static void launch_forces(const DevGrid &g, const ForceArgs &a, const ForceRings &fr, dim3 grid, cudaStream_t s)
 {
-  k_forces<NP><<<grid, 128, a.rings_a * sizeof(ForceRing), s>>>(g, a, fr);
+  launch(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
 }
 
 void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
@@ -997,7 +1014,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   a.nba = ga.x * ga.y;
   a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
   a.nbb = a.nbn + (a.npl > 0 ? g.nsm : 0);
-  k_force_rings<<<g.nr, RING_T, 0, s>>>(g, a, fr);
+  launch(k_force_rings, g.nr, RING_T, 0, s, g, a, fr);
   g_thorin_launches++;
   switch (a.npl) {
   case 0: launch_forces<0>(g, a, fr, ga, s); break;
@@ -1007,9 +1024,9 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   default: launch_forces<MAXPL_DEV>(g, a, fr, ga, s); break;
   }
   g_thorin_launches++;
-  k_forces_near<<<a.nbb, 128, 0, s>>>(g, a, fr);
+  launch(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
   g_thorin_launches++;
-  k_forces_final<<<2 + 2 * a.npl, 1024, 0, s>>>(g, a, scal);
+  launch(k_forces_final, 2 + 2 * a.npl, 1024, 0, s, g, a, scal);
   g_thorin_launches++;
 }
 
@@ -1101,6 +1118,7 @@ __device__ __forceinline__ bool acc_last_block(unsigned int *ticket)
 template <bool SET>
 __global__ void __launch_bounds__(RING_T) k_acc_reff(DevGrid g, AccArgs av, AccArgs *ap)
 {
+  pdl_wait();
   const AccArgs &a = SET ? av : *ap;
   if (a.nb == 0) return;                         // no annulus (only the device-resident DT launches this)
   const int ns = g.ns, ncells = (a.imax - a.imin + 1) * ns, nb = gridDim.x - 2;
@@ -1175,6 +1193,7 @@ __device__ __forceinline__ bool acc_cell(const DevGrid &g, const AccArgs &a, int
 // many multiprocessors.
 __global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *__restrict__ ap)
 {
+  pdl_wait();
   const AccArgs &a = *ap;
   if (a.nb == 0) return;                         // no annulus
   const int ncells = (a.imax - a.imin + 1) * g.ns;
@@ -1234,6 +1253,7 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *
 // momentum.
 __global__ void __launch_bounds__(ACC_BX) k_acc_apply(DevGrid g, const AccArgs *__restrict__ ap, double *__restrict__ scal)
 {
+  pdl_wait();
   const AccArgs &a = *ap;
   if (a.nb == 0) return;                         // no annulus
   const int ns = g.ns;
@@ -1279,12 +1299,12 @@ int aux_accrete_blocks(const DevGrid &g, int imin, int imax)
 void aux_accrete(const DevGrid &g, const AccArgs *a0, AccArgs *a_dev, int nb, double *scal, cudaStream_t s)
 {
   const int grid = nb < 2 * g.nsm ? nb : 2 * g.nsm;
-  if (a0) k_acc_reff<true><<<2 + grid, RING_T, 0, s>>>(g, *a0, a_dev);
-  else k_acc_reff<false><<<2 + grid, RING_T, 0, s>>>(g, AccArgs(), a_dev);
+  if (a0) launch(k_acc_reff<true>, 2 + grid, RING_T, 0, s, g, *a0, a_dev);
+  else launch(k_acc_reff<false>, 2 + grid, RING_T, 0, s, g, AccArgs(), a_dev);
   g_thorin_launches++;
-  k_acc_upper<<<2 * g.nsm, ACC_BX, 0, s>>>(g, a_dev);
+  launch(k_acc_upper, 2 * g.nsm, ACC_BX, 0, s, g, a_dev);
   g_thorin_launches++;
-  k_acc_apply<<<grid, ACC_BX, 0, s>>>(g, a_dev, scal);
+  launch(k_acc_apply, grid, ACC_BX, 0, s, g, a_dev, scal);
   g_thorin_launches++;
 }
 
@@ -1298,6 +1318,7 @@ __global__ void __launch_bounds__(RING_T) k_integrals(DevGrid g, const double *_
                                                       double omega_frame, double *__restrict__ part,
                                                       double *__restrict__ scal, unsigned int *ticket)
 {
+  pdl_wait();
   __shared__ bool last;
   const int i = blockIdx.x, nr = g.nr, ns = g.ns;
   const size_t row = (size_t)i * ns;
@@ -1333,9 +1354,9 @@ void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const 
                    unsigned int *ticket, cudaStream_t s)
 {
   if (pebbles)
-    k_integrals<true><<<g.nr, RING_T, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
+    launch(k_integrals<true>, g.nr, RING_T, 0, s, g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
   else
-    k_integrals<false><<<g.nr, RING_T, 0, s>>>(g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
+    launch(k_integrals<false>, g.nr, RING_T, 0, s, g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
   g_thorin_launches++;
 }
 
@@ -1350,6 +1371,7 @@ void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const 
 __global__ void k_open_inner(DevGrid g, double *__restrict__ rho, double *__restrict__ vr,
                              double *__restrict__ energy, int energy_eq, int damp_flux, double gasflux)
 {
+  pdl_wait();
   const int ns = g.ns, i = 1;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ns) return;
@@ -1374,6 +1396,7 @@ __global__ void k_open_inner(DevGrid g, double *__restrict__ rho, double *__rest
 __global__ void k_open_outer(DevGrid g, double *__restrict__ rho, double *__restrict__ vr,
                              double *__restrict__ energy, int energy_eq, int damp_flux, double gasflux)
 {
+  pdl_wait();
   const int ns = g.ns, i = g.nr - 1;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ns) return;
@@ -1413,6 +1436,7 @@ __global__ void __launch_bounds__(1024) k_nonreflecting(DevGrid g, double *__res
                                                         double *__restrict__ vr, double *__restrict__ energy,
                                                         const double *__restrict__ cs)
 {
+  pdl_wait();
   const int ns = g.ns, nr = g.nr;
   const bool inner = (blockIdx.x == 0);
   const int ia = inner ? 0 : nr - 2, ib = inner ? 1 : nr - 1;     // rings whose c_s are averaged
@@ -1457,6 +1481,7 @@ __global__ void __launch_bounds__(1024) k_nonreflecting(DevGrid g, double *__res
 __global__ void __launch_bounds__(1024) k_outer_source_mass(DevGrid g, double *__restrict__ rho,
                                                             double *__restrict__ vr, double penul_vr)
 {
+  pdl_wait();
   const int ns = g.ns, i = g.nr - 1;
   double *row = rho + (size_t)i * ns;
   const double avg = g.r.SigmaMed[i] - ring_sum_block(row, ns) / (double)ns;
@@ -1469,26 +1494,26 @@ __global__ void __launch_bounds__(1024) k_outer_source_mass(DevGrid g, double *_
 void aux_open_inner(const DevGrid &g, double *rho, double *vr, double *energy, int energy_eq, int damp_flux,
                     double gasflux, cudaStream_t s)
 {
-  k_open_inner<<<(g.ns + BX - 1) / BX, BX, 0, s>>>(g, rho, vr, energy, energy_eq, damp_flux, gasflux);
+  launch(k_open_inner, (g.ns + BX - 1) / BX, BX, 0, s, g, rho, vr, energy, energy_eq, damp_flux, gasflux);
   g_thorin_launches++;
 }
 
 void aux_open_outer(const DevGrid &g, double *rho, double *vr, double *energy, int energy_eq, int damp_flux,
                     double gasflux, cudaStream_t s)
 {
-  k_open_outer<<<(g.ns + BX - 1) / BX, BX, 0, s>>>(g, rho, vr, energy, energy_eq, damp_flux, gasflux);
+  launch(k_open_outer, (g.ns + BX - 1) / BX, BX, 0, s, g, rho, vr, energy, energy_eq, damp_flux, gasflux);
   g_thorin_launches++;
 }
 
 void aux_nonreflecting(const DevGrid &g, double *rho, double *vr, double *energy, const double *cs, cudaStream_t s)
 {
-  k_nonreflecting<<<2, 1024, 0, s>>>(g, rho, vr, energy, cs);
+  launch(k_nonreflecting, 2, 1024, 0, s, g, rho, vr, energy, cs);
   g_thorin_launches++;
 }
 
 void aux_outer_source_mass(const DevGrid &g, double *rho, double *vr, double penul_vr, cudaStream_t s)
 {
-  k_outer_source_mass<<<1, 1024, 0, s>>>(g, rho, vr, penul_vr);
+  launch(k_outer_source_mass, 1, 1024, 0, s, g, rho, vr, penul_vr);
   g_thorin_launches++;
 }
 
@@ -1499,6 +1524,7 @@ __global__ void k_parametric_cooling(DevGrid g, const double *__restrict__ rho, 
                                      const double *__restrict__ coolt, const double *__restrict__ qplusmed,
                                      double *__restrict__ enew, double gm1)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT];
   const int ns = g.ns;
   CELL_LOOP_2D
@@ -1513,7 +1539,7 @@ void aux_parametric_cooling(const DevGrid &g, const double *rho, const double *e
                             const double *divv, const double *coolt, const double *qplusmed, double *enew,
                             double gm1, cudaStream_t s)
 {
-  k_parametric_cooling<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, eint, qplus, divv, coolt, qplusmed, enew, gm1);
+  launch(k_parametric_cooling, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, eint, qplus, divv, coolt, qplusmed, enew, gm1);
   g_thorin_launches++;
 }
 
@@ -1553,6 +1579,7 @@ __global__ void __launch_bounds__(256) k_gas_accrete(DevGrid g, double *__restri
                                                      const double *__restrict__ cs, GasAccArgs a,
                                                      double *__restrict__ out)
 {
+  pdl_wait();
   const int ns = g.ns;
   const int nj = a.j_max - a.j_min + 1;
   const int ncell = (a.i_max - a.i_min + 1) * nj;
@@ -1599,7 +1626,7 @@ __global__ void __launch_bounds__(256) k_gas_accrete(DevGrid g, double *__restri
 void aux_gas_accrete(const DevGrid &g, double *dens, const double *vrad, const double *vtheta, const double *cs,
                      const GasAccArgs &a, double *out, cudaStream_t s)
 {
-  k_gas_accrete<<<1, 256, 0, s>>>(g, dens, vrad, vtheta, cs, a, out);
+  launch(k_gas_accrete, 1, 256, 0, s, g, dens, vrad, vtheta, cs, a, out);
   g_thorin_launches++;
 }
 
@@ -1609,6 +1636,7 @@ __global__ void k_drag_cell(const double *__restrict__ rho, const double *__rest
                             const double *__restrict__ vrad, const double *__restrict__ vtheta, int l, int ns,
                             double *__restrict__ out)
 {
+  pdl_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   out[0] = rho[l];
   out[1] = cs[l];
@@ -1621,7 +1649,7 @@ __global__ void k_drag_cell(const double *__restrict__ rho, const double *__rest
 void aux_drag_cell(const double *rho, const double *cs, const double *vrad, const double *vtheta, int l, int ns,
                    double *out, cudaStream_t s)
 {
-  k_drag_cell<<<1, 32, 0, s>>>(rho, cs, vrad, vtheta, l, ns, out);
+  launch(k_drag_cell, 1, 32, 0, s, rho, cs, vrad, vtheta, l, ns, out);
   g_thorin_launches++;
 }
 
@@ -1629,6 +1657,7 @@ void aux_drag_cell(const double *rho, const double *cs, const double *vrad, cons
 // frame's rotation rate changes by domega.
 __global__ void k_correct_vtheta(DevGrid g, double *__restrict__ vt, double domega)
 {
+  pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
   vt[l] -= domega * g.r.Rmed[i];
@@ -1636,6 +1665,6 @@ __global__ void k_correct_vtheta(DevGrid g, double *__restrict__ vt, double dome
 
 void aux_correct_vtheta(const DevGrid &g, double *vt, double domega, cudaStream_t s)
 {
-  k_correct_vtheta<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, vt, domega);
+  launch(k_correct_vtheta, grid2d(g.ns, g.nr, BX), BX, 0, s, g, vt, domega);
   g_thorin_launches++;
 }

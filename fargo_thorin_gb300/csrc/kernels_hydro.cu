@@ -59,6 +59,7 @@ struct SrcRing { double inv2, invrinf, ro, invdx2, supp, omega, oinv, cr, ct; };
 template <bool PEB>
 __global__ void __launch_bounds__(BX) k_sources(DevGrid g, SourceIO io)
 {
+  pdl_wait();
   __shared__ SrcRing ring[SRC_MAXRINGS];
   __shared__ double tab[64];
   const double dt = g.ctl[CTL_DT];
@@ -237,6 +238,7 @@ struct ViscRing { StressRing s; double irm, a, b, c, ra, rm, rc, rt, sr, st, er,
 
 __global__ void __launch_bounds__(BX) k_viscous(DevGrid g, ViscousIO io)
 {
+  pdl_wait();
   __shared__ ViscRing ring[VI_MAXRINGS + 3];
   __shared__ double s_tpp[2][BX], s_trp[2][BX], s_vt[BX], s_q[BX];
   const double dt = g.ctl[CTL_DT];
@@ -365,6 +367,7 @@ __global__ void __launch_bounds__(BX) k_viscous(DevGrid g, ViscousIO io)
 
 __global__ void __launch_bounds__(BX) k_heating(DevGrid g, HeatingIO io)
 {
+  pdl_wait();
   __shared__ StressRing ring[HT_MAXRINGS];
   const int ns = g.ns, nr = g.nr;
   const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
@@ -415,6 +418,7 @@ __global__ void __launch_bounds__(BX) k_heating(DevGrid g, HeatingIO io)
 __global__ void k_eos(DevGrid g, const double *__restrict__ rho, const double *__restrict__ energy,
                       double *__restrict__ temper, double *__restrict__ cs, double gm1, double gamma)
 {
+  pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
   // c_s = sqrt(gamma (gamma - 1) |e| / rho) = sqrt(gamma |T|)
@@ -678,6 +682,7 @@ struct DcRing { double c1, inv, invp, invdx, deltar2; };
 template <int LAW>
 __global__ void __launch_bounds__(BX) k_diffcoef(DevGrid g, DiffusionIO io)
 {
+  pdl_wait();
   __shared__ DcRing ring[DC_MAXRINGS];
   __shared__ unsigned long long smax[BX / 32][DC_MAXRINGS];
   __shared__ bool last;
@@ -798,6 +803,7 @@ __global__ void k_irradiation(DevGrid g, const double *__restrict__ rho, const d
                               double rstar, double tirr4fac, double opacity_drop, double taueff_c,
                               const double *__restrict__ rinf15, const double *__restrict__ rsup15)
 {
+  pdl_wait();
   const int ns = g.ns, nr = g.nr;
   CELL_LOOP_2D
   const double sqi = g.k.sqrt_adiabind_inv;
@@ -931,6 +937,7 @@ __global__ void __launch_bounds__(SOR_BX) k_sor_resid0(DevGrid g, const double *
                                                     const double *__restrict__ mljm, const double *__restrict__ rhs,
                                                     double *__restrict__ cw, SorCtl c)
 {
+  pdl_wait();
   const double omega = g.ctl[CTL_SOR_OMEGA];
   const int ns = g.ns, half = ns >> 1;
   const int i = blockIdx.y + 1;
@@ -972,6 +979,7 @@ struct MxRing { double ca, cb, ch; };
 template <bool RESID>
 __global__ void __launch_bounds__(BX) k_matrix(DevGrid g, MatrixIO io, SorCtl c)
 {
+  pdl_wait();
   __shared__ MxRing ring[MX_MAXRINGS + 1];
   __shared__ double sB[2][BX];
   const double dt = g.ctl[CTL_DT], omega = RESID ? g.ctl[CTL_SOR_OMEGA] : 0.0;
@@ -1086,12 +1094,6 @@ __device__ __forceinline__ bool sor_changed(double resid, double cw, double tn)
   return __double_as_longlong(__fma_rn(-tn, TH_SORPRECISION, resid * cw)) > 0LL;
 }
 
-// Programmatic dependent launch: the pass's blocks start while the pass before
-// drains; what a block does before sor_pdl_wait must not touch anything that
-// pass writes.
-__device__ __forceinline__ void sor_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void sor_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 struct SorRow { double ml, mlip, mlim, mljp, mljm, rhs, cw; };
 
 __global__ void __launch_bounds__(SOR_PX, SOR_POCC)
@@ -1112,8 +1114,9 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
   };
   SorRow m;
   if (idx < total) m = row_of(r, k);
-  sor_pdl_launch();
-  sor_pdl_wait();
+  // what a block does before this must not touch anything the pass before writes
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (*((volatile int *)c.done)) return;
   double a = 0.0;
   int ch = 0;
@@ -1410,6 +1413,7 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
 __global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, double *__restrict__ T,
                                 double *__restrict__ enew)
 {
+  pdl_wait();
   const int ns = g.ns, nr = g.nr;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y;
@@ -1486,6 +1490,7 @@ __device__ __forceinline__ void rd_load(const DevGrid &g, const RadialIO &io, co
 template <bool E, bool X>
 __global__ void __launch_bounds__(BX, 4) k_radial(DevGrid g, RadialIO io)
 {
+  pdl_wait();
   constexpr int NW = 4 + E + X;
   __shared__ RdRing ring[RD_MAXRINGS + 4];
   const double dt = g.ctl[CTL_DT];
@@ -1602,6 +1607,7 @@ __global__ void __launch_bounds__(BX, 4) k_radial(DevGrid g, RadialIO io)
 __global__ void k_label_from_ext(DevGrid g, const double *__restrict__ rho, const double *__restrict__ ext,
                                  double *__restrict__ label)
 {
+  pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
   label[l] = div_fast(ext[l], rho[l]);
@@ -1617,6 +1623,7 @@ __global__ void __launch_bounds__(RING_T) k_azi_rings(DevGrid g, const double *_
                                                       int *__restrict__ nshift, double *__restrict__ vmed,
                                                       double *__restrict__ vtemp)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT];
   const int i = blockIdx.x;
   const int ns = g.ns;
@@ -1666,6 +1673,7 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
                                                      int fast, const int *__restrict__ nshift,
                                                      const double *__restrict__ vmed, const double *__restrict__ vtemp)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT];
   __shared__ double s_a[AZ_TMAX], s_b[AZ_TMAX], s_c[AZ_TMAX];
   const int ns = g.ns, i = blockIdx.y, t = threadIdx.x, T = blockDim.x;
@@ -1771,6 +1779,7 @@ __global__ void k_velocities(DevGrid g, const double *__restrict__ rho, const do
                              const double *__restrict__ energy, double *__restrict__ temper, double *__restrict__ cs,
                              double gm1, double gamma)
 {
+  pdl_wait();
   const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
   const int ns = g.ns;
   CELL_LOOP_2D
@@ -1800,8 +1809,8 @@ void hydro_sources(const DevGrid &g, const SourceIO &io0, cudaStream_t s)
   // 0.15 rings a chunk: the ring below is read again, and the ring constants
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, SRC_MAXRINGS, 0.15);
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
-  if (io.pd) k_sources<true><<<grid, BX, 0, s>>>(g, io);
-  else k_sources<false><<<grid, BX, 0, s>>>(g, io);
+  if (io.pd) launch(k_sources<true>, grid, BX, 0, s, g, io);
+  else launch(k_sources<false>, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
@@ -1810,7 +1819,7 @@ void hydro_viscous(const DevGrid &g, const ViscousIO &io0, cudaStream_t s)
   ViscousIO io = io0;
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, VI_MAXRINGS, 1.8);
   const dim3 grid((g.ns + VI_COLS - 1) / VI_COLS, (g.nr + io.rings - 1) / io.rings);
-  k_viscous<<<grid, BX, 0, s>>>(g, io);
+  launch(k_viscous, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
@@ -1820,14 +1829,14 @@ void hydro_heating(const DevGrid &g, const HeatingIO &io0, cudaStream_t s)
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, HT_MAXRINGS, 0.2);
   if (io.rings < 3) io.rings = 3;                  // ring 0 is extrapolated by the thread of rings 1 and 2
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
-  k_heating<<<grid, BX, 0, s>>>(g, io);
+  launch(k_heating, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
 void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double *temper, double *cs, double gm1,
                double gg1, cudaStream_t s)
 {
-  k_eos<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, energy, temper, cs, gm1, gg1 / gm1);
+  launch(k_eos, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, energy, temper, cs, gm1, gg1 / gm1);
   g_thorin_launches++;
 }
 
@@ -1838,11 +1847,11 @@ void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io0, int law, cudaStrea
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, DC_MAXRINGS, 0.2, 8);
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
   switch (law) {
-  case THORIN_OPA_SM03: k_diffcoef<THORIN_OPA_SM03><<<grid, BX, 0, s>>>(g, io); break;
-  case THORIN_OPA_ZHU12: k_diffcoef<THORIN_OPA_ZHU12><<<grid, BX, 0, s>>>(g, io); break;
-  case THORIN_OPA_LP85: k_diffcoef<THORIN_OPA_LP85><<<grid, BX, 0, s>>>(g, io); break;
-  case THORIN_OPA_CONST: k_diffcoef<THORIN_OPA_CONST><<<grid, BX, 0, s>>>(g, io); break;
-  default: k_diffcoef<THORIN_OPA_BL94><<<grid, BX, 0, s>>>(g, io); break;
+  case THORIN_OPA_SM03: launch(k_diffcoef<THORIN_OPA_SM03>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_ZHU12: launch(k_diffcoef<THORIN_OPA_ZHU12>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_LP85: launch(k_diffcoef<THORIN_OPA_LP85>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_CONST: launch(k_diffcoef<THORIN_OPA_CONST>, grid, BX, 0, s, g, io); break;
+  default: launch(k_diffcoef<THORIN_OPA_BL94>, grid, BX, 0, s, g, io); break;
   }
   g_thorin_launches++;
 }
@@ -1851,7 +1860,7 @@ void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, co
                        double *qirr, double rstar, double tirr4fac, double opacity_drop, double taueff_c,
                        const double *rinf15, const double *rsup15, cudaStream_t s)
 {
-  k_irradiation<<<grid2d(g.ns, g.nr, BX), BX, 0, s>>>(g, rho, cs, opacity, flaring, qirr, rstar, tirr4fac, opacity_drop,
+  launch(k_irradiation, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, cs, opacity, flaring, qirr, rstar, tirr4fac, opacity_drop,
                                                       taueff_c, rinf15, rsup15);
   g_thorin_launches++;
 }
@@ -1870,8 +1879,8 @@ void hydro_matrix(const DevGrid &g, const MatrixIO &io0, const SorCtl *resid, cu
 {
   MatrixIO io = io0;
   io.rings = matrix_rings(g);
-  if (resid) k_matrix<true><<<matrix_grid(g), BX, 0, s>>>(g, io, *resid);
-  else k_matrix<false><<<matrix_grid(g), BX, 0, s>>>(g, io, SorCtl{});
+  if (resid) launch(k_matrix<true>, matrix_grid(g), BX, 0, s, g, io, *resid);
+  else launch(k_matrix<false>, matrix_grid(g), BX, 0, s, g, io, SorCtl{});
   g_thorin_launches++;
 }
 
@@ -1917,7 +1926,7 @@ void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const
                       const double *mljp, const double *mljm, const double *rhs, double *cw,
                       const SorCtl &c, cudaStream_t s)
 {
-  k_sor_resid0<<<sor_grid_resid(g), SOR_BX, 0, s>>>(g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c);
+  launch(k_sor_resid0, sor_grid_resid(g), SOR_BX, 0, s, g, T, ml, mlip, mlim, mljp, mljm, rhs, cw, c);
   g_thorin_launches++;
 }
 
@@ -2008,7 +2017,7 @@ void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double 
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)
 {
-  k_energy_from_t<<<grid2d(g.ns, g.nr + 1, BX), BX, 0, s>>>(g, rho, T, enew);
+  launch(k_energy_from_t, grid2d(g.ns, g.nr + 1, BX), BX, 0, s, g, rho, T, enew);
   g_thorin_launches++;
 }
 
@@ -2038,14 +2047,14 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
   rd.ext = S.w[6];
   rd.rings = chunk_rings(nr, ns, g.nsm, RD_MAXRINGS, 1.3);
   const dim3 rgrid((ns + BX - 1) / BX, (nr + rd.rings - 1) / rd.rings);
-  if (energy && label) k_radial<true, true><<<rgrid, BX, 0, s>>>(g, rd);
-  else if (energy) k_radial<true, false><<<rgrid, BX, 0, s>>>(g, rd);
-  else if (label) k_radial<false, true><<<rgrid, BX, 0, s>>>(g, rd);
-  else k_radial<false, false><<<rgrid, BX, 0, s>>>(g, rd);
+  if (energy && label) launch(k_radial<true, true>, rgrid, BX, 0, s, g, rd);
+  else if (energy) launch(k_radial<true, false>, rgrid, BX, 0, s, g, rd);
+  else if (label) launch(k_radial<false, true>, rgrid, BX, 0, s, g, rd);
+  else launch(k_radial<false, false>, rgrid, BX, 0, s, g, rd);
   g_thorin_launches++;
   // azimuthal step back into the momenta, the new energy, the tracer and
   // the new density
-  k_azi_rings<<<nr, RING_T, 0, s>>>(g, vt_in, S.nshift, S.vmed, S.vtemp);
+  launch(k_azi_rings, nr, RING_T, 0, s, g, vt_in, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   AziIO az;
   for (int k = 0; k < nq; k++) {
@@ -2056,16 +2065,16 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
   az.n = nq;
   const int T = azi_block(ns);
   const dim3 grid((ns + T - 2 * AZ_HALO - 1) / (T - 2 * AZ_HALO), nr);
-  if (nq == 7) k_azimuthal<7><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
-  else if (nq == 6) k_azimuthal<6><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
-  else k_azimuthal<5><<<grid, T, 0, s>>>(g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  if (nq == 7) launch(k_azimuthal<7>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else if (nq == 6) launch(k_azimuthal<6>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else launch(k_azimuthal<5>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   // velocities from the transported momenta
-  k_velocities<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,
+  launch(k_velocities, grid2d(ns, nr, BX), BX, 0, s, g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,
                                                  energy ? S.e_new : nullptr, energy ? temper : nullptr, cs, gm1, gg1 / gm1);
   g_thorin_launches++;
   if (label) {
-    k_label_from_ext<<<grid2d(ns, nr, BX), BX, 0, s>>>(g, S.rho_new, S.ext_new, label);
+    launch(k_label_from_ext, grid2d(ns, nr, BX), BX, 0, s, g, S.rho_new, S.ext_new, label);
     g_thorin_launches++;
   }
 }

@@ -103,6 +103,13 @@ __device__ __forceinline__ double warp_seq_sum(const double *row, int n)
   return acc;
 }
 
+// Start of a kernel launched by launch(): the kernel before it is done, and
+// the one after it may be placed.
+__device__ __forceinline__ void pdl_wait()
+{
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Block-wide reductions (fixed order: warp shuffles then warp partials) -----
 template <typename T, typename Op>
 __device__ __forceinline__ T warp_reduce(T v, Op op)

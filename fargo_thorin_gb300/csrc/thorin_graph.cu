@@ -18,6 +18,7 @@
 
 __global__ void k_g_dt_begin(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   S.g.ctl[CTL_DTEMP] = 0.0;
   GraphStats *st = S.st;
@@ -33,6 +34,7 @@ __global__ void k_g_dt_begin(StepDev S)
 // the remaining interval of the DT.
 __global__ void k_g_sub_begin(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   double *ctl = S.g.ctl;
   ctl[CTL_MASS_TAPER] = pl_mass_taper(ctl[CTL_TIME], S.c.mass_taper_param);
@@ -43,6 +45,7 @@ __global__ void k_g_sub_begin(StepDev S)
 // InitHeating (Planet.c:251) and EvaporatePebbles' fraction of this dt.
 __global__ void k_g_acc_init(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   for (int k = 0; k < S.npl; k++) { S.heat_val[k] = 0.0; S.heat_idx[k] = -1; }
   double facc = S.evaporation_rate * S.g.ctl[CTL_DT];
@@ -53,6 +56,7 @@ __global__ void k_g_acc_init(StepDev S)
 // AccretePebblesOntoPlanets' set-up for planet k.
 __global__ void k_g_acc_prep(StepDev S, int k)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   AccArgs a = *S.acc;
   pl_pebble_acc_prep(S.c, S.g.r.Rinf, S.g.r.Rsup, S.g.r.Rmed, S.sys, k, S.g.ctl[CTL_OMEGA_FRAME], S.g.ctl[CTL_DT],
@@ -63,6 +67,7 @@ __global__ void k_g_acc_prep(StepDev S, int k)
 // Heating1 and the planet's new mass and velocity after the accretion.
 __global__ void k_g_acc_finish(StepDev S, int k)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   const AccArgs &a = *S.acc;
   double dMp = 0.0, dPx = 0.0, dPy = 0.0;
@@ -83,6 +88,7 @@ __global__ void k_g_acc_finish(StepDev S, int k)
 // DampingTW04.
 __global__ void k_g_force_prep(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   double *ctl = S.g.ctl;
   ctl[CTL_DTEMP] += ctl[CTL_DT];
@@ -176,6 +182,7 @@ __device__ void nbody_step_warp(thorin_planets *sys, double dt)
 // (SourceEuler.c:251-268), one warp.
 __global__ void __launch_bounds__(32) k_g_planet_step(StepDev S)
 {
+  pdl_wait();
   thorin_planets *sys = S.sys;
   const double dt = S.g.ctl[CTL_DT];
   if (threadIdx.x == 0) {
@@ -201,6 +208,7 @@ __global__ void __launch_bounds__(32) k_g_planet_step(StepDev S)
 // the whole graph.
 __global__ void k_g_sor_begin(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   double *ctl = S.g.ctl;
   double omega = ctl[CTL_SOR_OMEGA] + ctl[CTL_SOR_DOMEGA], domega = ctl[CTL_SOR_DOMEGA];
@@ -215,6 +223,7 @@ __global__ void k_g_sor_begin(StepDev S)
 // reversal when the solve took more sweeps than the last.
 __global__ void k_g_sor_end(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   GraphStats *st = S.st;
   const int done = *S.sor.done, n = *S.sor.niter;
@@ -232,6 +241,7 @@ __global__ void k_g_sor_end(StepDev S)
 // (dtemp < 0.999999999 DT, SourceEuler.c:229).
 __global__ void k_g_sub_end(StepDev S)
 {
+  pdl_wait();
   if (threadIdx.x != 0) return;
   double *ctl = S.g.ctl;
   GraphStats *st = S.st;
@@ -246,14 +256,13 @@ __global__ void k_g_sub_end(StepDev S)
   cudaGraphSetConditional(S.h_sub, more);
 }
 
-#define ONE_BLOCK <<<1, 32, 0, s>>>
-void graph_dt_begin(const StepDev &S, cudaStream_t s) { k_g_dt_begin ONE_BLOCK(S); g_thorin_launches++; }
-void graph_sub_begin(const StepDev &S, cudaStream_t s) { k_g_sub_begin ONE_BLOCK(S); g_thorin_launches++; }
-void graph_acc_init(const StepDev &S, cudaStream_t s) { k_g_acc_init ONE_BLOCK(S); g_thorin_launches++; }
-void graph_acc_prep(const StepDev &S, int k, cudaStream_t s) { k_g_acc_prep ONE_BLOCK(S, k); g_thorin_launches++; }
-void graph_acc_finish(const StepDev &S, int k, cudaStream_t s) { k_g_acc_finish ONE_BLOCK(S, k); g_thorin_launches++; }
-void graph_force_prep(const StepDev &S, cudaStream_t s) { k_g_force_prep ONE_BLOCK(S); g_thorin_launches++; }
-void graph_planet_step(const StepDev &S, cudaStream_t s) { k_g_planet_step ONE_BLOCK(S); g_thorin_launches++; }
-void graph_sor_begin(const StepDev &S, cudaStream_t s) { k_g_sor_begin ONE_BLOCK(S); g_thorin_launches++; }
-void graph_sor_end(const StepDev &S, cudaStream_t s) { k_g_sor_end ONE_BLOCK(S); g_thorin_launches++; }
-void graph_sub_end(const StepDev &S, cudaStream_t s) { k_g_sub_end ONE_BLOCK(S); g_thorin_launches++; }
+void graph_dt_begin(const StepDev &S, cudaStream_t s) { launch(k_g_dt_begin, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_sub_begin(const StepDev &S, cudaStream_t s) { launch(k_g_sub_begin, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_acc_init(const StepDev &S, cudaStream_t s) { launch(k_g_acc_init, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_acc_prep(const StepDev &S, int k, cudaStream_t s) { launch(k_g_acc_prep, 1, 32, 0, s, S, k); g_thorin_launches++; }
+void graph_acc_finish(const StepDev &S, int k, cudaStream_t s) { launch(k_g_acc_finish, 1, 32, 0, s, S, k); g_thorin_launches++; }
+void graph_force_prep(const StepDev &S, cudaStream_t s) { launch(k_g_force_prep, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_planet_step(const StepDev &S, cudaStream_t s) { launch(k_g_planet_step, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_sor_begin(const StepDev &S, cudaStream_t s) { launch(k_g_sor_begin, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_sor_end(const StepDev &S, cudaStream_t s) { launch(k_g_sor_end, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_sub_end(const StepDev &S, cudaStream_t s) { launch(k_g_sub_end, 1, 32, 0, s, S); g_thorin_launches++; }

@@ -78,6 +78,7 @@ constexpr int conv_smem() { return (CIN / 8) * 3 * WN_HALO_W * 16 + 9 * CIN * N 
 template <int CIN, int N, int MODE>
 __global__ void __launch_bounds__(128, 4) k_wn_conv(ConvArgs a)
 {
+  pdl_wait();
   constexpr int K = 9 * CIN, KG = K / 8, C8 = CIN / 8;
   constexpr int A_BYTES = C8 * 3 * WN_HALO_W * 16, B_BYTES = KG * N * 16, LBO_A = 3 * WN_HALO_W * 16;
   constexpr uint32_t IDESC = umma::idesc_bf16(128, N);
@@ -225,6 +226,7 @@ struct WgradShape {
 template <int CIN, int N>
 __global__ void __launch_bounds__(128) k_wn_wgrad(WgradArgs a)
 {
+  pdl_wait();
   using S = WgradShape<CIN, N>;
   constexpr uint32_t IDESC = umma::idesc_bf16(128, N);
   extern __shared__ unsigned char smem_raw[];
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(128) k_wn_wgrad(WgradArgs a)
 __global__ void k_wn_wgrad_reduce(const float *__restrict__ part, int nblk, int cin, int cinp, int cout, int n,
                                   float *__restrict__ gw)
 {
+  pdl_wait();
   const int R = 9 * cinp;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < R * n) {
@@ -373,6 +376,7 @@ __global__ void k_wn_wgrad_reduce(const float *__restrict__ part, int nblk, int 
 __global__ void k_wn_pack(const float *__restrict__ w, int cin, int cout, int cinp, int coutp, bf16 *__restrict__ wk,
                           bf16 *__restrict__ wt)
 {
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int nk = coutp * 9 * cinp;
   if (idx < nk) {
@@ -389,6 +393,7 @@ __global__ void k_wn_pack(const float *__restrict__ w, int cin, int cout, int ci
 // per 8 channels of an output cell
 __global__ void k_wn_pool(const bf16 *__restrict__ a, bf16 *__restrict__ p, int B, int H, int W)
 {
+  pdl_wait();
   const long long n = (long long)B * (H / 2) * (W / 2) * (WN_C / 8);
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
@@ -416,6 +421,7 @@ __global__ void k_wn_pool(const bf16 *__restrict__ a, bf16 *__restrict__ p, int 
 __global__ void k_wn_upadd(const bf16 *__restrict__ low, const bf16 *__restrict__ skip, bf16 *__restrict__ u, int B,
                            int H, int W)
 {
+  pdl_wait();
   const long long n = (long long)B * H * W * (WN_C / 8);
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
@@ -439,6 +445,7 @@ __global__ void k_wn_upadd(const bf16 *__restrict__ low, const bf16 *__restrict_
 __global__ void k_wn_relu_mask(const float *__restrict__ g, const bf16 *__restrict__ act, bf16 *__restrict__ out,
                                long long n)
 {
+  pdl_wait();
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
   out[idx] = __float2bfloat16_rn(__bfloat162float(act[idx]) > 0.f ? g[idx] : 0.f);
@@ -449,6 +456,7 @@ __global__ void k_wn_relu_mask(const float *__restrict__ g, const bf16 *__restri
 __global__ void k_wn_downsum_mask(const float *__restrict__ gu, const bf16 *__restrict__ act, bf16 *__restrict__ out,
                                   int B, int H, int W)
 {
+  pdl_wait();
   const long long n = (long long)B * (H / 2) * (W / 2) * WN_C;
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
@@ -468,6 +476,7 @@ __global__ void k_wn_downsum_mask(const float *__restrict__ gu, const bf16 *__re
 __global__ void k_wn_unpool_mask(const float *__restrict__ ga, const float *__restrict__ gp, const bf16 *__restrict__ act,
                                  bf16 *__restrict__ out, int B, int H, int W)
 {
+  pdl_wait();
   const long long n = (long long)B * H * W * WN_C;
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= n) return;
@@ -485,6 +494,7 @@ __global__ void k_wn_unpool_mask(const float *__restrict__ ga, const float *__re
 __global__ void k_wn_loss(const float *__restrict__ y, const float *__restrict__ t, int B, int H, int W, float inv_n,
                           bf16 *__restrict__ gy16, double *__restrict__ lpart)
 {
+  pdl_wait();
   const long long P = (long long)B * H * W;
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   double l = 0.0;
@@ -509,6 +519,7 @@ __global__ void k_wn_loss(const float *__restrict__ y, const float *__restrict__
 // ordered sum of n partials times scale -> *out (one warp)
 __global__ void k_wn_sum(const double *__restrict__ part, int n, double scale, double *__restrict__ out)
 {
+  pdl_wait();
   double s = 0.0;
   for (int k = threadIdx.x; k < n; k += 32) s += part[k];
   s = warp_reduce(s, OpAdd());
@@ -520,6 +531,7 @@ __global__ void k_wn_sum(const double *__restrict__ part, int n, double scale, d
 __global__ void k_wn_sum_omega(const double *__restrict__ part, int n, const double *__restrict__ omega, double a,
                                double b, double *__restrict__ out)
 {
+  pdl_wait();
   double s = 0.0;
   for (int k = threadIdx.x; k < n; k += 32) s += part[k];
   s = warp_reduce(s, OpAdd());
@@ -528,6 +540,7 @@ __global__ void k_wn_sum_omega(const double *__restrict__ part, int n, const dou
 
 __global__ void k_wn_sqnorm(const float *__restrict__ g, int n, double *__restrict__ part)
 {
+  pdl_wait();
   double s = 0.0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) s += (double)g[k] * g[k];
   s = block_reduce(s, OpAdd(), 0.0);
@@ -538,6 +551,7 @@ __global__ void k_wn_adam(float *__restrict__ w, const float *__restrict__ g, fl
                           float *__restrict__ v, int n, float lr, float b1, float b2, float eps, float bc1, float bc2,
                           const double *__restrict__ sqnorm, float max_norm)
 {
+  pdl_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const double nrm = sqrt(*sqnorm);
@@ -570,6 +584,7 @@ __device__ __forceinline__ double sor_resid(const double *T, const SorSys &m, in
 // (part[grid + block]), grid-stride, block order
 __global__ void k_wn_scale(int nr, int ns, const double *__restrict__ T, SorSys m, double *__restrict__ part)
 {
+  pdl_wait();
   double s = 0.0, sr = 0.0;
   const long long n = (long long)(nr - 2) * ns;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
@@ -620,6 +635,7 @@ __global__ void k_wn_features(int nr, int ns, int fc, const double *__restrict__
                               const double *__restrict__ scale, const double *__restrict__ prev, bf16 *__restrict__ x,
                               double *__restrict__ jac)
 {
+  pdl_wait();
   const int H = nr / fc, W = ns / fc;
   const long long n = (long long)H * W;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -689,6 +705,7 @@ __device__ __forceinline__ float wn_up_weight(int i, int I, int n, bool periodic
 __global__ void k_wn_apply(int nr, int ns, int fc, double *__restrict__ T, const double *__restrict__ jac,
                            const float *__restrict__ y, const double *__restrict__ scale)
 {
+  pdl_wait();
   const long long n = (long long)(nr - 2) * ns;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -703,6 +720,7 @@ __global__ void k_wn_apply(int nr, int ns, int fc, double *__restrict__ T, const
 __global__ void k_wn_target(int nr, int ns, int fc, const double *__restrict__ tconv, const double *__restrict__ tk,
                             const double *__restrict__ jac, const double *__restrict__ scale, float *__restrict__ tgt)
 {
+  pdl_wait();
   const int H = nr / fc, W = ns / fc;
   const long long n = (long long)H * W;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -724,6 +742,7 @@ __global__ void k_wn_target(int nr, int ns, int fc, const double *__restrict__ t
 __global__ void k_wn_tpred(int nr, int ns, int fc, const double *__restrict__ tk, const double *__restrict__ jac,
                            const float *__restrict__ y, const double *__restrict__ scale, double *__restrict__ tp)
 {
+  pdl_wait();
   const long long n = (long long)nr * ns;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -736,6 +755,7 @@ __global__ void k_wn_tpred(int nr, int ns, int fc, const double *__restrict__ tk
 __global__ void k_wn_res(int nr, int ns, const double *__restrict__ tp, SorSys m, const double *__restrict__ sr,
                          float *__restrict__ rs, double *__restrict__ part)
 {
+  pdl_wait();
   const long long n = (long long)nr * ns;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   double acc = 0.0;
@@ -758,6 +778,7 @@ __global__ void k_wn_res(int nr, int ns, const double *__restrict__ tp, SorSys m
 __global__ void k_wn_res_grad(int nr, int ns, const float *__restrict__ rs, SorSys m, const double *__restrict__ scale,
                               const double *__restrict__ sr, float wres, double inv_n, float *__restrict__ gf)
 {
+  pdl_wait();
   const long long n = (long long)nr * ns;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -785,6 +806,7 @@ __global__ void k_wn_out_grad(int nr, int ns, int fc, const float *__restrict__ 
                               const float *__restrict__ tgt, float wsup, double inv_nc, bf16 *__restrict__ gy16,
                               double *__restrict__ part)
 {
+  pdl_wait();
   const int H = nr / fc, W = ns / fc;
   const long long n = (long long)H * W;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -822,6 +844,7 @@ __global__ void k_wn_out_grad(int nr, int ns, int fc, const float *__restrict__ 
 // dscal[0] = wres * dscal[4] + wsup * dscal[5]
 __global__ void k_wn_total(double *dscal, float wres, float wsup)
 {
+  pdl_wait();
   dscal[0] = (double)wres * dscal[4] + (double)wsup * dscal[5];
 }
 
@@ -831,6 +854,7 @@ __global__ void k_wn_total(double *dscal, float wres, float wsup)
 __global__ void k_wn_record(long long n, const double *__restrict__ tconv, const double *__restrict__ tstart,
                             double *__restrict__ hist, int nh, const double *__restrict__ dt, double *__restrict__ dts)
 {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q < n) {
     for (int k = nh - 1; k > 0; k--) hist[k * n + q] = hist[(k - 1) * n + q];
@@ -853,6 +877,7 @@ struct WsCoef { double c[WS_MAXORDER][WS_MAXORDER]; };
 __global__ void k_ws_delta(long long cells, const double *__restrict__ hist, int order, const double *__restrict__ dt,
                            const double *__restrict__ dts, WsCoef cf, double *__restrict__ u)
 {
+  pdl_wait();
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= cells) return;
   int m = 0;
@@ -873,6 +898,7 @@ __global__ void k_ws_line(int nr, int ns, const double *__restrict__ T, const do
                           const double *__restrict__ cw, const double *__restrict__ omega, double *__restrict__ vq,
                           double *__restrict__ part)
 {
+  pdl_wait();
   double ra = 0.0, aa = 0.0;
   const long long n = (long long)(nr - 2) * ns, cells = (long long)nr * ns;
   const double iw = 1.0 / *omega;
@@ -900,6 +926,7 @@ __global__ void k_ws_line(int nr, int ns, const double *__restrict__ T, const do
 // out[0] = s, out[1] += s (a running sum for the statistics)
 __global__ void k_ws_step(const double *__restrict__ part, int nb, double *__restrict__ out)
 {
+  pdl_wait();
   double ra = 0.0, aa = 0.0;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     ra += part[b];
@@ -922,6 +949,7 @@ __global__ void k_ws_step(const double *__restrict__ part, int nb, double *__res
 __global__ void k_ws_apply(int nr, int ns, double *__restrict__ T, const double *__restrict__ vq,
                            const double *__restrict__ step, const double *__restrict__ dts)
 {
+  pdl_wait();
   const long long n = (long long)(nr - 2) * ns, cells = (long long)nr * ns;
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n || !(dts[0] > 0.0)) return;
@@ -990,7 +1018,7 @@ static int conv_launch(thorin_warmnet *n, const bf16 *in, const bf16 *wk, const 
   const long long wave = per_sm * n->nsm;
   const int grid = (int)(tiles < wave ? tiles : wave);
   ConvArgs a{in, wk, bias, coutr, out, B, H, W, n->err};
-  k_wn_conv<CIN, N, MODE><<<grid, 128, SM, s>>>(a);
+  launch(k_wn_conv<CIN, N, MODE>, grid, 128, SM, s, a);
   g_thorin_launches++;
   return THORIN_OK;
 }
@@ -1008,11 +1036,11 @@ static int wgrad_launch(thorin_warmnet *n, int layer, const bf16 *in, const bf16
   const long long chunks = ((long long)B * H * W + 127) / 128;
   const int grid = (int)(chunks < n->part_blocks ? chunks : n->part_blocks);
   WgradArgs a{in, gout, n->part, B, H, W, n->err};
-  k_wn_wgrad<CIN, N><<<grid, 128, S::SMEM, s>>>(a);
+  launch(k_wn_wgrad<CIN, N>, grid, 128, S::SMEM, s, a);
   g_thorin_launches++;
   const LayerDef L = layer_def(layer);
   const int tot = 9 * L.cinp * N + L.cout;
-  k_wn_wgrad_reduce<<<nblk(tot), 256, 0, s>>>(n->part, grid, L.cin, L.cinp, L.cout, N, n->g + layer_off(layer));
+  launch(k_wn_wgrad_reduce, nblk(tot), 256, 0, s, n->part, grid, L.cin, L.cinp, L.cout, N, n->g + layer_off(layer));
   g_thorin_launches++;
   return THORIN_OK;
 }
@@ -1021,7 +1049,7 @@ static void pack_all(thorin_warmnet *n, cudaStream_t s)
 {
   for (int l = 0; l < WN_NL; l++) {
     const LayerDef L = layer_def(l);
-    k_wn_pack<<<nblk(2LL * L.coutp * 9 * L.cinp), 256, 0, s>>>(n->w + layer_off(l), L.cin, L.cout, L.cinp, L.coutp,
+    launch(k_wn_pack, nblk(2LL * L.coutp * 9 * L.cinp), 256, 0, s, n->w + layer_off(l), L.cin, L.cout, L.cinp, L.coutp,
                                                               n->wk[l], n->wt[l]);
     g_thorin_launches++;
   }
@@ -1040,11 +1068,11 @@ static int wn_forward(thorin_warmnet *n, int B, cudaStream_t s)
   int h[4] = {H, H / 2, H / 4, H / 8}, w[4] = {W, W / 2, W / 4, W / 8};
   bf16 **A = n->act;
   auto pool = [&](const bf16 *a, bf16 *p, int lv) {
-    k_wn_pool<<<nblk((long long)B * h[lv + 1] * w[lv + 1] * (WN_C / 8)), 256, 0, s>>>(a, p, B, h[lv], w[lv]);
+    launch(k_wn_pool, nblk((long long)B * h[lv + 1] * w[lv + 1] * (WN_C / 8)), 256, 0, s, a, p, B, h[lv], w[lv]);
     g_thorin_launches++;
   };
   auto upadd = [&](const bf16 *low, const bf16 *skip, bf16 *u, int lv) {
-    k_wn_upadd<<<nblk((long long)B * h[lv] * w[lv] * (WN_C / 8)), 256, 0, s>>>(low, skip, u, B, h[lv], w[lv]);
+    launch(k_wn_upadd, nblk((long long)B * h[lv] * w[lv] * (WN_C / 8)), 256, 0, s, low, skip, u, B, h[lv], w[lv]);
     g_thorin_launches++;
   };
   RCHK_WN(conv_launch<16, 32, 0>(n, n->x, n->wk[0], bias_of(n, 0), 32, A[A0], B, h[0], w[0], s));
@@ -1076,46 +1104,46 @@ static int wn_backward(thorin_warmnet *n, int B, cudaStream_t s, bool mse_loss =
   const unsigned lb = nblk(P0);
   double *lpart = n->dscal + 8;
   if (mse_loss) {       // otherwise the caller filled gy16 and the loss
-    k_wn_loss<<<lb, 256, 0, s>>>(n->y, n->tgt, B, H, W, inv_n, A[GY16], lpart);
+    launch(k_wn_loss, lb, 256, 0, s, n->y, n->tgt, B, H, W, inv_n, A[GY16], lpart);
     g_thorin_launches++;
-    k_wn_sum<<<1, 32, 0, s>>>(lpart, (int)lb, (double)inv_n, n->dscal);
+    launch(k_wn_sum, 1, 32, 0, s, lpart, (int)lb, (double)inv_n, n->dscal);
     g_thorin_launches++;
   }
   auto cnt = [&](int lv) { return (long long)B * h[lv] * w[lv] * WN_C; };
   // out layer
   RCHK_WN(wgrad_launch<32, 16>(n, 7, A[B0], A[GY16], B, h[0], w[0], s));
   RCHK_WN(conv_launch<16, 32, 2>(n, A[GY16], n->wt[7], nullptr, 0, n->gf[0], B, h[0], w[0], s));
-  k_wn_relu_mask<<<nblk(cnt(0)), 256, 0, s>>>(n->gf[0], A[B0], n->gb[0], cnt(0));
+  launch(k_wn_relu_mask, nblk(cnt(0)), 256, 0, s, n->gf[0], A[B0], n->gb[0], cnt(0));
   g_thorin_launches++;
   // d0 (input u0 = up(b1) + a0)
   RCHK_WN(wgrad_launch<32, 32>(n, 6, A[U0], n->gb[0], B, h[0], w[0], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[0], n->wt[6], nullptr, 0, n->ga[0], B, h[0], w[0], s));
-  k_wn_downsum_mask<<<nblk(cnt(1)), 256, 0, s>>>(n->ga[0], A[B1], n->gb[1], B, h[0], w[0]);
+  launch(k_wn_downsum_mask, nblk(cnt(1)), 256, 0, s, n->ga[0], A[B1], n->gb[1], B, h[0], w[0]);
   g_thorin_launches++;
   // d1
   RCHK_WN(wgrad_launch<32, 32>(n, 5, A[U1], n->gb[1], B, h[1], w[1], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[1], n->wt[5], nullptr, 0, n->ga[1], B, h[1], w[1], s));
-  k_wn_downsum_mask<<<nblk(cnt(2)), 256, 0, s>>>(n->ga[1], A[B2], n->gb[2], B, h[1], w[1]);
+  launch(k_wn_downsum_mask, nblk(cnt(2)), 256, 0, s, n->ga[1], A[B2], n->gb[2], B, h[1], w[1]);
   g_thorin_launches++;
   // d2
   RCHK_WN(wgrad_launch<32, 32>(n, 4, A[U2], n->gb[2], B, h[2], w[2], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[2], n->wt[4], nullptr, 0, n->ga[2], B, h[2], w[2], s));
-  k_wn_downsum_mask<<<nblk(cnt(3)), 256, 0, s>>>(n->ga[2], A[A3], n->gb[3], B, h[2], w[2]);
+  launch(k_wn_downsum_mask, nblk(cnt(3)), 256, 0, s, n->ga[2], A[A3], n->gb[3], B, h[2], w[2]);
   g_thorin_launches++;
   // e3 (input p3 = pool(a2))
   RCHK_WN(wgrad_launch<32, 32>(n, 3, A[P3], n->gb[3], B, h[3], w[3], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[3], n->wt[3], nullptr, 0, n->gf[3], B, h[3], w[3], s));
-  k_wn_unpool_mask<<<nblk(cnt(2)), 256, 0, s>>>(n->ga[2], n->gf[3], A[A2], n->gb[2], B, h[2], w[2]);
+  launch(k_wn_unpool_mask, nblk(cnt(2)), 256, 0, s, n->ga[2], n->gf[3], A[A2], n->gb[2], B, h[2], w[2]);
   g_thorin_launches++;
   // e2
   RCHK_WN(wgrad_launch<32, 32>(n, 2, A[P2], n->gb[2], B, h[2], w[2], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[2], n->wt[2], nullptr, 0, n->gf[2], B, h[2], w[2], s));
-  k_wn_unpool_mask<<<nblk(cnt(1)), 256, 0, s>>>(n->ga[1], n->gf[2], A[A1], n->gb[1], B, h[1], w[1]);
+  launch(k_wn_unpool_mask, nblk(cnt(1)), 256, 0, s, n->ga[1], n->gf[2], A[A1], n->gb[1], B, h[1], w[1]);
   g_thorin_launches++;
   // e1
   RCHK_WN(wgrad_launch<32, 32>(n, 1, A[P1], n->gb[1], B, h[1], w[1], s));
   RCHK_WN(conv_launch<32, 32, 2>(n, n->gb[1], n->wt[1], nullptr, 0, n->gf[1], B, h[1], w[1], s));
-  k_wn_unpool_mask<<<nblk(cnt(0)), 256, 0, s>>>(n->ga[0], n->gf[1], A[A0], n->gb[0], B, h[0], w[0]);
+  launch(k_wn_unpool_mask, nblk(cnt(0)), 256, 0, s, n->ga[0], n->gf[1], A[A0], n->gb[0], B, h[0], w[0]);
   g_thorin_launches++;
   // e0
   RCHK_WN(wgrad_launch<16, 32>(n, 0, n->x, n->gb[0], B, h[0], w[0], s));
@@ -1126,13 +1154,13 @@ static int wn_adam(thorin_warmnet *n, float lr, float b1, float b2, float eps, f
 {
   const int np = THORIN_WN_NPARAMS;
   double *part = n->dscal + 8;
-  k_wn_sqnorm<<<64, 256, 0, s>>>(n->g, np, part);
+  launch(k_wn_sqnorm, 64, 256, 0, s, n->g, np, part);
   g_thorin_launches++;
-  k_wn_sum<<<1, 32, 0, s>>>(part, 64, 1.0, n->dscal + 1);
+  launch(k_wn_sum, 1, 32, 0, s, part, 64, 1.0, n->dscal + 1);
   g_thorin_launches++;
   n->adam_t++;
   const float bc1 = 1.f - powf(b1, (float)n->adam_t), bc2 = 1.f - powf(b2, (float)n->adam_t);
-  k_wn_adam<<<nblk(np), 256, 0, s>>>(n->w, n->g, n->m, n->v, np, lr, b1, b2, eps, bc1, bc2, n->dscal + 1, max_norm);
+  launch(k_wn_adam, nblk(np), 256, 0, s, n->w, n->g, n->m, n->v, np, lr, b1, b2, eps, bc1, bc2, n->dscal + 1, max_norm);
   g_thorin_launches++;
   pack_all(n, s);
   return THORIN_OK;
@@ -1164,20 +1192,20 @@ int wn_sor_predict(thorin_warmnet *n, int nr, int ns, int fc, double *T, const d
   double *part = n->dscal + 8;
   const int sb = 2 * n->nsm;
   if (jscale && omega_dev) {   // omega on the device (device-resident DT)
-    k_wn_sum_omega<<<1, 32, 0, s>>>(jscale, 1, omega_dev, (double)(nr - 2), (double)ns, n->dscal + 2);
+    launch(k_wn_sum_omega, 1, 32, 0, s, jscale, 1, omega_dev, (double)(nr - 2), (double)ns, n->dscal + 2);
     g_thorin_launches += 1;
   } else if (jscale) {      // sum of omega |r / Ml| from the solve's own residual pass
-    k_wn_sum<<<1, 32, 0, s>>>(jscale, 1, 1.0 / (omega * (double)(nr - 2) * ns), n->dscal + 2);
+    launch(k_wn_sum, 1, 32, 0, s, jscale, 1, 1.0 / (omega * (double)(nr - 2) * ns), n->dscal + 2);
     g_thorin_launches += 1;
   } else {
-    k_wn_scale<<<sb, 256, 0, s>>>(nr, ns, T, m, part);
-    k_wn_sum<<<1, 32, 0, s>>>(part, sb, 1.0 / ((double)(nr - 2) * ns), n->dscal + 2);
+    launch(k_wn_scale, sb, 256, 0, s, nr, ns, T, m, part);
+    launch(k_wn_sum, 1, 32, 0, s, part, sb, 1.0 / ((double)(nr - 2) * ns), n->dscal + 2);
     g_thorin_launches += 2;
   }
-  k_wn_features<<<nblk((long long)(nr / fc) * (ns / fc)), 256, 0, s>>>(nr, ns, fc, T, m, n->dscal + 2, prev, n->x, jac);
+  launch(k_wn_features, nblk((long long)(nr / fc) * (ns / fc)), 256, 0, s, nr, ns, fc, T, m, n->dscal + 2, prev, n->x, jac);
   g_thorin_launches += 1;
   RCHK_WN(wn_forward(n, 1, s));
-  k_wn_apply<<<nblk((long long)(nr - 2) * ns), 256, 0, s>>>(nr, ns, fc, T, jac, n->y, n->dscal + 2);
+  launch(k_wn_apply, nblk((long long)(nr - 2) * ns), 256, 0, s, nr, ns, fc, T, jac, n->y, n->dscal + 2);
   g_thorin_launches++;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? THORIN_OK : wn_fail("predict kernels", e);
@@ -1198,21 +1226,21 @@ int wn_sor_train(thorin_warmnet *n, int nr, int ns, int fc, const double *tk, co
   const int sb = 2 * n->nsm;
   const long long cells = (long long)nr * ns, ncells = (long long)(nr / fc) * (ns / fc);
   const double inv_n = 1.0 / ((double)(nr - 2) * ns), inv_nc = 1.0 / (double)ncells;
-  k_wn_scale<<<sb, 256, 0, s>>>(nr, ns, tk, m, part);
-  k_wn_sum<<<1, 32, 0, s>>>(part, sb, inv_n, n->dscal + 2);
-  k_wn_sum<<<1, 32, 0, s>>>(part + sb, sb, inv_n, n->dscal + 3);
-  k_wn_features<<<nblk(ncells), 256, 0, s>>>(nr, ns, fc, tk, m, n->dscal + 2, prev, n->x, jac);
-  k_wn_target<<<nblk(ncells), 256, 0, s>>>(nr, ns, fc, tconv, tk, jac, n->dscal + 2, n->tgt);
+  launch(k_wn_scale, sb, 256, 0, s, nr, ns, tk, m, part);
+  launch(k_wn_sum, 1, 32, 0, s, part, sb, inv_n, n->dscal + 2);
+  launch(k_wn_sum, 1, 32, 0, s, part + sb, sb, inv_n, n->dscal + 3);
+  launch(k_wn_features, nblk(ncells), 256, 0, s, nr, ns, fc, tk, m, n->dscal + 2, prev, n->x, jac);
+  launch(k_wn_target, nblk(ncells), 256, 0, s, nr, ns, fc, tconv, tk, jac, n->dscal + 2, n->tgt);
   g_thorin_launches += 5;
   RCHK_WN(wn_forward(n, 1, s));
   float *rs = n->gf[0], *gfine = n->gf[0] + cells;    // free until the backward pass (>= 8 * cells floats)
-  k_wn_tpred<<<nblk(cells), 256, 0, s>>>(nr, ns, fc, tk, jac, n->y, n->dscal + 2, scratch);
-  k_wn_res<<<nblk(cells), 256, 0, s>>>(nr, ns, scratch, m, n->dscal + 3, rs, part);
-  k_wn_sum<<<1, 32, 0, s>>>(part, (int)nblk(cells), inv_n, n->dscal + 4);
-  k_wn_res_grad<<<nblk(cells), 256, 0, s>>>(nr, ns, rs, m, n->dscal + 2, n->dscal + 3, WRES, inv_n, gfine);
-  k_wn_out_grad<<<nblk(ncells), 256, 0, s>>>(nr, ns, fc, gfine, n->y, n->tgt, WSUP, inv_nc, n->act[GY16], part);
-  k_wn_sum<<<1, 32, 0, s>>>(part, (int)nblk(ncells), inv_nc, n->dscal + 5);
-  k_wn_total<<<1, 1, 0, s>>>(n->dscal, WRES, WSUP);
+  launch(k_wn_tpred, nblk(cells), 256, 0, s, nr, ns, fc, tk, jac, n->y, n->dscal + 2, scratch);
+  launch(k_wn_res, nblk(cells), 256, 0, s, nr, ns, scratch, m, n->dscal + 3, rs, part);
+  launch(k_wn_sum, 1, 32, 0, s, part, (int)nblk(cells), inv_n, n->dscal + 4);
+  launch(k_wn_res_grad, nblk(cells), 256, 0, s, nr, ns, rs, m, n->dscal + 2, n->dscal + 3, WRES, inv_n, gfine);
+  launch(k_wn_out_grad, nblk(ncells), 256, 0, s, nr, ns, fc, gfine, n->y, n->tgt, WSUP, inv_nc, n->act[GY16], part);
+  launch(k_wn_sum, 1, 32, 0, s, part, (int)nblk(ncells), inv_nc, n->dscal + 5);
+  launch(k_wn_total, 1, 1, 0, s, n->dscal, WRES, WSUP);
   g_thorin_launches += 7;
   RCHK_WN(wn_backward(n, 1, s, false));
   RCHK_WN(wn_adam(n, lr, 0.9f, 0.999f, 1e-8f, 1.0f, s));
@@ -1226,7 +1254,7 @@ int wn_record_update(int nr, int ns, const double *tconv, const double *tstart, 
                      const double *dt, double *dts, cudaStream_t s)
 {
   const long long cells = (long long)nr * ns;
-  k_wn_record<<<nblk(cells), 256, 0, s>>>(cells, tconv, tstart, hist, nh, dt, dts);
+  launch(k_wn_record, nblk(cells), 256, 0, s, cells, tconv, tstart, hist, nh, dt, dts);
   g_thorin_launches++;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? THORIN_OK : wn_fail("record kernel", e);
@@ -1259,10 +1287,10 @@ int ws_extrapolate(int nr, int ns, double *T, const double *hist, int order, con
   const long long cells = (long long)nr * ns;
   const SorSys m{ml, mlip, mlim, mljp, mljm, rhs};
   const int nb = 2 * nsm;
-  k_ws_delta<<<nblk(cells), 256, 0, s>>>(cells, hist, order, dt, dts, cf, scratch);
-  k_ws_line<<<nb, 256, 0, s>>>(nr, ns, T, scratch, m, cw, omega, vq, part);
-  k_ws_step<<<1, 256, 0, s>>>(part, nb, step);
-  k_ws_apply<<<nblk((long long)(nr - 2) * ns), 256, 0, s>>>(nr, ns, T, vq, step, dts);
+  launch(k_ws_delta, nblk(cells), 256, 0, s, cells, hist, order, dt, dts, cf, scratch);
+  launch(k_ws_line, nb, 256, 0, s, nr, ns, T, scratch, m, cw, omega, vq, part);
+  launch(k_ws_step, 1, 256, 0, s, part, nb, step);
+  launch(k_ws_apply, nblk((long long)(nr - 2) * ns), 256, 0, s, nr, ns, T, vq, step, dts);
   g_thorin_launches += 4;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? THORIN_OK : wn_fail("extrapolation kernels", e);
