@@ -108,22 +108,46 @@ __global__ void k_g_force_prep(StepDev S)
   ctl[CTL_INDY_PL] = S.indirect_term ? -ays : 0.0;
 }
 
-// The N-body step of thorin_planet.cuh (pl_nbody_step_n) by one warp: lane
+// The N-body step of thorin_planet.cuh (pl_nbody_step_n) by two warps.  Lane
 // 3 i + c holds component c of body i's position and velocity (N <= 9 bodies,
 // 27 lanes), so an update of the state is one FP64 instruction instead of 3 N,
 // and a body's distance to another is formed from its three lanes' squares by
 // shuffles.  Every sum keeps the order of the host's loops (a body's partners
 // in ascending order, the star first), and 2 k and 1 k are exact products, so
-// the results are the host's bits.  A warp gets one FP64 instruction per 64
-// cycles whatever the lanes do, so one thread took 7.8 us a step (2.0 ms for
-// the 256 steps of two bodies, longer than the hydro substep of a small disk);
-// this takes about 19 FP64 instructions a stage instead of 62.  A 192x576 disk's
-// DT of two substeps as a graph: 6.6 -> 2.9 ms.
-__device__ void nbody_step_warp(thorin_planets *sys, double dt)
+// the results are the host's bits.
+// A warp gets one FP64 instruction per 64 cycles whatever the lanes do, and
+// 1024 accelerations in line were longer than the hydro substep of a small
+// disk.  But of a step's four only two are in line: a0 and a1 need no other, a2
+// needs a0 and a3 needs a1.  So one warp (on another sub-partition) takes a0, a2 and
+// the new positions, the other one a1, a3 and the new velocities, 39 FP64
+// instructions each with two bodies, where one warp had 84: a DT of one substep of
+// a 24x72 disk as a graph 866 -> 518 us.
+
+// Acceleration of the lane's component at positions xt.
+__device__ __forceinline__ double nbody_acc(double xt, double m, int N, int body, int c)
 {
+  const int b0 = 3 * body;                         // the body's first lane
+  double a = 0.0;
+  for (int k = 1; k < N; k++) {
+    // partner k - 1 of the other bodies in ascending order; lanes of one
+    // body take the same one, and every lane stays in the loop
+    const int p = (k <= body) ? k - 1 : k;
+    const double d = __shfl_sync(TH_FULL, xt, 3 * p + c) - xt;
+    const double q = d * d;
+    const double r2 = (__shfl_sync(TH_FULL, q, b0) + __shfl_sync(TH_FULL, q, b0 + 1)) + __shfl_sync(TH_FULL, q, b0 + 2);
+    const double ir3 = div_fast(1.0, r2 * sqrt_fast(r2));
+    const double f = __shfl_sync(TH_FULL, m, 3 * p) * d * ir3;
+    a = (k == 1) ? f : a + f;
+  }
+  return a;
+}
+
+// By a block of two warps; ends with a barrier.
+__device__ void nbody_step_pair(thorin_planets *sys, double dt)
+{
+  __shared__ double sa0[32], sa2[32], sv2[32], sxn[32], svn[32];
   const int N = sys->nb + 1;
   const int lane = threadIdx.x & 31, body = min(lane / 3, N - 1), c = lane - 3 * (lane / 3);
-  const int b0 = 3 * body;                         // the body's first lane
   const double *px = (c == 0) ? sys->x : (c == 1) ? sys->y : sys->z;
   const double *pv = (c == 0) ? sys->vx : (c == 1) ? sys->vy : sys->vz;
   double x = body > 0 ? px[body - 1] : 0.0, v = body > 0 ? pv[body - 1] : 0.0;
@@ -138,49 +162,51 @@ __device__ void nbody_step_warp(thorin_planets *sys, double dt)
   }
   x -= cx / M;
   v -= cv / M;
+  __syncthreads();                                 // both have read the state
   const int nsteps = 256;
-  const double h = dt / nsteps, h6 = h / 6.0;
-  for (int s = 0; s < nsteps; s++) {
-    double sx = 0.0, sv = 0.0, kx = 0.0, kv = 0.0;
-#pragma unroll
-    for (int stage = 0; stage < 4; stage++) {
-      const double ch = (stage == 0) ? 0.0 : (stage == 3) ? 1.0 * h : 0.5 * h;
-      const double w = (stage == 1 || stage == 2) ? 2.0 : 1.0;
-      const double xt = (stage == 0) ? x : x + ch * kx;
-      const double vt = (stage == 0) ? v : v + ch * kv;
-      double a = 0.0;
-      for (int k = 1; k < N; k++) {
-        // partner k - 1 of the other bodies in ascending order; lanes of one
-        // body take the same one, and every lane stays in the loop
-        const int p = (k <= body) ? k - 1 : k;
-        const double d = __shfl_sync(TH_FULL, xt, 3 * p + c) - xt;
-        const double q = d * d;
-        const double r2 = (__shfl_sync(TH_FULL, q, b0) + __shfl_sync(TH_FULL, q, b0 + 1)) +
-                          __shfl_sync(TH_FULL, q, b0 + 2);
-        const double ir3 = div_fast(1.0, r2 * sqrt_fast(r2));
-        const double f = __shfl_sync(TH_FULL, m, 3 * p) * d * ir3;
-        a = (k == 1) ? f : a + f;
-      }
-      kx = vt;
-      kv = a;
-      sx = (stage == 0) ? kx : __fma_rn(w, kx, sx);
-      sv = (stage == 0) ? kv : __fma_rn(w, kv, sv);
+  const double h = dt / nsteps, h6 = h / 6.0, hh = 0.5 * h;
+  if (threadIdx.x < 32) {
+    for (int s = 0; s < nsteps; s++) {
+      const double a0 = nbody_acc(x, m, N, body, c);
+      sa0[lane] = a0;
+      const double v1 = v + hh * a0, x2 = x + hh * v1;
+      const double a2 = nbody_acc(x2, m, N, body, c);
+      sa2[lane] = a2;
+      const double v3 = v + h * a2;
+      __syncthreads();                             // a0, a2 and v2
+      x += h6 * (__fma_rn(2.0, sv2[lane], __fma_rn(2.0, v1, v)) + v3);
+      sxn[lane] = x;
+      __syncthreads();                             // the new x and v
+      v = svn[lane];
     }
-    x += h6 * sx;
-    v += h6 * sv;
+  } else {
+    for (int s = 0; s < nsteps; s++) {
+      const double x1 = x + hh * v;
+      const double a1 = nbody_acc(x1, m, N, body, c);
+      const double v2 = v + hh * a1;
+      sv2[lane] = v2;
+      const double x3 = x + h * v2;
+      const double a3 = nbody_acc(x3, m, N, body, c);
+      __syncthreads();
+      v += h6 * (__fma_rn(2.0, sa2[lane], __fma_rn(2.0, a1, sa0[lane])) + a3);
+      svn[lane] = v;
+      __syncthreads();
+      x = sxn[lane];
+    }
   }
   const double xh = x - __shfl_sync(TH_FULL, x, c), vh = v - __shfl_sync(TH_FULL, v, c);
-  if (lane >= 3 && lane < 3 * N) {
+  if (threadIdx.x >= 3 && threadIdx.x < 3 * N) {   // of the first warp
     double *ox = (c == 0) ? sys->x : (c == 1) ? sys->y : sys->z;
     double *ov = (c == 0) ? sys->vx : (c == 1) ? sys->vy : sys->vz;
     ox[body - 1] = xh;
     ov[body - 1] = vh;
   }
+  __syncthreads();
 }
 
 // AdvanceSystemFromDisk with DampingTW04, the N-body step and RotatePsys
-// (SourceEuler.c:251-268), one warp.
-__global__ void __launch_bounds__(32) k_g_planet_step(StepDev S)
+// (SourceEuler.c:251-268), two warps.
+__global__ void __launch_bounds__(64) k_g_planet_step(StepDev S)
 {
   pdl_wait();
   thorin_planets *sys = S.sys;
@@ -197,9 +223,8 @@ __global__ void __launch_bounds__(32) k_g_planet_step(StepDev S)
     const double ind[2] = {S.scal[SC_INDX], S.scal[SC_INDY]};
     pl_advance_from_disk(S.c, sys, dt, ind, rrho, rcs);
   }
-  __syncwarp();
-  if (sys->nb > 0) nbody_step_warp(sys, dt);
-  __syncwarp();
+  __syncthreads();
+  if (sys->nb > 0) nbody_step_pair(sys, dt);
   if (threadIdx.x == 0) pl_rotate(sys, S.g.ctl[CTL_OMEGA_FRAME] * dt);
 }
 
@@ -262,7 +287,7 @@ void graph_acc_init(const StepDev &S, cudaStream_t s) { launch(k_g_acc_init, 1, 
 void graph_acc_prep(const StepDev &S, int k, cudaStream_t s) { launch(k_g_acc_prep, 1, 32, 0, s, S, k); g_thorin_launches++; }
 void graph_acc_finish(const StepDev &S, int k, cudaStream_t s) { launch(k_g_acc_finish, 1, 32, 0, s, S, k); g_thorin_launches++; }
 void graph_force_prep(const StepDev &S, cudaStream_t s) { launch(k_g_force_prep, 1, 32, 0, s, S); g_thorin_launches++; }
-void graph_planet_step(const StepDev &S, cudaStream_t s) { launch(k_g_planet_step, 1, 32, 0, s, S); g_thorin_launches++; }
+void graph_planet_step(const StepDev &S, cudaStream_t s) { launch(k_g_planet_step, 1, 64, 0, s, S); g_thorin_launches++; }
 void graph_sor_begin(const StepDev &S, cudaStream_t s) { launch(k_g_sor_begin, 1, 32, 0, s, S); g_thorin_launches++; }
 void graph_sor_end(const StepDev &S, cudaStream_t s) { launch(k_g_sor_end, 1, 32, 0, s, S); g_thorin_launches++; }
 void graph_sub_end(const StepDev &S, cudaStream_t s) { launch(k_g_sub_end, 1, 32, 0, s, S); g_thorin_launches++; }
