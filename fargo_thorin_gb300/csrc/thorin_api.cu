@@ -140,6 +140,9 @@ struct thorin_disk {
   TransportScratch ts_peb;
   cudaStream_t s_peb = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_cs = nullptr, ev_cfl = nullptr, ev_forces = nullptr;   // their results are on the host
+  int (*host_side)(void *) = nullptr;   // host work that the substep has still to do (run_host_side)
+  void *host_arg = nullptr;
   double *partials, *scal;
   int *iscal, *nshift, *heat_idx_d, *damp_rings_d;
   double *heat_val_d;
@@ -482,6 +485,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   CUCHK(cudaMallocHost((void **)&d->scal_h, 256 * sizeof(double)));
   CUCHK(cudaMallocHost((void **)&d->iscal_h, 64 * sizeof(int)));
   CUCHK(cudaMallocHost((void **)&d->csmean_h, n1 * sizeof(double)));
+  for (cudaEvent_t *e : {&d->ev_cs, &d->ev_cfl, &d->ev_forces}) CUCHK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   // SOR control block
   const int sb = sor_blocks(d->g);
   double *sp;
@@ -715,6 +719,7 @@ extern "C" int thorin_gpu_destroy(thorin_disk *d)
     cudaStreamDestroy(d->s_pl);
   }
   for (int q = 0; q < 4; q++) cudaEventDestroy(d->ev[q]);
+  for (cudaEvent_t e : {d->ev_cs, d->ev_cfl, d->ev_forces}) cudaEventDestroy(e);
   if (d->s_peb) {
     cudaStreamSynchronize(d->s_peb);
     cudaEventDestroy(d->ev_fork);
@@ -1270,16 +1275,28 @@ static void cfl_launches(thorin_disk *d)
           (p.viscosity_alpha || p.viscosity != 0.0), d->partials, cfl_args(d), d->scal, d->iscal, d->s);
 }
 
-extern "C" int thorin_gpu_cfl(thorin_disk *d, double dt_remaining, double invdtreb_sq, int *n_sub)
+static int cfl_begin(thorin_disk *d, double dt_remaining, double invdtreb_sq)
 {
   set_ctl(d, {{CTL_DELTAT, dt_remaining}, {CTL_INVDTREB, invdtreb_sq}});
   cfl_launches(d);
   d->cfl_first = 0;
   KCHECK("cfl kernels");
   CUCHK(cudaMemcpyAsync(d->iscal_h, d->iscal, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, d->s));
-  CUCHK(cudaStreamSynchronize(d->s));
+  CUCHK(cudaEventRecord(d->ev_cfl, d->s));
+  return THORIN_OK;
+}
+
+static int cfl_end(thorin_disk *d, int *n_sub)
+{
+  CUCHK(cudaEventSynchronize(d->ev_cfl));
   *n_sub = d->iscal_h[IS_NSUB];
   return THORIN_OK;
+}
+
+extern "C" int thorin_gpu_cfl(thorin_disk *d, double dt_remaining, double invdtreb_sq, int *n_sub)
+{
+  RCHK(cfl_begin(d, dt_remaining, invdtreb_sq));
+  return cfl_end(d, n_sub);
 }
 
 extern "C" int thorin_gpu_stokes(thorin_disk *d)
@@ -1309,7 +1326,7 @@ static void heating1(thorin_disk *d, double Mp, double dMp, double Xp, double Yp
 extern "C" int thorin_gpu_accrete(thorin_disk *d, thorin_planets *sys, double dt)
 {
   const thorin_params &p = d->p;
-  {
+  if (p.pebbles && p.evaporation_rate > 0.0) {
     double facc = p.evaporation_rate * dt;                         // EvaporatePebbles' fraction
     if (facc > 1.0) facc = 1.0;
     set_ctl(d, {{CTL_DT, dt}, {CTL_OMEGA_FRAME, d->OmegaFrame}, {CTL_FACC_EVAP, facc}});
@@ -1411,15 +1428,22 @@ static ForceArgs force_args(const thorin_disk *d, int npl)
   return a;
 }
 
-extern "C" int thorin_gpu_forces(thorin_disk *d, thorin_planets *sys, double mass_taper, double indirect[2],
-                                 double *ring_rho, double *ring_cs)
+// What of the state before the hydro substep the host needs with the forces'
+// results: UpdateLog's interpolation at each planet.
+struct ForceRead {
+  int npl, torques;
+  int inside[MAXPL_DEV], two[MAXPL_DEV];
+  double frac[MAXPL_DEV], cspl[MAXPL_DEV], time;
+};
+
+// FillForcesArrays and the copy of its results; ring_cs (may be NULL): the
+// ring mean of c_s at each planet.  csmean_h must be current.
+static int forces_begin(thorin_disk *d, thorin_planets *sys, double mass_taper, double *ring_cs, ForceRead *fr)
 {
   const thorin_params &p = d->p;
   const int npl = sys->nb;
-  if (npl > MAXPL_DEV) { g_last_error = "more planets than the force kernel handles"; return THORIN_ERR_ARG; }
   DevPlanet pl[MAXPL_DEV];
   double axs = 0.0, ays = 0.0;
-  CUCHK(cudaStreamSynchronize(d->s));        // csmean_h is current
   for (int k = 0; k < npl; k++)
     pl_force_planet(d->plc, d->Rsup.data(), d->csmean_h, d->OmegaInv.data(), sys, k, mass_taper, &pl[k], &axs, &ays);
   if (npl > 0) CUCHK(cudaMemcpyAsync(d->planets_d, pl, npl * sizeof(DevPlanet), cudaMemcpyHostToDevice, d->s));
@@ -1427,65 +1451,87 @@ extern "C" int thorin_gpu_forces(thorin_disk *d, thorin_planets *sys, double mas
   set_ctl(d, {{CTL_MASS_TAPER, mass_taper}, {CTL_INDX_PL, indx_pl}, {CTL_INDY_PL, indy_pl}});
   aux_forces(d->g, force_args(d, npl), d->fr, d->scal, d->s);
   KCHECK("force kernels");
-  // DampingTW04 needs the ring means of Sigma (and c_s) at each planet
+  fr->npl = npl;
+  fr->torques = d->torque_pending;
+  fr->time = d->PhysicalTime;
   for (int k = 0; k < npl; k++) {
+    // DampingTW04 needs the ring means of Sigma (and c_s) at each planet
     const double r = sqrt(sys->x[k] * sys->x[k] + sys->y[k] * sys->y[k]);
-    if (ring_rho) ring_rho[k] = 0.0;
     if (ring_cs) ring_cs[k] = 0.0;
-    if (r >= d->Rinf[0] && r <= d->Rsup[d->nr - 1]) {
+    fr->inside[k] = (r >= d->Rinf[0] && r <= d->Rsup[d->nr - 1]);
+    if (fr->inside[k]) {
       const int i = ring_of(d, r);
       aux_ring_mean_at(d->g, d->rho, i, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->s);
       if (ring_cs) ring_cs[k] = d->csmean_h[i];
     }
-  }
-  // UpdateLog (Force.c:27-70) needs Sigma's ring means either side of each planet
-  int tq_ring[MAXPL_DEV];
-  const int torques = d->torque_pending;
-  if (torques) {
-    for (int k = 0; k < npl; k++) {
-      const double r = sqrt(sys->x[k] * sys->x[k] + sys->y[k] * sys->y[k]);
-      tq_ring[k] = (int)global_ifrac(d, r);
-      aux_ring_mean_at(d->g, d->rho, tq_ring[k], d->scal + SC_TORQUE + 2 * k, d->s);
-      if (tq_ring[k] + 1 <= d->nr) aux_ring_mean_at(d->g, d->rho, tq_ring[k] + 1, d->scal + SC_TORQUE + 2 * k + 1, d->s);
+    // UpdateLog (Force.c:27-70) needs Sigma's ring means either side of each planet
+    if (fr->torques) {
+      const double ifrac = global_ifrac(d, r), frac = ifrac - floor(ifrac);
+      const int ii = (int)ifrac;
+      fr->two[k] = (ii + 1 <= d->nr);
+      fr->frac[k] = frac;
+      fr->cspl[k] = d->csmean_h[ii] * (1.0 - frac) + (fr->two[k] ? d->csmean_h[ii + 1] : 0.0) * frac;
+      aux_ring_means(d->g, d->rho, d->scal + SC_TORQUE + 2 * k, nullptr, nullptr, ii, fr->two[k] ? 2 : 1, d->s);
     }
   }
   CUCHK(cudaMemcpyAsync(d->scal_h, d->scal, 128 * sizeof(double), cudaMemcpyDeviceToHost, d->s));
-  CUCHK(cudaStreamSynchronize(d->s));
-  for (int k = 0; k < npl; k++) {
+  CUCHK(cudaEventRecord(d->ev_forces, d->s));
+  return THORIN_OK;
+}
+
+static int forces_end(thorin_disk *d, thorin_planets *sys, const ForceRead &fr, double indirect[2], double *ring_rho)
+{
+  const thorin_params &p = d->p;
+  CUCHK(cudaEventSynchronize(d->ev_forces));
+  for (int k = 0; k < fr.npl; k++) {
     sys->ax[k] = d->scal_h[SC_PLANET_A + 2 * k];
     sys->ay[k] = d->scal_h[SC_PLANET_A + 2 * k + 1];
-    const double r = sqrt(sys->x[k] * sys->x[k] + sys->y[k] * sys->y[k]);
-    if (ring_rho && r >= d->Rinf[0] && r <= d->Rsup[d->nr - 1]) ring_rho[k] = d->scal_h[SC_PLANET_A + 2 * MAXPL_DEV + k];
+    if (ring_rho) ring_rho[k] = fr.inside[k] ? d->scal_h[SC_PLANET_A + 2 * MAXPL_DEV + k] : 0.0;
   }
-  if (torques) {
-    for (int k = 0; k < npl; k++) {
+  if (fr.torques) {
+    for (int k = 0; k < fr.npl; k++) {
       const double x = sys->x[k], y = sys->y[k], ax = sys->ax[k], ay = sys->ay[k], m = sys->mass[k];
-      const double r2 = x * x + y * y, r = sqrt(r2);
-      const double ifrac = global_ifrac(d, r), frac = ifrac - floor(ifrac);
-      const int ii = tq_ring[k];
-      const double rho_hi = (ii + 1 <= d->nr) ? d->scal_h[SC_TORQUE + 2 * k + 1] : 0.0;
-      const double cs_hi = (ii + 1 <= d->nr) ? d->csmean_h[ii + 1] : 0.0;
+      const double r2 = x * x + y * y, r = sqrt(r2), frac = fr.frac[k];
+      const double rho_hi = fr.two[k] ? d->scal_h[SC_TORQUE + 2 * k + 1] : 0.0;
       const double rhopl = d->scal_h[SC_TORQUE + 2 * k] * (1.0 - frac) + rho_hi * frac;
-      const double cspl = d->csmean_h[ii] * (1.0 - frac) + cs_hi * frac;
       const double omega = pow(r, -1.5);
-      const double h = cspl / (omega * r) * (1.0 / sqrt(p.adiabind));
+      const double h = fr.cspl[k] / (omega * r) * (1.0 / sqrt(p.adiabind));
       double norm = m * omega * r2 / h;
       norm *= norm;
       norm *= rhopl;
       const double tq = x * ay - y * ax;
       thorin_torque &t = d->torques[k];
-      t.time = d->PhysicalTime;
+      t.time = fr.time;
       t.torque = tq;
       t.torque_norm = tq * m * p.adiabind / norm;
       t.x = x; t.y = y; t.ax = ax; t.ay = ay;
     }
-    d->ntorque = npl;
+    d->ntorque = fr.npl;
     d->torque_pending = 0;
   }
   // IndirectTerm of the disk (the planets' part is only added to the gas)
   indirect[0] = d->scal_h[SC_INDX];
   indirect[1] = d->scal_h[SC_INDY];
   return THORIN_OK;
+}
+
+extern "C" int thorin_gpu_forces(thorin_disk *d, thorin_planets *sys, double mass_taper, double indirect[2],
+                                 double *ring_rho, double *ring_cs)
+{
+  if (sys->nb > MAXPL_DEV) { g_last_error = "more planets than the force kernel handles"; return THORIN_ERR_ARG; }
+  CUCHK(cudaStreamSynchronize(d->s));        // csmean_h is current
+  ForceRead fr;
+  RCHK(forces_begin(d, sys, mass_taper, ring_cs, &fr));
+  return forces_end(d, sys, fr, indirect, ring_rho);
+}
+
+// Host work that a substep left to be done while the GPU is busy.
+static int run_host_side(thorin_disk *d)
+{
+  if (!d->host_side) return THORIN_OK;
+  int (*f)(void *) = d->host_side;
+  d->host_side = nullptr;
+  return f(d->host_arg);
 }
 
 extern "C" int thorin_gpu_request_torques(thorin_disk *d)
@@ -1590,6 +1636,7 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
   }
   if (d->timing) CUCHK(cudaEventRecord(d->ev[0], d->s));
   if (d->sor_direct) {
+    RCHK(run_host_side(d));
     // THORIN_SOR_DIRECT: the same kernels (no graph condition) as plain
     // launches in chunks of sor_loop_k sweeps, the done flag read after each
     // chunk; kernel profilers list these, not kernels inside conditional
@@ -1613,6 +1660,7 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
   }
   if (d->timing) CUCHK(cudaEventRecord(d->ev[1], d->s));
   CUCHK(cudaMemcpyAsync(d->iscal_h + IS_SOR_DONE, d->sor.done, 2 * sizeof(int), cudaMemcpyDeviceToHost, d->s));
+  RCHK(run_host_side(d));
   CUCHK(cudaStreamSynchronize(d->s));
   const int done = d->iscal_h[IS_SOR_DONE], n = d->iscal_h[IS_SOR_DONE + 1];
   if (!done || n < 1) {
@@ -1885,6 +1933,7 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
   aux_viscosity_rings(d->g, d->vp, d->s);
   if (!d->capturing)
     CUCHK(cudaMemcpyAsync(d->csmean_h, d->ring[R_CSMEAN], d->nr * sizeof(double), cudaMemcpyDeviceToHost, d->s));
+  if (!d->capturing) CUCHK(cudaEventRecord(d->ev_cs, d->s));
   if (p.pebbles) CUCHK(cudaStreamWaitEvent(d->s, d->ev_join, 0));     // join the pebble transport
   KCHECK("hydro kernels");
   if (d->capturing) return status;     // clock and crash flag stay on the device
@@ -2018,6 +2067,23 @@ static void frame_point(int guiding_center, const thorin_planets *sys, double *x
   }
 }
 
+// The planets' side of a substep after its forces are launched.
+struct PlanetSide {
+  thorin_disk *d;
+  thorin_planets *sys;
+  ForceRead fr;
+  double dt, ind[2], rrho[THORIN_MAXPLANETS], rcs[THORIN_MAXPLANETS];
+};
+
+static int planet_side(PlanetSide *q)
+{
+  RCHK(forces_end(q->d, q->sys, q->fr, q->ind, q->rrho));
+  advance_from_disk(q->d, q->sys, q->dt, q->ind, q->rrho, q->rcs);
+  if (q->d->p.aerodynamic_drag) RCHK(thorin_gpu_drag(q->d, q->sys, q->dt));
+  pl_nbody_step(q->sys, q->dt);
+  return THORIN_OK;
+}
+
 extern "C" int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys)
 {
   const thorin_params &p = d->p;
@@ -2039,42 +2105,73 @@ extern "C" int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys)
     RCHK(rc);
     dt = DT / (double)n;
   }
+  // The planets' side of a substep (the kick from the disk's forces and the
+  // N-body step) is host work that the hydro substep does not read, unless the
+  // frame follows a planet; and the forces need the CFL's dt only where planets
+  // accrete before them.  So the host launches the forces before it waits for
+  // the CFL, and does the planets' side, a wait and 30 us of RK4 steps, while the
+  // hydro substep runs (run_host_side, before the solve's own wait).  DTs: 24x72 436 ->
+  // 404 us, 256x768 isothermal (two substeps) 886 -> 816 us.
+  const bool beside = !p.corotating && !p.aerodynamic_drag;
+  bool forces_first = beside && !p.pebbles && !p.prescribed_accretion && !p.sloppy_cfl;
+  for (int k = 0; k < sys->nb; k++) forces_first = forces_first && !(sys->acc[k] > 1e-10);
+  CUCHK(cudaStreamSynchronize(d->s));          // csmean_h is current
   while (dtemp < 0.999999999 * DT) {
     d->MassTaper = pl_mass_taper(d->PhysicalTime, p.mass_taper);
+    PlanetSide ps;
+    ps.d = d;
+    ps.sys = sys;
     if (!p.sloppy_cfl) {
       const double invdtreb_sq = pl_min_step_for_rebound(sys);
       int n;
-      RCHK(thorin_gpu_cfl(d, DT - dtemp, invdtreb_sq, &n));
+      RCHK(cfl_begin(d, DT - dtemp, invdtreb_sq));
+      if (forces_first) {
+        CUCHK(cudaEventSynchronize(d->ev_cs));
+        RCHK(forces_begin(d, sys, d->MassTaper, ps.rcs, &ps.fr));
+      }
+      RCHK(cfl_end(d, &n));
       dt = (DT - dtemp) / (double)n;
     } else if (p.pebbles) {
       aux_stokes(d->g, d->rho, d->psize, d->tau, d->s);       // PebbleStokesNumbers, every substep
     }
     RCHK(thorin_gpu_accrete(d, sys, dt));
     dtemp += dt;
-    double ind[2], rrho[THORIN_MAXPLANETS], rcs[THORIN_MAXPLANETS];
+    ps.dt = dt;
     double xmark, ymark;                                     // GetPsysInfo (MARK)
     frame_point(p.guiding_center, sys, &xmark, &ymark);
-    RCHK(thorin_gpu_forces(d, sys, d->MassTaper, ind, rrho, rcs));
-    advance_from_disk(d, sys, dt, ind, rrho, rcs);
-    if (p.aerodynamic_drag) RCHK(thorin_gpu_drag(d, sys, dt));
-    pl_nbody_step(sys, dt);
-    if (p.corotating) {
-      // GetPsysInfo (GET): the angle planet 0 (or its guiding centre) moved
-      // through; the frame follows it and the azimuthal velocities are
-      // corrected (SourceEuler.c:261-267, CorrectVtheta SideEuler.c:505-519)
-      double x, y;
-      frame_point(p.guiding_center, sys, &x, &y);
-      const double d2 = sqrt(x * x + y * y), d1 = sqrt(xmark * xmark + ymark * ymark);
-      const double cross = xmark * y - x * ymark;
-      const double OmegaNew = asin(cross / (d1 * d2)) / dt;
-      const double domega = OmegaNew - d->OmegaFrame;
-      aux_correct_vtheta(d->g, d->vtheta, domega, d->s);
-      if (p.pebbles) aux_correct_vtheta(d->g, d->pvtheta, domega, d->s);
-      d->OmegaFrame = OmegaNew;
+    if (!forces_first) {
+      if (p.sloppy_cfl) CUCHK(cudaEventSynchronize(d->ev_cs));
+      RCHK(forces_begin(d, sys, d->MassTaper, ps.rcs, &ps.fr));
     }
-    pl_rotate(sys, d->OmegaFrame * dt);
-    int s = thorin_gpu_hydro(d, dt);
+    if (beside) {
+      d->host_arg = &ps;
+      d->host_side = [](void *q) {
+        PlanetSide *s = (PlanetSide *)q;
+        RCHK(planet_side(s));
+        pl_rotate(s->sys, s->d->OmegaFrame * s->dt);
+        return THORIN_OK;
+      };
+    } else {
+      RCHK(planet_side(&ps));
+      if (p.corotating) {
+        // GetPsysInfo (GET): the angle planet 0 (or its guiding centre) moved
+        // through; the frame follows it and the azimuthal velocities are
+        // corrected (SourceEuler.c:261-267, CorrectVtheta SideEuler.c:505-519)
+        double x, y;
+        frame_point(p.guiding_center, sys, &x, &y);
+        const double d2 = sqrt(x * x + y * y), d1 = sqrt(xmark * xmark + ymark * ymark);
+        const double cross = xmark * y - x * ymark;
+        const double OmegaNew = asin(cross / (d1 * d2)) / dt;
+        const double domega = OmegaNew - d->OmegaFrame;
+        aux_correct_vtheta(d->g, d->vtheta, domega, d->s);
+        if (p.pebbles) aux_correct_vtheta(d->g, d->pvtheta, domega, d->s);
+        d->OmegaFrame = OmegaNew;
+      }
+      pl_rotate(sys, d->OmegaFrame * dt);
+    }
+    const int s = thorin_gpu_hydro(d, dt), sp = run_host_side(d);
     if (s != THORIN_OK && s != THORIN_ERR_SOR_MAXIT) return s;
+    RCHK(sp);
     if (s != THORIN_OK) status = s;
     nsub++;
   }
