@@ -367,7 +367,7 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
                                                                       viscous, upper, bound);
     g_thorin_launches++;
   }
-  launch(k_cfl_cells, grid2d(g.ns, g.nr - 1, 256), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
+  launch_fp64(k_cfl_cells, grid2d(g.ns, g.nr - 1, 256), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
                                                           bound, top);
   g_thorin_launches++;
   launch(k_cfl_final, 1, 1024, 0, s, g, cr, f0, scal, iscal, bound, top);
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(1024) k_forces_final(DevGrid g, ForceArgs a, d
 template <int NP>
 static void launch_forces(const DevGrid &g, const ForceArgs &a, const ForceRings &fr, dim3 grid, cudaStream_t s)
 {
-  launch(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
+  launch_fp64(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
 }
 
 void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
@@ -1014,7 +1014,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   a.nba = ga.x * ga.y;
   a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
   a.nbb = a.nbn + (a.npl > 0 ? g.nsm : 0);
-  launch(k_force_rings, g.nr, RING_T, 0, s, g, a, fr);
+  launch_fp64(k_force_rings, g.nr, RING_T, 0, s, g, a, fr);
   g_thorin_launches++;
   switch (a.npl) {
   case 0: launch_forces<0>(g, a, fr, ga, s); break;
@@ -1024,7 +1024,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   default: launch_forces<MAXPL_DEV>(g, a, fr, ga, s); break;
   }
   g_thorin_launches++;
-  launch(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
+  launch_fp64(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
   g_thorin_launches++;
   launch(k_forces_final, 2 + 2 * a.npl, 1024, 0, s, g, a, scal);
   g_thorin_launches++;

@@ -1809,8 +1809,8 @@ void hydro_sources(const DevGrid &g, const SourceIO &io0, cudaStream_t s)
   // 0.15 rings a chunk: the ring below is read again, and the ring constants
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, SRC_MAXRINGS, 0.15);
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
-  if (io.pd) launch(k_sources<true>, grid, BX, 0, s, g, io);
-  else launch(k_sources<false>, grid, BX, 0, s, g, io);
+  if (io.pd) launch_fp64(k_sources<true>, grid, BX, 0, s, g, io);
+  else launch_fp64(k_sources<false>, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
@@ -1819,7 +1819,7 @@ void hydro_viscous(const DevGrid &g, const ViscousIO &io0, cudaStream_t s)
   ViscousIO io = io0;
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, VI_MAXRINGS, 1.8);
   const dim3 grid((g.ns + VI_COLS - 1) / VI_COLS, (g.nr + io.rings - 1) / io.rings);
-  launch(k_viscous, grid, BX, 0, s, g, io);
+  launch_fp64(k_viscous, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
@@ -1829,7 +1829,7 @@ void hydro_heating(const DevGrid &g, const HeatingIO &io0, cudaStream_t s)
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, HT_MAXRINGS, 0.2);
   if (io.rings < 3) io.rings = 3;                  // ring 0 is extrapolated by the thread of rings 1 and 2
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
-  launch(k_heating, grid, BX, 0, s, g, io);
+  launch_fp64(k_heating, grid, BX, 0, s, g, io);
   g_thorin_launches++;
 }
 
@@ -1847,11 +1847,11 @@ void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io0, int law, cudaStrea
   io.rings = chunk_rings(g.nr, g.ns, g.nsm, DC_MAXRINGS, 0.2, 8);
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
   switch (law) {
-  case THORIN_OPA_SM03: launch(k_diffcoef<THORIN_OPA_SM03>, grid, BX, 0, s, g, io); break;
-  case THORIN_OPA_ZHU12: launch(k_diffcoef<THORIN_OPA_ZHU12>, grid, BX, 0, s, g, io); break;
-  case THORIN_OPA_LP85: launch(k_diffcoef<THORIN_OPA_LP85>, grid, BX, 0, s, g, io); break;
-  case THORIN_OPA_CONST: launch(k_diffcoef<THORIN_OPA_CONST>, grid, BX, 0, s, g, io); break;
-  default: launch(k_diffcoef<THORIN_OPA_BL94>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_SM03: launch_fp64(k_diffcoef<THORIN_OPA_SM03>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_ZHU12: launch_fp64(k_diffcoef<THORIN_OPA_ZHU12>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_LP85: launch_fp64(k_diffcoef<THORIN_OPA_LP85>, grid, BX, 0, s, g, io); break;
+  case THORIN_OPA_CONST: launch_fp64(k_diffcoef<THORIN_OPA_CONST>, grid, BX, 0, s, g, io); break;
+  default: launch_fp64(k_diffcoef<THORIN_OPA_BL94>, grid, BX, 0, s, g, io); break;
   }
   g_thorin_launches++;
 }
@@ -1860,7 +1860,7 @@ void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, co
                        double *qirr, double rstar, double tirr4fac, double opacity_drop, double taueff_c,
                        const double *rinf15, const double *rsup15, cudaStream_t s)
 {
-  launch(k_irradiation, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, cs, opacity, flaring, qirr, rstar, tirr4fac, opacity_drop,
+  launch_fp64(k_irradiation, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, cs, opacity, flaring, qirr, rstar, tirr4fac, opacity_drop,
                                                       taueff_c, rinf15, rsup15);
   g_thorin_launches++;
 }
@@ -1879,8 +1879,8 @@ void hydro_matrix(const DevGrid &g, const MatrixIO &io0, const SorCtl *resid, cu
 {
   MatrixIO io = io0;
   io.rings = matrix_rings(g);
-  if (resid) launch(k_matrix<true>, matrix_grid(g), BX, 0, s, g, io, *resid);
-  else launch(k_matrix<false>, matrix_grid(g), BX, 0, s, g, io, SorCtl{});
+  if (resid) launch_fp64(k_matrix<true>, matrix_grid(g), BX, 0, s, g, io, *resid);
+  else launch_fp64(k_matrix<false>, matrix_grid(g), BX, 0, s, g, io, SorCtl{});
   g_thorin_launches++;
 }
 
@@ -2047,10 +2047,10 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
   rd.ext = S.w[6];
   rd.rings = chunk_rings(nr, ns, g.nsm, RD_MAXRINGS, 1.3);
   const dim3 rgrid((ns + BX - 1) / BX, (nr + rd.rings - 1) / rd.rings);
-  if (energy && label) launch(k_radial<true, true>, rgrid, BX, 0, s, g, rd);
-  else if (energy) launch(k_radial<true, false>, rgrid, BX, 0, s, g, rd);
-  else if (label) launch(k_radial<false, true>, rgrid, BX, 0, s, g, rd);
-  else launch(k_radial<false, false>, rgrid, BX, 0, s, g, rd);
+  if (energy && label) launch_fp64(k_radial<true, true>, rgrid, BX, 0, s, g, rd);
+  else if (energy) launch_fp64(k_radial<true, false>, rgrid, BX, 0, s, g, rd);
+  else if (label) launch_fp64(k_radial<false, true>, rgrid, BX, 0, s, g, rd);
+  else launch_fp64(k_radial<false, false>, rgrid, BX, 0, s, g, rd);
   g_thorin_launches++;
   // azimuthal step back into the momenta, the new energy, the tracer and
   // the new density
@@ -2065,12 +2065,12 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
   az.n = nq;
   const int T = azi_block(ns);
   const dim3 grid((ns + T - 2 * AZ_HALO - 1) / (T - 2 * AZ_HALO), nr);
-  if (nq == 7) launch(k_azimuthal<7>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
-  else if (nq == 6) launch(k_azimuthal<6>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
-  else launch(k_azimuthal<5>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  if (nq == 7) launch_fp64(k_azimuthal<7>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else if (nq == 6) launch_fp64(k_azimuthal<6>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
+  else launch_fp64(k_azimuthal<5>, grid, T, 0, s, g, az, vt_in, fast, S.nshift, S.vmed, S.vtemp);
   g_thorin_launches++;
   // velocities from the transported momenta
-  launch(k_velocities, grid2d(ns, nr, BX), BX, 0, s, g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,
+  launch_fp64(k_velocities, grid2d(ns, nr, BX), BX, 0, s, g, S.rho_new, S.mom[0], S.mom[1], S.mom[2], S.mom[3], vr, vt, damp_vrad, drin, drout,
                                                  energy ? S.e_new : nullptr, energy ? temper : nullptr, cs, gm1, gg1 / gm1);
   g_thorin_launches++;
   if (label) {

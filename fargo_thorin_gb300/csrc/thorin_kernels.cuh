@@ -183,7 +183,7 @@ extern std::atomic<long long> g_thorin_launches;
 // 1.181 / 1.175 ms, 128x384 0.522 / 0.508 / 0.499 / 0.499 / 0.515.
 #define PDL_BLOCKS 304
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+inline void launch_upto(size_t most, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
 {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at = {};
@@ -194,8 +194,27 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &at;
-  cfg.numAttrs = ((size_t)grid.x * grid.y * grid.z <= PDL_BLOCKS) ? 1 : 0;
+  cfg.numAttrs = ((size_t)grid.x * grid.y * grid.z <= most) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+{
+  launch_upto(PDL_BLOCKS, kernel, grid, block, smem, s, std::forward<A>(args)...);
+}
+
+// For the kernels that the FP64 pipe bounds: placed early, their blocks gather
+// on the multiprocessors that the kernel before leaves first, and the fullest of
+// these sets the time, so only grids of up to half the multiprocessors go
+// early.  Limits of 0 / 76 / 152 / 304 blocks, ms a substep: 24x72 0.263 / 0.242 /
+// 0.241 / 0.237, 64x192 0.281 / 0.270 / 0.296 / 0.296, 96x288 0.317 / 0.313 / 0.310 /
+// 0.333, from 128x384 on the same.
+#define PDL_BLOCKS_FP64 76
+template <typename... P, typename... A>
+inline void launch_fp64(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+{
+  launch_upto(PDL_BLOCKS_FP64, kernel, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 // kernels_hydro.cu
