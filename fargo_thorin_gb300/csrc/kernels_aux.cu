@@ -61,15 +61,16 @@ void aux_ring_means(const DevGrid &g, const double *f0, double *o0, const double
   g_thorin_launches++;
 }
 
-__global__ void k_set_ctl(double *__restrict__ ctl, CtlSet v)
+__global__ void k_set_ctl(double *__restrict__ ctl, CtlSet v, int *crash)
 {
   pdl_wait();
+  if (crash && threadIdx.x == 0) *crash = 0;
   if (threadIdx.x < (unsigned)v.n) ctl[v.idx[threadIdx.x]] = v.val[threadIdx.x];
 }
 
-void aux_set_ctl(double *ctl, const CtlSet &v, cudaStream_t s)
+void aux_set_ctl(double *ctl, const CtlSet &v, int *crash, cudaStream_t s)
 {
-  launch(k_set_ctl, 1, 32, 0, s, ctl, v);
+  launch(k_set_ctl, 1, 32, 0, s, ctl, v, crash);
   g_thorin_launches++;
 }
 
@@ -78,9 +79,19 @@ void aux_ring_mean(const DevGrid &g, const double *f, double *out, cudaStream_t 
   aux_ring_means(g, f, out, nullptr, nullptr, 0, g.nr, s);
 }
 
-void aux_ring_mean_at(const DevGrid &g, const double *f, int ring, double *out, cudaStream_t s)
+// The means of the rings r.ring[] to r.out[].
+__global__ void __launch_bounds__(RING_T) k_ring_list(int ns, const double *__restrict__ f, RingList r)
 {
-  aux_ring_means(g, f, out, nullptr, nullptr, ring, 1, s);
+  pdl_wait();
+  const double a = ring_sum(f + (size_t)r.ring[blockIdx.x] * ns, ns);
+  if (threadIdx.x == 0) *r.out[blockIdx.x] = a / (double)ns;
+}
+
+void aux_ring_list(const DevGrid &g, const double *f, const RingList &r, cudaStream_t s)
+{
+  if (r.n <= 0) return;
+  launch(k_ring_list, r.n, RING_T, 0, s, g.ns, f, r);
+  g_thorin_launches++;
 }
 
 // FViscosity at Rmed[i] and Rinf[i] (Viscosity.c:26-54).  The ring index
@@ -100,19 +111,28 @@ __device__ __forceinline__ double fvisc(const ViscParams &v, double rad, double 
   return nu;
 }
 
-__global__ void k_viscosity_rings(DevGrid g, ViscParams v)
+// Ring means of the sound speed (and, with alpha_flock, of the temperature)
+// with each ring's viscosity from them, one block per ring.
+__global__ void __launch_bounds__(RING_T) k_sound_rings(DevGrid g, ViscParams v, const double *__restrict__ cs,
+                                                        const double *__restrict__ temper, double *__restrict__ csmean,
+                                                        double *__restrict__ tempmean)
 {
   pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.nr) return;
-  const double cs = g.r.csmean[i], tm = g.r.tempmean[i];
-  g.r.nu_med[i] = fvisc(v, g.r.Rmed[i], cs, tm, g.r.Rmed15[i]);
-  g.r.nu_inf[i] = fvisc(v, g.r.Rinf[i], cs, tm, g.r.Rinf15[i]);
+  const int i = blockIdx.x, ns = g.ns;
+  const double c = ring_sum(cs + (size_t)i * ns, ns) / (double)ns;
+  double t = tempmean[i];
+  if (temper) t = ring_sum(temper + (size_t)i * ns, ns) / (double)ns;
+  if (threadIdx.x != 0) return;
+  csmean[i] = c;
+  tempmean[i] = t;
+  g.r.nu_med[i] = fvisc(v, g.r.Rmed[i], c, t, g.r.Rmed15[i]);
+  g.r.nu_inf[i] = fvisc(v, g.r.Rinf[i], c, t, g.r.Rinf15[i]);
 }
 
-void aux_viscosity_rings(const DevGrid &g, const ViscParams &v, cudaStream_t s)
+void aux_sound_rings(const DevGrid &g, const ViscParams &v, const double *cs, const double *temper, double *csmean,
+                     double *tempmean, cudaStream_t s)
 {
-  launch(k_viscosity_rings, (g.nr + 127) / 128, 128, 0, s, g, v);
+  launch(k_sound_rings, g.nr, RING_T, 0, s, g, v, cs, v.alpha_flock ? temper : nullptr, csmean, tempmean);
   g_thorin_launches++;
 }
 
@@ -313,8 +333,9 @@ __global__ void __launch_bounds__(1024) k_cfl_final(DevGrid g, CflRings cr, CflF
 {
   pdl_wait();
   // the remaining part of the DT and MinStepForRebound's rate come from the
-  // disk's control block; so does the CFL's substep length, written back
-  const double deltaT = g.ctl[CTL_DELTAT], invdtreb_sq = g.ctl[CTL_INVDTREB], dts = scal[SC_DTSTELLAR];
+  // host (own) or the disk's control block, which receives the substep length
+  const double deltaT = f.own ? f.deltaT : g.ctl[CTL_DELTAT], invdtreb_sq = f.own ? f.invdtreb_sq : g.ctl[CTL_INVDTREB],
+               dts = scal[SC_DTSTELLAR];
   const unsigned long long mg = top[0], mp = top[1];
   long long shear = __double_as_longlong(1e30);
   for (int i = threadIdx.x; i < g.nr - 1; i += blockDim.x) {
@@ -367,7 +388,7 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
                                                                       viscous, upper, bound);
     g_thorin_launches++;
   }
-  launch_fp64(k_cfl_cells, grid2d(g.ns, g.nr - 1, 256), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
+  launch(k_cfl_cells, grid2d(g.ns, g.nr - 1, 256), 256, 0, s, g, vr, vt, cs, pvr, pvt, cr, pebbles, fast, viscous, upper,
                                                           bound, top);
   g_thorin_launches++;
   launch(k_cfl_final, 1, 1024, 0, s, g, cr, f0, scal, iscal, bound, top);
@@ -398,8 +419,22 @@ void aux_evaporate(const DevGrid &g, const double *T, double *pdens, cudaStream_
 // ---------------------------------------------------------------------------
 // Damping boundaries (DampingBoundary, SideEuler.c:368-419, and DampPebbles,
 // SideEuler.c:423-456).  Only rings inside the damping zones are launched.
+// pd: the pebbles in the same launch (NULL: not).
+__device__ __forceinline__ void damp_peb_cell(const DevGrid &g, int i, int l, double dt, double omega_frame,
+                                              double *pd, double *pvr, double *pvt)
+{
+  const double lambda = g.r.WaveKiller[i] * dt;
+  const double d0 = g.r.PebDensInit[i], vr0 = g.r.PebVradInit[i];
+  const double vt0 = g.r.PebVthetaInit[i] - g.r.Rmed[i] * omega_frame;
+  pd[l] = div_fast(pd[l] + lambda * d0, 1.0 + lambda);
+  pvr[l] = div_fast(pvr[l] + lambda * vr0, 1.0 + lambda);
+  pvt[l] = div_fast(pvt[l] + lambda * vt0, 1.0 + lambda);
+}
+
 __global__ void k_damp_gas(DevGrid g, double *__restrict__ vrad, double *__restrict__ rho, double *__restrict__ vtheta,
-                           double *__restrict__ energy, const int *__restrict__ rings, const double *__restrict__ vr0r, int damp_init, int damp_flux, int energy_eq)
+                           double *__restrict__ energy, const int *__restrict__ rings, const double *__restrict__ vr0r,
+                           int damp_init, int damp_flux, int energy_eq, double *__restrict__ pd,
+                           double *__restrict__ pvr, double *__restrict__ pvt)
 {
   pdl_wait();
   const double dt = g.ctl[CTL_DT], omega_frame = g.ctl[CTL_OMEGA_FRAME];
@@ -419,15 +454,16 @@ __global__ void k_damp_gas(DevGrid g, double *__restrict__ vrad, double *__restr
     if (energy_eq) energy[l] = div_fast(energy[l] + lambda * e0, 1.0 + lambda);
   }
   if (damp_flux) rho[l] = div_fast(rho[l] + lambda * g.r.SigmaMed[i], 1.0 + lambda);
+  if (pd) damp_peb_cell(g, i, l, dt, omega_frame, pd, pvr, pvt);
 }
 
 void aux_damp_gas(const DevGrid &g, double *vrad, double *rho, double *vtheta, double *energy, const int *rings,
-                  int nrings, const double *vr0r, int damp_init, int damp_flux,
-                  int energy_eq, cudaStream_t s)
+                  int nrings, const double *vr0r, int damp_init, int damp_flux, int energy_eq, double *pd, double *pvr,
+                  double *pvt, cudaStream_t s)
 {
   if (nrings <= 0) return;
-  launch(k_damp_gas, grid2d(g.ns, nrings, BX), BX, 0, s, g, vrad, rho, vtheta, energy, rings, vr0r,
-                                                     damp_init, damp_flux, energy_eq);
+  launch(k_damp_gas, grid2d(g.ns, nrings, BX), BX, 0, s, g, vrad, rho, vtheta, energy, rings, vr0r, damp_init, damp_flux,
+         energy_eq, pd, pvr, pvt);
   g_thorin_launches++;
 }
 
@@ -466,12 +502,7 @@ __global__ void k_damp_peb(DevGrid g, double *__restrict__ pd, double *__restric
   if (j >= ns) return;
   const int i = rings[blockIdx.y];
   const int l = j + i * ns;
-  const double lambda = g.r.WaveKiller[i] * dt;
-  const double d0 = g.r.PebDensInit[i], vr0 = g.r.PebVradInit[i];
-  const double vt0 = g.r.PebVthetaInit[i] - g.r.Rmed[i] * omega_frame;
-  pd[l] = div_fast(pd[l] + lambda * d0, 1.0 + lambda);
-  pvr[l] = div_fast(pvr[l] + lambda * vr0, 1.0 + lambda);
-  pvt[l] = div_fast(pvt[l] + lambda * vt0, 1.0 + lambda);
+  damp_peb_cell(g, i, l, dt, omega_frame, pd, pvr, pvt);
 }
 
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s)
@@ -506,9 +537,21 @@ void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s)
 // k_force_rings, one block per ring: the ring-mean Stokes number, the scale
 // heights of the ring means and the 10-node vertical average of the star's
 // pull for the ring-mean column, one node per lane of the first warp.
-__global__ void __launch_bounds__(RING_T) k_force_rings(DevGrid g, ForceArgs a, ForceRings fr)
+// It also leaves the planets and control values of the host path (hp.n >= 0)
+// for the kernels after it.
+__global__ void __launch_bounds__(RING_T) k_force_rings(DevGrid g, ForceArgs a, ForceRings fr, HostPlanets hp)
 {
   pdl_wait();
+  if (blockIdx.x == 0 && hp.n >= 0) {
+    const double *from = (const double *)hp.pl;
+    double *to = (double *)a.pl_out;
+    for (int k = threadIdx.x; k < hp.n * (int)(sizeof(DevPlanet) / sizeof(double)); k += RING_T) to[k] = from[k];
+    if (threadIdx.x == 0) {
+      g.ctl[CTL_MASS_TAPER] = hp.mass_taper;
+      g.ctl[CTL_INDX_PL] = hp.indx;
+      g.ctl[CTL_INDY_PL] = hp.indy;
+    }
+  }
   const int i = blockIdx.x, lane = threadIdx.x;
   const double H = g.r.csmean[i] * g.r.OmegaInv[i] * g.k.sqrt_adiabind_inv;
   const double r2 = g.r.Rmed2[i];
@@ -974,11 +1017,11 @@ __global__ void __launch_bounds__(1024) k_forces_final(DevGrid g, ForceArgs a, d
 template <int NP>
 static void launch_forces(const DevGrid &g, const ForceArgs &a, const ForceRings &fr, dim3 grid, cudaStream_t s)
 {
-  launch_fp64(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
+  launch(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
 }
 
-void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
-                double *scal, cudaStream_t s)
+void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
+                cudaStream_t s)
 {
   ForceArgs a = a0;
   for (int pass = 0; pass < 2; pass++) {
@@ -1014,7 +1057,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   a.nba = ga.x * ga.y;
   a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
   a.nbb = a.nbn + (a.npl > 0 ? g.nsm : 0);
-  launch_fp64(k_force_rings, g.nr, RING_T, 0, s, g, a, fr);
+  launch(k_force_rings, g.nr, RING_T, 0, s, g, a, fr, hp);
   g_thorin_launches++;
   switch (a.npl) {
   case 0: launch_forces<0>(g, a, fr, ga, s); break;
@@ -1024,7 +1067,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
   default: launch_forces<MAXPL_DEV>(g, a, fr, ga, s); break;
   }
   g_thorin_launches++;
-  launch_fp64(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
+  launch(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
   g_thorin_launches++;
   launch(k_forces_final, 2 + 2 * a.npl, 1024, 0, s, g, a, scal);
   g_thorin_launches++;

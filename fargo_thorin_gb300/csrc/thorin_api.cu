@@ -906,6 +906,13 @@ static double cs_iso_host(const thorin_disk *d, int i)
   return aspect_ratio_host(d, r) * sqrt(1.0 * 1.0 / r) * pow(r, d->p.flaring_index);
 }
 
+// The ring means of c_s (and, with alpha_flock, of the temperature) and the
+// viscosity from them.
+static void sound_rings(thorin_disk *d, bool temper)
+{
+  aux_sound_rings(d->g, d->vp, d->cs, temper ? d->temper : nullptr, d->ring[R_CSMEAN], d->ring[R_TEMPMEAN], d->s);
+}
+
 // ComputeSoundSpeed, ComputePressureField, ComputeTemperatureField and the
 // ring means that depend on them (Init.c:131-133).
 static int eos_refresh(thorin_disk *d)
@@ -918,9 +925,7 @@ static int eos_refresh(thorin_disk *d)
     RCHK(upload_ring(d, R_CSISO, c));
     aux_iso_eos(d->g, d->rho, d->ring[R_CSISO], d->cs, d->press, d->temper, 1, 1, 1, d->s);
   }
-  aux_ring_mean(d->g, d->cs, d->ring[R_CSMEAN], d->s);
-  if (d->p.alpha_flock) aux_ring_mean(d->g, d->temper, d->ring[R_TEMPMEAN], d->s);
-  aux_viscosity_rings(d->g, d->vp, d->s);
+  sound_rings(d, true);
   CUCHK(cudaMemcpyAsync(d->csmean_h, d->ring[R_CSMEAN], d->nr * sizeof(double), cudaMemcpyDeviceToHost, d->s));
   return THORIN_OK;
 }
@@ -1147,9 +1152,7 @@ extern "C" int thorin_gpu_refresh(thorin_disk *d, int flags)
   if (flags == THORIN_REFRESH_RING_MEANS) {
     // a state put back as it was at the end of a DT (fields, c_s and T
     // included): the ring means and viscosities the next substep reads
-    aux_ring_mean(d->g, d->cs, d->ring[R_CSMEAN], d->s);
-    if (p.alpha_flock) aux_ring_mean(d->g, d->temper, d->ring[R_TEMPMEAN], d->s);
-    aux_viscosity_rings(d->g, d->vp, d->s);
+    sound_rings(d, true);
     CUCHK(cudaMemcpyAsync(d->csmean_h, d->ring[R_CSMEAN], d->nr * sizeof(double), cudaMemcpyDeviceToHost, d->s));
     CUCHK(cudaStreamSynchronize(d->s));
     return THORIN_OK;
@@ -1241,12 +1244,12 @@ extern "C" int thorin_planet_from_elements(thorin_planets *sys, int k, float mas
 }
 
 // Writes control-block values (stream-ordered) for the kernels that follow.
-static void set_ctl(thorin_disk *d, std::initializer_list<std::pair<int, double>> kv, cudaStream_t s = nullptr)
+static void set_ctl(thorin_disk *d, std::initializer_list<std::pair<int, double>> kv, int *crash = nullptr)
 {
   CtlSet v;
   v.n = 0;
   for (const auto &e : kv) { v.idx[v.n] = e.first; v.val[v.n] = e.second; v.n++; }
-  aux_set_ctl(d->ctl, v, s ? s : d->s);
+  aux_set_ctl(d->ctl, v, crash, d->s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1267,18 +1270,21 @@ static CflFinal cfl_args(const thorin_disk *d)
   return f;
 }
 
-static void cfl_launches(thorin_disk *d)
+static void cfl_launches(thorin_disk *d, const CflFinal &fin)
 {
   const thorin_params &p = d->p;
   if (p.pebbles) aux_stokes(d->g, d->rho, d->psize, d->tau, d->s);       // PebbleStokesNumbers
   aux_cfl(d->g, d->vrad, d->vtheta, d->cs, d->pvrad, d->pvtheta, d->cfl, p.pebbles, p.fast_transport,
-          (p.viscosity_alpha || p.viscosity != 0.0), d->partials, cfl_args(d), d->scal, d->iscal, d->s);
+          (p.viscosity_alpha || p.viscosity != 0.0), d->partials, fin, d->scal, d->iscal, d->s);
 }
 
 static int cfl_begin(thorin_disk *d, double dt_remaining, double invdtreb_sq)
 {
-  set_ctl(d, {{CTL_DELTAT, dt_remaining}, {CTL_INVDTREB, invdtreb_sq}});
-  cfl_launches(d);
+  CflFinal fin = cfl_args(d);
+  fin.own = 1;
+  fin.deltaT = dt_remaining;
+  fin.invdtreb_sq = invdtreb_sq;
+  cfl_launches(d, fin);
   d->cfl_first = 0;
   KCHECK("cfl kernels");
   CUCHK(cudaMemcpyAsync(d->iscal_h, d->iscal, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, d->s));
@@ -1422,7 +1428,7 @@ static ForceArgs force_args(const thorin_disk *d, int npl)
   a.col = d->force_col;
   a.near = d->force_near;
   a.ticket = d->ticket + 8;
-  a.pl = d->planets_d;
+  a.pl = a.pl_out = d->planets_d;
   a.npl = npl; a.pebbles = p.pebbles; a.exclude_hill = p.exclude_hill; a.pebble_gravity = p.pebble_gravity;
   a.pebble_alpha = p.pebble_alpha; a.hillcut = p.hillcut;
   return a;
@@ -1442,15 +1448,19 @@ static int forces_begin(thorin_disk *d, thorin_planets *sys, double mass_taper, 
 {
   const thorin_params &p = d->p;
   const int npl = sys->nb;
-  DevPlanet pl[MAXPL_DEV];
+  HostPlanets hp;
   double axs = 0.0, ays = 0.0;
   for (int k = 0; k < npl; k++)
-    pl_force_planet(d->plc, d->Rsup.data(), d->csmean_h, d->OmegaInv.data(), sys, k, mass_taper, &pl[k], &axs, &ays);
-  if (npl > 0) CUCHK(cudaMemcpyAsync(d->planets_d, pl, npl * sizeof(DevPlanet), cudaMemcpyHostToDevice, d->s));
-  const double indx_pl = p.indirect_term ? -axs : 0.0, indy_pl = p.indirect_term ? -ays : 0.0;
-  set_ctl(d, {{CTL_MASS_TAPER, mass_taper}, {CTL_INDX_PL, indx_pl}, {CTL_INDY_PL, indy_pl}});
-  aux_forces(d->g, force_args(d, npl), d->fr, d->scal, d->s);
+    pl_force_planet(d->plc, d->Rsup.data(), d->csmean_h, d->OmegaInv.data(), sys, k, mass_taper, &hp.pl[k], &axs, &ays);
+  hp.n = npl;
+  hp.mass_taper = mass_taper;
+  hp.indx = p.indirect_term ? -axs : 0.0;
+  hp.indy = p.indirect_term ? -ays : 0.0;
+  aux_forces(d->g, force_args(d, npl), d->fr, hp, d->scal, d->s);
   KCHECK("force kernels");
+  RingList rl;
+  rl.n = 0;
+  auto ring_mean = [&](int i, double *out) { rl.ring[rl.n] = i; rl.out[rl.n++] = out; };
   fr->npl = npl;
   fr->torques = d->torque_pending;
   fr->time = d->PhysicalTime;
@@ -1461,7 +1471,7 @@ static int forces_begin(thorin_disk *d, thorin_planets *sys, double mass_taper, 
     fr->inside[k] = (r >= d->Rinf[0] && r <= d->Rsup[d->nr - 1]);
     if (fr->inside[k]) {
       const int i = ring_of(d, r);
-      aux_ring_mean_at(d->g, d->rho, i, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->s);
+      ring_mean(i, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k);
       if (ring_cs) ring_cs[k] = d->csmean_h[i];
     }
     // UpdateLog (Force.c:27-70) needs Sigma's ring means either side of each planet
@@ -1471,9 +1481,11 @@ static int forces_begin(thorin_disk *d, thorin_planets *sys, double mass_taper, 
       fr->two[k] = (ii + 1 <= d->nr);
       fr->frac[k] = frac;
       fr->cspl[k] = d->csmean_h[ii] * (1.0 - frac) + (fr->two[k] ? d->csmean_h[ii + 1] : 0.0) * frac;
-      aux_ring_means(d->g, d->rho, d->scal + SC_TORQUE + 2 * k, nullptr, nullptr, ii, fr->two[k] ? 2 : 1, d->s);
+      ring_mean(ii, d->scal + SC_TORQUE + 2 * k);
+      if (fr->two[k]) ring_mean(ii + 1, d->scal + SC_TORQUE + 2 * k + 1);
     }
   }
+  aux_ring_list(d->g, d->rho, rl, d->s);
   CUCHK(cudaMemcpyAsync(d->scal_h, d->scal, 128 * sizeof(double), cudaMemcpyDeviceToHost, d->s));
   CUCHK(cudaEventRecord(d->ev_forces, d->s));
   return THORIN_OK;
@@ -1717,6 +1729,14 @@ static int iterate_relaxation(thorin_disk *d)
 // EnergySources.c:201-335).  Leaves the new energy in d->energy.
 static int capture_sor(thorin_disk *d);
 
+// The relaxation parameter of the next solve: a step of the schedule, which
+// turns at the bounds (EnergySources.c:298-305).
+static double next_omega(const thorin_disk *d)
+{
+  const double omega = d->omega + d->domega;
+  return omega > TH_OMEGAUPPER ? TH_OMEGAUPPER : (omega < 1.0 ? 1.0 : omega);
+}
+
 static int energy_step(thorin_disk *d, double dt)
 {
   const thorin_params &p = d->p;
@@ -1786,11 +1806,10 @@ static int energy_step(thorin_disk *d, double dt)
     d->omega = d->omegabest;
     d->Niterlast = d->Niterbest;
   }
-  d->omega += d->domega;
-  if (d->omega > TH_OMEGAUPPER) { d->omega = TH_OMEGAUPPER; d->domega = -d->domega; }
-  if (d->omega < 1.0) { d->omega = 1.0; d->domega = -d->domega; }
-  if (!first) {
-    set_ctl(d, {{CTL_SOR_OMEGA, d->omega}});
+  const double omega = next_omega(d);
+  if (omega != d->omega + d->domega) d->domega = -d->domega;
+  d->omega = omega;
+  if (!first) {                        // the control block has it since the substep's start
     hydro_matrix(d->g, mx, &d->sor, d->s);
     KCHECK("energy kernels");
   }
@@ -1839,32 +1858,48 @@ static void transport_fluid(thorin_disk *d, double **rho, const double *vr_in, c
 extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
 {
   const thorin_params &p = d->p;
-  if (!d->capturing) set_ctl(d, {{CTL_DT, dt}, {CTL_OMEGA_FRAME, d->OmegaFrame}});
+  if (!d->capturing)                   // on the device in the DT graph; the crash flag is cleared too
+    set_ctl(d, {{CTL_DT, dt}, {CTL_OMEGA_FRAME, d->OmegaFrame}, {CTL_SOR_OMEGA, next_omega(d)}}, d->iscal + IS_CRASH);
   const int damp = p.damping;
-  auto boundary = [&]() {                // ApplyBoundaryCondition (SideEuler.c:490-503)
+  // ApplyBoundaryCondition (SideEuler.c:490-503) up to the damping
+  auto boundary_open = [&]() {
     if (p.open_inner) aux_open_inner(d->g, d->rho, d->vrad, d->energy, p.energy_eq, p.damp_flux, p.gasflux, d->s);
     if (p.open_outer) aux_open_outer(d->g, d->rho, d->vrad, d->energy, p.energy_eq, p.damp_flux, p.gasflux, d->s);
     if (p.non_reflecting) {
       if (p.energy_eq) {                   // ComputeSoundSpeed: c_s, its ring means and the viscosity
         hydro_eos(d->g, d->rho, d->energy, nullptr, d->cs, d->gm1, d->gg1, d->s);
-        aux_ring_mean(d->g, d->cs, d->ring[R_CSMEAN], d->s);
-        aux_viscosity_rings(d->g, d->vp, d->s);
+        sound_rings(d, false);
       }
       aux_nonreflecting(d->g, d->rho, d->vrad, d->energy, d->cs, d->s);
     }
     if (p.outer_source_mass)
       aux_outer_source_mass(d->g, d->rho, d->vrad, p.imposed_disk_drift * pow((d->Rinf[d->nr - 1] / 1.0), -p.sigma_slope),
                             d->s);
-    if (damp) aux_damp_gas(d->g, d->vrad, d->rho, d->vtheta, d->energy, d->damp_rings_d, d->ndamp, d->ring[R_DAMPVR0], p.damp_init, p.damp_flux, p.energy_eq, d->s);
   };
-  // ApplyBoundaryCondition, DetectCrash, ComputePressureField (SourceEuler.c:271-292)
-  boundary();
-  CUCHK(cudaMemsetAsync(d->iscal + IS_CRASH, 0, sizeof(int), d->s));
-  aux_crash(d->g, p.pebbles ? d->pdens : d->energy, d->iscal + IS_CRASH, d->s);
+  auto damp_gas = [&](bool pebbles) {
+    aux_damp_gas(d->g, d->vrad, d->rho, d->vtheta, d->energy, d->damp_rings_d, d->ndamp, d->ring[R_DAMPVR0], p.damp_init,
+                 p.damp_flux, p.energy_eq, pebbles ? d->pdens : nullptr, d->pvrad, d->pvtheta, d->s);
+  };
+  auto boundary = [&]() {
+    boundary_open();
+    if (damp) damp_gas(false);
+  };
+  // ApplyBoundaryCondition, DetectCrash, ComputePressureField (SourceEuler.c:
+  // 271-292); with pebbles the crash test is of their density, which only their
+  // own damping (SourceTermsPebbles', after the test) changes, so both fluids
+  // are damped in one launch
+  if (p.pebbles) {
+    boundary_open();
+    aux_crash(d->g, d->pdens, d->iscal + IS_CRASH, d->s);
+    if (damp) damp_gas(true);
+    else aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s);
+  } else {
+    boundary();
+    aux_crash(d->g, d->energy, d->iscal + IS_CRASH, d->s);
+  }
   if (!p.energy_eq) aux_iso_eos(d->g, d->rho, nullptr, d->cs, d->press, d->temper, 0, 1, 0, d->s);
   // SourceTermsPebbles (Pebbles.c:550-613), SubStep1 (SourceEuler.c:319-415),
   // SubStep1Pebbles and ParticleDiffusion
-  if (p.pebbles) aux_damp_peb(d->g, d->pdens, d->pvrad, d->pvtheta, d->damp_rings_d, d->ndamp, d->s);
   SourceIO src = {};
   src.rho = d->rho; src.vr = d->vrad; src.vt = d->vtheta; src.energy = d->energy;
   src.press = p.energy_eq ? nullptr : d->press;
@@ -1928,9 +1963,7 @@ extern "C" int thorin_gpu_hydro(thorin_disk *d, double dt)
     if (p.energy_eq) hydro_eos(d->g, d->rho, d->energy, d->temper, d->cs, d->gm1, d->gg1, d->s);
   }
   if (!p.energy_eq) aux_iso_eos(d->g, d->rho, nullptr, d->cs, d->press, d->temper, 0, 0, 1, d->s);
-  aux_ring_mean(d->g, d->cs, d->ring[R_CSMEAN], d->s);
-  if (p.alpha_flock) aux_ring_mean(d->g, d->temper, d->ring[R_TEMPMEAN], d->s);
-  aux_viscosity_rings(d->g, d->vp, d->s);
+  sound_rings(d, true);
   if (!d->capturing)
     CUCHK(cudaMemcpyAsync(d->csmean_h, d->ring[R_CSMEAN], d->nr * sizeof(double), cudaMemcpyDeviceToHost, d->s));
   if (!d->capturing) CUCHK(cudaEventRecord(d->ev_cs, d->s));
@@ -2284,9 +2317,9 @@ static int capture_substep(thorin_disk *d)
   StepDev &S = d->capS;
   const int npl = S.npl;
   graph_sub_begin(S, d->s);
-  cfl_launches(d);
+  cfl_launches(d, cfl_args(d));
   if (p.pebbles) {
-    graph_acc_init(S, d->s);
+    if (npl == 0) graph_acc_init(S, d->s);
     const int nb_max = aux_accrete_blocks(d->g, 0, d->nr - 1);
     for (int k = 0; k < npl; k++) {
       graph_acc_prep(S, k, d->s);
@@ -2295,8 +2328,10 @@ static int capture_substep(thorin_disk *d)
     }
     if (p.evaporation_rate > 0.0) aux_evaporate(d->g, d->temper, d->pdens, d->s);
   }
-  graph_force_prep(S, d->s);
-  aux_forces(d->g, force_args(d, npl), d->fr, d->scal, d->s);
+  if (!p.pebbles || npl == 0) graph_force_prep(S, d->s);      // else with the last planet's accretion
+  HostPlanets hp;
+  hp.n = -1;                           // they are on the device
+  aux_forces(d->g, force_args(d, npl), d->fr, hp, d->scal, d->s);
   for (int k = 0; k < npl; k++)
     graph_ring_mean_at(d->g, d->rho, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->ring_info_d + k, d->s);
   // the planet kick and N-body step run beside the hydro substep, which does

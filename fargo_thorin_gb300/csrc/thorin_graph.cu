@@ -43,53 +43,38 @@ __global__ void k_g_sub_begin(StepDev S)
 }
 
 // InitHeating (Planet.c:251) and EvaporatePebbles' fraction of this dt.
-__global__ void k_g_acc_init(StepDev S)
+__device__ void acc_init(const StepDev &S)
 {
-  pdl_wait();
-  if (threadIdx.x != 0) return;
   for (int k = 0; k < S.npl; k++) { S.heat_val[k] = 0.0; S.heat_idx[k] = -1; }
   double facc = S.evaporation_rate * S.g.ctl[CTL_DT];
   if (facc > 1.0) facc = 1.0;
   S.g.ctl[CTL_FACC_EVAP] = facc;
 }
 
-// AccretePebblesOntoPlanets' set-up for planet k.
+__global__ void k_g_acc_init(StepDev S)
+{
+  pdl_wait();
+  if (threadIdx.x == 0) acc_init(S);
+}
+
+// AccretePebblesOntoPlanets' set-up for planet k (the first: InitHeating too).
 __global__ void k_g_acc_prep(StepDev S, int k)
 {
   pdl_wait();
   if (threadIdx.x != 0) return;
+  if (k == 0) acc_init(S);
   AccArgs a = *S.acc;
   pl_pebble_acc_prep(S.c, S.g.r.Rinf, S.g.r.Rsup, S.g.r.Rmed, S.sys, k, S.g.ctl[CTL_OMEGA_FRAME], S.g.ctl[CTL_DT],
                      ACC_BX, &a);
   *S.acc = a;
 }
 
-// Heating1 and the planet's new mass and velocity after the accretion.
-__global__ void k_g_acc_finish(StepDev S, int k)
-{
-  pdl_wait();
-  if (threadIdx.x != 0) return;
-  const AccArgs &a = *S.acc;
-  double dMp = 0.0, dPx = 0.0, dPy = 0.0;
-  if (a.nb > 0) { dMp = S.scal[SC_ACC_DM]; dPx = S.scal[SC_ACC_DPX]; dPy = S.scal[SC_ACC_DPY]; }
-  if (S.accret_heating) {
-    int idx;
-    double add;
-    if (pl_heating1(S.c, S.g.r.Rsup, S.g.r.Surf, S.g.ctl[CTL_TIME], a.Mp, dMp, a.Xp, a.Yp, S.g.ctl[CTL_DT], &idx, &add)) {
-      S.heat_idx[k] = idx;
-      S.heat_val[k] += add;
-    }
-  }
-  pl_pebble_acc_finish(S.sys, k, a, dMp, dPx, dPy);
-}
-
 // dtemp += dt (SourceEuler.c:249), then FillForcesArrays' per-planet
 // constants, the planets' indirect term and each planet's ring for
 // DampingTW04.
-__global__ void k_g_force_prep(StepDev S)
+__device__ void force_prep(const StepDev &S)
 {
-  pdl_wait();
-  if (threadIdx.x != 0) return;
+  S.iscal[IS_CRASH] = 0;
   double *ctl = S.g.ctl;
   ctl[CTL_DTEMP] += ctl[CTL_DT];
   double axs = 0.0, ays = 0.0;
@@ -106,6 +91,33 @@ __global__ void k_g_force_prep(StepDev S)
   }
   ctl[CTL_INDX_PL] = S.indirect_term ? -axs : 0.0;
   ctl[CTL_INDY_PL] = S.indirect_term ? -ays : 0.0;
+}
+
+__global__ void k_g_force_prep(StepDev S)
+{
+  pdl_wait();
+  if (threadIdx.x == 0) force_prep(S);
+}
+
+// Heating1 and the planet's new mass and velocity after the accretion; after
+// the last planet's the forces' set-up.
+__global__ void k_g_acc_finish(StepDev S, int k)
+{
+  pdl_wait();
+  if (threadIdx.x != 0) return;
+  const AccArgs &a = *S.acc;
+  double dMp = 0.0, dPx = 0.0, dPy = 0.0;
+  if (a.nb > 0) { dMp = S.scal[SC_ACC_DM]; dPx = S.scal[SC_ACC_DPX]; dPy = S.scal[SC_ACC_DPY]; }
+  if (S.accret_heating) {
+    int idx;
+    double add;
+    if (pl_heating1(S.c, S.g.r.Rsup, S.g.r.Surf, S.g.ctl[CTL_TIME], a.Mp, dMp, a.Xp, a.Yp, S.g.ctl[CTL_DT], &idx, &add)) {
+      S.heat_idx[k] = idx;
+      S.heat_val[k] += add;
+    }
+  }
+  pl_pebble_acc_finish(S.sys, k, a, dMp, dPx, dPy);
+  if (k == S.npl - 1) force_prep(S);
 }
 
 // The N-body step of thorin_planet.cuh (pl_nbody_step_n) by two warps.  Lane

@@ -115,7 +115,23 @@ struct CflRings {
 
 struct CflFinal {
   int pebbles, first_call;
+  int own;                     // deltaT and invdtreb_sq are here (else in the control block)
   double deltaT, invdtreb_sq, minimum_step, maximum_step, first_step, twopi_cfl_ns;
+};
+
+// The planets and control values that the host path hands to the force
+// kernels (n < 0: they are on the device).
+struct HostPlanets {
+  int n;
+  double mass_taper, indx, indy;
+  DevPlanet pl[MAXPL_DEV];
+};
+
+// Single rings whose means are wanted.
+struct RingList {
+  int n;
+  int ring[3 * MAXPL_DEV];
+  double *out[3 * MAXPL_DEV];
 };
 
 struct ForceRings {
@@ -138,6 +154,7 @@ struct ForceArgs {
   unsigned char *near;        // cells left to k_forces_near
   unsigned int *ticket;       // of k_forces_final
   const DevPlanet *pl;
+  DevPlanet *pl_out;           // the same, for the host path's copy
   int npl, pebbles, exclude_hill, pebble_gravity;
   double pebble_alpha, hillcut;   // the mass taper is read from the control block
   // vertical quadrature weights exp(-z_m^2 / 2H^2) at z_m = (m - 1/2) 3H/N,
@@ -258,16 +275,17 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
 void aux_ring_means(const DevGrid &g, const double *f0, double *o0, const double *f1, double *o1, int ring0, int nrings,
                     cudaStream_t s);
 void aux_ring_mean(const DevGrid &g, const double *f, double *out, cudaStream_t s);
-void aux_ring_mean_at(const DevGrid &g, const double *f, int ring, double *out, cudaStream_t s);
-void aux_viscosity_rings(const DevGrid &g, const ViscParams &v, cudaStream_t s);
+void aux_ring_list(const DevGrid &g, const double *f, const RingList &r, cudaStream_t s);
+void aux_sound_rings(const DevGrid &g, const ViscParams &v, const double *cs, const double *temper, double *csmean,
+                     double *tempmean, cudaStream_t s);
 void aux_stokes(const DevGrid &g, const double *rho, const double *psize, double *tau, cudaStream_t s);
 void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double *cs, const double *pvr, const double *pvt,
              const CflRings &cr, int pebbles, int fast, int viscous, double *part, const CflFinal &f0, double *scal,
              int *iscal, cudaStream_t s);
 void aux_evaporate(const DevGrid &g, const double *T, double *pdens, cudaStream_t s);
 void aux_damp_gas(const DevGrid &g, double *vrad, double *rho, double *vtheta, double *energy, const int *rings,
-                  int nrings, const double *vr0r, int damp_init, int damp_flux,
-                  int energy_eq, cudaStream_t s);
+                  int nrings, const double *vr0r, int damp_init, int damp_flux, int energy_eq, double *pd, double *pvr,
+                  double *pvt, cudaStream_t s);
 void aux_open_inner(const DevGrid &g, double *rho, double *vr, double *energy, int energy_eq, int damp_flux,
                     double gasflux, cudaStream_t s);
 void aux_open_outer(const DevGrid &g, double *rho, double *vr, double *energy, int energy_eq, int damp_flux,
@@ -286,14 +304,15 @@ void aux_iso_eos(const DevGrid &g, const double *rho, const double *csr, double 
                  int set_cs, int set_press, int set_temper, cudaStream_t s);
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s);
 void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s);
-void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr,
-                double *scal, cudaStream_t s);
+void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
+                cudaStream_t s);
 // Pebble accretion with the arguments a0, which go to a_dev, or, with a0 NULL,
 // with those at a_dev; nb: aux_accrete_blocks of the widest annulus possible.
 void aux_accrete(const DevGrid &g, const AccArgs *a0, AccArgs *a_dev, int nb, double *scal, cudaStream_t s);
-// Control block writes (host path): up to 6 (index, value) pairs.
+// Control block writes (host path): up to 6 (index, value) pairs; crash (may
+// be NULL): cleared.
 struct CtlSet { int n; int idx[6]; double val[6]; };
-void aux_set_ctl(double *ctl, const CtlSet &v, cudaStream_t s);
+void aux_set_ctl(double *ctl, const CtlSet &v, int *crash, cudaStream_t s);
 int aux_accrete_blocks(const DevGrid &g, int imin, int imax);
 void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const double *vt, const double *e,
                    const double *pd, const double *pvt, double omega_frame, int pebbles, double *part, double *scal,
