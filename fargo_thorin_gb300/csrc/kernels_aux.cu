@@ -1141,6 +1141,30 @@ __device__ double column_mass_warp(double a, double b, double Hpeb)
 // 67 (a third of it the copy of the result and the wait for it).
 // acc[] scalars: 0 Reff, 1 vrel, 2 Mt, 3 limiter, 4-5 the ring means.
 
+// Sums of N values over a block of BS threads, valid in every thread: a warp
+// per value adds the threads' (the warps' FP64 instructions go side by side,
+// where block reductions one after another took 10 N of 64 cycles each).
+template <int N, int BS>
+__device__ __forceinline__ void acc_block_sums(double v[N])
+{
+  __shared__ double sh[N][BS];
+  __shared__ double out[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) sh[k][threadIdx.x] = v[k];
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w < N) {
+    double a = sh[w][lane];
+#pragma unroll
+    for (int q = 1; q < BS / 32; q++) a += sh[w][lane + 32 * q];
+    a = warp_reduce(a, OpAdd());
+    if (lane == 0) out[w] = a;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; k++) v[k] = out[k];
+}
+
 __device__ __forceinline__ bool acc_last_block(unsigned int *ticket)
 {
   __shared__ bool last;
@@ -1169,7 +1193,7 @@ __global__ void __launch_bounds__(RING_T) k_acc_reff(DevGrid g, AccArgs av, AccA
     const double *tau = a.tau + (size_t)a.imin * ns;
     double t = 0.0;
     for (int q = (blockIdx.x - 2) * RING_T + threadIdx.x; q < ncells; q += nb * RING_T) t += tau[q];
-    t = block_reduce(t, OpAdd(), 0.0);
+    acc_block_sums<1, RING_T>(&t);
     if (threadIdx.x == 0) a.part[blockIdx.x - 2] = t;
   } else {
     const int i = a.iflow + blockIdx.x;          // vt1D[nrad] is zero in the reference
@@ -1181,19 +1205,20 @@ __global__ void __launch_bounds__(RING_T) k_acc_reff(DevGrid g, AccArgs av, AccA
   if (!acc_last_block(a.ticket)) return;
   double ts = 0.0;
   for (int b = threadIdx.x; b < nb; b += RING_T) ts += __ldcg(a.part + b);
-  ts = block_reduce(ts, OpAdd(), 0.0);
+  acc_block_sums<1, RING_T>(&ts);
   if (threadIdx.x == 0) {
-    const double tau_mean = ts / (double)ncells;
+    const double tau_mean = div_fast(ts, (double)ncells);
     const double flow = __ldcg(a.acc + 4) * (1.0 - a.frac) + __ldcg(a.acc + 5) * a.frac + a.Rp * a.omega_frame;
-    const double flowx = -flow * a.Yp / a.Rp, flowy = flow * a.Xp / a.Rp;
-    const double vrel = sqrt((a.VXp - flowx) * (a.VXp - flowx) + (a.VYp - flowy) * (a.VYp - flowy) + a.VZp * a.VZp);
-    const double Mt = sqrt(1.0 / 3.0) * cube_rn(vrel) / a.Omegap;
+    const double flowx = div_fast(-flow * a.Yp, a.Rp), flowy = div_fast(flow * a.Xp, a.Rp);
+    const double vrel =
+        sqrt_fast((a.VXp - flowx) * (a.VXp - flowx) + (a.VYp - flowy) * (a.VYp - flowy) + a.VZp * a.VZp);
+    const double Mt = div_fast(sqrt(1.0 / 3.0) * cube_rn(vrel), a.Omegap);
     double Reff;
     if (a.Mp < Mt) {
-      const double Rbondi = a.Mp / vrel / vrel, tbondi = Rbondi / vrel;
-      Reff = Rbondi * sqrt(tau_mean * a.Rp15 / tbondi);
+      const double Rbondi = div_fast(div_fast(a.Mp, vrel), vrel), tbondi = div_fast(Rbondi, vrel);
+      Reff = Rbondi * sqrt_fast(div_fast(tau_mean * a.Rp15, tbondi));
     } else {
-      Reff = a.Rhill * pow(tau_mean / 0.1, 1.0 / 3.0);
+      Reff = a.Rhill * pow(div_fast(tau_mean, 0.1), 1.0 / 3.0);
     }
     if (Reff > a.Rhill) Reff = a.Rhill;
     a.acc[0] = Reff;
@@ -1219,8 +1244,8 @@ __device__ __forceinline__ bool acc_cell(const DevGrid &g, const AccArgs &a, int
   const double R2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
   if (!(R2 <= Reff2)) return false;
   const double H = __dmul_rn(__dmul_rn(a.cs[l], g.r.OmegaInv[i]), g.k.sqrt_adiabind_inv);
-  Hpeb = __dmul_rn(H, __dsqrt_rn(__ddiv_rn(a.pebble_alpha, a.tau[l])));
-  const double h = __dsqrt_rn(__dsub_rn(Reff2, R2));
+  Hpeb = __dmul_rn(H, sqrt_fast(div_fast(a.pebble_alpha, a.tau[l])));
+  const double h = sqrt_fast(__dsub_rn(Reff2, R2));
   zmin = __dsub_rn(a.Zp, h);
   zmax = __dadd_rn(a.Zp, h);
   return true;
@@ -1260,15 +1285,14 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *
     if (inside) {
       const double pd = a.pdens[l];
       const double mcell = g.r.Surf[i] * pd;
-      const double vdp = pd / Hpeb * g.k.sqrt2pi_inv;
+      const double vdp = div_fast(pd, Hpeb) * g.k.sqrt2pi_inv;
       double dM = vdp * g.r.Surf[i] * cm;
       if (dM > mcell) dM = 0.99999999 * mcell;
       a.macc[l] = dM;
       v[0] += dM; v[1] += Hpeb; v[2] += pd; v[3] += 1.0;
     }
   }
-  if (__syncthreads_or(v[3] > 0.0))
-    for (int k = 0; k < 4; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  if (__syncthreads_or(v[3] > 0.0)) acc_block_sums<4, ACC_BX>(v);
   if (threadIdx.x == 0)
     for (int k = 0; k < 4; k++) a.part[4 * blockIdx.x + k] = v[k];
   if (!acc_last_block(a.ticket)) return;
@@ -1276,19 +1300,19 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_upper(DevGrid g, const AccArgs *
   for (int k = 0; k < 4; k++) v[k] = 0.0;
   for (int b = threadIdx.x; b < nb; b += ACC_BX)
     for (int k = 0; k < 4; k++) v[k] += __ldcg(a.part + 4 * b + k);
-  for (int k = 0; k < 4; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  acc_block_sums<4, ACC_BX>(v);
   if (threadIdx.x == 0) {
     const double dmu = v[0];
     double Hpeb_mean = v[1], pdens_mean = v[2];
     const int nc = (int)v[3];
-    if (nc > 0) { Hpeb_mean /= (double)nc; pdens_mean /= (double)nc; }
+    if (nc > 0) { Hpeb_mean = div_fast(Hpeb_mean, (double)nc); pdens_mean = div_fast(pdens_mean, (double)nc); }
     const double Reff = a.acc[0], vrel = a.acc[1], Mt = a.acc[2];
     const double veloc = (a.Mp < Mt) ? vrel : Reff * a.Omegap;
     double dM_model;
     if (Hpeb_mean < Reff) dM_model = 2.0 * Reff * veloc * pdens_mean;
-    else dM_model = TH_PI * Reff * Reff * veloc * pdens_mean / Hpeb_mean * g.k.sqrt2pi_inv;
+    else dM_model = div_fast(TH_PI * Reff * Reff * veloc * pdens_mean, Hpeb_mean) * g.k.sqrt2pi_inv;
     dM_model *= a.dt;
-    a.acc[3] = (dmu > dM_model) ? dM_model / dmu : 1.0;
+    a.acc[3] = (dmu > dM_model) ? div_fast(dM_model, dmu) : 1.0;
   }
 }
 
@@ -1314,14 +1338,13 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_apply(DevGrid g, const AccArgs *
       const double dM = up * limiter;
       a.macc[l] = 0.0;
       const double mcell = g.r.Surf[i] * a.pdens[l];
-      double pd = (mcell - dM) / g.r.Surf[i];
+      double pd = div_fast(mcell - dM, g.r.Surf[i]);
       if (pd < 0.0) pd = 1.e-20;
       a.pdens[l] = pd;
       v[0] += dM; v[1] += dM * vxc; v[2] += dM * vyc;
     }
   }
-  if (__syncthreads_or(v[0] != 0.0))
-    for (int k = 0; k < 3; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  if (__syncthreads_or(v[0] != 0.0)) acc_block_sums<3, ACC_BX>(v);
   if (threadIdx.x == 0)
     for (int k = 0; k < 3; k++) a.part[3 * blockIdx.x + k] = v[k];
   if (!acc_last_block(a.ticket)) return;
@@ -1329,7 +1352,7 @@ __global__ void __launch_bounds__(ACC_BX) k_acc_apply(DevGrid g, const AccArgs *
   for (int k = 0; k < 3; k++) v[k] = 0.0;
   for (int b = threadIdx.x; b < nb; b += ACC_BX)
     for (int k = 0; k < 3; k++) v[k] += __ldcg(a.part + 3 * b + k);
-  for (int k = 0; k < 3; k++) v[k] = block_reduce(v[k], OpAdd(), 0.0);
+  acc_block_sums<3, ACC_BX>(v);
   if (threadIdx.x == 0) { scal[SC_ACC_DM] = v[0]; scal[SC_ACC_DPX] = v[1]; scal[SC_ACC_DPY] = v[2]; }
 }
 
