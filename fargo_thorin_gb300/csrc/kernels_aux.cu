@@ -1138,7 +1138,7 @@ __device__ double column_mass_warp(double a, double b, double Hpeb)
 // the reference.  A launch on a small disk is mostly latency: the nine
 // launches before this, with the arguments, the ring means and each sum a
 // launch of its own, took 91 us of a substep at 128x384, these take
-// 67 (a third of it the copy of the result and the wait for it).
+// 51 (a third of it the copy of the result and the wait for it).
 // acc[] scalars: 0 Reff, 1 vrel, 2 Mt, 3 limiter, 4-5 the ring means.
 
 // Sums of N values over a block of BS threads, valid in every thread: a warp
