@@ -139,17 +139,17 @@ void aux_sound_rings(const DevGrid &g, const ViscParams &v, const double *cs, co
 // ---------------------------------------------------------------------------
 // PebbleStokesNumbers (Pebbles.c:280-300).
 __global__ void k_stokes(DevGrid g, const double *__restrict__ rho, const double *__restrict__ psize,
-                         double *__restrict__ tau)
+                         double *__restrict__ tau, double c)
 {
   pdl_wait();
   const int ns = g.ns;
   CELL_LOOP_2D
-  tau[l] = div_fast((2.0 * g.k.pebbulkdens * g.k.sqrt_adiabind_inv) * psize[l], rho[l]);
+  tau[l] = div_fast(c * psize[l], rho[l]);
 }
 
 void aux_stokes(const DevGrid &g, const double *rho, const double *psize, double *tau, cudaStream_t s)
 {
-  launch(k_stokes, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, psize, tau);
+  launch(k_stokes, grid2d(g.ns, g.nr, BX), BX, 0, s, g, rho, psize, tau, 2.0 * g.k.pebbulkdens * g.k.sqrt_adiabind_inv);
   g_thorin_launches++;
 }
 

@@ -476,12 +476,11 @@ __device__ double opacity_BL94(double vd, double rho2cgs, double T)
   if (grains) {
     // k1 = kappa0 T^2, k2 = kappa1 T^-7, k3 = kappa2 T^0.5;
     // t1 = (k1^-2 + k2^-2)^-2, x = k3 / (1 + 1e22 T^-10), k = (t1 + x^4)^(1/4),
-    // rearranged to two divisions
+    // rearranged to two divisions; x only enters squared, so without the root
     const double T2 = T * T, T4 = T2 * T2, T5 = T4 * T, T10 = T5 * T5, T14 = T10 * T4;
-    const double k3 = kappa[2] * sqrt_fast(T);
     const double ik = div_fast(T4, __fma_rn(2.5e-33 * T14, T4, 2.5e7));         // 1 / (k1^-2 + k2^-2) = T^4 / (2.5e7 + 2.5e-33 T^18)
-    const double x = div_fast(k3 * T10, T10 + 1.0e22);
-    const double x2 = x * x;
+    const double u = div_fast(T10, T10 + 1.0e22);
+    const double x2 = (kappa[2] * kappa[2]) * T * (u * u);
     k = root4(__fma_rn(ik, ik, x2 * x2));
   } else if (T > 0.0 && rho > 0.0) {
     // T <= TEMPB(i, j) compared as logarithms: ln T <= (ln(kappa_j / kappa_i)
@@ -1656,7 +1655,11 @@ __global__ void __launch_bounds__(RING_T) k_azi_rings(DevGrid g, const double *_
     const double invdt = 1.0 / dt, dpinvns = 2.0 * TH_PI / (double)ns;
     vmed[i] = vm;
     nshift[i] = (int)(long long)Nround;
-    vtemp[i] = (Ntilde - Nround) * g.r.Rmed[i] * invdt * dpinvns;
+    const double v = (Ntilde - Nround) * g.r.Rmed[i] * invdt * dpinvns;
+    // of the uniform pass: v, the face coefficient and the flux's ring factor
+    vtemp[3 * i] = v;
+    vtemp[3 * i + 1] = __fma_rn(-v, dt * g.r.InvDxtheta[i], v > 0.0 ? 1.0 : -1.0);
+    vtemp[3 * i + 2] = (g.r.Rsup[i] - g.r.Rinf[i]) * dt * v;
   }
 }
 
@@ -1705,17 +1708,16 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
   for (int k = 0; k < NQ; k++) q[k] = io.src[k][rowo + j];
   const double vface = vt[rowo + j];
   const double vsub = fast ? vmed[i] : 0.0;
-  const double vuni = fast ? vtemp[i] : 0.0;
   const int npass = fast ? 2 : 1;
   for (int pass = 0; pass < npass; pass++) {
-    const double v = (pass == 1) ? vuni : (vface - vsub);
+    const double v = (pass == 1) ? vtemp[3 * i] : (vface - vsub);
     const bool up = __double_as_longlong(v) > 0LL; // v > 0.0: upwind cell of the left face is j-1
     // face value q* = q_up +/- (dxtheta -/+ v dt) dq_up with the slope dq kept
     // without its 1/dxtheta factor, which goes into csg = +/-1 - v dt/dxtheta
     // instead.  The upwind choice differs between neighbouring cells, so it
     // selects operands (integer moves) and every face value is one FMA,
     // fma(csg, dq_up, q_up), rather than two predicated ones.
-    const double csg = __fma_rn(-v, dtinvdx, up ? 1.0 : -1.0);
+    const double csg = (pass == 1) ? vtemp[3 * i + 1] : __fma_rn(-v, dtinvdx, up ? 1.0 : -1.0);
     // RhoStar at the left face (ComputeStarTheta of the density)
     const double rho = q[NQ - 1];
     s_a[t] = rho;
@@ -1728,8 +1730,9 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
     s_c[t] = drho;
     __syncthreads();
     const double rs = __fma_rn(csg, up ? s_c[tm] : drho, up ? rho_m : rho);
-    const double cf = dxrad * rs * v;              // flux = dxrad Q* RhoStar v
-    const double rcp = div_fast(1.0, rho + 1e-20); // 1 / (RhoInt + 1e-20)
+    const double cf = (pass == 1) ? vtemp[3 * i + 2] * rs : dxrad * rs * v;   // flux = dxrad Q* RhoStar v
+    // 1 / (RhoInt + 1e-20); from 2^-13 on the sum is RhoInt
+    const double rcp = div_fast(1.0, __double2hiint(rho) >= 0x3f200000 ? rho : rho + 1e-20);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NQ; k++) {

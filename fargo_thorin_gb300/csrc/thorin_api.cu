@@ -114,7 +114,7 @@ enum {  // ring arrays kept on the device
   R_WAVEKILLER, R_RMED15, R_RINF15, R_RSUP15, R_COSTAB, R_SINTAB, R_SIGMAMED, R_ENERGYMED, R_VTHETAMED, R_PEBDENS0,
   R_PEBVRAD0, R_PEBVTHETA0, R_CSMEAN, R_TEMPMEAN, R_NUMED, R_NUINF, R_INVDXTHETA, R_INVDXTHETA2, R_SUPPTORQUE,
   R_DELTAR2, R_CFLDXRAD, R_CFLDXTHETA, R_CFLMINDX, R_CFLDEN5, R_VMOY, R_PVTMED, R_HAVR, R_PHAVR, R_AGR0, R_PAGR0,
-  R_STARW, R_VMED, R_VTEMP, R_DAMPVR0, R_CSISO, R_COOLT, R_QPLUSMED, R_DRSQ, R_OMEGA,
+  R_STARW, R_VMED, R_DAMPVR0, R_CSISO, R_COOLT, R_QPLUSMED, R_DRSQ, R_OMEGA,
   R_COUNT
 };
 
@@ -453,7 +453,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   RCHK(dalloc(d, (void **)&d->nshift, n1 * sizeof(int)));
   d->ts.nshift = d->nshift;
   d->ts.vmed = d->ring[R_VMED];
-  d->ts.vtemp = d->ring[R_VTEMP];
+  RCHK(dalloc(d, (void **)&d->ts.vtemp, 3 * n1 * sizeof(double)));
   if (d->p.pebbles) {
     TransportScratch &P = d->ts_peb;
     P = TransportScratch{};
@@ -465,7 +465,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     P.w[6] = P.ext_new = nullptr;
     RCHK(dalloc(d, (void **)&P.nshift, n1 * sizeof(int)));
     RCHK(dalloc(d, (void **)&P.vmed, n1 * sizeof(double)));
-    RCHK(dalloc(d, (void **)&P.vtemp, n1 * sizeof(double)));
+    RCHK(dalloc(d, (void **)&P.vtemp, 3 * n1 * sizeof(double)));
     CUCHK(cudaStreamCreateWithFlags(&d->s_peb, cudaStreamNonBlocking));
     CUCHK(cudaEventCreateWithFlags(&d->ev_fork, cudaEventDisableTiming));
     CUCHK(cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming));
