@@ -67,6 +67,7 @@ struct ConvArgs {
   int coutr;
   void *out;
   int B, H, W;
+  int rings;                                       // rings of a strip per unit of work
   int *err;
 };
 
@@ -88,9 +89,19 @@ __global__ void __launch_bounds__(128, 4) k_wn_conv(ConvArgs a)
   uint32_t *tslot = (uint32_t *)(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
 
-  for (int c = tid; c < N * KG; c += 128) {
-    const int n = c / KG, kg = c - n * KG;
-    *(uint4 *)(sB + kg * N * 16 + n * 16) = *(const uint4 *)(a.wk + (size_t)n * K + kg * 8);
+  {                                                        // every load in flight before the first store
+    constexpr int NW = (N * KG + 127) / 128;
+    uint4 w[NW];
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+      const int c = tid + 128 * k;
+      if (c < N * KG) w[k] = __ldg((const uint4 *)(a.wk + (size_t)(c / KG) * K + c % KG * 8));
+    }
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+      const int c = tid + 128 * k;
+      if (c < N * KG) *(uint4 *)(sB + c % KG * N * 16 + c / KG * 16) = w[k];
+    }
   }
   if (tid == 0) umma::mbar_init(bar, 1);
   if (warp == 0) umma::tmem_alloc(tslot, 32);
@@ -103,95 +114,101 @@ __global__ void __launch_bounds__(128, 4) k_wn_conv(ConvArgs a)
   // beside the next tile's loads
   auto bias = [&](int n) { return (MODE != 2 && n < a.coutr) ? __ldg(a.bias + n) : 0.f; };
 
-  const int tpr = (a.W + 127) / 128;                       // tiles per ring
-  const long long ntiles = (long long)a.B * a.H * tpr;
-  // A tile stages rings i-1, i, i+1 over cells p0-1 .. p0+128 (azimuth
-  // wrapped).  The global loads of the next tile are issued into registers
-  // as soon as this tile's MMAs are issued, so their latency overlaps the
-  // MMA wait and the epilogue; every load of the thread is in flight before
-  // the first store.
-  constexpr int NCH = 3 * WN_HALO_W * C8, PER = (NCH + 127) / 128;
+  const int tpr = (a.W + 127) / 128;                       // strips of 128 cells per ring
+  const int nch = (a.H + a.rings - 1) / a.rings;           // chunks of a.rings rings per strip
+  const long long nunits = (long long)a.B * nch * tpr;
+  // A block walks the rings of a strip chunk with the rings i-1, i, i+1 over
+  // cells p0-1 .. p0+128 (azimuth wrapped) staged in three slots (ring mod 3), so
+  // each ring of the chunk is read once instead of by three tiles.  The next
+  // ring's loads are issued into registers as soon as this ring's MMAs are
+  // issued, so their latency overlaps the MMA wait and the epilogue.  The eight
+  // convolutions of a 512x1536 prediction: 219 us with a tile a ring, 194 with
+  // strips, 180 with the weights' loads all in flight (their gather was most of
+  // the small levels' 11 us); five blocks per multiprocessor instead of four: 213.
+  constexpr int NCH = WN_HALO_W * C8, PER = (NCH + 127) / 128;
   uint4 val[PER];
-  auto load_tile = [&](long long tile) {
-    const long long ring = tile / tpr;
-    const int p0 = (int)(tile - ring * tpr) * 128;
-    const int i = (int)(ring % a.H);
-    const long long rbase = ring - i;
+  auto load_ring = [&](long long rbase, int ii, int p0) {
 #pragma unroll
     for (int k = 0; k < PER; k++) {
       const int ch = tid + 128 * k;
       val[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (ch < NCH) {
-        const int c8 = ch % C8, rest = ch / C8, pp = rest % WN_HALO_W, rr = rest / WN_HALO_W;
-        const int ii = i + rr - 1;
+      if (ch < NCH && ii >= 0 && ii < a.H) {
+        const int c8 = ch % C8, pp = ch / C8;
         int jj = p0 - 1 + pp;
         jj = jj < 0 ? jj + a.W : (jj >= a.W ? jj % a.W : jj);
-        if (ii >= 0 && ii < a.H) val[k] = __ldg((const uint4 *)(a.in + ((rbase + ii) * a.W + jj) * CIN + c8 * 8));
+        val[k] = __ldg((const uint4 *)(a.in + ((rbase + ii) * a.W + jj) * CIN + c8 * 8));
       }
+    }
+  };
+  auto store_ring = [&](int slot) {
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int ch = tid + 128 * k;
+      if (ch < NCH) *(uint4 *)(sA + ((ch % C8 * 3 + slot) * WN_HALO_W + ch / C8) * 16) = val[k];
     }
   };
   uint32_t phase = 0;
   bool ok = true;
-  if ((long long)blockIdx.x < ntiles) load_tile(blockIdx.x);
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long ring = tile / tpr;                     // b * H + i
-    const int p0 = (int)(tile - ring * tpr) * 128;
+  for (long long unit = blockIdx.x; unit < nunits && ok; unit += gridDim.x) {
+    const int p0 = (int)(unit % tpr) * 128, i0 = (int)(unit / tpr % nch) * a.rings, i1 = min(i0 + a.rings, a.H);
+    const long long rbase = unit / tpr / nch * a.H;
+    load_ring(rbase, i0 - 1, p0);
+    store_ring((i0 + 2) % 3);
+    load_ring(rbase, i0, p0);
+    store_ring(i0 % 3);
+    load_ring(rbase, i0 + 1, p0);
+    for (int i = i0; i < i1; i++) {
+      const long long ring = rbase + i;                      // b * H + i
+      store_ring((i + 1) % 3);
+      umma::fence_smem_async();
+      __syncthreads();
+      if (tid == 0) {
+        umma::fence_after_sync();
+        const uint32_t a0 = umma::smem_addr(sA), b0 = umma::smem_addr(sB);
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int ch = tid + 128 * k;
-      if (ch < NCH) {
-        const int c8 = ch % C8, rest = ch / C8, pp = rest % WN_HALO_W, rr = rest / WN_HALO_W;
-        *(uint4 *)(sA + ((c8 * 3 + rr) * WN_HALO_W + pp) * 16) = val[k];
-      }
-    }
-    umma::fence_smem_async();
-    __syncthreads();
-    if (tid == 0) {
-      umma::fence_after_sync();
-      const uint32_t a0 = umma::smem_addr(sA), b0 = umma::smem_addr(sB);
+        for (int t = 0; t < 9; t++) {
+          const int rr = (i + 2 + t / 3) % 3, pp = t % 3;    // ring 1 + dr, first cell 1 + dphi
 #pragma unroll
-      for (int t = 0; t < 9; t++) {
-        const int rr = t / 3, pp = t % 3;                  // ring 1 + dr, first cell 1 + dphi
-#pragma unroll
-        for (int ks = 0; ks < CIN / 16; ks++)
-          umma::mma_bf16(tmem, umma::desc(a0 + ((2 * ks * 3 + rr) * WN_HALO_W + pp) * 16, LBO_A, 128),
-                         umma::desc(b0 + (t * (CIN / 16) + ks) * 2 * N * 16, N * 16, 128), IDESC, t > 0 || ks > 0);
-      }
-      umma::mma_commit(bar);
-    }
-    __syncwarp();
-    if (tile + gridDim.x < ntiles) load_tile(tile + gridDim.x);   // registers only: sA is the MMA's until the wait
-    ok = umma::mbar_wait(bar, phase, WN_WAIT);
-    ok = __syncthreads_and(ok);
-    phase ^= 1u;
-    if (!ok) break;
-    umma::fence_after_sync();
-    float v[N];
-    umma::tmem_ld<N>(tmem + ((uint32_t)(warp * 32) << 16), v);
-    const bool live = p0 + tid < a.W;
-    const long long p = ring * a.W + p0 + tid;
-    if (live) {
-      if (MODE == 0) {
-        uint4 *dst = (uint4 *)((bf16 *)a.out + p * N);
-#pragma unroll
-        for (int q = 0; q < N / 8; q++) {
-          __nv_bfloat162 h[4];
-#pragma unroll
-          for (int e = 0; e < 4; e++)
-            h[e] = __floats2bfloat162_rn(fmaxf(v[8 * q + 2 * e] + bias(8 * q + 2 * e), 0.f),
-                                         fmaxf(v[8 * q + 2 * e + 1] + bias(8 * q + 2 * e + 1), 0.f));
-          dst[q] = *(uint4 *)h;
+          for (int ks = 0; ks < CIN / 16; ks++)
+            umma::mma_bf16(tmem, umma::desc(a0 + ((2 * ks * 3 + rr) * WN_HALO_W + pp) * 16, LBO_A, 128),
+                           umma::desc(b0 + (t * (CIN / 16) + ks) * 2 * N * 16, N * 16, 128), IDESC, t > 0 || ks > 0);
         }
-      } else if (MODE == 1) {
-        ((float *)a.out)[p] = v[0] + bias(0);
-      } else {
-        float4 *dst = (float4 *)((float *)a.out + p * N);
-#pragma unroll
-        for (int q = 0; q < N / 4; q++) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        umma::mma_commit(bar);
       }
+      __syncwarp();
+      if (i + 1 < i1) load_ring(rbase, i + 2, p0);           // registers only: sA is the MMA's until the wait
+      ok = umma::mbar_wait(bar, phase, WN_WAIT);
+      ok = __syncthreads_and(ok);
+      phase ^= 1u;
+      if (!ok) break;
+      umma::fence_after_sync();
+      float v[N];
+      umma::tmem_ld<N>(tmem + ((uint32_t)(warp * 32) << 16), v);
+      const bool live = p0 + tid < a.W;
+      const long long p = ring * a.W + p0 + tid;
+      if (live) {
+        if (MODE == 0) {
+          uint4 *dst = (uint4 *)((bf16 *)a.out + p * N);
+#pragma unroll
+          for (int q = 0; q < N / 8; q++) {
+            __nv_bfloat162 h[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+              h[e] = __floats2bfloat162_rn(fmaxf(v[8 * q + 2 * e] + bias(8 * q + 2 * e), 0.f),
+                                           fmaxf(v[8 * q + 2 * e + 1] + bias(8 * q + 2 * e + 1), 0.f));
+            dst[q] = *(uint4 *)h;
+          }
+        } else if (MODE == 1) {
+          ((float *)a.out)[p] = v[0] + bias(0);
+        } else {
+          float4 *dst = (float4 *)((float *)a.out + p * N);
+#pragma unroll
+          for (int q = 0; q < N / 4; q++) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+      }
+      umma::fence_before_sync();
+      __syncthreads();
     }
-    umma::fence_before_sync();
-    __syncthreads();
   }
   if (!ok) {
     if (tid == 0) atomicExch(a.err, 1);
@@ -1016,8 +1033,11 @@ static int conv_launch(thorin_warmnet *n, const bf16 *in, const bf16 *wk, const 
   constexpr long long per_sm = 4;
   const long long tiles = (long long)B * H * ((W + 127) / 128);
   const long long wave = per_sm * n->nsm;
-  const int grid = (int)(tiles < wave ? tiles : wave);
-  ConvArgs a{in, wk, bias, coutr, out, B, H, W, n->err};
+  // as many rings a unit as leave one wave of units
+  const int rings = (int)((tiles + wave - 1) / wave);
+  const long long units = (long long)B * ((H + rings - 1) / rings) * ((W + 127) / 128);
+  const int grid = (int)(units < wave ? units : wave);
+  ConvArgs a{in, wk, bias, coutr, out, B, H, W, rings, n->err};
   launch(k_wn_conv<CIN, N, MODE>, grid, 128, SM, s, a);
   g_thorin_launches++;
   return THORIN_OK;
