@@ -2,11 +2,11 @@
 // transport of the AlgoGas substep (src_main/SourceEuler.c:319-586,
 // Viscosity.c:85-260, EnergySources.c:75-856, TransportEuler.c:34-505).
 //
-// Each kernel keeps the reference's per-cell operation order (products and
-// sums associate left to right exactly as written in the C source) so that,
-// compiled without FMA contraction, results match the reference bit for bit
-// wherever no transcendental function is involved.
+// The kernels are bound by the FP64 pipe, so their arithmetic is regrouped for
+// few FP64 instructions (each says how); results agree with the reference's
+// operation order to rounding, and integer decisions are exact.
 #include <cstdio>
+#include <type_traits>
 #include "thorin_kernels.cuh"
 
 #define CELL_LOOP_2D                                                        \
@@ -683,8 +683,8 @@ __device__ __forceinline__ double opacity_law(const DevConst &k, double vd, doub
 // (FluxLimiterValue, :684-698) of s = 4 |grad T| / (rho kappa T) needs only s^2
 // below s = 2, where it is 2 / (3 + sqrt(9 + 10 s^2)); both forms give 1/5 at
 // s = 2.  The diffusion coefficient's division and the limiter's are one.
-// FP64-bound: 81 FP64 instructions a cell with the Bell & Lin opacity, 120
-// before; 512x1536: 182 -> 138 us, with the minimum over the blocks.
+// FP64-bound: 79 FP64 instructions a cell with the Bell & Lin opacity, 120
+// before; 512x1536: 182 -> 136 us, with the minimum over the blocks.
 // Rings per block: chunks of at most 8, as the inner, hotter rings take the
 // longer opacity branches and short chunks spread them (512x1536: 133 / 138 / 157
 // us with 3 / 6 / 11 rings; 1024x3072: 486 / 500 / 543 us with 8 / 16 / 21).
@@ -1680,8 +1680,11 @@ __global__ void __launch_bounds__(RING_T) k_azi_rings(DevGrid g, const double *_
 // last bits only.  The FP64 pipe bounds it: six FP64 instructions per quantity
 // and pass (the quotient, its difference, the face value, the flux and two for
 // the update; the slopes run on the FP32 and integer pipes, vl_slope).
-// 512x1536: 231 -> 147 us with the gas's six quantities (151 -> 92 FP64
-// instructions a cell).
+// The two passes are separate code: with the choice made per pass at run time
+// both passes' FP64 instructions were issued under predicates.
+// 1024x3072: 556 us with the gas's six quantities and 87 FP64 instructions a
+// cell (588 us and 91 under predicates, 917 us and 151 with the slopes on the
+// FP64 pipe).
 #define AZ_HALO 4
 #define AZ_TMAX 512
 
@@ -1708,16 +1711,18 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
   for (int k = 0; k < NQ; k++) q[k] = io.src[k][rowo + j];
   const double vface = vt[rowo + j];
   const double vsub = fast ? vmed[i] : 0.0;
-  const int npass = fast ? 2 : 1;
-  for (int pass = 0; pass < npass; pass++) {
-    const double v = (pass == 1) ? vtemp[3 * i] : (vface - vsub);
+  // the residual velocity's pass or the uniform one, whose v, face coefficient
+  // and flux factor are the ring's
+  auto wind = [&](auto uniform) {
+    constexpr bool U = decltype(uniform)::value;
+    const double v = U ? vtemp[3 * i] : (vface - vsub);
     const bool up = __double_as_longlong(v) > 0LL; // v > 0.0: upwind cell of the left face is j-1
     // face value q* = q_up +/- (dxtheta -/+ v dt) dq_up with the slope dq kept
     // without its 1/dxtheta factor, which goes into csg = +/-1 - v dt/dxtheta
     // instead.  The upwind choice differs between neighbouring cells, so it
     // selects operands (integer moves) and every face value is one FMA,
     // fma(csg, dq_up, q_up), rather than two predicated ones.
-    const double csg = (pass == 1) ? vtemp[3 * i + 1] : __fma_rn(-v, dtinvdx, up ? 1.0 : -1.0);
+    const double csg = U ? vtemp[3 * i + 1] : __fma_rn(-v, dtinvdx, up ? 1.0 : -1.0);
     // RhoStar at the left face (ComputeStarTheta of the density)
     const double rho = q[NQ - 1];
     s_a[t] = rho;
@@ -1730,9 +1735,8 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
     s_c[t] = drho;
     __syncthreads();
     const double rs = __fma_rn(csg, up ? s_c[tm] : drho, up ? rho_m : rho);
-    const double cf = (pass == 1) ? vtemp[3 * i + 2] * rs : dxrad * rs * v;   // flux = dxrad Q* RhoStar v
-    // 1 / (RhoInt + 1e-20); from 2^-13 on the sum is RhoInt
-    const double rcp = div_fast(1.0, __double2hiint(rho) >= 0x3f200000 ? rho : rho + 1e-20);
+    const double cf = U ? vtemp[3 * i + 2] * rs : dxrad * rs * v;   // flux = dxrad Q* RhoStar v
+    const double rcp = div_fast(1.0, rho + 1e-20); // 1 / (RhoInt + 1e-20)
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NQ; k++) {
@@ -1760,7 +1764,9 @@ __global__ void __launch_bounds__(AZ_TMAX) k_azimuthal(DevGrid g, AziIO io, cons
       __syncthreads();
       q[k] = __fma_rn(F - s_b[tp], invsurf, q[k]);
     }
-  }
+  };
+  wind(std::false_type());
+  if (fast) wind(std::true_type());
   const int x = t - AZ_HALO;
   if (x >= 0 && x < seg && j0 + x < ns) {
     int jo = j;
