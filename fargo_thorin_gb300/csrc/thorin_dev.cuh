@@ -84,9 +84,6 @@ struct DevGrid {
   int sor_tpsm;                          // SOR pass: resident threads per multiprocessor (0: 1536)
 };
 
-__device__ __forceinline__ int jp_of(int j, int ns) { return (j == ns - 1) ? 0 : j + 1; }
-__device__ __forceinline__ int jm_of(int j, int ns) { return (j == 0) ? ns - 1 : j - 1; }
-
 // Sum of row[0..n) in strictly left-to-right order (the reference's
 // sequential ring sums, e.g. mpi_make1Dprofile, mpiTasks.c:26-32), computed by
 // one warp: lanes load coalesced chunks, the running sum walks the chunk in
@@ -432,10 +429,9 @@ __device__ __forceinline__ double div_fast(double x, double d)
   return x / d;
 }
 
-// Square root and reciprocal square root in three FP64 instructions each:
-// the estimate y of 1/sqrt(x), then s = x y with the residual x - s^2 formed
-// exactly (Markstein's correction as in div_fast), or one Newton-Raphson step
-// of y.  thorin_selftest_sqrt measures both on the GPU.
+// Square root in three FP64 instructions: the estimate y of 1/sqrt(x), then
+// s = x y with the residual x - s^2 formed exactly (Markstein's correction as in
+// div_fast).  thorin_selftest_sqrt measures it on the GPU.
 __device__ __forceinline__ double sqrt_fast(double x)
 {
   if (exp_ok(x) && __double2hiint(x) > 0) {
@@ -445,17 +441,6 @@ __device__ __forceinline__ double sqrt_fast(double x)
     return __fma_rn(r, half_i(y), s);
   }
   return sqrt(x);
-}
-
-__device__ __forceinline__ double rsqrt_fast(double x)
-{
-  if (exp_ok(x) && __double2hiint(x) > 0) {
-    const double y = rsqrt_est(x);
-    const double t = x * y;
-    const double e = __fma_rn(-t, y, 1.0);
-    return __fma_rn(half_i(y), e, y);
-  }
-  return rsqrt(x);
 }
 
 // y (1 + rel) for |rel| below 2^-40: rel in units of y's last place, rounded to

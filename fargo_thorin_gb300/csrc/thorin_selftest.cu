@@ -1,5 +1,5 @@
 // thorin_selftest.cu -- on-device checks of the kernels' division and square
-// root routines (div_fast, div_slope, vl_slope, sqrt_fast, rsqrt_fast) against the IEEE
+// root routines (div_fast, div_slope, vl_slope, sqrt_fast) against the IEEE
 // operations, conditional graph nodes, and the FP64 FMA peak.
 #include <string>
 #include "thorin_kernels.cuh"
@@ -65,33 +65,28 @@ extern "C" int thorin_selftest_division(long long n, unsigned long long seed, do
   return THORIN_OK;
 }
 
-// sqrt_fast against sqrt, rsqrt_fast against 1 / sqrt(x) (two roundings,
-// so one ulp of distance is expected there): out[0] mismatches of sqrt,
-// out[1] and out[2] the largest distances in ulp.
+// sqrt_fast against sqrt: out[0] mismatches, out[1] the largest distance in ulp.
 __global__ void k_selftest_sqrt(long long n, unsigned long long seed, double emax, unsigned long long *__restrict__ out)
 {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double x = fabs(st_value(seed + (unsigned long long)t, emax));
   const long long a = __double_as_longlong(sqrt(x)), b = __double_as_longlong(sqrt_fast(x));
-  const long long c = __double_as_longlong(1.0 / sqrt(x)), e = __double_as_longlong(rsqrt_fast(x));
-  const unsigned long long u = (unsigned long long)(a > b ? a - b : b - a), v = (unsigned long long)(c > e ? c - e : e - c);
+  const unsigned long long u = (unsigned long long)(a > b ? a - b : b - a);
   if (u) {
     atomicAdd(out, 1ULL);
     atomicMax(out + 1, u);
   }
-  if (v > 1ULL) atomicMax(out + 2, v);
 }
 
 extern "C" int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_exponent,
-                                    unsigned long long *mismatches, unsigned long long *max_ulp,
-                                    unsigned long long *max_ulp_rsqrt)
+                                    unsigned long long *mismatches, unsigned long long *max_ulp)
 {
-  if (n < 1 || !mismatches || !max_ulp || !max_ulp_rsqrt || !(max_exponent >= 0.0 && max_exponent <= 1000.0)) {
+  if (n < 1 || !mismatches || !max_ulp || !(max_exponent >= 0.0 && max_exponent <= 1000.0)) {
     g_last_error = "selftest_sqrt: n >= 1, 0 <= max_exponent <= 1000 and output pointers required";
     return THORIN_ERR_ARG;
   }
-  unsigned long long *dev = nullptr, host[3] = {0ULL, 0ULL, 0ULL};
+  unsigned long long *dev = nullptr, host[2] = {0ULL, 0ULL};
   cudaError_t e = cudaMalloc((void **)&dev, sizeof(host));
   if (e == cudaSuccess) e = cudaMemset(dev, 0, sizeof(host));
   if (e == cudaSuccess) {
@@ -106,7 +101,6 @@ extern "C" int thorin_selftest_sqrt(long long n, unsigned long long seed, double
   }
   *mismatches = host[0];
   *max_ulp = host[1];
-  *max_ulp_rsqrt = host[2];
   return THORIN_OK;
 }
 

@@ -313,11 +313,12 @@ int thorin_gpu_algogas_graph(thorin_disk *d, thorin_planets *sys);
  * THORIN_ERR_ARG with the reason in thorin_gpu_last_error(). */
 int thorin_gpu_graph_supported(thorin_disk *d, const thorin_planets *sys);
 
-/* Launch shape of the SOR sweeps (no counterpart in the reference): sweeps
- * per run of the sweep loop's body (1..64, default 8) and the resident
+/* Launch shape of the SOR sweeps (no counterpart in the reference) where they
+ * are launches of their own, on disks above 2.4 million cells: sweeps
+ * per run of the sweep loop's body (1..64, default 8) and the most resident
  * threads per multiprocessor of a colour pass (128..2048 in steps of 128,
- * default 1536).  Results do not depend on either; the ensemble autotuner
- * picks them per disk size.  The disk's graphs are rebuilt at their next
+ * default 1536; the kernel holds at most 1024).  Results do not depend on
+ * either; the ensemble autotuner picks them per disk size.  The disk's graphs are rebuilt at their next
  * use. */
 int thorin_gpu_set_launch_shape(thorin_disk *d, int sor_loop_sweeps, int sor_threads_per_sm);
 int thorin_gpu_get_launch_shape(thorin_disk *d, int *sor_loop_sweeps, int *sor_threads_per_sm);
@@ -431,12 +432,10 @@ int thorin_selftest_exp(long long n, unsigned long long seed, double range, doub
                         unsigned long long *max_ulp_exp, unsigned long long *max_ulp_pow);
 
 /* Compares the kernels' square root routine with IEEE square root on n
- * random operands (exponents in [-max_exponent, max_exponent]) and the
- * reciprocal square root with 1 / sqrt(x): results that differ from sqrt, the
- * largest distance from it, and the largest distance of the reciprocal square
- * root beyond one ulp (0: none). */
+ * random operands (exponents in [-max_exponent, max_exponent]): results that
+ * differ and the largest distance in ulp (0: none). */
 int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_exponent, unsigned long long *mismatches,
-                         unsigned long long *max_ulp, unsigned long long *max_ulp_rsqrt);
+                         unsigned long long *max_ulp);
 
 /* Self-test of the conditional CUDA graph nodes behind the SOR sweep loop:
  * a kernel that sets an IF node's condition to 0 must skip its body

@@ -67,18 +67,14 @@ def test_van_leer_slope_bound(max_exponent, seed):
 @pytest.mark.parametrize("max_exponent,seed", [(40.0, 6), (300.0, 7), (1000.0, 8)])
 def test_square_roots_match_ieee(max_exponent, seed):
     """sqrt_fast is Markstein-corrected like the division: at most one ulp
-    from sqrt, in practice identical.  rsqrt_fast has one rounded product and
-    one Newton-Raphson step (error below 1.5 ulp) against 1 / sqrt(x), itself
-    up to 1 ulp off: at most 2 ulp apart."""
+    from sqrt, in practice identical."""
     from fargo_thorin_gb300 import _lib
     lib = _lib.load()
     n = 1 << 26
-    mis, ulp, ulpr = C.c_ulonglong(), C.c_ulonglong(), C.c_ulonglong()
-    _lib.check(lib.thorin_selftest_sqrt(n, seed, max_exponent, C.byref(mis), C.byref(ulp), C.byref(ulpr)),
-               "selftest_sqrt")
+    mis, ulp = C.c_ulonglong(), C.c_ulonglong()
+    _lib.check(lib.thorin_selftest_sqrt(n, seed, max_exponent, C.byref(mis), C.byref(ulp)), "selftest_sqrt")
     assert ulp.value <= 1
     assert mis.value <= n // 1000000
-    assert ulpr.value <= 2
 
 
 def test_graph_conditional_nodes():
