@@ -1042,17 +1042,23 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, con
     if (pass) a.isig30 = 1.0 / sig;
     else a.isig10 = 1.0 / sig;
   }
-  // rings per block: chunks long enough that the block sums and the ring
-  // constants are a small part, and at least about six blocks per
-  // multiprocessor; for the near cells fewer, as all their work may lie in a
-  // few chunks
+  // rings per block: the chunk with the least work on the busiest
+  // multiprocessor, which runs four blocks at a time and uses 1 - (1 - n / 4)^2
+  // of the FP64 pipe with n of them left, the ring and planet constants and the
+  // block sums counted as two rings.  24x72 16.6 -> 9.4 us, 128x384 17.3 -> 11.5,
+  // 512x1536 65.7 -> 61, 1024x3072 243 -> 224 (some six blocks a multiprocessor and
+  // at least four rings before).  For the near cells at most four rings, as all
+  // their work may lie in a few chunks
   const int nbx = (g.ns + 127) / 128;
-  auto rings = [&](int blocks, int lo, int hi) {
-    const int r = (int)((long long)g.nr * nbx / (g.nsm * blocks));
-    return r < lo ? lo : (r > hi ? hi : r);
-  };
-  a.rings_a = rings(6, 4, 32);
-  a.rings_b = rings(40, 1, 4);
+  a.rings_a = 1;
+  double best = 1e300;
+  for (int r = 1; r <= 32; r++) {
+    const int n = (nbx * ((g.nr + r - 1) / r) + g.nsm - 1) / g.nsm, part = n & 3;
+    const double q = 1.0 - 0.25 * part, w = ((n - part) + (part ? part / (1.0 - q * q) : 0.0)) * (r + 2);
+    if (w < best) { best = w; a.rings_a = r; }
+  }
+  const int rb = (int)((long long)g.nr * nbx / (g.nsm * 40));
+  a.rings_b = rb < 1 ? 1 : (rb > 4 ? 4 : rb);
   const dim3 ga(nbx, (g.nr + a.rings_a - 1) / a.rings_a);
   a.nba = ga.x * ga.y;
   a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
