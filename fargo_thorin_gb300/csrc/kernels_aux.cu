@@ -930,21 +930,19 @@ __global__ void __launch_bounds__(128) k_forces_near(DevGrid g, ForceArgs a, For
     for (int k = 0; k < a.npl; k++) {
       const DevPlanet &P = a.pl[k];
       if (!(P.rmorevert2 > 0.0)) continue;
-      // rings that reach within two Hill radii of the planet's radius
+      // rings that reach within two Hill radii of the planet's radius: from the
+      // first with Rsup >= rp - rh to the last with Rinf <= rp + rh, counted by the
+      // lanes (radii are positive, so their bits compare as integers); two
+      // bisections were 20 dependent loads, a third of the kernel on a small disk
       const double rp = sqrt(P.x * P.x + P.y * P.y), rh = 2.001 * P.rhill;
-      int lo = 0, hi = g.nr;
-      while (lo < hi) {                              // first ring with Rsup >= rp - rh
-        const int mid = (lo + hi) >> 1;
-        if (g.r.Rsup[mid] < rp - rh) lo = mid + 1;
-        else hi = mid;
+      const long long below = __double_as_longlong(rp - rh), above = __double_as_longlong(rp + rh);
+      int imin = 0, lo = 0;
+      for (int i = lane; i < g.nr; i += 32) {
+        imin += __double_as_longlong(g.r.Rsup[i]) < below ? 1 : 0;
+        lo += __double_as_longlong(g.r.Rinf[i]) <= above ? 1 : 0;
       }
-      const int imin = lo;
-      hi = g.nr;
-      while (lo < hi) {                              // first ring with Rinf > rp + rh
-        const int mid = (lo + hi) >> 1;
-        if (g.r.Rinf[mid] <= rp + rh) lo = mid + 1;
-        else hi = mid;
-      }
+      imin = __reduce_add_sync(TH_FULL, imin);
+      lo = __reduce_add_sync(TH_FULL, lo);
       const long long ncells = (long long)(lo - imin) * ns;
       for (long long base = gw; base < ncells; base += 32LL * nw) {   // warp-uniform
         const long long q = base + (long long)lane * nw;
@@ -974,9 +972,14 @@ __global__ void __launch_bounds__(128) k_forces_near(DevGrid g, ForceArgs a, For
     if (threadIdx.x < nq) a.part[(size_t)threadIdx.x * nb + b] = 0.0;
     return;
   }
-  for (int q = 0; q < nq; q++) {
-    const double v = block_reduce_smem<128>(acc[q], OpAdd());
-    if (threadIdx.x == 0) a.part[(size_t)q * nb + b] = v;
+  // a warp per quantity adds the threads' values
+  extern __shared__ double near_sums[];              // [nq][128]
+  for (int q = 0; q < nq; q++) near_sums[q * 128 + threadIdx.x] = acc[q];
+  __syncthreads();
+  for (int q = threadIdx.x >> 5; q < nq; q += 4) {
+    const double *v = near_sums + q * 128 + (threadIdx.x & 31);
+    const double t = warp_reduce((v[0] + v[32]) + (v[64] + v[96]), OpAdd());
+    if ((threadIdx.x & 31) == 0) a.part[(size_t)q * nb + b] = t;
   }
 }
 
@@ -1073,7 +1076,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, con
   default: launch_forces<MAXPL_DEV>(g, a, fr, ga, s); break;
   }
   g_thorin_launches++;
-  launch(k_forces_near, a.nbb, 128, 0, s, g, a, fr);
+  launch(k_forces_near, a.nbb, 128, (2 + 2 * a.npl) * 128 * sizeof(double), s, g, a, fr);
   g_thorin_launches++;
   launch(k_forces_final, 2 + 2 * a.npl, 1024, 0, s, g, a, scal);
   g_thorin_launches++;
