@@ -396,23 +396,36 @@ void aux_cfl(const DevGrid &g, const double *vr, const double *vt, const double 
 }
 
 // ---------------------------------------------------------------------------
-// EvaporatePebbles (Pebbles.c:834-864).
+// EvaporatePebbles (Pebbles.c:834-864).  One load and one comparison a cell but
+// where it is hot, so a thread takes EVAP_CPT cells with an integer comparison
+// (a cell a thread and FP64: 28 us on the 1024x3072 disk, now 11.5).
+#define EVAP_CPT 8
 __global__ void k_evaporate(DevGrid g, const double *__restrict__ T, double *__restrict__ pdens)
 {
   pdl_wait();
   const double facc = g.ctl[CTL_FACC_EVAP];
-  const int ns = g.ns;
-  CELL_LOOP_2D
-  if (T[l] > g.k.evaptemp) {
-    double d = pdens[l] * (1.0 - facc);
-    if (d < 1.0e-8) d = 1.0e-8;
-    pdens[l] = d;
+  const int ns = g.ns, row = blockIdx.y * ns, j0 = blockIdx.x * (BX * EVAP_CPT) + threadIdx.x;
+  double t[EVAP_CPT];
+#pragma unroll
+  for (int m = 0; m < EVAP_CPT; m++) t[m] = (j0 + m * BX < ns) ? T[row + j0 + m * BX] : 0.0;
+  // T > evaptemp > 0 on the bits: a negative T is below, a NaN is not above
+  const long long e = __double_as_longlong(g.k.evaptemp);
+#pragma unroll
+  for (int m = 0; m < EVAP_CPT; m++) {
+    const int j = j0 + m * BX, l = row + j;
+    const long long b = __double_as_longlong(t[m]);
+    if (j < ns && (e > 0 ? b > e && b <= 0x7ff0000000000000LL : t[m] > g.k.evaptemp)) {
+      asm volatile("" ::: "memory");               // a branch: under predicates the FP64 pipe is busy all the same
+      double d = pdens[l] * (1.0 - facc);
+      if (d < 1.0e-8) d = 1.0e-8;
+      pdens[l] = d;
+    }
   }
 }
 
 void aux_evaporate(const DevGrid &g, const double *T, double *pdens, cudaStream_t s)
 {
-  launch(k_evaporate, grid2d(g.ns, g.nr, BX), BX, 0, s, g, T, pdens);
+  launch(k_evaporate, grid2d(g.ns, g.nr, BX * EVAP_CPT), BX, 0, s, g, T, pdens);
   g_thorin_launches++;
 }
 

@@ -1422,22 +1422,30 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
 }
 
 // After SOR: boundary rings adopt their neighbours' temperature and the
-// energy is rebuilt, E = rho T c_v (EnergySources.c:319-334).
-__global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, double *__restrict__ T,
-                                double *__restrict__ enew)
+// energy is rebuilt, E = rho T c_v (EnergySources.c:319-334).  EFT_CPT cells a
+// thread, their loads in flight together; 1024x3072: 28 -> 17 us (75 MB at copy
+// speed: 11).
+#define EFT_CPT 4
+__global__ void k_energy_from_t(DevGrid g, const double *__restrict__ rho, double *T, double *__restrict__ enew)
 {
   pdl_wait();
-  const int ns = g.ns, nr = g.nr;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  if (j >= ns) return;
-  const int l = j + i * ns;
-  if (i == nr) { enew[l] = 0.0; return; }
-  double t;
-  if (i == 0) { t = T[l + ns]; T[l] = t; }
-  else if (i == nr - 1) { t = T[l - ns]; T[l] = t; }
-  else t = T[l];
-  enew[l] = rho[l] * t * g.k.cv;
+  const int ns = g.ns, nr = g.nr, i = blockIdx.y, j0 = blockIdx.x * (BX * EFT_CPT) + threadIdx.x;
+  const int row = i * ns, from = (i == 0) ? row + ns : (i == nr - 1) ? row - ns : row;
+  double t[EFT_CPT], r[EFT_CPT];
+#pragma unroll
+  for (int m = 0; m < EFT_CPT; m++) {
+    const int j = j0 + m * BX;
+    const bool in = j < ns && i < nr;
+    t[m] = in ? T[from + j] : 0.0;
+    r[m] = in ? rho[row + j] : 0.0;
+  }
+#pragma unroll
+  for (int m = 0; m < EFT_CPT; m++) {
+    const int j = j0 + m * BX;
+    if (j >= ns) continue;
+    if (from != row && i < nr) T[row + j] = t[m];
+    enew[row + j] = (i < nr) ? r[m] * t[m] * g.k.cv : 0.0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2040,7 +2048,7 @@ void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double 
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)
 {
-  launch(k_energy_from_t, grid2d(g.ns, g.nr + 1, BX), BX, 0, s, g, rho, T, enew);
+  launch(k_energy_from_t, grid2d(g.ns, g.nr + 1, BX * EFT_CPT), BX, 0, s, g, rho, T, enew);
   g_thorin_launches++;
 }
 
