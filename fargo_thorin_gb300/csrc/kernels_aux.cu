@@ -1,6 +1,7 @@
 // kernels_aux.cu -- ring means, viscosity per ring, CFL, pebble source terms,
 // damping boundaries, disk forces with their reductions, pebble accretion,
 // conservation integrals.
+#include <algorithm>
 #include "thorin_kernels.cuh"
 #include "thorin_graph.cuh"
 
@@ -1036,8 +1037,37 @@ static void launch_forces(const DevGrid &g, const ForceArgs &a, const ForceRings
   launch(k_forces<NP>, grid, 128, a.rings_a * sizeof(ForceRing), s, g, a, fr);
 }
 
-void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
-                cudaStream_t s)
+// Blocks of the force kernels.
+struct ForceShape { int nbx, rings_a, rings_b, nba, nbn, nbb; };
+
+static ForceShape force_shape(const DevGrid &g, int npl)
+{
+  // rings per block: the chunk with the least work on the busiest
+  // multiprocessor, which runs four blocks at a time and uses 1 - (1 - n / 4)^2
+  // of the FP64 pipe with n of them left, the ring and planet constants and the
+  // block sums counted as two rings.  24x72 16.6 -> 9.4 us, 128x384 17.3 -> 11.5,
+  // 512x1536 65.7 -> 61, 1024x3072 243 -> 224 (some six blocks a multiprocessor and
+  // at least four rings before).  For the near cells at most four rings, as all
+  // their work may lie in a few chunks
+  ForceShape q;
+  q.nbx = (g.ns + 127) / 128;
+  q.rings_a = 1;
+  double best = 1e300;
+  for (int r = 1; r <= 32; r++) {
+    const int n = (q.nbx * ((g.nr + r - 1) / r) + g.nsm - 1) / g.nsm, part = n & 3;
+    const double u = 1.0 - 0.25 * part, w = ((n - part) + (part ? part / (1.0 - u * u) : 0.0)) * (r + 2);
+    if (w < best) { best = w; q.rings_a = r; }
+  }
+  const int rb = (int)((long long)g.nr * q.nbx / (g.nsm * 40));
+  q.rings_b = rb < 1 ? 1 : (rb > 4 ? 4 : rb);
+  q.nba = q.nbx * ((g.nr + q.rings_a - 1) / q.rings_a);
+  q.nbn = q.nbx * ((g.nr + q.rings_b - 1) / q.rings_b);
+  q.nbb = q.nbn + (npl > 0 ? g.nsm : 0);
+  return q;
+}
+
+int aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
+               cudaStream_t s)
 {
   ForceArgs a = a0;
   for (int pass = 0; pass < 2; pass++) {
@@ -1058,27 +1088,14 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, con
     if (pass) a.isig30 = 1.0 / sig;
     else a.isig10 = 1.0 / sig;
   }
-  // rings per block: the chunk with the least work on the busiest
-  // multiprocessor, which runs four blocks at a time and uses 1 - (1 - n / 4)^2
-  // of the FP64 pipe with n of them left, the ring and planet constants and the
-  // block sums counted as two rings.  24x72 16.6 -> 9.4 us, 128x384 17.3 -> 11.5,
-  // 512x1536 65.7 -> 61, 1024x3072 243 -> 224 (some six blocks a multiprocessor and
-  // at least four rings before).  For the near cells at most four rings, as all
-  // their work may lie in a few chunks
-  const int nbx = (g.ns + 127) / 128;
-  a.rings_a = 1;
-  double best = 1e300;
-  for (int r = 1; r <= 32; r++) {
-    const int n = (nbx * ((g.nr + r - 1) / r) + g.nsm - 1) / g.nsm, part = n & 3;
-    const double q = 1.0 - 0.25 * part, w = ((n - part) + (part ? part / (1.0 - q * q) : 0.0)) * (r + 2);
-    if (w < best) { best = w; a.rings_a = r; }
-  }
-  const int rb = (int)((long long)g.nr * nbx / (g.nsm * 40));
-  a.rings_b = rb < 1 ? 1 : (rb > 4 ? 4 : rb);
-  const dim3 ga(nbx, (g.nr + a.rings_a - 1) / a.rings_a);
-  a.nba = ga.x * ga.y;
-  a.nbn = nbx * ((g.nr + a.rings_b - 1) / a.rings_b);
-  a.nbb = a.nbn + (a.npl > 0 ? g.nsm : 0);
+  const ForceShape q = force_shape(g, a.npl);
+  if ((size_t)(2 + 2 * a.npl) * (q.nba + q.nbb) > a.part_size) return THORIN_ERR_NOMEM;
+  a.rings_a = q.rings_a;
+  a.rings_b = q.rings_b;
+  a.nba = q.nba;
+  a.nbn = q.nbn;
+  a.nbb = q.nbb;
+  const dim3 ga(q.nbx, q.nba / q.nbx);
   launch(k_force_rings, g.nr, RING_T, 0, s, g, a, fr, hp);
   g_thorin_launches++;
   switch (a.npl) {
@@ -1093,6 +1110,7 @@ void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, con
   g_thorin_launches++;
   launch(k_forces_final, 2 + 2 * a.npl, 1024, 0, s, g, a, scal);
   g_thorin_launches++;
+  return THORIN_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1446,6 +1464,20 @@ void aux_integrals(const DevGrid &g, const double *rho, const double *vr, const 
   else
     launch(k_integrals<false>, g.nr, RING_T, 0, s, g, rho, vr, vt, e, pd, pvt, omega_frame, part, scal, ticket);
   g_thorin_launches++;
+}
+
+// Doubles that the kernels of this file write to a disk's reduction scratch,
+// from the grids they are launched with: the CFL's two floats a block, the
+// forces' 2 + 2 npl values a block, the accretion's four values of two blocks
+// a multiprocessor, the integrals' five a ring.
+size_t aux_partials(const DevGrid &g, int npl)
+{
+  const ForceShape q = force_shape(g, npl);
+  const dim3 c = grid2d(g.ns, g.nr - 1, 256 * CFL_CPT);
+  size_t n = (size_t)c.x * c.y;
+  n = std::max(n, (size_t)(2 + 2 * npl) * (q.nba + q.nbb));
+  n = std::max(n, (size_t)4 * 2 * g.nsm);
+  return std::max(n, (size_t)5 * g.nr);
 }
 
 // ---------------------------------------------------------------------------

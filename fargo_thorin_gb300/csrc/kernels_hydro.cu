@@ -1871,11 +1871,20 @@ void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double
   g_thorin_launches++;
 }
 
+// 0.2 rings a chunk: the difference with the ring below and the ring constants
+static int diffcoef_rings(const DevGrid &g) { return chunk_rings(g.nr, g.ns, g.nsm, DC_MAXRINGS, 0.2, 8); }
+
+// Doubles of a disk's reduction scratch that k_diffcoef writes, one a block.
+size_t hydro_partials(const DevGrid &g)
+{
+  const int r = diffcoef_rings(g);
+  return (size_t)((g.ns + BX - 1) / BX) * ((g.nr + r - 1) / r);
+}
+
 void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io0, int law, cudaStream_t s)
 {
   DiffusionIO io = io0;
-  // 0.2 rings a chunk: the difference with the ring below and the ring constants
-  io.rings = chunk_rings(g.nr, g.ns, g.nsm, DC_MAXRINGS, 0.2, 8);
+  io.rings = diffcoef_rings(g);
   const dim3 grid((g.ns + BX - 1) / BX, (g.nr + io.rings - 1) / io.rings);
   switch (law) {
   case THORIN_OPA_SM03: launch_fp64(k_diffcoef<THORIN_OPA_SM03>, grid, BX, 0, s, g, io); break;

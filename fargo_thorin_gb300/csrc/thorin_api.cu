@@ -143,7 +143,8 @@ struct thorin_disk {
   cudaEvent_t ev_cs = nullptr, ev_cfl = nullptr, ev_forces = nullptr;   // their results are on the host
   int (*host_side)(void *) = nullptr;   // host work that the substep has still to do (run_host_side)
   void *host_arg = nullptr;
-  double *partials, *scal;
+  double *partials, *scal;           // partials: reduction scratch of partials_size doubles
+  size_t partials_size;
   int *iscal, *nshift, *heat_idx_d, *damp_rings_d;
   double *heat_val_d;
   double *force_col;                 // indirect term per column (ForceArgs::col)
@@ -407,6 +408,25 @@ static int check_supported(const thorin_params &p)
   return THORIN_OK;
 }
 
+// Doubles of a disk's reduction scratch: the most that any kernel's blocks
+// write, with as many planets as the force kernels take.
+static size_t partials_size(const DevGrid &g) { return std::max(aux_partials(g, MAXPL_DEV), hydro_partials(g)); }
+
+extern "C" int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, long long *need, long long *held)
+{
+  if (nrad < 4 || nsec < 4 || npl < 0 || npl > MAXPL_DEV || nsm < 1 || !need || !held) {
+    g_last_error = "selftest_partials: nrad, nsec >= 4, 0 to 8 planets, nsm >= 1 and output pointers required";
+    return THORIN_ERR_ARG;
+  }
+  DevGrid g = {};
+  g.nr = nrad;
+  g.ns = nsec;
+  g.nsm = nsm;
+  *need = (long long)std::max(aux_partials(g, npl), hydro_partials(g));
+  *held = (long long)partials_size(g);
+  return THORIN_OK;
+}
+
 extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
 {
   if (!pin || !out) return THORIN_ERR_ARG;
@@ -470,9 +490,8 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     CUCHK(cudaEventCreateWithFlags(&d->ev_fork, cudaEventDisableTiming));
     CUCHK(cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming));
   }
-  // reduction scratch: enough partials for every reduction kernel
-  const size_t nb = (size_t)((d->ns + 127) / 128 + 2) * (size_t)(d->nr + 2) + (size_t)d->g.nsm;
-  RCHK(dalloc(d, (void **)&d->partials, nb * (2 + 2 * MAXPL_DEV + 6) * sizeof(double)));
+  d->partials_size = partials_size(d->g);
+  RCHK(dalloc(d, (void **)&d->partials, d->partials_size * sizeof(double)));
   RCHK(dalloc(d, (void **)&d->scal, 256 * sizeof(double)));
   RCHK(dalloc(d, (void **)&d->iscal, 64 * sizeof(int)));
   RCHK(dalloc(d, (void **)&d->ticket, 16 * sizeof(unsigned int)));
@@ -1425,6 +1444,7 @@ static ForceArgs force_args(const thorin_disk *d, int npl)
   a.rho = d->rho; a.cs = d->cs; a.tau = d->tau; a.pdens = d->pdens;
   a.agr = d->agr; a.agt = d->agt; a.pagr = d->pagr; a.pagt = d->pagt;
   a.part = d->partials;
+  a.part_size = d->partials_size;
   a.col = d->force_col;
   a.near = d->force_near;
   a.ticket = d->ticket + 8;
@@ -1432,6 +1452,13 @@ static ForceArgs force_args(const thorin_disk *d, int npl)
   a.npl = npl; a.pebbles = p.pebbles; a.exclude_hill = p.exclude_hill; a.pebble_gravity = p.pebble_gravity;
   a.pebble_alpha = p.pebble_alpha; a.hillcut = p.hillcut;
   return a;
+}
+
+static int launch_forces(thorin_disk *d, int npl, const HostPlanets &hp)
+{
+  const int rc = aux_forces(d->g, force_args(d, npl), d->fr, hp, d->scal, d->s);
+  if (rc != THORIN_OK) g_last_error = "forces: the reduction scratch is too small";
+  return rc;
 }
 
 // What of the state before the hydro substep the host needs with the forces'
@@ -1456,7 +1483,7 @@ static int forces_begin(thorin_disk *d, thorin_planets *sys, double mass_taper, 
   hp.mass_taper = mass_taper;
   hp.indx = p.indirect_term ? -axs : 0.0;
   hp.indy = p.indirect_term ? -ays : 0.0;
-  aux_forces(d->g, force_args(d, npl), d->fr, hp, d->scal, d->s);
+  RCHK(launch_forces(d, npl, hp));
   KCHECK("force kernels");
   RingList rl;
   rl.n = 0;
@@ -2331,7 +2358,7 @@ static int capture_substep(thorin_disk *d)
   if (!p.pebbles || npl == 0) graph_force_prep(S, d->s);      // else with the last planet's accretion
   HostPlanets hp;
   hp.n = -1;                           // they are on the device
-  aux_forces(d->g, force_args(d, npl), d->fr, hp, d->scal, d->s);
+  RCHK(launch_forces(d, npl, hp));
   for (int k = 0; k < npl; k++)
     graph_ring_mean_at(d->g, d->rho, d->scal + SC_PLANET_A + 2 * MAXPL_DEV + k, d->ring_info_d + k, d->s);
   // the planet kick and N-body step run beside the hydro substep, which does

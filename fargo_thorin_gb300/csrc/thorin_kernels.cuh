@@ -150,6 +150,7 @@ struct ForceArgs {
   const double *rho, *cs, *tau, *pdens;
   double *agr, *agt, *pagr, *pagt;
   double *part;               // [2 + 2*npl][nblocks]
+  size_t part_size;           // doubles at part
   double *col;                // [2][ns]: the indirect term of each column (radial, and azimuthal between j-1 and j)
   unsigned char *near;        // cells left to k_forces_near
   unsigned int *ticket;       // of k_forces_final
@@ -240,6 +241,7 @@ void hydro_viscous(const DevGrid &g, const ViscousIO &io, cudaStream_t s);
 void hydro_heating(const DevGrid &g, const HeatingIO &io, cudaStream_t s);
 void hydro_eos(const DevGrid &g, const double *rho, const double *energy, double *temper, double *cs, double gm1,
                double gg1, cudaStream_t s);
+size_t hydro_partials(const DevGrid &g);
 void hydro_diffcoef(const DevGrid &g, const DiffusionIO &io, int law, cudaStream_t s);
 void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, const double *opacity, double *flaring,
                        double *qirr, double rstar, double tirr4fac, double opacity_drop, double taueff_c,
@@ -272,6 +274,7 @@ void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const 
                      double drout, double *temper, double *cs, double gm1, double gg1, cudaStream_t s);
 
 // kernels_aux.cu
+size_t aux_partials(const DevGrid &g, int npl);
 void aux_ring_means(const DevGrid &g, const double *f0, double *o0, const double *f1, double *o1, int ring0, int nrings,
                     cudaStream_t s);
 void aux_ring_mean(const DevGrid &g, const double *f, double *out, cudaStream_t s);
@@ -304,8 +307,9 @@ void aux_iso_eos(const DevGrid &g, const double *rho, const double *csr, double 
                  int set_cs, int set_press, int set_temper, cudaStream_t s);
 void aux_damp_peb(const DevGrid &g, double *pd, double *pvr, double *pvt, const int *rings, int nrings, cudaStream_t s);
 void aux_crash(const DevGrid &g, const double *f, int *flag, cudaStream_t s);
-void aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
-                cudaStream_t s);
+// THORIN_ERR_NOMEM, without a launch, when the block sums do not fit a0.part_size.
+int aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, const HostPlanets &hp, double *scal,
+               cudaStream_t s);
 // Pebble accretion with the arguments a0, which go to a_dev, or, with a0 NULL,
 // with those at a_dev; nb: aux_accrete_blocks of the widest annulus possible.
 void aux_accrete(const DevGrid &g, const AccArgs *a0, AccArgs *a_dev, int nb, double *scal, cudaStream_t s);

@@ -437,6 +437,11 @@ int thorin_selftest_exp(long long n, unsigned long long seed, double range, doub
 int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_exponent, unsigned long long *mismatches,
                          unsigned long long *max_ulp);
 
+/* Size of a disk's reduction scratch, without a GPU: the doubles that the
+ * launches of an nrad x nsec disk with npl planets write on a GPU of nsm
+ * multiprocessors, and those that thorin_gpu_create allocates for the disk. */
+int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, long long *need, long long *held);
+
 /* Self-test of the conditional CUDA graph nodes behind the SOR sweep loop:
  * a kernel that sets an IF node's condition to 0 must skip its body
  * (*if_zero = 0) and to 1 run it once (*if_one = 1); only then a WHILE node
