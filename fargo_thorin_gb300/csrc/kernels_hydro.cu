@@ -2036,9 +2036,9 @@ int hydro_sor_grid_fits(const DevGrid &g, int maxiters)
   return n * sms >= q.nb;
 }
 
-void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
-                    const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                    void *x, double eps, int maxiters, int shared, cudaStream_t s)
+cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                           const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                           void *x, double eps, int maxiters, int shared, cudaStream_t s)
 {
   const SorGridShape q = sor_grid_shape(g, shared);
   cudaLaunchConfig_t cfg = {};
@@ -2052,7 +2052,7 @@ void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const SorSystem m = {ml, mlip, mlim, mljp, mljm, rhs, cw};
-  cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res);
+  return cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res);
 }
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)

@@ -165,6 +165,8 @@ struct thorin_disk {
   int graph_npl = -1;                // planets the graph was built for
   int capturing = 0;                 // launches are being captured into the DT graph
   StepDev capS;
+  int one_refused = 0;               // the solve's cooperative launch, or a graph that holds it, was refused
+  int graph_fault = 0;               // THORIN_FAULT_*: failure that the next DT graph's capture meets
   cudaGraph_t capture_sor_body = nullptr;   // body of the SOR loop node, filled after the substep capture
   cudaStream_t s_pl = nullptr;       // the planet step's branch of the substep graph
   double *cap_ptr[11] = {};          // the buffers the DT graph was captured with (graph_roles order)
@@ -1640,10 +1642,18 @@ static int sor_loop_graph(thorin_disk *d)
 }
 
 // The sweeps of a solve as one launch (sor_one).
-static void sor_one_launch(thorin_disk *d)
+static int sor_one_launch(thorin_disk *d)
 {
-  hydro_sor_grid(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs, d->sor_cw, d->sor, d->sor_x,
-                 d->p.sor_eps, d->p.sor_maxiters, d->sor_shared, d->s);
+  const bool fake = d->capturing && d->graph_fault == THORIN_FAULT_SOLVE_REFUSED;
+  const cudaError_t e = fake ? cudaErrorNotSupported
+                             : hydro_sor_grid(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs,
+                                              d->sor_cw, d->sor, d->sor_x, d->p.sor_eps, d->p.sor_maxiters,
+                                              d->sor_shared, d->s);
+  if (e == cudaSuccess) return THORIN_OK;
+  cudaGetLastError();
+  g_last_error = std::string("cooperative launch of the SOR solve: ") + cudaGetErrorString(e);
+  d->one_refused = 1;
+  return THORIN_ERR_CUDA;
 }
 
 // SuccessiveOverrelaxation driver: the start residual (and the learned warm
@@ -1690,7 +1700,7 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
     }
   } else {
     if (d->sor_one) {
-      sor_one_launch(d);
+      RCHK(sor_one_launch(d));
     } else {
       RCHK(sor_loop_graph(d));
       CUCHK(cudaGraphLaunch(d->sor_loop, d->s));
@@ -2290,7 +2300,7 @@ static int capture_sor(thorin_disk *d)
                           d->ws_vq, d->ws_part, d->ws_step, d->g.nsm, d->s));
   }
   if (d->sor_one) {
-    sor_one_launch(d);
+    RCHK(sor_one_launch(d));
   } else {
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg;
@@ -2370,14 +2380,22 @@ static int capture_substep(thorin_disk *d)
   // the hydro substep, with the buffers' roles restored at the end
   double *const f0[5] = {d->rho, d->vrad, d->vtheta, d->energy, d->pdens};
   double *const sc0[6] = {d->vrad_new, d->vtheta_new, d->energy_new, d->t_rho_gas, d->t_e_gas, d->t_rho_peb};
-  const int rc = thorin_gpu_hydro(d, 0.0);
+  int rc = thorin_gpu_hydro(d, 0.0);
   double *f1[5] = {d->rho, d->vrad, d->vtheta, d->energy, d->pdens};
-  const size_t bytes = d->fsize * sizeof(double);
-  for (int q = 0; q < 5; q++)
-    if (f1[q] && f1[q] != f0[q]) CUCHK(cudaMemcpyAsync(f0[q], f1[q], bytes, cudaMemcpyDeviceToDevice, d->s));
+  // whatever fails, the buffers have their roles back
   d->rho = f0[0]; d->vrad = f0[1]; d->vtheta = f0[2]; d->energy = f0[3]; d->pdens = f0[4];
   d->vrad_new = sc0[0]; d->vtheta_new = sc0[1]; d->energy_new = sc0[2];
   d->t_rho_gas = sc0[3]; d->t_e_gas = sc0[4]; d->t_rho_peb = sc0[5];
+  const size_t bytes = d->fsize * sizeof(double);
+  for (int q = 0; q < 5 && rc == THORIN_OK; q++) {
+    if (!f1[q] || f1[q] == f0[q]) continue;
+    const cudaError_t e = (d->graph_fault == THORIN_FAULT_COPY) ? cudaErrorUnknown
+                          : cudaMemcpyAsync(f0[q], f1[q], bytes, cudaMemcpyDeviceToDevice, d->s);
+    if (e != cudaSuccess) {
+      g_last_error = std::string("device-resident DT, state back into its buffers: ") + cudaGetErrorString(e);
+      rc = THORIN_ERR_CUDA;
+    }
+  }
   CUCHK(cudaStreamWaitEvent(d->s, d->ev_pl_join, 0));
   if (rc != THORIN_OK) return rc;
   graph_sub_end(S, d->s);
@@ -2483,7 +2501,10 @@ static int capture_dt_graph(thorin_disk *d, int npl)
     cudaGraph_t tmp;
     e = cudaStreamEndCapture(d->s, &tmp);
   }
-  if (e == cudaSuccess && rc == THORIN_OK) e = cudaGraphInstantiate(&exec, G, 0);
+  if (e == cudaSuccess && rc == THORIN_OK) {
+    e = cudaGraphInstantiate(&exec, G, 0);
+    if (e != cudaSuccess && d->sor_one) d->one_refused = 1;
+  }
   if (G) cudaGraphDestroy(G);
   cudaGetLastError();
   if (rc != THORIN_OK) return rc;
@@ -2499,18 +2520,32 @@ static int capture_dt_graph(thorin_disk *d, int npl)
   return THORIN_OK;
 }
 
+// Where the solve's cooperative launch is refused (a conditional node's body
+// takes none under MPS: the launch or the graph's instantiation fails), the
+// launches of the passes take its place.  Any other failure is the caller's.
 static int build_dt_graph(thorin_disk *d, int npl)
 {
+  d->one_refused = 0;
   int rc = capture_dt_graph(d, npl);
-  if (rc != THORIN_OK && d->sor_one) {
-    // a conditional node's body takes no cooperative launch under MPS: the
-    // launches of the passes instead
+  if (rc != THORIN_OK && d->one_refused) {
+    const std::string first = g_last_error;
     const int one = d->sor_one;
     d->sor_one = 0;
     rc = capture_dt_graph(d, npl);
     d->sor_one = one;
+    if (rc != THORIN_OK) g_last_error = first + "; with launched sweeps: " + g_last_error;
   }
+  d->graph_fault = 0;
   return rc;
+}
+
+extern "C" int thorin_selftest_graph_fault(thorin_disk *d, int fault)
+{
+  if (!d || fault < 0 || fault > THORIN_FAULT_COPY) return THORIN_ERR_ARG;
+  CUCHK(cudaStreamSynchronize(d->s));
+  if (d->dt_graph) { cudaGraphExecDestroy(d->dt_graph); d->dt_graph = nullptr; }
+  d->graph_fault = fault;
+  return THORIN_OK;
 }
 
 // Uploads what the graph reads (planets, clock, frame, omega schedule) and

@@ -265,9 +265,9 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
 // the GPU.
 #define SOR_GRID_RECORDS 1024
 int hydro_sor_grid_fits(const DevGrid &g, int maxiters);
-void hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
-                    const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                    void *x, double eps, int maxiters, int shared, cudaStream_t s);
+cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
+                           const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
+                           void *x, double eps, int maxiters, int shared, cudaStream_t s);
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s);
 void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
                      double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,

@@ -442,6 +442,15 @@ int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_expone
  * multiprocessors, and those that thorin_gpu_create allocates for the disk. */
 int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, long long *need, long long *held);
 
+/* Failures of a DT graph's capture, by faked return codes of host calls: the
+ * disk's DT graph is dropped and its next build meets the fault once.  The
+ * solve's cooperative launch refused: the graph is built with launched sweeps.
+ * A copy of the state refused: thorin_gpu_algogas_graph returns
+ * THORIN_ERR_CUDA, and the disk is as it was. */
+#define THORIN_FAULT_SOLVE_REFUSED 1
+#define THORIN_FAULT_COPY          2
+int thorin_selftest_graph_fault(thorin_disk *d, int fault);
+
 /* Self-test of the conditional CUDA graph nodes behind the SOR sweep loop:
  * a kernel that sets an IF node's condition to 0 must skip its body
  * (*if_zero = 0) and to 1 run it once (*if_one = 1); only then a WHILE node
