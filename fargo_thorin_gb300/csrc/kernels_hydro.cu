@@ -470,6 +470,7 @@ __device__ double opacity_BL94(double vd, double rho2cgs, double T)
       else grains = (T <= TEMPB(2, 3));
     } else {
       grains = (T <= TEMPB(2, 3));
+      if (grains && T < 0.0) return sqrt(T);                 // not a number, as the reference's T^(1/2)
     }
   }
   double k;
