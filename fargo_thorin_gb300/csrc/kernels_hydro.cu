@@ -764,9 +764,10 @@ __global__ void __launch_bounds__(BX) k_diffcoef(DevGrid g, DiffusionIO io)
     // DiffusionTimestep's min of deltar2 / D: deltar2 is a ring constant and
     // correctly rounded division is monotone, so for D > 0 the minimum of a
     // ring is deltar2 / max D; other D (which only a crashed state holds) are
-    // divided cell by cell as the reference does
+    // divided cell by cell as the reference does (a D that is not a number
+    // counts for nothing, and must not hide the ring's others)
     unsigned hi = (unsigned)__double2hiint(D), lo = (unsigned)__double2loint(D);
-    if (!(__double_as_longlong(D) > 0LL)) {
+    if ((unsigned long long)__double_as_longlong(D) - 1ULL >= 0x7ff0000000000000ULL) {
       hi = lo = 0u;
       const double t = div_fast(R.deltar2, D);
       if (in && t < dtl) dtl = t;

@@ -1,6 +1,7 @@
 """A cell whose energy has turned negative (the crash test of a disk with
-pebbles looks at their density alone) shows in the opacity, as in the reference: T^(1/2) of the
-Bell & Lin grains is not a number there."""
+pebbles looks at their density alone) shows in the opacity and is left out of
+the diffusion time step, as in the reference: T^(1/2) of the Bell & Lin grains
+is not a number there, and no comparison with it holds."""
 import numpy as np
 import pytest
 
@@ -10,6 +11,8 @@ from fargo_thorin_gb300 import workloads
 
 pytestmark = pytest.mark.gpu
 NR, NS = 16, 96
+T2SI = 1.32712440018e20 / (8.3144598 / (2.4 * 0.001)) / 149597870700.0       # K of a code unit
+UT = (149597870700.0 ** 3 / 1.32712440018e20) ** 0.5                          # s of a code unit
 
 
 def _step(cells):
@@ -48,3 +51,42 @@ def test_opacity_of_a_negative_temperature():
         # the tolerance of the oracle comparisons (test_gpu_parity)
         assert H.rel_l2(a[~bad], b[~bad]) < 1e-11, f
     d.close()
+
+
+@pytest.mark.parametrize("factor", [-1.0, np.nan])
+def test_diffusion_time_step_without_the_cells_that_are_not_numbers(factor):
+    """DiffusionTimestep's minimum over the other cells, whichever ring the bad
+    one lies in: dr^2 / (2 D) restated from the state (FluxLimiterValue and
+    DiffusionCoefs, EnergySources.c:556-605, 684-696, 833-856).  One short
+    hydro substep; what it changes of the state is of order 1e-9."""
+    from fargo_thorin_gb300 import _lib
+    from fargo_thorin_gb300.disk import GpuDisk
+    p = workloads.params_for("disk1", NR, NS)
+    p.sor_maxiters = 5
+    sig = 5.670367e-8 / 1.98855e30 * UT ** 3 * T2SI ** 4
+    for i in range(NR):
+        d = GpuDisk(p)
+        d.init_default()
+        H.start_state(d, p, {"dens": d.get(0), "temper": d.get(8)})
+        rho, e = (np.array(d.get(H.FIELD_IDS[f])[:NR * NS]).reshape(NR, NS) for f in ("dens", "energy"))
+        e[i, 37] *= factor
+        d.set(H.FIELD_IDS["energy"], e)
+        d.set_sor_state(1.0, 1e-3, 50)
+        _lib.check(d.L.thorin_gpu_stokes(d.h), "stokes")
+        _lib.check(d.L.thorin_gpu_hydro(d.h, 1.0e-9), "hydro", ok=(0, 4))
+        T = e * (p.adiabind - 1.0) / rho
+        rin, rout, rmed, _ = (np.asarray(a)[:, None] for a in d.rings())
+        kap = np.asarray(d.get(H.FIELD_IDS["opacity"])[:NR * NS]).reshape(NR, NS)
+        fac = np.sqrt(2.0 * np.pi) * np.sqrt(np.abs(T)) * rmed ** 1.5 / (rho * kap)
+        gr = np.vstack([np.zeros((1, NS)), np.diff(T, axis=0) / np.diff(rmed, axis=0)])
+        gt = (T - np.roll(T, 1, axis=1)) / (2.0 * np.pi / NS * rmed)
+        grad = np.zeros((NR, NS))
+        grad[1:-1] = np.hypot(0.5 * (gr[2:] + gr[1:-1]), 0.5 * (np.roll(gt, -1, axis=1) + gt)[1:-1])
+        grad[0], grad[-1] = grad[1], grad[-2]
+        s = 4.0 * grad * fac / T
+        lim = np.where(s <= 2.0, 2.0 / (3.0 + np.sqrt(9.0 + 10.0 * s * s)),
+                       10.0 / (10.0 * s + 9.0 + np.sqrt(np.abs(81.0 + 180.0 * s))))
+        dt = 0.5 * (rout - rin) ** 2 / (lim * 16.0 * sig * T ** 3 * fac)
+        assert np.isnan(dt[i, 37])
+        assert abs(d.dt_stellar() / np.nanmin(dt) - 1.0) < 1e-6, i
+        d.close()
