@@ -50,7 +50,7 @@ static int chunk_rings(int nr, int ns, int nsm, int most, double extra, int slot
 // (pressure, half of the velocity average, the pebble-to-gas ratio); quotients
 // by the same sums of densities share a reciprocal; the difference of the
 // ratios of two columns is one quotient.  FP64-bound: about 30 FP64
-// instructions a cell for the gas (40 before) and 97 with pebbles (135 in three
+// instructions a cell for the gas (40 before) and 98 with pebbles (135 in three
 // kernels).  512x1536: 161 us, 213 us in three kernels.
 #define SRC_MAXRINGS 24
 
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(BX) k_sources(DevGrid g, SourceIO io)
 {
   pdl_wait();
   __shared__ SrcRing ring[SRC_MAXRINGS];
-  __shared__ double tab[64];
+  __shared__ double tab[128];
   const double dt = g.ctl[CTL_DT];
   const int ns = g.ns, nr = g.nr;
   const int i0 = blockIdx.y * io.rings, i1 = min(i0 + io.rings, nr);
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(BX) k_sources(DevGrid g, SourceIO io)
       R.ct = div_fast(-g.r.nu_med[i], io.schmidt) * io.invdxtheta[i];
     }
   }
-  if (PEB && threadIdx.x >= 64) tab[threadIdx.x - 64] = c_exp64[threadIdx.x - 64];
+  if (PEB) tab[threadIdx.x] = c_exp64[threadIdx.x];
   __syncthreads();
   const int j = blockIdx.x * BX + threadIdx.x;
   if (j >= ns) return;

@@ -518,9 +518,12 @@ __device__ __forceinline__ double unit_quotient(double r)
 // exp(x) by table (P. T. P. Tang, ACM Trans. Math. Softw. 15(2):144-157,
 // 1989): n the integer nearest 64 x / ln 2, r = x - n ln 2 / 64 in two steps,
 // exp(x) = 2^(n div 64) 2^((n mod 64)/64) (1 + (r + r^2 (1/2 + r/6 + t))) with
-// the tail t = r^2/24 + r^3/120 + r^4/720, below 1.3e-6, in FP32.  Eight FP64
-// instructions.  tab: exp_table's 64 powers of 2^(1/64), in shared memory.
-__constant__ double c_exp64[64] = {
+// the tail t = r^2/24 + r^3/120 + r^4/720, below 1.3e-6, in FP32.  The powers of
+// 2^(1/64) are rounded values and their remainders (c_exp64, copied to shared
+// memory: tab): with the rounded ones alone, an FP64 instruction less, the
+// largest error was 1.02 ulp, and CUDA's exp has 0.87; with both it is 0.56.
+// Nine FP64 instructions.
+__constant__ double c_exp64[128] = {
     1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
     1.0442737824274138, 1.0556451783605572, 1.0671404006768237, 1.0787607977571199,
     1.0905077326652577, 1.102382583307841, 1.1143867425958924, 1.1265216186082418,
@@ -536,7 +539,23 @@ __constant__ double c_exp64[64] = {
     1.681792830507429, 1.7001063537185235, 1.718619298122478, 1.7373338352737062,
     1.7562521603732995, 1.7753764925265212, 1.7947090750031072, 1.8142521755003989,
     1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
-    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
+    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951,
+    0.0, -1.5234778603368577e-17, 5.109225028973444e-17, 7.600838874027088e-18,
+    8.551889705537965e-17, 1.759325738772092e-18, -7.899853966841582e-17, -6.656660436056593e-17,
+    -3.046782079812471e-17, 5.2660368715706944e-17, 1.0410278456845571e-16, 5.165856758795457e-17,
+    8.912812676025408e-17, 3.250710218863827e-17, 3.8292048369240935e-17, 5.554203254218079e-17,
+    3.982015231465646e-17, 6.644981499252301e-17, -7.712630692681488e-17, -1.89878163130253e-17,
+    4.658027591836937e-17, -6.7113898212968784e-18, 2.667932131342186e-18, 1.713594918243561e-17,
+    2.5382502794888315e-17, -7.181536135519454e-17, -2.8587312100388614e-17, 8.927282594831732e-17,
+    7.70094837980299e-17, 9.593797919118849e-17, -6.770511658794786e-17, -9.614213209051323e-17,
+    -9.667293313452913e-17, -1.2031642489053655e-17, -3.0237581349939873e-17, -5.600377186075216e-17,
+    -3.483994556892796e-17, 1.4192920154284036e-17, -1.016455327754295e-16, -1.1024941712342561e-16,
+    7.949834809697621e-17, 3.7812070533575275e-17, -1.0136916471278304e-17, -1.0094406542311964e-16,
+    2.4707192569797888e-17, -6.712955084707084e-17, -1.0125679913674773e-16, 5.8909926967131e-17,
+    8.199010020581497e-17, -8.0237193703977e-18, -1.851380418263111e-17, 3.164389299292957e-17,
+    2.960140695448873e-17, 6.429731796556572e-17, 1.8227458427912087e-17, -9.969531538920349e-17,
+    3.283107224245627e-17, 9.761887490727594e-17, -6.122763413004143e-17, 3.4034035352165297e-17,
+    -1.0619946056195963e-16, 1.0332385960676326e-16, 8.960767791036668e-17, 4.0388753109278167e-17};
 
 __device__ __forceinline__ double float_to_double(float f)
 {
@@ -568,7 +587,7 @@ __device__ __forceinline__ double exp_fast(double x, const double *tab)
     const double q = __fma_rn(r, 0.16666666666666666, 0.5) + float_to_double(t);
     const double e = __fma_rn(r * r, q, r);
     const double T = tab[n & 63];
-    const double y = __fma_rn(T, e, T);
+    const double y = T + __fma_rn(T, e, tab[64 + (n & 63)]);
     return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
   }
   return exp(x);

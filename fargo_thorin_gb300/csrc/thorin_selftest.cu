@@ -333,8 +333,8 @@ extern "C" int thorin_selftest_slope_division(long long n, unsigned long long se
 __global__ void k_selftest_exp(long long n, unsigned long long seed, double range, double emax,
                                unsigned long long *__restrict__ out)
 {
-  __shared__ double tab[64];
-  if (threadIdx.x < 64) tab[threadIdx.x] = c_exp64[threadIdx.x];
+  __shared__ double tab[128];
+  if (threadIdx.x < 128) tab[threadIdx.x] = c_exp64[threadIdx.x];
   __syncthreads();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -372,6 +372,43 @@ extern "C" int thorin_selftest_exp(long long n, unsigned long long seed, double 
   }
   *max_ulp_exp = host[0];
   *max_ulp_pow = host[1];
+  return THORIN_OK;
+}
+
+// exp_fast and exp of n values.
+__global__ void k_selftest_exp_values(int n, const double *__restrict__ x, double *__restrict__ fast,
+                                      double *__restrict__ cuda)
+{
+  __shared__ double tab[128];
+  if (threadIdx.x < 128) tab[threadIdx.x] = c_exp64[threadIdx.x];
+  __syncthreads();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  fast[t] = exp_fast(x[t], tab);
+  cuda[t] = exp(x[t]);
+}
+
+extern "C" int thorin_selftest_exp_values(int n, const double *x, double *fast, double *cuda)
+{
+  if (n < 1 || n > (1 << 28) || !x || !fast || !cuda) {
+    g_last_error = "selftest_exp_values: 1 <= n <= 2^28 and array pointers required";
+    return THORIN_ERR_ARG;
+  }
+  double *dev = nullptr;
+  const size_t bytes = (size_t)n * sizeof(double);
+  cudaError_t e = cudaMalloc((void **)&dev, 3 * bytes);
+  if (e == cudaSuccess) e = cudaMemcpy(dev, x, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_selftest_exp_values<<<(n + 255) / 256, 256>>>(n, dev, dev + n, dev + 2 * (size_t)n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(fast, dev + n, bytes, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(cuda, dev + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+  if (dev) cudaFree(dev);
+  if (e != cudaSuccess) {
+    g_last_error = std::string("selftest_exp_values: ") + cudaGetErrorString(e);
+    return THORIN_ERR_CUDA;
+  }
   return THORIN_OK;
 }
 

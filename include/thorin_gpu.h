@@ -431,6 +431,9 @@ int thorin_selftest_vl_slope(long long n, unsigned long long seed, double max_ex
 int thorin_selftest_exp(long long n, unsigned long long seed, double range, double max_exponent,
                         unsigned long long *max_ulp_exp, unsigned long long *max_ulp_pow);
 
+/* The kernels' exponential and CUDA's exp of n host values, to host arrays. */
+int thorin_selftest_exp_values(int n, const double *x, double *fast, double *cuda);
+
 /* Compares the kernels' square root routine with IEEE square root on n
  * random operands (exponents in [-max_exponent, max_exponent]): results that
  * differ and the largest distance in ulp (0: none). */
