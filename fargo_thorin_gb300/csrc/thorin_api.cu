@@ -156,20 +156,23 @@ struct thorin_disk {
   // device-resident DT (thorin_gpu_algogas_graph): the instantiated graph of
   // one DT, the planets and counters it keeps on the device, and the state
   // of the capture that builds it
-  cudaGraphExec_t dt_graph = nullptr;
+  // DT graphs: of a disk advanced alone, and beside others (sor_shared is part of
+  // the captured solve's launch)
+  cudaGraphExec_t dt_graph[2] = {nullptr, nullptr};
   thorin_planets *sys_d = nullptr, *sys_h = nullptr;   // device copy, pinned staging copy
   GraphStats *gst_d = nullptr, *gst_h = nullptr;
   int *ring_info_d = nullptr;
   AccArgs *acc_args_g = nullptr;     // the graph's own accretion arguments (its buffers' pointers)
   double *ctl_h = nullptr;           // pinned staging of the control block
-  int graph_npl = -1;                // planets the graph was built for
+  int graph_npl[2] = {-1, -1};       // planets the graphs were built for
+  int graph_builds[2] = {0, 0};      // times each was built
   int capturing = 0;                 // launches are being captured into the DT graph
   StepDev capS;
   int one_refused = 0;               // the solve's cooperative launch, or a graph that holds it, was refused
   int graph_fault = 0;               // THORIN_FAULT_*: failure that the next DT graph's capture meets
   cudaGraph_t capture_sor_body = nullptr;   // body of the SOR loop node, filled after the substep capture
   cudaStream_t s_pl = nullptr;       // the planet step's branch of the substep graph
-  double *cap_ptr[11] = {};          // the buffers the DT graph was captured with (graph_roles order)
+  double *cap_ptr[11] = {};          // the buffers the DT graphs were captured with (graph_roles order)
   cudaEvent_t ev_pl_fork = nullptr, ev_pl_join = nullptr;
   AccArgs *acc_args_d;               // pebble accretion arguments on the device
   SorCtl sor;
@@ -622,6 +625,14 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   return THORIN_OK;
 }
 
+static void drop_dt_graphs(thorin_disk *d)
+{
+  for (cudaGraphExec_t &g : d->dt_graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 // Update history of the warm start with at least nh slots (zeroed, no time
 // step recorded); a larger history replaces the old one.
 static int ws_history(thorin_disk *d, int nh)
@@ -640,10 +651,7 @@ static int ws_history(thorin_disk *d, int nh)
     cudaFree(d->ws_prev);
     d->ws_prev = nullptr;
   }
-  if (d->dt_graph) {                               // the DT graph holds the old history's address
-    cudaGraphExecDestroy(d->dt_graph);
-    d->dt_graph = nullptr;
-  }
+  drop_dt_graphs(d);                               // they hold the old history's address
   RCHK(dalloc(d, (void **)&d->ws_prev, (size_t)nh * cells * sizeof(double)));
   CUCHK(cudaMemsetAsync(d->ws_dts, 0, THORIN_WS_MAX_ORDER * sizeof(double), d->s));
   d->ws_nh = nh;
@@ -677,10 +685,7 @@ extern "C" int thorin_gpu_warmstart(thorin_disk *d, thorin_warmnet *n, int mode,
   if (d->ws_dts)                                   // every attach starts without recorded updates
     CUCHK(cudaMemsetAsync(d->ws_dts, 0, THORIN_WS_MAX_ORDER * sizeof(double), d->s));
   d->ws_f = f;
-  if (d->dt_graph && (d->ws_net != n || d->ws_mode != mode)) {
-    cudaGraphExecDestroy(d->dt_graph);            // the DT graph holds the warm start's launches or not
-    d->dt_graph = nullptr;
-  }
+  if (d->ws_net != n || d->ws_mode != mode) drop_dt_graphs(d);   // they hold the warm start's launches or not
   d->ws_net = n;
   d->ws_mode = mode;
   d->ws_lr = lr;
@@ -696,10 +701,7 @@ extern "C" int thorin_gpu_warmstart_order(thorin_disk *d, int order)
   if (order == d->ws_order) return THORIN_OK;
   d->ws_order = order;
   if (d->ws_mode == THORIN_WS_EXTRAPOLATE) RCHK(ws_history(d, order));
-  if (d->dt_graph) {                               // the order is baked into the DT graph's launch
-    cudaGraphExecDestroy(d->dt_graph);
-    d->dt_graph = nullptr;
-  }
+  drop_dt_graphs(d);                               // the order is baked into their launches
   return THORIN_OK;
 }
 
@@ -729,7 +731,7 @@ extern "C" int thorin_gpu_destroy(thorin_disk *d)
   cudaFreeHost(d->csmean_h);
   if (d->nshift_h) cudaFreeHost(d->nshift_h);
   if (d->sor_loop) cudaGraphExecDestroy(d->sor_loop);
-  if (d->dt_graph) cudaGraphExecDestroy(d->dt_graph);
+  drop_dt_graphs(d);
   if (d->sys_h) cudaFreeHost(d->sys_h);
   if (d->gst_h) cudaFreeHost(d->gst_h);
   if (d->ctl_h) cudaFreeHost(d->ctl_h);
@@ -2428,10 +2430,10 @@ static const char *graph_unsupported(const thorin_disk *d, const thorin_planets 
   return nullptr;
 }
 
-static int capture_dt_graph(thorin_disk *d, int npl)
+static int capture_dt_graph(thorin_disk *d, int npl, int slot)
 {
   const thorin_params &p = d->p;
-  if (d->dt_graph) { cudaGraphExecDestroy(d->dt_graph); d->dt_graph = nullptr; }
+  if (d->dt_graph[slot]) { cudaGraphExecDestroy(d->dt_graph[slot]); d->dt_graph[slot] = nullptr; }
   if (!d->sys_d) {
     RCHK(dalloc(d, (void **)&d->sys_d, sizeof(thorin_planets)));
     RCHK(dalloc(d, (void **)&d->gst_d, sizeof(GraphStats)));
@@ -2512,8 +2514,9 @@ static int capture_dt_graph(thorin_disk *d, int npl)
     g_last_error = std::string("device-resident DT graph: ") + cudaGetErrorString(e);
     return THORIN_ERR_CUDA;
   }
-  d->dt_graph = exec;
-  d->graph_npl = npl;
+  d->dt_graph[slot] = exec;
+  d->graph_npl[slot] = npl;
+  d->graph_builds[slot]++;
   double **roles[11];
   graph_roles(d, roles);
   for (int k = 0; k < 11; k++) d->cap_ptr[k] = *roles[k];
@@ -2523,15 +2526,15 @@ static int capture_dt_graph(thorin_disk *d, int npl)
 // Where the solve's cooperative launch is refused (a conditional node's body
 // takes none under MPS: the launch or the graph's instantiation fails), the
 // launches of the passes take its place.  Any other failure is the caller's.
-static int build_dt_graph(thorin_disk *d, int npl)
+static int build_dt_graph(thorin_disk *d, int npl, int slot)
 {
   d->one_refused = 0;
-  int rc = capture_dt_graph(d, npl);
+  int rc = capture_dt_graph(d, npl, slot);
   if (rc != THORIN_OK && d->one_refused) {
     const std::string first = g_last_error;
     const int one = d->sor_one;
     d->sor_one = 0;
-    rc = capture_dt_graph(d, npl);
+    rc = capture_dt_graph(d, npl, slot);
     d->sor_one = one;
     if (rc != THORIN_OK) g_last_error = first + "; with launched sweeps: " + g_last_error;
   }
@@ -2539,11 +2542,19 @@ static int build_dt_graph(thorin_disk *d, int npl)
   return rc;
 }
 
+extern "C" int thorin_selftest_graph_builds(thorin_disk *d, int *alone, int *beside)
+{
+  if (!d || !alone || !beside) return THORIN_ERR_ARG;
+  *alone = d->graph_builds[0];
+  *beside = d->graph_builds[1];
+  return THORIN_OK;
+}
+
 extern "C" int thorin_selftest_graph_fault(thorin_disk *d, int fault)
 {
   if (!d || fault < 0 || fault > THORIN_FAULT_COPY) return THORIN_ERR_ARG;
   CUCHK(cudaStreamSynchronize(d->s));
-  if (d->dt_graph) { cudaGraphExecDestroy(d->dt_graph); d->dt_graph = nullptr; }
+  drop_dt_graphs(d);
   d->graph_fault = fault;
   return THORIN_OK;
 }
@@ -2552,18 +2563,21 @@ extern "C" int thorin_selftest_graph_fault(thorin_disk *d, int fault)
 // launches one DT on the disk's stream; thorin_gpu_graph_finish reads back.
 static int graph_launch(thorin_disk *d, const thorin_planets *sys)
 {
-  if (!d->dt_graph || d->graph_npl != sys->nb) RCHK(build_dt_graph(d, sys->nb));
   // the host path swaps buffers between the state fields and their scratch
-  // partners; the graph reads the buffers it was captured with, so the state
+  // partners; the graphs read the buffers they were captured with, so the state
   // goes back into those first (each field's buffers are its own, so no copy
-  // overwrites another field)
-  double **roles[11];
-  graph_roles(d, roles);
-  const size_t bytes = d->fsize * sizeof(double);
-  for (int k = 0; k < 5; k++)
-    if (*roles[k] && *roles[k] != d->cap_ptr[k])
-      CUCHK(cudaMemcpyAsync(d->cap_ptr[k], *roles[k], bytes, cudaMemcpyDeviceToDevice, d->s));
-  for (int k = 0; k < 11; k++) *roles[k] = d->cap_ptr[k];
+  // overwrites another field), also before a second graph is captured
+  if (d->dt_graph[0] || d->dt_graph[1]) {
+    double **roles[11];
+    graph_roles(d, roles);
+    const size_t bytes = d->fsize * sizeof(double);
+    for (int k = 0; k < 5; k++)
+      if (*roles[k] && *roles[k] != d->cap_ptr[k])
+        CUCHK(cudaMemcpyAsync(d->cap_ptr[k], *roles[k], bytes, cudaMemcpyDeviceToDevice, d->s));
+    for (int k = 0; k < 11; k++) *roles[k] = d->cap_ptr[k];
+  }
+  const int slot = d->sor_one && d->sor_shared;
+  if (!d->dt_graph[slot] || d->graph_npl[slot] != sys->nb) RCHK(build_dt_graph(d, sys->nb, slot));
   *d->sys_h = *sys;
   CUCHK(cudaMemcpyAsync(d->sys_d, d->sys_h, sizeof(thorin_planets), cudaMemcpyHostToDevice, d->s));
   set_ctl(d, {{CTL_TIME, d->PhysicalTime}, {CTL_OMEGA_FRAME, d->OmegaFrame}, {CTL_SOR_OMEGA, d->omega},
@@ -2571,7 +2585,7 @@ static int graph_launch(thorin_disk *d, const thorin_planets *sys)
   d->gst_h->niterlast = d->Niterlast;
   CUCHK(cudaMemcpyAsync(&d->gst_d->niterlast, &d->gst_h->niterlast, sizeof(int), cudaMemcpyHostToDevice, d->s));
   if (d->timing) CUCHK(cudaEventRecord(d->ev[2], d->s));
-  CUCHK(cudaGraphLaunch(d->dt_graph, d->s));
+  CUCHK(cudaGraphLaunch(d->dt_graph[slot], d->s));
   if (d->timing) CUCHK(cudaEventRecord(d->ev[3], d->s));
   CUCHK(cudaMemcpyAsync(d->sys_h, d->sys_d, sizeof(thorin_planets), cudaMemcpyDeviceToHost, d->s));
   CUCHK(cudaMemcpyAsync(d->gst_h, d->gst_d, sizeof(GraphStats), cudaMemcpyDeviceToHost, d->s));
@@ -2623,7 +2637,7 @@ extern "C" int thorin_gpu_set_launch_shape(thorin_disk *d, int sor_loop_sweeps, 
   d->sor_loop_k = sor_loop_sweeps;
   d->g.sor_tpsm = sor_threads_per_sm;
   if (d->sor_loop) { cudaGraphExecDestroy(d->sor_loop); d->sor_loop = nullptr; }
-  if (d->dt_graph) { cudaGraphExecDestroy(d->dt_graph); d->dt_graph = nullptr; }
+  drop_dt_graphs(d);
   return THORIN_OK;
 }
 
@@ -2672,7 +2686,7 @@ extern "C" int thorin_ensemble_algogas_graph(thorin_disk **disks, thorin_planets
   std::vector<int> launched(n, 0);
   for (int k = 0; k < n; k++) {
     thorin_disk *d = disks[k];
-    thorin_disk_share(d, n > 1);                   // for the graph if it is built now
+    thorin_disk_share(d, n > 1);                   // picks the graph
     int rc = thorin_gpu_graph_supported(d, systems[k]);
     if (rc == THORIN_OK && graph_host_dt(d)) rc = thorin_gpu_algogas(d, systems[k]);
     else if (rc == THORIN_OK) { rc = graph_launch(d, systems[k]); launched[k] = (rc == THORIN_OK); }

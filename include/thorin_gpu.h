@@ -306,7 +306,9 @@ int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys);
  * boundaries and opacity laws; other options are rejected with
  * THORIN_ERR_ARG (thorin_gpu_graph_supported says which).  No torque log
  * records are made.  The graph is built at the first call for the current
- * number of planets. */
+ * number of planets; a disk that is also advanced beside others
+ * (thorin_ensemble_algogas_graph) keeps a second one for that, whose solves
+ * leave them room. */
 int thorin_gpu_algogas_graph(thorin_disk *d, thorin_planets *sys);
 
 /* THORIN_OK if thorin_gpu_algogas_graph covers this disk and system, else
@@ -453,6 +455,10 @@ int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, long long *ne
 #define THORIN_FAULT_SOLVE_REFUSED 1
 #define THORIN_FAULT_COPY          2
 int thorin_selftest_graph_fault(thorin_disk *d, int fault);
+
+/* How often a disk's DT graphs were built: the one it is advanced with alone
+ * and the one for thorin_ensemble_algogas_graph with other disks. */
+int thorin_selftest_graph_builds(thorin_disk *d, int *alone, int *beside);
 
 /* Self-test of the conditional CUDA graph nodes behind the SOR sweep loop:
  * a kernel that sets an IF node's condition to 0 must skip its body
