@@ -526,8 +526,6 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   d->sor.niter = ip + 1;
   d->sor.changed = ip + 2;
   d->sor.abort = ip + 3;
-  CUCHK(cudaMemset(sp, 0, 8 * sizeof(double)));
-  CUCHK(cudaMemset(ip, 0, 8 * sizeof(int)));
   d->sor.ticket = d->ticket;
   d->sor.cond = 0;
   d->sor.has_cond = 0;
@@ -537,11 +535,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   }
   if (const char *ed = getenv("THORIN_SOR_DIRECT")) d->sor_direct = (atoi(ed) != 0);
   d->sor_one = !d->sor_direct && hydro_sor_grid_fits(d->g, d->p.sor_maxiters);
-  if (d->sor_one) {
-    const size_t bytes = 16 * (2 * (size_t)(d->nr - 2) * d->ns + SOR_GRID_RECORDS);
-    RCHK(dalloc(d, &d->sor_x, bytes));
-    CUCHK(cudaMemset(d->sor_x, 0, bytes));
-  }
+  if (d->sor_one) RCHK(dalloc(d, &d->sor_x, 16 * (2 * (size_t)(d->nr - 2) * d->ns + SOR_GRID_RECORDS)));
   fill_rings(d);
   {
     PlConst &c = d->plc;                 // constants of the planet side of a substep
