@@ -534,7 +534,8 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
     if (k >= 1 && k <= 64) d->sor_loop_k = k;
   }
   if (const char *ed = getenv("THORIN_SOR_DIRECT")) d->sor_direct = (atoi(ed) != 0);
-  d->sor_one = !d->sor_direct && hydro_sor_grid_fits(d->g, d->p.sor_maxiters);
+  const char *es = getenv("THORIN_SOR_PASSES");     // sweeps as launches, in the WHILE nodes, on any disk
+  d->sor_one = !d->sor_direct && !(es && atoi(es) != 0) && hydro_sor_grid_fits(d->g, d->p.sor_maxiters);
   if (d->sor_one) RCHK(dalloc(d, &d->sor_x, 16 * (2 * (size_t)(d->nr - 2) * d->ns + SOR_GRID_RECORDS)));
   fill_rings(d);
   {
