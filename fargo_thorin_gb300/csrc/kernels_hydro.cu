@@ -1952,6 +1952,8 @@ static dim3 sor_grid_pass(const DevGrid &g, bool capped = true)
   return dim3((unsigned)(nblk < wave ? nblk : wave));
 }
 
+int hydro_sor_pass_blocks(const DevGrid &g) { return (int)sor_grid_pass(g).x; }
+
 static dim3 sor_grid_resid(const DevGrid &g)
 {
   return dim3((g.ns + SOR_BX * SOR_CPT - 1) / (SOR_BX * SOR_CPT), g.nr - 2);

@@ -166,6 +166,7 @@ struct thorin_disk {
   double *ctl_h = nullptr;           // pinned staging of the control block
   int graph_npl[2] = {-1, -1};       // planets the graphs were built for
   int graph_builds[2] = {0, 0};      // times each was built
+  int graph_sweeps[2] = {0, 0};      // their solves are launched sweeps
   int capturing = 0;                 // launches are being captured into the DT graph
   StepDev capS;
   int one_refused = 0;               // the solve's cooperative launch, or a graph that holds it, was refused
@@ -2512,6 +2513,7 @@ static int capture_dt_graph(thorin_disk *d, int npl, int slot)
   d->dt_graph[slot] = exec;
   d->graph_npl[slot] = npl;
   d->graph_builds[slot]++;
+  d->graph_sweeps[slot] = loop;
   double **roles[11];
   graph_roles(d, roles);
   for (int k = 0; k < 11; k++) d->cap_ptr[k] = *roles[k];
@@ -2632,7 +2634,23 @@ extern "C" int thorin_gpu_set_launch_shape(thorin_disk *d, int sor_loop_sweeps, 
   d->sor_loop_k = sor_loop_sweeps;
   d->g.sor_tpsm = sor_threads_per_sm;
   if (d->sor_loop) { cudaGraphExecDestroy(d->sor_loop); d->sor_loop = nullptr; }
-  drop_dt_graphs(d);
+  for (int k = 0; k < 2; k++)                       // a solve in one launch has no part in the shape
+    if (d->dt_graph[k] && d->graph_sweeps[k]) {
+      cudaGraphExecDestroy(d->dt_graph[k]);
+      d->dt_graph[k] = nullptr;
+    }
+  return THORIN_OK;
+}
+
+extern "C" int thorin_gpu_sweep_blocks(thorin_disk *d, int sor_threads_per_sm, int *blocks)
+{
+  if (!d || !blocks || sor_threads_per_sm < 128 || sor_threads_per_sm > 2048 || sor_threads_per_sm % 128) {
+    g_last_error = "sweep blocks: 128..2048 SOR threads per SM in steps of 128";
+    return THORIN_ERR_ARG;
+  }
+  DevGrid g = d->g;
+  g.sor_tpsm = sor_threads_per_sm;
+  *blocks = d->sor_one ? 0 : hydro_sor_pass_blocks(g);
   return THORIN_OK;
 }
 

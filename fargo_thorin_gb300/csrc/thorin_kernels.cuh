@@ -249,6 +249,7 @@ void hydro_irradiation(const DevGrid &g, const double *rho, const double *cs, co
 // resid: also the start of the SOR solve (NULL: the matrix alone)
 void hydro_matrix(const DevGrid &g, const MatrixIO &io, const SorCtl *resid, cudaStream_t s);
 int sor_blocks(const DevGrid &g);
+int hydro_sor_pass_blocks(const DevGrid &g);     // blocks of a colour pass
 void hydro_sor_resid0(const DevGrid &g, const double *T, const double *ml, const double *mlip, const double *mlim,
                       const double *mljp, const double *mljm, const double *rhs, double *cw,
                       const SorCtl &c, cudaStream_t s);

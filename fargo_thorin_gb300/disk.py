@@ -99,6 +99,14 @@ class GpuDisk:
         _lib.check(self.L.thorin_gpu_get_launch_shape(self.h, C.byref(a), C.byref(b)), "get_launch_shape")
         return a.value, b.value
 
+    def sweep_launches(self, sor_loop_sweeps: int, sor_threads_per_sm: int):
+        """How a solve's sweeps are launched with a launch shape: (sweeps per
+        run of the loop body, blocks of a colour pass); None where a solve is
+        one launch, whatever the shape."""
+        n = C.c_int()
+        _lib.check(self.L.thorin_gpu_sweep_blocks(self.h, sor_threads_per_sm, C.byref(n)), "sweep_blocks")
+        return (sor_loop_sweeps, n.value) if n.value else None
+
     def integrals(self):
         vals = [C.c_double() for _ in range(5)]
         _lib.check(self.L.thorin_gpu_integrals(self.h, *[C.byref(v) for v in vals]), "integrals")

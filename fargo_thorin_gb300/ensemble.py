@@ -231,6 +231,8 @@ class Ensemble:
         then, in graph mode, the SOR launch shape of each disk size in turn
         (sweeps per run of the sweep loop, resident threads per SM of a
         colour pass), keeping a size's best before the next size is tried.
+        A shape whose launches have been timed is not tried again, so sizes
+        whose solves are one launch have none to try.
         Returns the schedule and the time of every candidate."""
         trials = []
 
@@ -251,7 +253,13 @@ class Ensemble:
                 best, best_t = cand, t
         if best["mode"] == "graph":
             for nr in sorted({d.nr for d in self.disks}, reverse=True):
+                def launches(shape):
+                    return tuple(d.sweep_launches(*shape) for d in self.disks if d.nr == nr)
+                tried = {launches((8, 1536))}               # the default that the mode was timed with
                 for shape in shapes[1:]:
+                    if launches(shape) in tried:
+                        continue
+                    tried.add(launches(shape))
                     cand = {"mode": "graph", "shapes": dict(best["shapes"])}
                     cand["shapes"][nr] = shape
                     t = time_of(cand)

@@ -320,10 +320,14 @@ int thorin_gpu_graph_supported(thorin_disk *d, const thorin_planets *sys);
  * per run of the sweep loop's body (1..64, default 8) and the most resident
  * threads per multiprocessor of a colour pass (128..2048 in steps of 128,
  * default 1536; the kernel holds at most 1024).  Results do not depend on
- * either; the ensemble autotuner picks them per disk size.  The disk's graphs are rebuilt at their next
- * use. */
+ * either; the ensemble autotuner picks them per disk size.  The disk's graphs
+ * that hold sweeps are rebuilt at their next use.  thorin_gpu_sweep_blocks
+ * says how many blocks a colour pass has with that many threads, 0 on a disk
+ * whose solve is one launch: thread counts with the same blocks are the same
+ * launches. */
 int thorin_gpu_set_launch_shape(thorin_disk *d, int sor_loop_sweeps, int sor_threads_per_sm);
 int thorin_gpu_get_launch_shape(thorin_disk *d, int *sor_loop_sweeps, int *sor_threads_per_sm);
+int thorin_gpu_sweep_blocks(thorin_disk *d, int sor_threads_per_sm, int *blocks);
 
 /* Conservation integrals (SideEuler.c:26-80,523-565), summed on the device. */
 int thorin_gpu_integrals(thorin_disk *d, double *mass, double *momentum,
