@@ -1998,9 +1998,10 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
 // the coefficients of its first res pairs (whole warps') in shared memory.
 // A solve alone on the GPU takes up to 1024 threads of a multiprocessor and
 // 200 KB of its memory; with shared set (disks of an ensemble advanced
-// together) it takes three quarters of the multiprocessors and at most half of
-// each, so that two solves and the other disks' kernels fit beside each other:
-// a DT of eight disks of 128 to 512 rings takes 12.7 ms (13.0 on all
+// together) it takes three quarters of the multiprocessors and up to 1.15
+// million cells at most half of each (above, the temperatures alone fill more
+// than 110 KB), so that two solves and the other disks' kernels fit beside each
+// other: a DT of eight disks of 128 to 512 rings takes 12.7 ms (13.0 on all
 // multiprocessors, 14.2 with the larger blocks); alone the smaller blocks cost
 // 333x1002 3.85 us a pass instead of 3.3, 512x1536 6.8 instead of 6.1.
 struct SorGridShape { int nb, nt, R, res; size_t smem; };
@@ -2021,23 +2022,45 @@ static SorGridShape sor_grid_shape(const DevGrid &g, int shared)
   return q;
 }
 
+// The most dynamic shared memory of a block.
+#define SOR_GRID_SMEM (227 * 1024 - 256)
+
+// Whether either shape of a disk is within the kernel's limits; *smem (may be
+// NULL): the larger one's shared memory.
+bool hydro_sor_grid_within(const DevGrid &g, int maxiters, long long *smem)
+{
+  if (g.nr < 3 || (g.ns & 1) || (long long)g.ns * (g.nr - 2) > SOR_GRID_CELLS || maxiters >= (1 << 24) - 2) return false;
+  size_t most = 0;
+  bool ok = true;
+  for (int shared = 0; shared < 2; shared++) {
+    const SorGridShape q = sor_grid_shape(g, shared);
+    most = q.smem > most ? q.smem : most;
+    ok = ok && q.smem <= SOR_GRID_SMEM && q.nb < SOR_GRID_RECORDS;
+  }
+  if (smem) *smem = (long long)most;
+  return ok;
+}
+
 int hydro_sor_grid_fits(const DevGrid &g, int maxiters)
 {
-  if (g.nr < 3 || (g.ns & 1) || (long long)g.ns * (g.nr - 2) > SOR_GRID_CELLS || maxiters >= (1 << 24) - 2) return 0;
-  const SorGridShape q = sor_grid_shape(g, 0);     // the larger blocks
-  if (q.smem > 227 * 1024 - 256 || q.nb >= SOR_GRID_RECORDS) return 0;
-  int dev = 0, coop = 0, sms = 0, n = 0;
+  if (!hydro_sor_grid_within(g, maxiters, nullptr)) return 0;
+  int dev = 0, coop = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || !coop) {
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || !coop ||
+      cudaFuncSetAttribute(k_sor_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, SOR_GRID_SMEM) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  if (cudaFuncSetAttribute(k_sor_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 256) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sor_grid, q.nt + 32, q.smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
+  for (int shared = 0; shared < 2; shared++) {
+    const SorGridShape q = sor_grid_shape(g, shared);
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sor_grid, q.nt + 32, q.smem) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    if (n * sms < q.nb) return 0;
   }
-  return n * sms >= q.nb;
+  return 1;
 }
 
 cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,

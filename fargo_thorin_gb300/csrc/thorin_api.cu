@@ -433,6 +433,21 @@ extern "C" int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, lo
   return THORIN_OK;
 }
 
+extern "C" int thorin_selftest_solve_shape(int nrad, int nsec, int nsm, int *within, long long *smem)
+{
+  if (nrad < 4 || nsec < 4 || nsm < 1 || !within || !smem) {
+    g_last_error = "selftest_solve_shape: nrad, nsec >= 4, nsm >= 1 and output pointers required";
+    return THORIN_ERR_ARG;
+  }
+  DevGrid g = {};
+  g.nr = nrad;
+  g.ns = nsec;
+  g.nsm = nsm;
+  *smem = 0;
+  *within = hydro_sor_grid_within(g, 1000, smem);
+  return THORIN_OK;
+}
+
 extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
 {
   if (!pin || !out) return THORIN_ERR_ARG;

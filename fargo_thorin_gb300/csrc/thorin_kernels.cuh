@@ -266,6 +266,7 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
 // the GPU.
 #define SOR_GRID_RECORDS 1024
 int hydro_sor_grid_fits(const DevGrid &g, int maxiters);
+bool hydro_sor_grid_within(const DevGrid &g, int maxiters, long long *smem);
 cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
                            const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
                            void *x, double eps, int maxiters, int shared, cudaStream_t s);

@@ -451,6 +451,11 @@ int thorin_selftest_sqrt(long long n, unsigned long long seed, double max_expone
  * multiprocessors, and those that thorin_gpu_create allocates for the disk. */
 int thorin_selftest_partials(int nrad, int nsec, int npl, int nsm, long long *need, long long *held);
 
+/* Whether an nrad x nsec disk's SOR solve is within the limits of one launch on
+ * a GPU of nsm multiprocessors, alone and beside other disks, and the larger
+ * shape's shared memory a block, in bytes (without a GPU). */
+int thorin_selftest_solve_shape(int nrad, int nsec, int nsm, int *within, long long *smem);
+
 /* Failures of a DT graph's capture, by faked return codes of host calls: the
  * disk's DT graph is dropped and its next build meets the fault once.  The
  * solve's cooperative launch refused: the graph is built with launched sweeps.
