@@ -63,6 +63,7 @@ SIGNATURES = {
     "thorin_selftest_partials": (C.c_int, [C.c_int] * 4 + [C.POINTER(C.c_longlong)] * 2),
     "thorin_selftest_graph_fault": (C.c_int, [_P, C.c_int]),
     "thorin_selftest_solve_shape": (C.c_int, [C.c_int] * 3 + [C.POINTER(C.c_int), C.POINTER(C.c_longlong)]),
+    "thorin_selftest_solve_wait": (C.c_int, [_P, C.c_int]),
     "thorin_selftest_graph_builds": (C.c_int, [_P] + [C.POINTER(C.c_int)] * 2),
     "thorin_selftest_graph_conditional": (C.c_int, [C.POINTER(C.c_int)] * 3),
     "thorin_selftest_graph_nested": (C.c_int, [C.POINTER(C.c_int)] * 2),

@@ -1213,8 +1213,9 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
 // still in the other of x's two buffers.  So a solve runs one sweep more than
 // it needs.  The updates are the passes' own, bit for bit.
 // All blocks are resident together (cooperative launch); each wait has a
-// limit, after which the solve ends without a verdict, and the caller reports
-// that.
+// limit, after which its block ends the solve for all (*abort) and the caller
+// reports that, also when the verdict was out already: such a block has not
+// written its temperatures.
 // us a pass, launches / here: 24x72 6.2 / 2.25, 128x384 5.7 / 1.9, 256x768 6.8 /
 // 2.5, 333x1002 8.0 / 3.3, 384x1152 8.6 / 3.9, 512x1536 10.8 / 6.0, 640x1920 12.9 /
 // 9.1, 700x2100 15.2 / 11.1, 850x2550 19.3 / 18.9, 1024x3072 25.8 / 28.2: there the
@@ -1222,7 +1223,6 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
 // last two.  Coefficients all streamed: 192x576 2.8 (2.1 in shared memory),
 // 333x1002 3.4, 640x1920 9.7.
 #define SOR_GRID_CELLS 2400000        // largest disk (cells of rings 1 .. nr-2)
-#define SOR_GRID_SPIN (1 << 22)       // loads of one wait, about 3 s
 
 __device__ __forceinline__ void x_load(const ulonglong2 *p, unsigned long long &v, unsigned long long &tag)
 {
@@ -1236,12 +1236,13 @@ __device__ __forceinline__ void x_store(ulonglong2 *p, unsigned long long v, uns
                ::"l"(p), "l"(v), "l"(tag) : "memory");
 }
 
-// Loads until the tag (shifted right) is there; false when the wait ran out.
-__device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long want, int shift, int *abort,
+// Loads until the tag (shifted right) is there; false when the wait ran out,
+// here (spin loads) or in another block.
+__device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long want, int shift, int spin, int *abort,
                                        unsigned long long &v, unsigned long long &tag)
 {
   for (int n = 1; (tag >> shift) != want; n++) {
-    if ((n & 1023) == 0 && (n >= SOR_GRID_SPIN || *(volatile int *)abort)) {
+    if (n >= spin || ((n & 1023) == 0 && *(volatile int *)abort)) {
       *(volatile int *)abort = 1;
       return false;
     }
@@ -1253,7 +1254,7 @@ __device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long w
 struct SorSystem { const double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *cw; };
 
 __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, SorCtl c, ulonglong2 *x, double eps,
-                                           int maxiters, int R, int res)
+                                           int maxiters, int R, int res, int spin)
 {
   extern __shared__ double sm[];
   __shared__ int sdec[2];
@@ -1294,7 +1295,7 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         ch = 0;
         for (int k = lane; k < nb; k += 32) {
           tag = ~want << 13;
-          if (!x_wait(rec + k, want, 13, c.abort, v, tag)) { dead = true; break; }
+          if (!x_wait(rec + k, want, 13, spin, c.abort, v, tag)) { dead = true; break; }
           s += __longlong_as_double((long long)v);
           ch += (int)(tag & 8191u);
         }
@@ -1314,7 +1315,7 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         }
       } else {
         tag = ~(ep | (unsigned)n);
-        if (lane == 0) dead = !x_wait(verdict, ep | (unsigned)n, 0, c.abort, v, tag);
+        if (lane == 0) dead = !x_wait(verdict, ep | (unsigned)n, 0, spin, c.abort, v, tag);
         dead = __any_sync(TH_FULL, dead);
         dec = dead ? 0 : (int)__shfl_sync(TH_FULL, (unsigned)v, 0);
       }
@@ -1382,15 +1383,15 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         const double own = so[p], tc = sT[col * Pm + p];
         double tip, tim, ts;
         if (xup) {
-          if (!x_wait(xo + p + half, want, 0, c.abort, v0, t0)) dead = true;
+          if (!x_wait(xo + p + half, want, 0, spin, c.abort, v0, t0)) dead = true;
           tip = __longlong_as_double((long long)v0);
         } else tip = (p + half < P) ? so[p + half] : T[(size_t)(nr - 1) * ns + (jr ^ col)];
         if (xdn) {
-          if (!x_wait(xo + p - half, want, 0, c.abort, v1, t1)) dead = true;
+          if (!x_wait(xo + p - half, want, 0, spin, c.abort, v1, t1)) dead = true;
           tim = __longlong_as_double((long long)v1);
         } else tim = (p >= half) ? so[p - half] : T[jr ^ col];
         if (xsd) {
-          if (!x_wait(xo + sd, want, 0, c.abort, v2, t2)) dead = true;
+          if (!x_wait(xo + sd, want, 0, spin, c.abort, v2, t2)) dead = true;
           ts = __longlong_as_double((long long)v2);
         } else ts = so[sd];
         double resid = __fma_rn(tc, w.ml, -w.rhs);
@@ -2065,7 +2066,7 @@ int hydro_sor_grid_fits(const DevGrid &g, int maxiters)
 
 cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
                            const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                           void *x, double eps, int maxiters, int shared, cudaStream_t s)
+                           void *x, double eps, int maxiters, int shared, int spin, cudaStream_t s)
 {
   const SorGridShape q = sor_grid_shape(g, shared);
   cudaLaunchConfig_t cfg = {};
@@ -2079,7 +2080,7 @@ cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const SorSystem m = {ml, mlip, mlim, mljp, mljm, rhs, cw};
-  return cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res);
+  return cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res, spin);
 }
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)

@@ -219,6 +219,7 @@ struct thorin_disk {
   int sor_loop_k = 8;            // sweeps per run of the loop body
   int sor_direct = 0;            // sweeps as plain stream launches (for kernel profilers)
   int sor_one = 0;               // a solve is one cooperative launch
+  int sor_spin = SOR_GRID_SPIN;  // loads of one of its waits
   int sor_shared = 0;            // its blocks leave room for other disks' (set by the ensemble calls)
   void *sor_x = nullptr;         // cells exchanged between the blocks of k_sor_grid
   double heatsrc[THORIN_MAXPLANETS];
@@ -538,7 +539,7 @@ extern "C" int thorin_gpu_create(const thorin_params *pin, thorin_disk **out)
   d->sor.jscale = sp + 2;
   d->sor.epoch = (unsigned long long *)(sp + 3);
   d->sor.ipart = ip + 8;
-  d->sor.done = ip;
+  d->sor.done = ip;                                // the four are read back together
   d->sor.niter = ip + 1;
   d->sor.changed = ip + 2;
   d->sor.abort = ip + 3;
@@ -1661,7 +1662,7 @@ static int sor_one_launch(thorin_disk *d)
   const cudaError_t e = fake ? cudaErrorNotSupported
                              : hydro_sor_grid(d->g, d->temper, d->ml, d->mlip, d->mlim, d->mljp, d->mljm, d->rhs,
                                               d->sor_cw, d->sor, d->sor_x, d->p.sor_eps, d->p.sor_maxiters,
-                                              d->sor_shared, d->s);
+                                              d->sor_shared, d->sor_spin, d->s);
   if (e == cudaSuccess) return THORIN_OK;
   cudaGetLastError();
   g_last_error = std::string("cooperative launch of the SOR solve: ") + cudaGetErrorString(e);
@@ -1721,10 +1722,15 @@ static int sor_solve(thorin_disk *d, double omega, int *niter, int *capped, bool
     KCHECK("SOR sweep kernels");
   }
   if (d->timing) CUCHK(cudaEventRecord(d->ev[1], d->s));
-  CUCHK(cudaMemcpyAsync(d->iscal_h + IS_SOR_DONE, d->sor.done, 2 * sizeof(int), cudaMemcpyDeviceToHost, d->s));
+  int *out = d->iscal_h + IS_SOR_OUT;              // done, niter, changed, abort
+  CUCHK(cudaMemcpyAsync(out, d->sor.done, 4 * sizeof(int), cudaMemcpyDeviceToHost, d->s));
   RCHK(run_host_side(d));
   CUCHK(cudaStreamSynchronize(d->s));
-  const int done = d->iscal_h[IS_SOR_DONE], n = d->iscal_h[IS_SOR_DONE + 1];
+  const int done = out[0], n = out[1];
+  if (out[3]) {
+    g_last_error = "a wait of the SOR solve ran out";
+    return THORIN_ERR_TIMEOUT;
+  }
   if (!done || n < 1) {
     g_last_error = "SOR loop ended without an exit decision";
     return THORIN_ERR_CUDA;
@@ -2554,6 +2560,15 @@ static int build_dt_graph(thorin_disk *d, int npl, int slot)
   return rc;
 }
 
+extern "C" int thorin_selftest_solve_wait(thorin_disk *d, int loads)
+{
+  if (!d || loads < 0) return THORIN_ERR_ARG;
+  CUCHK(cudaStreamSynchronize(d->s));
+  drop_dt_graphs(d);                               // the limit is baked into their launches
+  d->sor_spin = loads ? loads : SOR_GRID_SPIN;
+  return THORIN_OK;
+}
+
 extern "C" int thorin_selftest_graph_builds(thorin_disk *d, int *alone, int *beside)
 {
   if (!d || !alone || !beside) return THORIN_ERR_ARG;
@@ -2632,6 +2647,7 @@ static int graph_finish(thorin_disk *d, thorin_planets *sys)
     CUCHK(cudaEventElapsedTime(&ms, d->ev[2], d->ev[3]));
     d->st.step_time_ms = ms;
   }
+  if (g.error == 4) { g_last_error = "a wait of the SOR solve ran out"; return THORIN_ERR_TIMEOUT; }
   if (g.error == 1) { g_last_error = "SOR loop ended without an exit decision"; return THORIN_ERR_CUDA; }
   if (g.error == 2) { g_last_error = "substep bound of the device-resident DT reached"; return THORIN_ERR_STATE; }
   if (g.error == 3) { g_last_error = "non-positive substep length"; return THORIN_ERR_STATE; }

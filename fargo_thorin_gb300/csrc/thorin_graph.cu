@@ -265,6 +265,7 @@ __global__ void k_g_sor_end(StepDev S)
   GraphStats *st = S.st;
   const int done = *S.sor.done, n = *S.sor.niter;
   if (!done || n < 1) st->error = 1;
+  if (*S.sor.abort) st->error = 4;                 // the solve is void, whatever done says
   if (done == 2) st->capped = 1;
   st->sor_calls++;
   st->sor_sweeps += n;

@@ -24,7 +24,8 @@ enum {
   SC_RCS = 96,                // device-resident DT: ring mean of c_s at each planet, taken before the hydro
   SC_CFLTOP = 104             // bits of the CFL's largest sums of squared rates (gas, pebbles)
 };
-enum { IS_NSUB = 0, IS_SOR_DONE, IS_SOR_NITER, IS_SOR_CHANGED, IS_CRASH, IS_COUNT, IS_CFL_BOUND = 32 };
+enum { IS_NSUB = 0, IS_SOR_DONE, IS_SOR_NITER, IS_SOR_CHANGED, IS_CRASH, IS_COUNT, IS_CFL_BOUND = 32,
+       IS_SOR_OUT = 40 };         // of the host copy: done, niter, changed, abort of the solve
 
 // Red-black SOR control block (device pointers).
 struct SorCtl {
@@ -38,7 +39,7 @@ struct SorCtl {
   int *changed;
   double *jscale;         // sum over the start of |resid| * omega/Ml (k_sor_resid0)
   unsigned long long *epoch;    // number of this solve (k_sor_grid's tags)
-  int *abort;             // a wait of k_sor_grid ran out
+  int *abort;             // a wait of k_sor_grid ran out: the solve is void, done or not
   // Condition of the graph's WHILE node around the sweeps: the completion
   // step sets it to 0 together with done (has_cond 0: no such node)
   cudaGraphConditionalHandle cond;
@@ -263,13 +264,14 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
 // The whole solve in one cooperative launch, where
 // hydro_sor_grid_fits; x: 32 bytes a cell of rings 1 .. nr-2 and
 // 16 SOR_GRID_RECORDS more, zero at first; shared: other disks are at work on
-// the GPU.
+// the GPU; spin: loads of one wait before it gives up.
 #define SOR_GRID_RECORDS 1024
+#define SOR_GRID_SPIN (1 << 22)       // about 3 s
 int hydro_sor_grid_fits(const DevGrid &g, int maxiters);
 bool hydro_sor_grid_within(const DevGrid &g, int maxiters, long long *smem);
 cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const double *mlip, const double *mlim,
                            const double *mljp, const double *mljm, const double *rhs, const double *cw, const SorCtl &c,
-                           void *x, double eps, int maxiters, int shared, cudaStream_t s);
+                           void *x, double eps, int maxiters, int shared, int spin, cudaStream_t s);
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s);
 void hydro_transport(const DevGrid &g, double **rho, const double *vr_in, const double *vt_in, double *vr, double *vt,
                      double **energy, double *label, const TransportScratch &S, int fast, int damp_vrad, double drin,

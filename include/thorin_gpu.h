@@ -465,6 +465,11 @@ int thorin_selftest_solve_shape(int nrad, int nsec, int nsm, int *within, long l
 #define THORIN_FAULT_COPY          2
 int thorin_selftest_graph_fault(thorin_disk *d, int fault);
 
+/* Limit of the waits of a disk's solve in one launch: loads before a wait gives
+ * up and the call returns THORIN_ERR_TIMEOUT (0: the default, about 3 s).  The
+ * state is void after that; the GPU stays usable. */
+int thorin_selftest_solve_wait(thorin_disk *d, int loads);
+
 /* How often a disk's DT graphs were built: the one it is advanced with alone
  * and the one for thorin_ensemble_algogas_graph with other disks. */
 int thorin_selftest_graph_builds(thorin_disk *d, int *alone, int *beside);
