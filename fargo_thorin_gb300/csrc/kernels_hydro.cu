@@ -533,7 +533,7 @@ __device__ double opacity_ZHU12(double vd, double rho2cgs, double T)
   if (Tf > 0.0f && rf > 0.0f && Tf < 1e30f && rf < 1e30f) {
     const float lt = 0.30103f * __log2f(Tf), lp = 0.30103f * __log2f(rf) + lt + 7.5395978f;   // log10(8.3144598e7 / 2.4)
     const float d1 = lt - (2.23567f + 0.01899f * (lp - 5.0f)), d2 = lt - (2.30713f + 0.01899f * (lp - 5.0f));
-    const bool ice = d1 < -1e-3f, silicate = d1 > 1e-3f && d2 > 1e-3f && lt < 2.8017f - 1e-3f;      // (17.08 + 1.5 2.30713) / 7.332
+    const bool ice = d1 < -1e-3f, silicate = d1 > 1e-3f && d2 > 1e-3f && lt < 2.8015132f - 1e-3f;      // (17.08 + 1.5 2.30713) / 7.332
     // the last rule's floor 3.586 lt - 16.85 is far below either
     if ((ice || silicate) && lt < 3.0f) return (ice ? 0.0033011936420003054 : 0.001443128488200116) * (T * sqrt_fast(T));  // 10^-2.481329, 10^-2.840695
   }
