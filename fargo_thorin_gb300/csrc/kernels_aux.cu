@@ -1114,8 +1114,8 @@ int aux_forces(const DevGrid &g, const ForceArgs &a0, const ForceRings &fr, cons
 }
 
 // ---------------------------------------------------------------------------
-// AccretePebblesOntoPlanets for one planet (Pebbles.c:353-539), one block.
-// The annulus [imin, imax] holding the Hill sphere is searched; cells within
+// AccretePebblesOntoPlanets for one planet (Pebbles.c:353-539).  The annulus
+// [imin, imax] holding the Hill sphere is searched; cells within
 // the effective accretion radius give up pebbles up to the model rate.
 
 // Trapzd and IntegrateColumnMass (Pebbles.c:302-349) for one cell, evaluated
@@ -1183,7 +1183,8 @@ __device__ double column_mass_warp(double a, double b, double Hpeb)
 
 // Sums of N values over a block of BS threads, valid in every thread: a warp
 // per value adds the threads' (the warps' FP64 instructions go side by side,
-// where block reductions one after another took 10 N of 64 cycles each).
+// where block reductions one after another took 10 N of them in line, 64 cycles
+// each in a warp that is alone).
 template <int N, int BS>
 __device__ __forceinline__ void acc_block_sums(double v[N])
 {

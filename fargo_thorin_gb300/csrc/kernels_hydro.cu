@@ -51,7 +51,7 @@ static int chunk_rings(int nr, int ns, int nsm, int most, double extra, int slot
 // by the same sums of densities share a reciprocal; the difference of the
 // ratios of two columns is one quotient.  FP64-bound: about 30 FP64
 // instructions a cell for the gas (40 before) and 98 with pebbles (135 in three
-// kernels).  512x1536: 161 us, 213 us in three kernels.
+// kernels).  512x1536: 157 us, 213 us in three kernels.
 #define SRC_MAXRINGS 24
 
 struct SrcRing { double inv2, invrinf, ro, invdx2, supp, omega, oinv, cr, ct; };
@@ -1070,8 +1070,8 @@ __global__ void __launch_bounds__(BX) k_matrix(DevGrid g, MatrixIO io, SorCtl c)
 // One colour pass of a sweep.  Each cell costs seven FP64 instructions: the
 // residual as five FMAs, its absolute value added to the L1 norm, and the
 // update T - resid * (omega/Ml) as one FMA (omega/Ml prepared once per solve
-// by k_sor_resid0); the change test delta > T*SORPRECISION runs on the integer
-// pipe (sor_changed).  That is 22 us of the FP64 pipe for a pass of the
+// by k_matrix, or k_sor_resid0); the change test delta > T*SORPRECISION runs
+// on the integer pipe (sor_changed).  That is 22 us of the FP64 pipe for a pass of the
 // 1024x3072 disk, 17 us of DRAM traffic (seven coefficient arrays and T, 118
 // MB), and the latency of a pass's start and end, so:
 // * one wave of blocks strides over the colour's cells, 10 a thread on that
@@ -1181,7 +1181,7 @@ k_sor_pass(DevGrid g, double *__restrict__ T, const double *__restrict__ ml, con
   cs = block_reduce(cs, OpAddI(), 0);
   if (threadIdx.x == 0) {
     const double r0 = *c.normres0;
-    const int n = __ldcg(c.niter) + 1;             // this sweep's number (k_sor_resid0 set 0)
+    const int n = __ldcg(c.niter) + 1;             // this sweep's number (the start residual set 0)
     *c.normres = s;
     *c.changed = cs;
     *c.niter = n;

@@ -2282,13 +2282,14 @@ extern "C" int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys)
 //
 //   [k_g_dt_begin] -> WHILE(h_sub) {  one substep:
 //       k_g_sub_begin, Stokes numbers, CFL (dt into the control block),
-//       InitHeating, per planet: accretion set-up, v_theta ring means,
-//       accretion kernels, Heating1 + planet update; evaporation,
-//       force constants, FillForcesArrays, DampingTW04 ring means,
+//       per planet: accretion set-up (the first: InitHeating), three accretion
+//       kernels, Heating1 + planet update (the last: force constants);
+//       evaporation, FillForcesArrays, DampingTW04 ring means,
 //       planet kick + N-body step + rotation (a branch beside the hydro),
 //       the hydro substep of the host path (pebble transport on a parallel
-//       branch) with the SOR solve as   k_g_sor_begin, residual,
-//       WHILE(h_sor) { sweeps }, k_g_sor_end,
+//       branch) with the SOR solve as   k_g_sor_begin, matrix with the start
+//       residual, [warm start], k_sor_grid or WHILE(h_sor) { sweeps },
+//       k_g_sor_end,
 //       copies that put the state back into the buffers the next run of the
 //       body reads, k_g_sub_end (clock, counters, loop condition)  }
 //
@@ -2299,9 +2300,9 @@ extern "C" int thorin_gpu_algogas(thorin_disk *d, thorin_planets *sys)
 // started in.  The first DT of a disk (omega calibration) runs on the host
 // path; planets are kept on the device for the DT.
 
-// Inserts the SOR sweep loop into the capture, after the omega schedule and
-// the matrix with the start residual: the warm start, a WHILE node whose body
-// (captured later into d->capS) holds the sweeps, then the counters.
+// Inserts the SOR solve into the capture, after the omega schedule and the
+// matrix with the start residual: the warm start, the solve's one launch or a
+// WHILE node whose body (captured later) holds the sweeps, then the counters.
 static int capture_sor(thorin_disk *d)
 {
   StepDev &S = d->capS;

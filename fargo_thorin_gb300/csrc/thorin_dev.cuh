@@ -117,7 +117,6 @@ __device__ __forceinline__ T warp_reduce(T v, Op op)
 
 struct OpAdd { __device__ double operator()(double a, double b) const { return a + b; } };
 struct OpMin { __device__ double operator()(double a, double b) const { return b < a ? b : a; } };
-struct OpMax { __device__ double operator()(double a, double b) const { return b > a ? b : a; } };
 struct OpAddI { __device__ int operator()(int a, int b) const { return a + b; } };
 
 // Result valid in thread 0.  blockDim.x must be a multiple of 32 (<= 1024).
@@ -219,18 +218,19 @@ __device__ __forceinline__ void integral_ring(const double *__restrict__ rho, co
 }
 
 // Reciprocal and reciprocal square root estimates without the FP64 pipe.
-// GB300 issues an FP64 warp instruction every 76 cycles of a sub-partition
-// (1.68 lanes per clock and SM, any mix of adds, products and FMAs) and FP32
-// and integer ones in 1 to 4, so an estimate that takes about 25 of those and
+// GB300 issues an FP64 warp instruction every 64 cycles of a sub-partition that
+// is at it alone and every 76 with all four (1.68 lanes per clock and SM, any
+// mix of adds, products and FMAs), and FP32 and integer ones in 1 to 4, so an estimate that takes about 25 of those and
 // no FP64 instruction is nearly free beside the FP64 work of any kernel here.
 // The mantissa m of the operand is split into a 24-bit FP32 part and an FP32
 // remainder, m = mh + ml; one Newton-Raphson step (to second order) from the
 // hardware's FP32 estimate y0 gives the correction y - y0 in FP32, which is
 // added to the bits of y0 as a 64-bit integer in units of 2^-53 of the
 // binade [0.5, 1].  Relative error below 2^-43 even for an FP32 estimate 2 ulp
-// off (the form before this, the hardware's FP64 estimate with one FP64
-// Newton-Raphson step, had 2^-40 and cost two FP64 instructions).  Operands: normal numbers with exponents in
-// [-500, 500] (the callers check).
+// off; measured 213 units of 2^-53 (the form before this, the hardware's FP64
+// estimate with one FP64 Newton-Raphson step, had 2^-40 and cost two FP64
+// instructions).  Operands: normal numbers with exponents in [-500, 500] (the
+// callers check).
 __device__ __forceinline__ double est_assemble(float y0, float corr, int hi_shift)
 {
   const int k = __float2int_rn(corr * 4503599627370496.0f);            // corr * 2^52, |k| < 2^31
@@ -306,10 +306,11 @@ __device__ __forceinline__ double div_slope(double x, double d)
 // (24 bits and the remainder in FP32); the sum is a two-sum, the quotient
 // b / (a + b) the hardware's reciprocal estimate with one correction from the
 // exact FP32 residual, and the pair's low part is added to the high part's
-// bits in units of their last place.  Relative error below 2^-42.  Differences
+// bits in units of their last place.  Relative error below 2^-42, measured 441
+// units of 2^-53 (963 with a reciprocal estimate one ulp off).  Differences
 // more than 2^60 apart, zero, not finite or near the ends of the exponent
 // range take the FP64 form (div_slope).  About 60 FP32 and integer
-// instructions in place of three FP64 ones (228 cycles of a sub-partition).
+// instructions in place of three FP64 ones (228 cycles of a busy sub-partition).
 // With WEIGHTED the sum is w a + b (the radial step's unequal ring spacings),
 // w = wh + wl as an FP32 pair, w64 the same in FP64.
 template <bool WEIGHTED>

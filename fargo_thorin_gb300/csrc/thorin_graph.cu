@@ -127,10 +127,10 @@ __global__ void k_g_acc_finish(StepDev S, int k)
 // shuffles.  Every sum keeps the order of the host's loops (a body's partners
 // in ascending order, the star first), and 2 k and 1 k are exact products, so
 // the results are the host's bits.
-// A warp gets one FP64 instruction per 64 cycles whatever the lanes do, and
-// 1024 accelerations in line were longer than the hydro substep of a small
-// disk.  But of a step's four only two are in line: a0 and a1 need no other, a2
-// needs a0 and a3 needs a1.  So one warp (on another sub-partition) takes a0, a2 and
+// A warp alone on its sub-partition gets one FP64 instruction per 64 cycles
+// whatever the lanes do, and 1024 accelerations in line were longer than the
+// hydro substep of a small disk.  But of a step's four only two are in line: a0
+// and a1 need no other, a2 needs a0 and a3 needs a1.  So one warp (on another sub-partition) takes a0, a2 and
 // the new positions, the other one a1, a3 and the new velocities, 39 FP64
 // instructions each with two bodies, where one warp had 84: a DT of one substep of
 // a 24x72 disk as a graph 866 -> 518 us.

@@ -37,7 +37,7 @@ struct SorCtl {
   double *normres0;
   double *normres;
   int *changed;
-  double *jscale;         // sum over the start of |resid| * omega/Ml (k_sor_resid0)
+  double *jscale;         // sum over the start of |resid| * omega/Ml (with the start residual)
   unsigned long long *epoch;    // number of this solve (k_sor_grid's tags)
   int *abort;             // a wait of k_sor_grid ran out: the solve is void, done or not
   // Condition of the graph's WHILE node around the sweeps: the completion
