@@ -1237,12 +1237,15 @@ __device__ __forceinline__ void x_store(ulonglong2 *p, unsigned long long v, uns
 }
 
 // Loads until the tag (shifted right) is there; false when the wait ran out,
-// here (spin loads) or in another block.
+// here or in another block.  FEW: a limit of `spin` loads, for the test of this;
+// as a comparison of every load it costs 128x384 2.34 -> 2.44 us a pass, so the
+// usual limit is looked at once in 1024.
+template <bool FEW>
 __device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long want, int shift, int spin, int *abort,
                                        unsigned long long &v, unsigned long long &tag)
 {
   for (int n = 1; (tag >> shift) != want; n++) {
-    if (n >= spin || ((n & 1023) == 0 && *(volatile int *)abort)) {
+    if (FEW ? n >= spin : (n & 1023) == 0 && (n >= SOR_GRID_SPIN || *(volatile int *)abort)) {
       *(volatile int *)abort = 1;
       return false;
     }
@@ -1253,6 +1256,7 @@ __device__ __forceinline__ bool x_wait(const ulonglong2 *p, unsigned long long w
 
 struct SorSystem { const double *ml, *mlip, *mlim, *mljp, *mljm, *rhs, *cw; };
 
+template <bool FEW>
 __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, SorCtl c, ulonglong2 *x, double eps,
                                            int maxiters, int R, int res, int spin)
 {
@@ -1295,7 +1299,7 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         ch = 0;
         for (int k = lane; k < nb; k += 32) {
           tag = ~want << 13;
-          if (!x_wait(rec + k, want, 13, spin, c.abort, v, tag)) { dead = true; break; }
+          if (!x_wait<FEW>(rec + k, want, 13, spin, c.abort, v, tag)) { dead = true; break; }
           s += __longlong_as_double((long long)v);
           ch += (int)(tag & 8191u);
         }
@@ -1315,7 +1319,7 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         }
       } else {
         tag = ~(ep | (unsigned)n);
-        if (lane == 0) dead = !x_wait(verdict, ep | (unsigned)n, 0, spin, c.abort, v, tag);
+        if (lane == 0) dead = !x_wait<FEW>(verdict, ep | (unsigned)n, 0, spin, c.abort, v, tag);
         dead = __any_sync(TH_FULL, dead);
         dec = dead ? 0 : (int)__shfl_sync(TH_FULL, (unsigned)v, 0);
       }
@@ -1383,15 +1387,15 @@ __global__ void __maxnreg__(64) k_sor_grid(DevGrid g, double *T, SorSystem m, So
         const double own = so[p], tc = sT[col * Pm + p];
         double tip, tim, ts;
         if (xup) {
-          if (!x_wait(xo + p + half, want, 0, spin, c.abort, v0, t0)) dead = true;
+          if (!x_wait<FEW>(xo + p + half, want, 0, spin, c.abort, v0, t0)) dead = true;
           tip = __longlong_as_double((long long)v0);
         } else tip = (p + half < P) ? so[p + half] : T[(size_t)(nr - 1) * ns + (jr ^ col)];
         if (xdn) {
-          if (!x_wait(xo + p - half, want, 0, spin, c.abort, v1, t1)) dead = true;
+          if (!x_wait<FEW>(xo + p - half, want, 0, spin, c.abort, v1, t1)) dead = true;
           tim = __longlong_as_double((long long)v1);
         } else tim = (p >= half) ? so[p - half] : T[jr ^ col];
         if (xsd) {
-          if (!x_wait(xo + sd, want, 0, spin, c.abort, v2, t2)) dead = true;
+          if (!x_wait<FEW>(xo + sd, want, 0, spin, c.abort, v2, t2)) dead = true;
           ts = __longlong_as_double((long long)v2);
         } else ts = so[sd];
         double resid = __fma_rn(tc, w.ml, -w.rhs);
@@ -2048,14 +2052,15 @@ int hydro_sor_grid_fits(const DevGrid &g, int maxiters)
   int dev = 0, coop = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || !coop ||
-      cudaFuncSetAttribute(k_sor_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, SOR_GRID_SMEM) != cudaSuccess) {
+      cudaFuncSetAttribute(k_sor_grid<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SOR_GRID_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sor_grid<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SOR_GRID_SMEM) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   for (int shared = 0; shared < 2; shared++) {
     const SorGridShape q = sor_grid_shape(g, shared);
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sor_grid, q.nt + 32, q.smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sor_grid<false>, q.nt + 32, q.smem) != cudaSuccess) {
       cudaGetLastError();
       return 0;
     }
@@ -2080,7 +2085,8 @@ cudaError_t hydro_sor_grid(const DevGrid &g, double *T, const double *ml, const 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const SorSystem m = {ml, mlip, mlim, mljp, mljm, rhs, cw};
-  return cudaLaunchKernelEx(&cfg, k_sor_grid, g, T, m, c, (ulonglong2 *)x, eps, maxiters, q.R, q.res, spin);
+  return cudaLaunchKernelEx(&cfg, spin < SOR_GRID_SPIN ? k_sor_grid<true> : k_sor_grid<false>, g, T, m, c,
+                            (ulonglong2 *)x, eps, maxiters, q.R, q.res, spin);
 }
 
 void hydro_energy_from_t(const DevGrid &g, const double *rho, double *T, double *enew, cudaStream_t s)

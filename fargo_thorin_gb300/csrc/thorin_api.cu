@@ -2563,7 +2563,7 @@ static int build_dt_graph(thorin_disk *d, int npl, int slot)
 
 extern "C" int thorin_selftest_solve_wait(thorin_disk *d, int loads)
 {
-  if (!d || loads < 0) return THORIN_ERR_ARG;
+  if (!d || loads < 0 || loads > SOR_GRID_SPIN) return THORIN_ERR_ARG;
   CUCHK(cudaStreamSynchronize(d->s));
   drop_dt_graphs(d);                               // the limit is baked into their launches
   d->sor_spin = loads ? loads : SOR_GRID_SPIN;

@@ -264,7 +264,7 @@ void hydro_sor_sweeps(const DevGrid &g, double *T, const double *ml, const doubl
 // The whole solve in one cooperative launch, where
 // hydro_sor_grid_fits; x: 32 bytes a cell of rings 1 .. nr-2 and
 // 16 SOR_GRID_RECORDS more, zero at first; shared: other disks are at work on
-// the GPU; spin: loads of one wait before it gives up.
+// the GPU; spin: loads of one wait before it gives up (at most SOR_GRID_SPIN).
 #define SOR_GRID_RECORDS 1024
 #define SOR_GRID_SPIN (1 << 22)       // about 3 s
 int hydro_sor_grid_fits(const DevGrid &g, int maxiters);
