@@ -57,6 +57,8 @@ SIGNATURES = {
     "thorin_selftest_slope_division": (C.c_int, [C.c_longlong, C.c_ulonglong, C.c_double,
                                                  C.POINTER(C.c_ulonglong)]),
     "thorin_selftest_vl_slope": (C.c_int, [C.c_longlong, C.c_ulonglong, C.c_double] + [C.POINTER(C.c_ulonglong)] * 2),
+    "thorin_selftest_vl_slope_weighted": (C.c_int, [C.c_longlong, C.c_ulonglong] + [C.c_double] * 2
+                                          + [C.POINTER(C.c_ulonglong)]),
     "thorin_selftest_exp": (C.c_int, [C.c_longlong, C.c_ulonglong] + [C.c_double] * 2 + [C.POINTER(C.c_ulonglong)] * 2),
     "thorin_selftest_exp_values": (C.c_int, [C.c_int] + [_D] * 3),
     "thorin_selftest_sqrt": (C.c_int, [C.c_longlong, C.c_ulonglong, C.c_double] + [C.POINTER(C.c_ulonglong)] * 2),

@@ -312,7 +312,8 @@ __device__ __forceinline__ double div_slope(double x, double d)
 // range take the FP64 form (div_slope).  About 60 FP32 and integer
 // instructions in place of three FP64 ones (228 cycles of a busy sub-partition).
 // With WEIGHTED the sum is w a + b (the radial step's unequal ring spacings),
-// w = wh + wl as an FP32 pair, w64 the same in FP64.
+// w = wh + wl as an FP32 pair, w64 the same in FP64; measured 535 units for w
+// within 1.05 of 1, 875 within a factor of 4.
 template <bool WEIGHTED>
 __device__ __forceinline__ double vl_slope_t(double a, double b, float wh, float wl, double w64)
 {

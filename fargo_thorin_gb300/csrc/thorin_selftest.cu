@@ -458,6 +458,50 @@ extern "C" int thorin_selftest_vl_slope(long long n, unsigned long long seed, do
   return THORIN_OK;
 }
 
+// The weighted slope of the radial step against a (b / (w a + b)), w in
+// [1 / wmax, wmax].
+__global__ void k_selftest_vl_slope_weighted(long long n, unsigned long long seed, double emax, double wmax,
+                                             unsigned long long *__restrict__ out)
+{
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const unsigned long long key = seed + 3ULL * (unsigned long long)t;
+  const double c = exp2((double)(int)(st_mix(key) % 201ULL) - 100.0);
+  const double a = st_value(key + 1ULL, emax) * c, b = st_value(key + 2ULL, emax) * c;
+  const double u = 2.0 * ((double)(st_mix(key + 7ULL * (unsigned long long)n) >> 11) * (1.0 / 9007199254740992.0)) - 1.0;
+  const double w = exp2(u * log2(wmax));
+  const float wh = (float)w, wl = (float)(w - (double)wh);         // as k_radial splits its ring ratio
+  const double ref = ((a > 0.0) == (b > 0.0)) ? a * (b / (w * a + b)) : 0.0;
+  const long long x = __double_as_longlong(ref), y = __double_as_longlong(vl_slope_t<true>(a, b, wh, wl, w));
+  const unsigned long long d = (unsigned long long)(x > y ? x - y : y - x);
+  if (d) atomicMax(out, d);
+}
+
+extern "C" int thorin_selftest_vl_slope_weighted(long long n, unsigned long long seed, double max_exponent,
+                                                 double max_weight, unsigned long long *max_ulp)
+{
+  if (n < 1 || !max_ulp || !(max_exponent >= 0.0 && max_exponent <= 300.0) || !(max_weight >= 1.0 && max_weight <= 1024.0)) {
+    g_last_error = "selftest_vl_slope_weighted: n >= 1, 0 <= max_exponent <= 300, 1 <= max_weight <= 1024 and an output "
+                   "pointer required";
+    return THORIN_ERR_ARG;
+  }
+  unsigned long long *dev = nullptr, host = 0ULL;
+  cudaError_t e = cudaMalloc((void **)&dev, sizeof(host));
+  if (e == cudaSuccess) e = cudaMemset(dev, 0, sizeof(host));
+  if (e == cudaSuccess) {
+    k_selftest_vl_slope_weighted<<<(unsigned)((n + 255) / 256), 256>>>(n, seed, max_exponent, max_weight, dev);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(&host, dev, sizeof(host), cudaMemcpyDeviceToHost);
+  if (dev) cudaFree(dev);
+  if (e != cudaSuccess) {
+    g_last_error = std::string("selftest_vl_slope_weighted: ") + cudaGetErrorString(e);
+    return THORIN_ERR_CUDA;
+  }
+  *max_ulp = host;
+  return THORIN_OK;
+}
+
 extern "C" int thorin_selftest_fp64_peak(double *gflops)
 {
   if (!gflops) {

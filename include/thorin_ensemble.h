@@ -9,6 +9,8 @@
  * disks that alone leave most multiprocessors idle run side by side.  A
  * disk's results do not depend on the worker count or the order: each
  * disk's kernels and reductions run in a fixed order on its own streams.
+ * (Alone and beside others a solve adds its residuals in another order, so the
+ * sweep counts could differ where a norm is within rounding of the threshold.)
  * No counterpart in the reference.
  */
 #ifndef THORIN_ENSEMBLE_H
@@ -45,7 +47,9 @@ int thorin_ensemble_tune(thorin_disk *const *disks, thorin_planets *const *syste
  * all launched on the disks' own streams from the calling thread before any
  * is waited for, so that the disks run side by side with no host round trip
  * inside the DT.  A disk's first DT runs on the host path (omega
- * calibration).  status[k] as for thorin_ensemble_algogas. */
+ * calibration).  With more than one disk each has a graph for this call, beside
+ * the one of thorin_gpu_algogas_graph, whose SOR solve takes three quarters of
+ * the multiprocessors.  status[k] as for thorin_ensemble_algogas. */
 int thorin_ensemble_algogas_graph(thorin_disk **disks, thorin_planets **systems, int n, int *status);
 
 #ifdef __cplusplus

@@ -431,6 +431,11 @@ int thorin_selftest_slope_division(long long n, unsigned long long seed, double 
 int thorin_selftest_vl_slope(long long n, unsigned long long seed, double max_exponent, unsigned long long *max_ulp,
                              unsigned long long *max_ulp_quotient);
 
+/* The same for the radial step's slope a b / (w a + b), the ratio w of its ring
+ * spacings in [1 / max_weight, max_weight]. */
+int thorin_selftest_vl_slope_weighted(long long n, unsigned long long seed, double max_exponent, double max_weight,
+                                      unsigned long long *max_ulp);
+
 /* Self-test of the kernels' exponential on [-range, range] and of x^(-3/2)
  * against CUDA's exp and 1 / (x sqrt(x)): n random operands; returns the
  * largest differences in ulps. */
@@ -466,7 +471,8 @@ int thorin_selftest_solve_shape(int nrad, int nsec, int nsm, int *within, long l
 int thorin_selftest_graph_fault(thorin_disk *d, int fault);
 
 /* Limit of the waits of a disk's solve in one launch: loads before a wait gives
- * up and the call returns THORIN_ERR_TIMEOUT (0: the default, about 3 s).  The
+ * up and the call returns THORIN_ERR_TIMEOUT (1 .. 2^22; 0: the default, 2^22,
+ * about 3 s).  The
  * state is void after that; the GPU stays usable. */
 int thorin_selftest_solve_wait(thorin_disk *d, int loads);
 

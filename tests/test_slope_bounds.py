@@ -24,3 +24,14 @@ def test_van_leer_slope_within_its_stated_error(max_exponent, seed):
     _lib.check(_lib.load().thorin_selftest_vl_slope(1 << 26, seed, max_exponent, C.byref(ulp), C.byref(q)), "vl_slope")
     print("slope: max", ulp.value, "ulp")
     assert ulp.value <= 2048 + 2                          # and the reference's two roundings
+
+
+@pytest.mark.parametrize("max_exponent,max_weight,seed", [(0.5, 1.05, 41), (20.0, 1.05, 42), (29.9, 2.0, 43),
+                                                          (32.0, 4.0, 44), (200.0, 64.0, 45)])
+def test_weighted_slope_within_its_stated_error(max_exponent, max_weight, seed):
+    """The radial step's slope: w enters as an FP32 pair (2^-48)."""
+    ulp = C.c_ulonglong()
+    _lib.check(_lib.load().thorin_selftest_vl_slope_weighted(1 << 26, seed, max_exponent, max_weight, C.byref(ulp)),
+               "vl_slope_weighted")
+    print("weighted slope: max", ulp.value, "ulp")
+    assert ulp.value <= 2048 + 3                          # and the reference's three roundings
