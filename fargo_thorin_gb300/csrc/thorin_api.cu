@@ -294,12 +294,19 @@ static void fill_rings(thorin_disk *d)
     }
 }
 
-static double fviscosity_host(const thorin_disk *d, int i_ring, double rad, const std::vector<double> &csm)
+static double fviscosity_host(const thorin_disk *d, int i_ring, double rad, const std::vector<double> &csm,
+                              const std::vector<double> &tm)
 {
-  // FViscosity (Viscosity.c:26-54) for the ring the reference's search finds.
+  // FViscosity (Viscosity.c:26-54) for the ring the reference's search finds;
+  // csm, tm: ring means of the sound speed and the temperature
   const thorin_params &p = d->p;
   double nu = p.viscosity;
   if (p.viscosity_alpha) nu = p.alpha_viscosity * csm[i_ring] * csm[i_ring] * pow(rad, 1.5);
+  if (p.alpha_flock) {
+    const double alpha =
+        (p.alpha_mri - p.alpha_dead) * (1.0 - tanh((p.tmri - tm[i_ring] * T2SI) / p.twidth)) / 2.0 + p.alpha_dead;
+    nu = alpha * csm[i_ring] * csm[i_ring] * pow(rad, 1.5);
+  }
   const double rmin = (p.cavity_radius - p.cavity_width * p.aspect_ratio);
   const double rmax = (p.cavity_radius + p.cavity_width * p.aspect_ratio);
   if (rad < rmin) nu *= p.cavity_ratio;
@@ -1060,22 +1067,24 @@ extern "C" int thorin_gpu_init_default(thorin_disk *d)
   }
   for (int i = 0; i < nr; i++)
     for (int j = 0; j < ns; j++) { rho[j + i * ns] = d->SigmaMed[i]; e[j + i * ns] = d->EnergyMed[i]; }
-  std::vector<double> csm(nr + 2, 0.0);
+  std::vector<double> csm(nr + 2, 0.0), tm(nr + 2, 0.0);
   for (int i = 0; i < nr; i++) {
-    double sacc = 0.0;
+    double sacc = 0.0, tacc = 0.0;
     const double csi = p.energy_eq ? 0.0 : cs_iso_host(d, i);
     for (int j = 0; j < ns; j++) {
       const int l = j + i * ns;
       cs[l] = p.energy_eq ? sqrt(p.adiabind * (p.adiabind - 1.0) * fabs(e[l]) / rho[l]) : csi;
       sacc += cs[l];
+      tacc += (p.energy_eq ? e[l] * (p.adiabind - 1.0) : rho[l] * cs[l] * cs[l]) * (1.0 / rho[l]);
     }
     csm[i] = sacc / (double)ns;
+    tm[i] = tacc / (double)ns;
   }
   if (p.parametric_cooling) {             // FillCoolingTime, FillQplus (Theo.c:103-129)
     std::vector<double> ct(nr + 2, 0.0), qm(nr + 2, 0.0);
     for (int i = 0; i < nr; i++) {
       ct[i] = p.cooling_time * pow(d->Rmed[i], 2.0 + 2.0 * p.flaring_index);
-      qm[i] = 2.25 * fviscosity_host(d, i, d->Rmed[i], csm) * p.sigma0 * pow(d->Rmed[i], -p.sigma_slope - 3.0);
+      qm[i] = 2.25 * fviscosity_host(d, i, d->Rmed[i], csm, tm) * p.sigma0 * pow(d->Rmed[i], -p.sigma_slope - 3.0);
     }
     RCHK(upload_ring(d, R_COOLT, ct));
     RCHK(upload_ring(d, R_QPLUSMED, qm));
@@ -1121,7 +1130,7 @@ extern "C" int thorin_gpu_init_default(thorin_disk *d)
     int ir;
     if (i == nr) { r = d->Rmed[nr - 1]; ri = d->Rinf[nr - 1]; ir = nr - 1; }
     else { r = d->Rmed[i]; ri = d->Rinf[i]; ir = i; }
-    const double viscosity = fviscosity_host(d, ir, r, csm);
+    const double viscosity = fviscosity_host(d, ir, r, csm, tm);
     for (int j = 0; j < ns; j++) {
       const int l = j + i * ns;
       const double rg = r, omega = sqrt(1.0 * 1.0 / rg / rg / rg);
