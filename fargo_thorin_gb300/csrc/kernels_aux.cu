@@ -1566,7 +1566,9 @@ __global__ void __launch_bounds__(1024) k_nonreflecting(DevGrid g, double *__res
   double dangle;
   if (inner) dangle = (pow(g.r.Rinf[1], -1.5) - 1.0) / (.5 * (csin + csout)) * (g.r.Rmed[1] - g.r.Rmed[0]);
   else dangle = (pow(g.r.Rinf[nr - 2], -1.5) - 1.0) / (.5 * (csin + csout)) * (g.r.Rmed[nr - 1] - g.r.Rmed[nr - 2]);
-  const int i_angle = (int)(dangle / 2.0 / TH_PI * (double)ns + .5);
+  // whole turns are taken off: the reference adds or takes off one, so in thin
+  // disks it leaves the ring (and the array), as the shear is longer than that
+  const int i_angle = (int)(dangle / 2.0 / TH_PI * (double)ns + .5) % ns;
   const int i = inner ? 1 : nr - 1;
   const int edge = inner ? 0 : nr - 1;
   const double sig = inner ? g.r.SigmaMed[1] : g.r.SigmaMed[nr - 2];
